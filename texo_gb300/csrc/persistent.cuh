@@ -17,15 +17,11 @@ namespace tgp {
 constexpr int kBlocksPerSm = 1;
 constexpr int kBatchBlocksPerSm = 4;
 
-// Grid barrier words (device memory, zeroed before each launch): an arrival
-// counter and, on its own 128-byte line, the generation every waiter polls.
-struct alignas(128) BarrierLine {
-  unsigned int count;
-  unsigned int pad[31];
-};
-struct GridBarrier {
-  BarrierLine root;                         // arrivals
-  unsigned int gen;                         // generation
+// Grid barrier words (device memory, zeroed before each launch): the
+// arrivals counted since the launch began and the error word, side by side
+// so that one 8-byte load polls both.
+struct alignas(128) GridBarrier {
+  unsigned int arrived;
   int error;                                // 1 when a bounded wait ran out
   unsigned int pad[30];
 };
