@@ -178,6 +178,21 @@ __device__ __forceinline__ long long tap_fixed(float q, float wx, float wy) {
   return __float2ll_rn(__fmul_rn(__fmul_rn(__fmul_rn(q, wx), wy), kFixF));
 }
 
+// The kThreads threads that run one virtual block's work: a whole block
+// (BAR 0), or one half of a double block (its own named barrier).
+template <int BAR>
+struct Group {
+  int tid;   // 0 .. kThreads - 1
+  __device__ __forceinline__ void sync() const {
+    if (BAR == 0)
+      __syncthreads();
+    else
+      asm volatile("bar.sync %0, %1;" ::"n"(BAR), "n"(kThreads) : "memory");
+  }
+};
+using Block = Group<0>;
+__device__ __forceinline__ Block whole_block() { return Block{(int)threadIdx.x}; }
+
 // ---- block reductions (fixed order within a block) --------------------------
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
@@ -193,38 +208,44 @@ __device__ __forceinline__ T warp_sum(T v) {
 // sub-partition) each fold an interleaved quarter with an xor tree, and
 // thread 0 folds the four results. `sh` needs kThreads + 4 slots; the result
 // is valid in thread 0. The order is fixed, so every block folds alike.
-template <typename Op>
-__device__ __forceinline__ double block_fold_fp64(double v, double* sh, Op op) {
-  __syncthreads();   // earlier readers of sh are done
-  sh[threadIdx.x] = v;
-  __syncthreads();
-  const int w = threadIdx.x >> 5;
+template <class G, typename Op>
+__device__ __forceinline__ double block_fold_fp64(const G& g, double v, double* sh, Op op) {
+  g.sync();   // earlier readers of sh are done
+  sh[g.tid] = v;
+  g.sync();
+  const int w = g.tid >> 5;
   if (w < 4) {
-    double s = sh[threadIdx.x];
-    for (int i = threadIdx.x + 128; i < (int)blockDim.x; i += 128) s = op(s, sh[i]);
+    double s = op(sh[g.tid], sh[g.tid + 128]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s = op(s, __shfl_xor_sync(0xffffffffu, s, o));
-    if ((threadIdx.x & 31) == 0) sh[kThreads + w] = s;
+    if ((g.tid & 31) == 0) sh[kThreads + w] = s;
   }
-  __syncthreads();
-  return threadIdx.x == 0 ? op(op(op(sh[kThreads], sh[kThreads + 1]), sh[kThreads + 2]), sh[kThreads + 3]) : 0.0;
+  g.sync();
+  return g.tid == 0 ? op(op(op(sh[kThreads], sh[kThreads + 1]), sh[kThreads + 2]), sh[kThreads + 3]) : 0.0;
 }
 struct FoldAdd {
   __device__ double operator()(double a, double b) const { return a + b; }
 };
-__device__ __forceinline__ double block_sum(double v, double* sh) { return block_fold_fp64(v, sh, FoldAdd()); }
+template <typename Op>
+__device__ __forceinline__ double block_fold_fp64(double v, double* sh, Op op) {
+  return block_fold_fp64(whole_block(), v, sh, op);
+}
+template <class G>
+__device__ __forceinline__ double block_sum(const G& g, double v, double* sh) {
+  return block_fold_fp64(g, v, sh, FoldAdd());
+}
 
 // Sum over the block; result valid in thread 0. `sh` needs kThreads/32 slots.
-template <typename T>
-__device__ __forceinline__ T block_sum(T v, T* sh) {
+template <class G, typename T>
+__device__ __forceinline__ T block_sum(const G& g, T v, T* sh) {
   v = warp_sum(v);
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  __syncthreads();
+  const int lane = g.tid & 31, w = g.tid >> 5;
+  g.sync();
   if (lane == 0) sh[w] = v;
-  __syncthreads();
+  g.sync();
   T r = 0;
-  if (threadIdx.x == 0)
-    for (int i = 0; i < (int)(blockDim.x >> 5); ++i) r += sh[i];
+  if (g.tid == 0)
+    for (int i = 0; i < kThreads / 32; ++i) r += sh[i];
   return r;
 }
 

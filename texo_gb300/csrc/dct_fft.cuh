@@ -7,9 +7,9 @@
 // s_0 = sqrt(1/n), s_k = sqrt(2/n). The inverse (DCT-III) forms
 // W_k = exp(-i pi k / 2n) (X_k / s_k + i X_{n-k} / s_{n-k}) (X_n = 0), takes
 // F = FFT_n(W) and reads x_{2j} = Re F_j / n, x_{2j+1} = Re F_{n-1-j} / n.
-// The FFT is an in-place radix-2 decimation-in-time transform in shared
-// memory over a group of vectors stored back to back, fed in bit-reversed
-// order.
+// The FFT is a radix-2 decimation-in-time transform over a group of vectors,
+// each thread keeping the two points of its butterfly in registers from
+// stage to stage.
 //
 // Every value inside a transform is a double-float: an unevaluated sum
 // hi + lo of two FP32 numbers, added with Knuth's two-sum and multiplied with
@@ -37,12 +37,16 @@
 namespace tgp {
 namespace fft {
 
-constexpr int kBuf = 2048;                       // complex double-float slots of the work buffer (32 KB)
-constexpr int kData = 1024;                      // slots a group's data takes at most (n <= 1024)
-constexpr int kPer = kData / kThreads;           // data slots per thread
+// Work buffer, in 16-byte slots: [0, exch) the butterflies' points crossing
+// between warps (two buffers), then the staged vectors (float2 a point), then
+// the tables of one axis up to 256 points. Lengths up to 512 take 512 points
+// a group, 1024 takes 1024 (two butterflies a thread).
+constexpr int kBuf = 2048;
+constexpr int kStage = 640;                      // float2 slots of one staged copy, padding included (512 points)
+constexpr int kTables = 512 + kStage;            // the tables' first slot
 
 struct Smem {
-  float4 buf[kBuf];   // (re.hi, im.hi, re.lo, im.lo)
+  float4 buf[kBuf];
 };
 
 // ---- double-float arithmetic ---------------------------------------------
@@ -108,26 +112,33 @@ __device__ __forceinline__ Axis axis_y(const Dev& d) {
 }
 
 // Up to 256 points the tables (n/2 twiddles, n post and n pre factors, n
-// 1/s_k) fit in the half of the buffer the data leaves free and are copied
-// there once per pass: the stages then read their twiddles from shared
-// memory instead of making an L2 round trip per stage (the persistent
-// kernel's grid barriers leave L1 cold).
+// 1/s_k) fit in the work buffer beside the data and are copied there: the
+// stages then read their twiddles from shared memory instead of making an L2
+// round trip per stage (the persistent kernel's grid barriers leave L1 cold).
+// With `there` they are in place already: the persistent kernel copies the
+// tables of a square grid once, both axes sharing them.
 constexpr int kTableLog = 8;
-__device__ __forceinline__ Axis stage_tables(const Axis& a, float4* buf) {
+template <class G>
+__device__ __forceinline__ Axis stage_tables(const G& g, const Axis& a, float4* buf, bool there) {
   if (a.logn > kTableLog) return a;
-  float4* tw = buf + kData;
+  float4* tw = buf + kTables;
   float4* post = tw + (a.n >> 1);
   float4* pre = post + a.n;
   float2* inv_s = reinterpret_cast<float2*>(pre + a.n);
-  __syncthreads();   // earlier readers of the buffer are done
-  for (int i = threadIdx.x; i < a.n; i += blockDim.x) {
-    if (i < (a.n >> 1)) tw[i] = a.tw[i];
-    post[i] = a.post[i];
-    pre[i] = a.pre[i];
-    inv_s[i] = a.inv_s[i];
+  if (!there) {
+    g.sync();   // earlier readers of the buffer are done
+    for (int i = g.tid; i < a.n; i += kThreads) {
+      if (i < (a.n >> 1)) tw[i] = a.tw[i];
+      post[i] = a.post[i];
+      pre[i] = a.pre[i];
+      inv_s[i] = a.inv_s[i];
+    }
+    g.sync();
   }
-  __syncthreads();
   return Axis{tw, post, pre, inv_s, a.n, a.logn};
+}
+__device__ __forceinline__ bool tables_stay(const Dev& d) {
+  return d.fft && d.logW == d.logH && d.logW <= kTableLog;
 }
 
 // Vectors transformed together: one butterfly per thread per stage (n/2
@@ -139,93 +150,201 @@ __device__ __forceinline__ int brev(int m, int logn) {
   return logn ? (int)(__brev((unsigned)m) >> (32 - logn)) : 0;
 }
 // position of sample i in Makhoul's order (and, for the inverse, the FFT
-// output index that holds sample i)
+// output index that holds sample i), and the sample at a position
 __device__ __forceinline__ int mak(int i, int n) { return (i & 1) ? n - 1 - (i >> 1) : (i >> 1); }
+__device__ __forceinline__ int unmak(int m, int n) { return m < (n >> 1) ? 2 * m : 2 * (n - 1 - m) + 1; }
+// staged slots, padded so that the strided accesses of the butterflies'
+// outputs meet different banks
+__device__ __forceinline__ int pad_k(int k) { return k + (k >> 2); }   // coefficients, four apart a lane
+__device__ __forceinline__ int pad_i(int i) { return i + (i >> 3); }   // samples, eight apart a lane
 
-// In-place radix-2 DIT over G vectors of length n (bit-reversed input).
-__device__ __forceinline__ void stages(float4* buf, int G, const Axis& a) {
-  const int half_n = a.n >> 1, total = G * half_n;
-  for (int s = 0; s < a.logn; ++s) {
-    const int half = 1 << s, step = half_n >> s;
-    __syncthreads();
-    for (int b = threadIdx.x; b < total; b += blockDim.x) {
-      const int g = b >> (a.logn - 1), j = b & (half_n - 1);
-      const int jj = j & (half - 1);
-      float4* p = buf + (g << a.logn) + ((j >> s) << (s + 1)) + jj;
-      const CDF w = cdf_load(a.tw[jj * step]);
-      const CDF u = cdf_load(p[0]);
-      const CDF t = cdf_mul(cdf_load(p[half]), w);
-      p[0] = cdf_store(CDF{df_add(u.re, t.re), df_add(u.im, t.im)});
-      p[half] = cdf_store(CDF{df_sub(u.re, t.re), df_sub(u.im, t.im)});
-    }
+// The radix-2 network. Positions are the bit-reversed input order: stage s
+// pairs the positions that differ in bit s. A thread holds, at stage s, the
+// two points whose positions agree with its thread index in every other bit,
+// and between the stages s - 1 and s it hands one of them to the thread whose
+// index differs in the bit that stands for position bit s; that index bit
+// then stands for bit s - 1. Lane bits stand for the high position bits (low
+// bits of the sample index, so that the staged samples are read without
+// conflicts) and trade with shuffles; the warp bits, if a vector spans
+// several warps, stand for the low ones and trade through shared memory, one
+// block barrier each: two exchanges of 256 points' seven. A transform is bound
+// by the latency of its chain on 8 warps; a block barrier and two trips
+// through shared memory for every stage were half of it. The butterflies'
+// values are the same, operation for operation. Measured: the three passes
+// of a 256 x 256 solve in the persistent loop, its three grid barriers
+// included, 28.8 -> 25.3 us; a 1024 x 1024 solve in the host engine (rows
+// forward / columns / rows inverse) 37 / 80 / 55 -> 25 / 68 / 33 us.
+// NB = 2 (1024 points): a thread runs two butterflies, whose points differ in
+// position bit 1 at stage 0.
+template <int NB>
+struct Place {
+  int L, n;      // log2 length, length
+  int vec;       // vector of the group
+  int p;         // position of the thread's first point at stage 0 (butterfly 0)
+  int lanes;     // index bits of a vector inside a warp
+  __device__ __forceinline__ Place(int tid, int logn) {
+    L = logn;
+    n = 1 << logn;
+    const int bits = logn - NB;                   // index bits of a vector
+    const int t = tid & ((1 << max(bits, 0)) - 1);
+    vec = tid >> max(bits, 0);
+    lanes = min(bits, 5);
+    p = brev(t & ((1 << max(lanes, 0)) - 1), logn) | ((t >> max(lanes, 0)) << NB);
   }
-  __syncthreads();
+};
+struct Pair {
+  CDF a, b;
+};
+
+__device__ __forceinline__ void butterfly(Pair& x, const CDF& w) {
+  const CDF t = cdf_mul(x.b, w);
+  x.b = CDF{df_sub(x.a.re, t.re), df_sub(x.a.im, t.im)};
+  x.a = CDF{df_add(x.a.re, t.re), df_add(x.a.im, t.im)};
 }
 
-// Forward: G real vectors x(g, i) (double-floats) -> buf holds V = FFT(v) in
-// natural order; X_k = Re(post_k V_k). With logG >= 0 the loads run with the
-// vector index fastest (G = 2^logG neighbouring columns of a row-major grid
-// are then read together), else with the sample index fastest.
-template <class Load>
-__device__ __forceinline__ void dct2(float4* buf, int G, const Axis& a, Load load, int logG = -1) {
-  __syncthreads();
-  for (int e = threadIdx.x; e < (G << a.logn); e += blockDim.x) {
-    int g, i;
-    if (logG >= 0) {
-      g = e & (G - 1);
-      i = e >> logG;
-    } else {
-      g = e >> a.logn;
-      i = e & (a.n - 1);
-    }
-    const DF x = load(g, i);
-    buf[(g << a.logn) + brev(mak(i, a.n), a.logn)] = make_float4(x.hi, 0.f, x.lo, 0.f);
+// Brings position bit s into the pairs (s >= 1).
+template <int NB, class G>
+__device__ __forceinline__ void exchange(const G& g, const Place<NB>& at, int s, Pair (&x)[NB], float4* exch) {
+  if (NB == 2 && s == 1) {   // between the thread's own butterflies
+    const CDF t = x[0].b;
+    x[0].b = x[NB - 1].a;
+    x[NB - 1].a = t;
+    return;
   }
-  stages(buf, G, a);
+  const bool up = (at.p >> s) & 1;
+  const int w = s - NB;                          // warp bit
+  if (w < at.L - NB - at.lanes) {                // through shared memory, the two buffers in turn
+    float4* e = exch + (w & 1) * NB * kThreads;
+#pragma unroll
+    for (int r = 0; r < NB; ++r) e[r * kThreads + g.tid] = cdf_store(up ? x[r].a : x[r].b);
+    g.sync();
+    const int from = g.tid ^ (32 << w);
+#pragma unroll
+    for (int r = 0; r < NB; ++r) {
+      const CDF v = cdf_load(e[r * kThreads + from]);
+      if (up)
+        x[r].a = v;
+      else
+        x[r].b = v;
+    }
+  } else {
+    const int m = 1 << (at.L - 1 - s);
+#pragma unroll
+    for (int r = 0; r < NB; ++r) {
+      const CDF q = up ? x[r].a : x[r].b;
+      CDF v;
+      v.re.hi = __shfl_xor_sync(0xffffffffu, q.re.hi, m);
+      v.re.lo = __shfl_xor_sync(0xffffffffu, q.re.lo, m);
+      v.im.hi = __shfl_xor_sync(0xffffffffu, q.im.hi, m);
+      v.im.lo = __shfl_xor_sync(0xffffffffu, q.im.lo, m);
+      if (up)
+        x[r].a = v;
+      else
+        x[r].b = v;
+    }
+  }
 }
-__device__ __forceinline__ DF coef(const Axis& a, const float4* buf, int g, int k) {
-  const CDF v = cdf_load(buf[(g << a.logn) + k]), p = cdf_load(a.post[k]);
+
+// Stages [from, L); on return pair r holds the outputs of frequencies (or
+// sample positions) out_index(at, r) and out_index(at, r) + n / 2.
+template <int NB, class G>
+__device__ __forceinline__ void stages(const G& g, const Place<NB>& at, int from, Pair (&x)[NB], const Axis& a,
+                                       float4* exch) {
+  for (int s = from; s < at.L; ++s) {
+    exchange(g, at, s, x, exch);
+#pragma unroll
+    for (int r = 0; r < NB; ++r) {
+      const int j = ((at.p >> 1) | r) & ((1 << s) - 1);
+      butterfly(x[r], cdf_load(a.tw[j << (at.L - 1 - s)]));
+    }
+  }
+}
+template <int NB>
+__device__ __forceinline__ int out_index(const Place<NB>& at, int r) {
+  return (at.p >> 1) | r;
+}
+
+// Forward: the vectors' real samples staged in Makhoul's order (st[vec * n +
+// m], conflict-free) -> V. The inputs are real and stage 0's twiddle is one,
+// so stage 0 is two real sums, formed from four staged samples by each of the
+// two threads that would trade them (no exchange before stage 1); the
+// products by one and the sums with zero that are left out change no value.
+template <int NB, class G>
+__device__ __forceinline__ void forward(const G& g, const Place<NB>& at, const float2* st, const Axis& a,
+                                        float4* exch, Pair (&x)[NB]) {
+  const DF zero{0.f, 0.f};
+  auto sample = [&](int m) {
+    const float2 v = st[(at.vec << at.L) + m];
+    return DF{v.x, v.y};
+  };
+  const int m = brev(at.p, at.L), h = at.n >> 1, q = at.n >> 2;
+  if (NB == 1 && at.L == 1) {
+    const DF u = sample(0), v = sample(1);
+    x[0] = Pair{{df_add(u, v), zero}, {df_sub(u, v), zero}};
+    return;
+  }
+  const int m0 = NB == 1 ? m & ~q : m;
+  const DF u0 = sample(m0), u1 = sample(m0 + h), v0 = sample(m0 + q), v1 = sample(m0 + h + q);
+#pragma unroll
+  for (int r = 0; r < NB; ++r) {
+    const bool odd = NB == 2 ? r == 1 : (at.p >> 1) & 1;   // position bit 0 after stage 0
+    const DF u = odd ? df_sub(u0, u1) : df_add(u0, u1), v = odd ? df_sub(v0, v1) : df_add(v0, v1);
+    const CDF w = cdf_load(a.tw[odd ? q : 0]);
+    const CDF t{df_mul(v, w.re), df_mul(v, w.im)};
+    x[r].a = CDF{df_add(u, t.re), t.im};
+    x[r].b = CDF{df_sub(u, t.re), df_neg(t.im)};
+  }
+  stages(g, at, 2, x, a, exch);
+}
+// X_k = Re(post_k V_k)
+__device__ __forceinline__ DF coef(const Axis& a, const CDF& v, int k) {
+  const CDF p = cdf_load(a.post[k]);
   return df_sub(df_mul(p.re, v.re), df_mul(p.im, v.im));
 }
 
-// Inverse: coefficients c(g, k) (double-floats) -> buf holds F; sample i of
-// vector g is Re buf[g n + mak(i, n)] / n. The coefficients may be read from
-// buf itself: every thread reads its W values before any is written.
-template <class Coef>
-__device__ __forceinline__ void dct3(float4* buf, int G, const Axis& a, Coef c) {
-  float4 w[kPer];
-  int at[kPer];
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < kPer; ++q) {
-    const int e = threadIdx.x + q * kThreads;
-    at[q] = -1;
-    if (e < (G << a.logn)) {
-      const int g = e >> a.logn, k = e & (a.n - 1);
-      const float2 sk = a.inv_s[k];
-      const DF ck = df_mul(c(g, k), DF{sk.x, sk.y});
-      DF cn = DF{0.f, 0.f};
-      if (k) {
-        const float2 sn = a.inv_s[a.n - k];
-        cn = df_mul(c(g, a.n - k), DF{sn.x, sn.y});
-      }
-      w[q] = cdf_store(cdf_mul(cdf_load(a.pre[k]), CDF{ck, cn}));
-      at[q] = (g << a.logn) + brev(k, a.logn);
+// Inverse: the coefficients X_k / s_k staged (st[vec * stride + pad_k(k)]) ->
+// F; sample unmak(m) of the vector is Re F_m / n.
+template <int NB, class G>
+__device__ __forceinline__ void inverse(const G& g, const Place<NB>& at, const float2* st, int stride, const Axis& a,
+                                        float4* exch, Pair (&x)[NB]) {
+  const float2* v = st + at.vec * stride;
+  auto w = [&](int k) {
+    const float2 c = v[pad_k(k)];
+    DF cn{0.f, 0.f};
+    if (k) {
+      const float2 r = v[pad_k(at.n - k)];
+      cn = DF{r.x, r.y};
     }
-  }
-  __syncthreads();
+    return cdf_mul(cdf_load(a.pre[k]), CDF{DF{c.x, c.y}, cn});
+  };
+  const int m = brev(at.p, at.L);
 #pragma unroll
-  for (int q = 0; q < kPer; ++q)
-    if (at[q] >= 0) buf[at[q]] = w[q];
-  stages(buf, G, a);
+  for (int r = 0; r < NB; ++r) {
+    const int k = m + r * (at.n >> 2);
+    const CDF u = w(k), t = w(k + (at.n >> 1));
+    x[r].a = CDF{df_add(u.re, t.re), df_add(u.im, t.im)};   // stage 0: twiddle one
+    x[r].b = CDF{df_sub(u.re, t.re), df_sub(u.im, t.im)};
+  }
+  stages(g, at, 1, x, a, exch);
 }
-// Re of an inverse-transform output slot, times 1/n (a power of two)
-__device__ __forceinline__ DF out_sample(const float4& v, float inv_n) { return df_scale(DF{v.x, v.z}, inv_n); }
+// an inverse output times 1/n (a power of two)
+__device__ __forceinline__ DF out_sample(const CDF& v, float inv_n) { return df_scale(v.re, inv_n); }
 // t1 / t2 as double-float grids
 __device__ __forceinline__ float2* df_grid(float* g) { return reinterpret_cast<float2*>(g); }
 __device__ __forceinline__ DF df_at(const float* g, size_t i) {
   const float2 v = reinterpret_cast<const float2*>(g)[i];
   return DF{v.x, v.y};
+}
+// the staged copies: NB = 1 has two (one filled while the other may still be
+// read by a vector of one or two warps, whose transforms cross no block
+// barrier), NB = 2 one (its exchanges' barriers lie between)
+template <int NB>
+__device__ __forceinline__ float2* stage_in(float4* buf) {
+  return reinterpret_cast<float2*>(buf + (NB == 1 ? 512 : 1024));
+}
+template <int NB>
+__device__ __forceinline__ float2* stage_out(float4* buf) {
+  return stage_in<NB>(buf) + (NB == 1 ? kStage : 0);
 }
 
 // Pass 1: t1 = rows-DCT(rho). With `mean` (fixed-point mean per field) the
@@ -233,116 +352,224 @@ __device__ __forceinline__ DF df_at(const float* g, size_t i) {
 // the transform exactly (as a double-float), is stored rounded to FP32, and
 // the physical overflow is counted into the IS_OVERFLOW / IS_OVER_BINS
 // partials.
-static __device__ void pass_rows_fwd(const Dev& d, Partials p, int vb, int nvb, Smem& sm, Shared& sh,
-                                     const long long* mean) {
-  const int W = d.g.Wb, H = d.g.Hb, G = min(group_size(d.logW), H);
-  const int gpf = (H + G - 1) / G, groups = gpf * d.K;
-  const Axis a = vb < groups ? stage_tables(axis_x(d), sm.buf) : axis_x(d);
+template <int NB, class G>
+static __device__ __forceinline__ void rows_fwd(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
+                                                Shared& sh, const long long* mean, bool tables) {
+  const int W = d.g.Wb, H = d.g.Hb, L = d.logW, GV = min(group_size(L), H), per = GV << L;
+  const int gpf = (H + GV - 1) / GV, groups = gpf * d.K;
+  const Axis a = vb < groups ? stage_tables(g, axis_x(d), buf, tables) : axis_x(d);
+  const Place<NB> at(g.tid, L);
+  const int stride = pad_k(W);
+  float2 *in = stage_in<NB>(buf), *out = stage_out<NB>(buf);
   long long ov[kMaxFields], cnt[kMaxFields];
 #pragma unroll
   for (int f = 0; f < kMaxFields; ++f) ov[f] = cnt[f] = 0;
   for (int t = vb; t < groups; t += nvb) {
-    const int f = t / gpf, y0 = (t % gpf) * G;
-    const size_t base = (size_t)f * d.B;
-    dct2(sm.buf, G, a, [&](int g, int x) -> DF {
-      const int y = y0 + g;
-      if (y >= H) return DF{0.f, 0.f};
-      const size_t i = base + (size_t)y * W + x;
-      if (!mean) return DF{d.rho[i], 0.f};
-      const long long q = d.phys[i];
-      const long long v = q + d.fill[i] - mean[f];
-      d.rho[i] = __ll2float_rn(v) * kInvFixF;
-      if (q > 0)
+    const int f = t / gpf, y0 = (t % gpf) * GV;
+    const size_t base = (size_t)f * d.B + (size_t)y0 * W;
+    g.sync();   // earlier readers of the buffer are done
+    long long o = 0, c = 0;
 #pragma unroll
-        for (int ff = 0; ff < kMaxFields; ++ff)
-          if (ff == f) {
-            ov[ff] += q;
-            cnt[ff] += 1;
+    for (int q = 0; q < 2 * NB; ++q) {
+      const int e = g.tid + q * kThreads;
+      if (e < per) {
+        DF x;
+        if (!mean) {
+          x = DF{d.rho[base + e], 0.f};
+        } else {
+          const long long ph = d.phys[base + e];
+          const long long v = ph + d.fill[base + e] - mean[f];
+          d.rho[base + e] = __ll2float_rn(v) * kInvFixF;
+          if (ph > 0) {
+            o += ph;
+            c += 1;
           }
-      return df_scale(df_from_ll(v), kInvFixF);
-    });
-    for (int e = threadIdx.x; e < (G << a.logn); e += blockDim.x) {
-      const int g = e >> a.logn, k = e & (W - 1), y = y0 + g;
-      if (y < H) {
-        const DF c = coef(a, sm.buf, g, k);
-        df_grid(d.t1)[base + (size_t)y * W + k] = make_float2(c.hi, c.lo);
+          x = df_scale(df_from_ll(v), kInvFixF);
+        }
+        in[(e & ~(W - 1)) + mak(e & (W - 1), W)] = make_float2(x.hi, x.lo);
       }
+    }
+#pragma unroll
+    for (int ff = 0; ff < kMaxFields; ++ff)
+      if (ff == f) {
+        ov[ff] += o;
+        cnt[ff] += c;
+      }
+    g.sync();
+    Pair x[NB];
+    const bool mine = at.vec < GV;   // fewer vectors than a group holds: idle threads trade zeros
+    Place<NB> pl = at;
+    if (!mine) pl.vec = 0;
+    forward(g, pl, in, a, buf, x);
+    if (mine)
+#pragma unroll
+      for (int r = 0; r < NB; ++r) {
+        const int k = out_index(at, r);
+        const DF c0 = coef(a, x[r].a, k), c1 = coef(a, x[r].b, k + (W >> 1));
+        out[at.vec * stride + pad_k(k)] = make_float2(c0.hi, c0.lo);
+        out[at.vec * stride + pad_k(k + (W >> 1))] = make_float2(c1.hi, c1.lo);
+      }
+    g.sync();
+#pragma unroll
+    for (int q = 0; q < 2 * NB; ++q) {
+      const int e = g.tid + q * kThreads;
+      if (e < per) df_grid(d.t1)[base + e] = out[(e >> L) * stride + pad_k(e & (W - 1))];
     }
   }
   if (mean)
-    for (int f = 0; f < d.K; ++f) {
-      write_partial(ov[f], islot(p, IS_OVERFLOW + f), vb, sh.l);
-      write_partial(cnt[f], islot(p, IS_OVER_BINS + f), vb, sh.l);
-    }
+#pragma unroll
+    for (int f = 0; f < kMaxFields; ++f)
+      if (f < d.K) {
+        write_partial(g, ov[f], islot(p, IS_OVERFLOW + f), vb, sh.l);
+        write_partial(g, cnt[f], islot(p, IS_OVER_BINS + f), vb, sh.l);
+      }
 }
 
 // Pass 2: t2 = cols-IDCT(cols-DCT(t1) * inv_eig), whole columns per group;
 // the scaled coefficients stay double-floats between the two transforms.
-static __device__ void pass_cols(const Dev& d, int vb, int nvb, Smem& sm) {
-  const int W = d.g.Wb, H = d.g.Hb, G = min(group_size(d.logH), W);
-  const int gpf = (W + G - 1) / G, groups = gpf * d.K;
-  const Axis a = vb < groups ? stage_tables(axis_y(d), sm.buf) : axis_y(d);
-  const int logG = 31 - __clz(G);
+template <int NB, class G>
+static __device__ __forceinline__ void cols(const G& g, const Dev& d, int vb, int nvb, float4* buf, bool tables) {
+  const int W = d.g.Wb, H = d.g.Hb, L = d.logH, GV = min(group_size(L), W), per = GV << L;
+  const int gpf = (W + GV - 1) / GV, groups = gpf * d.K;
+  const Axis a = vb < groups ? stage_tables(g, axis_y(d), buf, tables) : axis_y(d);
+  const Place<NB> at(g.tid, L);
+  const int stride = pad_k(H), logG = 31 - __clz(GV);
+  float2 *in = stage_in<NB>(buf), *mid = stage_out<NB>(buf);
   const float inv_n = 1.0f / (float)H;
   for (int t = vb; t < groups; t += nvb) {
-    const int f = t / gpf, x0 = (t % gpf) * G;
-    const size_t base = (size_t)f * d.B;
-    dct2(
-        sm.buf, G, a,
-        [&](int g, int y) -> DF {
-          const int x = x0 + g;
-          return x < W ? df_at(d.t1, base + (size_t)y * W + x) : DF{0.f, 0.f};
-        },
-        logG);
-    // scaled coefficients, in place (each slot read and written by one thread)
-    for (int e = threadIdx.x; e < (G << a.logn); e += blockDim.x) {
-      const int g = e & (G - 1), ky = e >> logG, x = x0 + g;
-      const int slot = (g << a.logn) + ky;
-      DF c = DF{0.f, 0.f};
-      if (x < W) c = df_mul(coef(a, sm.buf, g, ky), DF{d.inv_eig[(size_t)ky * W + x], 0.f});
-      sm.buf[slot] = make_float4(c.hi, 0.f, c.lo, 0.f);
+    const int f = t / gpf, x0 = (t % gpf) * GV;
+    const size_t base = (size_t)f * d.B + x0;
+    g.sync();   // earlier readers of the buffer are done
+#pragma unroll
+    for (int q = 0; q < 2 * NB; ++q) {   // neighbouring columns read together
+      const int e = g.tid + q * kThreads, v = e & (GV - 1), y = e >> logG;
+      if (e < per) in[(v << L) + mak(y, H)] = df_grid(d.t1)[base + (size_t)y * W + v];
     }
-    dct3(sm.buf, G, a, [&](int g, int k) -> DF {
-      const float4 v = sm.buf[(g << a.logn) + k];
-      return DF{v.x, v.z};
-    });
-    for (int e = threadIdx.x; e < (G << a.logn); e += blockDim.x) {
-      const int g = e & (G - 1), y = e >> logG, x = x0 + g;
-      if (x < W) {
-        const DF v = out_sample(sm.buf[(g << a.logn) + mak(y, H)], inv_n);
-        df_grid(d.t2)[base + (size_t)y * W + x] = make_float2(v.hi, v.lo);
+    const bool mine = at.vec < GV;
+    Place<NB> pl = at;
+    if (!mine) pl.vec = 0;
+    float ie[2 * NB];   // in flight while the samples are staged
+#pragma unroll
+    for (int r = 0; r < NB; ++r) {
+      const int k = out_index(at, r);
+      ie[2 * r] = d.inv_eig[(size_t)k * W + x0 + pl.vec];
+      ie[2 * r + 1] = d.inv_eig[(size_t)(k + (H >> 1)) * W + x0 + pl.vec];
+    }
+    g.sync();
+    Pair x[NB];
+    forward(g, pl, in, a, buf, x);
+    if (mine)
+#pragma unroll
+      for (int r = 0; r < NB; ++r) {
+        const int k = out_index(at, r);
+        const float2 s0 = a.inv_s[k], s1 = a.inv_s[k + (H >> 1)];
+        const DF c0 = df_mul(df_mul(coef(a, x[r].a, k), DF{ie[2 * r], 0.f}), DF{s0.x, s0.y});
+        const DF c1 = df_mul(df_mul(coef(a, x[r].b, k + (H >> 1)), DF{ie[2 * r + 1], 0.f}), DF{s1.x, s1.y});
+        mid[at.vec * stride + pad_k(k)] = make_float2(c0.hi, c0.lo);
+        mid[at.vec * stride + pad_k(k + (H >> 1))] = make_float2(c1.hi, c1.lo);
       }
+    g.sync();
+    inverse(g, pl, mid, stride, a, buf, x);
+    const int ostride = pad_i(H);
+    if (mine)
+#pragma unroll
+      for (int r = 0; r < NB; ++r) {
+        const int m = out_index(at, r);
+        const DF v0 = out_sample(x[r].a, inv_n), v1 = out_sample(x[r].b, inv_n);
+        in[at.vec * ostride + pad_i(unmak(m, H))] = make_float2(v0.hi, v0.lo);
+        in[at.vec * ostride + pad_i(unmak(m + (H >> 1), H))] = make_float2(v1.hi, v1.lo);
+      }
+    g.sync();
+#pragma unroll
+    for (int q = 0; q < 2 * NB; ++q) {
+      const int e = g.tid + q * kThreads, v = e & (GV - 1), y = e >> logG;
+      if (e < per) df_grid(d.t2)[base + (size_t)y * W + v] = in[v * ostride + pad_i(y)];
     }
   }
 }
 
 // Pass 3: phi = rows-IDCT(t2) and the energy partials <rho, phi>.
-static __device__ void pass_rows_inv(const Dev& d, Partials p, int vb, int nvb, Smem& sm, Shared& sh) {
-  const int W = d.g.Wb, H = d.g.Hb, G = min(group_size(d.logW), H);
-  const int gpf = (H + G - 1) / G, groups = gpf * d.K;
-  const Axis a = vb < groups ? stage_tables(axis_x(d), sm.buf) : axis_x(d);
+template <int NB, class G>
+static __device__ __forceinline__ void rows_inv(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
+                                                Shared& sh, bool tables) {
+  const int W = d.g.Wb, H = d.g.Hb, L = d.logW, GV = min(group_size(L), H), per = GV << L;
+  const int gpf = (H + GV - 1) / GV, groups = gpf * d.K;
+  const Axis a = vb < groups ? stage_tables(g, axis_x(d), buf, tables) : axis_x(d);
+  const Place<NB> at(g.tid, L);
+  const int stride = pad_k(W), ostride = pad_i(W);
+  float2* mid = stage_in<NB>(buf);
+  float* out = reinterpret_cast<float*>(stage_out<NB>(buf));
   const float inv_n = 1.0f / (float)W;
   double eacc[kMaxFields] = {0.0, 0.0, 0.0, 0.0};
   for (int t = vb; t < groups; t += nvb) {
-    const int f = t / gpf, y0 = (t % gpf) * G;
-    const size_t base = (size_t)f * d.B;
-    dct3(sm.buf, G, a, [&](int g, int k) -> DF {
-      const int y = y0 + g;
-      return y < H ? df_at(d.t2, base + (size_t)y * W + k) : DF{0.f, 0.f};
-    });
-    for (int e = threadIdx.x; e < (G << a.logn); e += blockDim.x) {
-      const int g = e >> a.logn, x = e & (W - 1), y = y0 + g;
-      if (y < H) {
-        const size_t i = base + (size_t)y * W + x;
-        const float v = df_float(out_sample(sm.buf[(g << a.logn) + mak(x, W)], inv_n));
-        d.phi[i] = v;
+    const int f = t / gpf, y0 = (t % gpf) * GV;
+    const size_t base = (size_t)f * d.B + (size_t)y0 * W;
+    float rho[2 * NB];
+    g.sync();   // earlier readers of the buffer are done
+#pragma unroll
+    for (int q = 0; q < 2 * NB; ++q) {
+      const int e = g.tid + q * kThreads;
+      if (e < per) {
+        const int k = e & (W - 1);
+        const float2 s = a.inv_s[k];
+        const DF c = df_mul(df_at(d.t2, base + e), DF{s.x, s.y});
+        mid[(e >> L) * stride + pad_k(k)] = make_float2(c.hi, c.lo);
+        rho[q] = d.rho[base + e];
+      }
+    }
+    g.sync();
+    Pair x[NB];
+    const bool mine = at.vec < GV;
+    Place<NB> pl = at;
+    if (!mine) pl.vec = 0;
+    inverse(g, pl, mid, stride, a, buf, x);
+    if (mine)
+#pragma unroll
+      for (int r = 0; r < NB; ++r) {
+        const int m = out_index(at, r);
+        out[at.vec * ostride + pad_i(unmak(m, W))] = df_float(out_sample(x[r].a, inv_n));
+        out[at.vec * ostride + pad_i(unmak(m + (W >> 1), W))] = df_float(out_sample(x[r].b, inv_n));
+      }
+    g.sync();
+#pragma unroll
+    for (int q = 0; q < 2 * NB; ++q) {
+      const int e = g.tid + q * kThreads;
+      if (e < per) {
+        const float v = out[(e >> L) * ostride + pad_i(e & (W - 1))];
+        d.phi[base + e] = v;
 #pragma unroll
         for (int ff = 0; ff < kMaxFields; ++ff)
-          if (ff == f) eacc[ff] += (double)(d.rho[i] * v);
+          if (ff == f) eacc[ff] += (double)(rho[q] * v);
       }
     }
   }
-  for (int f = 0; f < d.K; ++f) write_partial(eacc[f], pslot(p, SLOT_ENERGY + f), vb, sh.d);
+#pragma unroll
+  for (int f = 0; f < kMaxFields; ++f)
+    if (f < d.K) write_partial(g, eacc[f], pslot(p, SLOT_ENERGY + f), vb, sh.d);
+}
+
+template <class G>
+static __device__ void pass_rows_fwd(const G& g, const Dev& d, Partials p, int vb, int nvb, Smem& sm, Shared& sh,
+                                     const long long* mean, bool tables) {
+  if (d.logW == 10)
+    rows_fwd<2>(g, d, p, vb, nvb, sm.buf, sh, mean, tables);
+  else
+    rows_fwd<1>(g, d, p, vb, nvb, sm.buf, sh, mean, tables);
+}
+template <class G>
+static __device__ void pass_cols(const G& g, const Dev& d, int vb, int nvb, Smem& sm, bool tables) {
+  if (d.logH == 10)
+    cols<2>(g, d, vb, nvb, sm.buf, tables);
+  else
+    cols<1>(g, d, vb, nvb, sm.buf, tables);
+}
+template <class G>
+static __device__ void pass_rows_inv(const G& g, const Dev& d, Partials p, int vb, int nvb, Smem& sm, Shared& sh,
+                                     bool tables) {
+  if (d.logW == 10)
+    rows_inv<2>(g, d, p, vb, nvb, sm.buf, sh, tables);
+  else
+    rows_inv<1>(g, d, p, vb, nvb, sm.buf, sh, tables);
 }
 
 }  // namespace fft

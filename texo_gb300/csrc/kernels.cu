@@ -10,16 +10,16 @@ namespace tgp {
 __global__ void __launch_bounds__(kThreads) k_fft_rows_fwd(Dev d, Partials p) {
   __shared__ fft::Smem sm;
   __shared__ Shared sh;
-  fft::pass_rows_fwd(d, p, blockIdx.x, gridDim.x, sm, sh, nullptr);
+  fft::pass_rows_fwd(whole_block(), d, p, blockIdx.x, gridDim.x, sm, sh, nullptr, false);
 }
 __global__ void __launch_bounds__(kThreads) k_fft_cols(Dev d) {
   __shared__ fft::Smem sm;
-  fft::pass_cols(d, blockIdx.x, gridDim.x, sm);
+  fft::pass_cols(whole_block(), d, blockIdx.x, gridDim.x, sm, false);
 }
 __global__ void __launch_bounds__(kThreads) k_fft_rows_inv(Dev d, Partials p) {
   __shared__ fft::Smem sm;
   __shared__ Shared sh;
-  fft::pass_rows_inv(d, p, blockIdx.x, gridDim.x, sm, sh);
+  fft::pass_rows_inv(whole_block(), d, p, blockIdx.x, gridDim.x, sm, sh, false);
 }
 
 // The slice phase before tensor-core pass `step` (memory-bound, every block).

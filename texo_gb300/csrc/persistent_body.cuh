@@ -143,6 +143,8 @@ struct Ctx {
   unsigned long long nbar;
   unsigned long long* clock;   // shared [8] phase accumulators, [8] last mark, [9] barrier wait
 
+  bool tables;                 // the FFT tables stay in the work buffer
+
   unsigned ph = 0;             // barriers passed, counted by every thread
 
   __device__ bool sync() {
@@ -225,11 +227,11 @@ struct Ctx {
         // FFT form: rows (with the density preparation folded in), columns, rows
         fold_means();
         fft::Smem& fs = *reinterpret_cast<fft::Smem*>(gsm.fft);
-        for (int v = pb; v < V; v += np) fft::pass_rows_fwd(d, r.p, v, V, fs, sh, fmean);
+        for (int v = pb; v < V; v += np) fft::pass_rows_fwd(whole_block(), d, r.p, v, V, fs, sh, fmean, tables);
         if (!sync()) return false;
-        for (int v = pb; v < V; v += np) fft::pass_cols(d, v, V, fs);
+        for (int v = pb; v < V; v += np) fft::pass_cols(whole_block(), d, v, V, fs, tables);
         if (!sync()) return false;
-        for (int v = pb; v < V; v += np) fft::pass_rows_inv(d, r.p, v, V, fs, sh);
+        for (int v = pb; v < V; v += np) fft::pass_rows_inv(whole_block(), d, r.p, v, V, fs, sh, tables);
         if (!sync()) return false;
       } else {
         int st0 = 0;
@@ -498,7 +500,8 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
   }
   copy_words(&S, run);
   __syncthreads();
-  Ctx<LARGE> c{d, r, B, S, bar, &gen, &bar_failed, gsm, sh, rd, rl, coef, fvals, fmean, pb, np, Vn, 0ull, clock};
+  Ctx<LARGE> c{d, r, B, S, bar, &gen, &bar_failed, gsm, sh, rd, rl, coef, fvals, fmean, pb, np, Vn, 0ull, clock, fft::tables_stay(d)};
+  if (c.tables) fft::stage_tables(whole_block(), fft::axis_x(d), reinterpret_cast<fft::Smem*>(gsm.fft)->buf, false);
   const int n = d.nobj;
   unsigned done = 0;
   bool ok = true;

@@ -68,10 +68,14 @@ struct OpMin {
 };
 
 // Block sum of a per-thread value, written as partial vb (thread 0).
+template <class G, typename T>
+__device__ __forceinline__ void write_partial(const G& g, T v, T* slot, int vb, T* sh) {
+  T r = block_sum(g, v, sh);
+  if (g.tid == 0) slot[vb] = r;
+}
 template <typename T>
 __device__ __forceinline__ void write_partial(T v, T* slot, int vb, T* sh) {
-  T r = block_sum(v, sh);
-  if (threadIdx.x == 0) slot[vb] = r;
+  write_partial(whole_block(), v, slot, vb, sh);
 }
 struct FoldMax {
   __device__ double operator()(double a, double b) const { return fmax(a, b); }
