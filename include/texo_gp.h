@@ -447,9 +447,11 @@ int32_t texo_gp_stage_times(texo_gp_handle h, uint32_t reps, double* ms, uint32_
 const char* texo_gp_stage_name(uint32_t stage);
 /* Cumulative phase profile of the device engine since create/reset, in
  * microseconds, as seen by the persistent kernel's first block: out[0..7] =
- * scatter+WA, prep, transforms, gather+combine, preconditioner/init,
- * extrapolation, candidate, other; out[8] = time block 0 spent waiting in
- * grid barriers; out[9] = number of grid barriers. */
+ * scatter of the extrapolated point (with the origin's gradient), prep,
+ * transforms (with the wirelength beside them and a candidate's scatter),
+ * gather+combine, preconditioner/extrapolation/origin's wirelength, extra
+ * resets, candidate, other; out[8] = time block 0 spent waiting in grid
+ * barriers; out[9] = number of grid barriers. */
 int32_t texo_gp_device_profile(texo_gp_handle h, double out[10]);
 
 /* Per-iteration controller trace of the host engine (diagnostic, for parity

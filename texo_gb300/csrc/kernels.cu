@@ -59,11 +59,11 @@ __global__ void __launch_bounds__(kThreads) k_zero_energy(Dev d, Partials p, int
 }
 
 __global__ void __launch_bounds__(kThreads) k_init(Dev d, bool grids, bool wa) {
-  stage_init(d, blockIdx.x, gridDim.x, grids, wa);
+  stage_init(whole_block(), d, blockIdx.x, gridDim.x, grids, wa);
 }
 __global__ void __launch_bounds__(kThreads) k_scatter(Dev d, Partials p, const float2* pos) {
   __shared__ Shared sh;
-  stage_scatter(d, pos, p, blockIdx.x, gridDim.x, sh);
+  stage_scatter(whole_block(), d, pos, p, blockIdx.x, gridDim.x, sh);
 }
 // The tiled scatter's four passes (scatter_tiles.cuh).
 __global__ void __launch_bounds__(kThreads) k_tile_count(Dev d, const float2* pos) {
@@ -91,44 +91,44 @@ __global__ void __launch_bounds__(kThreads) k_spread_positions(Dev d, float2* ou
 }
 __global__ void __launch_bounds__(kThreads) k_wa(Dev d, Partials p, const float2* pos, double gamma) {
   __shared__ Shared sh;
-  stage_wa(d, pos, gamma, p, blockIdx.x, gridDim.x, sh);
+  stage_wa(whole_block(), d, pos, gamma, p, blockIdx.x, gridDim.x, sh.d);
 }
 __global__ void __launch_bounds__(kThreads) k_prep(Dev d, Partials p) {
   __shared__ Shared sh;
-  stage_prep(d, p, gridDim.x, blockIdx.x, gridDim.x, sh);
+  stage_prep(whole_block(), d, p, gridDim.x, blockIdx.x, gridDim.x, sh);
 }
 template <bool LARGE>
 __global__ void __launch_bounds__(kThreads) k_dct(Dev d, Partials p, int step) {
   __shared__ GemmShared sm;
   __shared__ Shared sh;
-  stage_dct_t<LARGE>(d, step, p, blockIdx.x, gridDim.x, sm, sh);
+  stage_dct_t<LARGE>(whole_block(), d, step, p, blockIdx.x, gridDim.x, sm, sh);
 }
 __global__ void __launch_bounds__(kThreads) k_gather(Dev d, Partials p, const float2* pos) {
   __shared__ Shared sh;
-  stage_gather(d, pos, p, blockIdx.x, gridDim.x, sh);
+  stage_gather(whole_block(), d, pos, p, blockIdx.x, gridDim.x, sh);
 }
 __global__ void __launch_bounds__(kThreads) k_combine(Dev d, Partials p, const double* coef, float2* gout) {
   __shared__ Shared sh;
-  stage_combine(d, coef, gout, p, blockIdx.x, gridDim.x, sh);
+  stage_combine(whole_block(), d, coef, gout, p, blockIdx.x, gridDim.x, sh);
 }
 __global__ void __launch_bounds__(kThreads) k_extrapolate(Dev d, Partials p, const float2* x, const float2* xp,
                                                          float e, float2* y) {
   __shared__ Shared sh;
-  stage_extrapolate(d, x, xp, e, y, p, blockIdx.x, gridDim.x, sh);
+  stage_extrapolate(whole_block(), d, x, xp, e, y, p, blockIdx.x, gridDim.x, sh);
 }
 __global__ void __launch_bounds__(kThreads) k_candidate(Dev d, Partials p, const float2* y, const float2* gy,
                                                        float invL, float2* c) {
   __shared__ Shared sh;
-  stage_candidate(d, y, gy, invL, c, p, blockIdx.x, gridDim.x, sh);
+  stage_candidate(whole_block(), d, y, gy, invL, c, p, blockIdx.x, gridDim.x, sh);
 }
 __global__ void __launch_bounds__(kThreads) k_kkt(Dev d, Partials p, const float2* x, const float2* g,
                                                  const float2* ref) {
   __shared__ Shared sh;
-  stage_kkt(d, x, g, ref, p, blockIdx.x, gridDim.x, sh);
+  stage_kkt(whole_block(), d, x, g, ref, p, blockIdx.x, gridDim.x, sh);
 }
 __global__ void __launch_bounds__(kThreads) k_precond(Dev d, Partials p, const double* lambda) {
   __shared__ Shared sh;
-  stage_precond(d, lambda, p, blockIdx.x, gridDim.x, sh);
+  stage_precond(whole_block(), d, lambda, p, blockIdx.x, gridDim.x, sh);
 }
 __global__ void __launch_bounds__(kThreads) k_hpwl(Dev d, Partials p, const float2* pos) {
   __shared__ Shared sh;

@@ -13,9 +13,9 @@ const void* batch_kernel_large();
 
 int persistent_blocks_per_sm() {
   int a = 0, b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, persistent_kernel_small(), kThreads, 0) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, persistent_kernel_small(), 2 * kThreads, 0) != cudaSuccess)
     return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, persistent_kernel_large(), kThreads, 0) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, persistent_kernel_large(), 2 * kThreads, 0) != cudaSuccess)
     return 0;
   return a < b ? a : b;
 }
@@ -38,7 +38,7 @@ int32_t enqueue_persistent(const Dev& d, const Reduce& r, const Buffers& b, RunB
   GridBarrier* bar = &dev->bar;
   void* args[] = {&dd, &rr, &bb, &run, &bar, &V};
   const void* fn = large_tiles(d) ? persistent_kernel_large() : persistent_kernel_small();
-  if (cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(kThreads), args, 0, s) != cudaSuccess) return TEXO_GP_ERR_CUDA;
+  if (cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(2 * kThreads), args, 0, s) != cudaSuccess) return TEXO_GP_ERR_CUDA;
   if (cudaMemcpyAsync(host, dev, sizeof(RunBlock), cudaMemcpyDeviceToHost, s) != cudaSuccess) return TEXO_GP_ERR_CUDA;
   return TEXO_GP_OK;
 }

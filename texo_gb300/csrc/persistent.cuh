@@ -6,14 +6,16 @@
 namespace tgp {
 
 // Co-resident blocks per SM of the persistent kernels. One instance alone
-// runs 1 per SM (up to 255 registers per thread; each instance has one
-// virtual block per SM, so a single launch covers all of them): at 42k cells
-// the loop is bound by its grid barriers and the FFT passes' latency, which
-// fewer, larger blocks cut (measured on GB300: 3633 it/s with 1 per SM, 3254
-// with 2, 2139 with 4). The batch kernel runs 4 per SM (64 registers): many
-// latency-bound instances share the GPU, and more resident warps win over
-// registers there (64 mixed jobs: 193 placements/s with 4 per SM against
-// 146 with 2).
+// runs one double block of 2 x 256 threads per SM (each instance has one
+// virtual block of 256 per SM, so a single launch covers all of them): at 42k
+// cells the loop is bound by its grid barriers and the latency of its phases,
+// which more blocks lengthen (with single blocks: 3633 it/s with 1 per SM,
+// 3254 with 2, 2139 with 4), while the second half runs the wirelength work
+// beside the transforms (device time of a 42k-cell placement 21.8 -> 17.2 ms,
+// with the phases it saves). The batch kernel runs 4 single blocks per SM (64
+// registers): many latency-bound instances share the GPU, and more resident
+// warps win over registers there (64 mixed jobs: 193 placements/s with 4 per
+// SM against 146 with 2).
 constexpr int kBlocksPerSm = 1;
 constexpr int kBatchBlocksPerSm = 4;
 
@@ -54,7 +56,7 @@ struct DevRun {
   double lambda[kMaxFields], e0[kMaxFields], inv_e0[kMaxFields], mstep, gamma;
   double best_max, best_tot;
   int have_prev_stationary, density_at_x;
-  double cur_overflow[kMaxFields], cur_energy[kMaxFields], cur_force[kMaxFields];
+  double cur_overflow[kMaxFields], cur_energy[kMaxFields];
   long long cur_overflow_fixed[kMaxFields];
   // Nesterov state (global_placement.rs:29-58)
   double a, L;
@@ -81,13 +83,13 @@ struct RunBlock {
 
 // Phase categories of DevRun::phase_ns.
 enum PhaseClock {
-  PC_SCATTER_WA = 0,   // scatter + WA (or WA alone) up to its barrier
+  PC_SCATTER_WA = 0,   // scatter of y + the origin's combination
   PC_PREP = 1,
-  PC_DCT = 2,          // the four transform GEMMs
+  PC_DCT = 2,          // the transforms and the WA beside them (a candidate's scatter included)
   PC_GATHER = 3,       // gather + combine
-  PC_PRECOND = 4,      // preconditioner / init / copies
-  PC_EXTRAP = 5,       // extrapolation + init
-  PC_CANDIDATE = 6,    // candidate + init
+  PC_PRECOND = 4,      // preconditioner, extrapolation, reset, the origin's WA
+  PC_EXTRAP = 5,       // a reset between two density evaluations of one step
+  PC_CANDIDATE = 6,    // candidate + reset
   PC_OTHER = 7
 };
 

@@ -2,7 +2,7 @@
 //
 // The kernel runs `optimize_density_once` (crates/texo-pnr/src/eplace.rs:439-582)
 // with `dynamic_nesterov_step` (crates/texo-pnr/src/global_placement.rs:121-335)
-// on the device. Stages are separated by a barrier over the instance's
+// on the device. Phases are separated by a barrier over the instance's
 // blocks; after each barrier every block reduces the partials it needs in the
 // same fixed order, so all blocks hold bit-identical scalars and take the same
 // branch. Thread 0 of each block keeps the controller state in shared memory;
@@ -12,6 +12,23 @@
 // instance's physical blocks loop over them. Partials are indexed by virtual
 // block, so an instance computes bit-identical results whether it runs alone
 // on every SM or shares one launch with other instances (batched serving).
+//
+// One iteration, with the usual origin whose density is known (X the origin,
+// Y the extrapolated point, C a candidate; "|" a grid barrier):
+//   preconditioner, Y, reset of the grids; WA(X) | scatter(Y), combine(X) |
+//   transforms(Y) | | ; WA(Y) | gather + combine(Y) |
+//   candidate C, reset of the grids | scatter(C) | transforms(C) | | ; WA(C) |
+//   gather + combine(C) |
+// The origin's gradient costs no phase of its own (its WA runs beside the
+// preconditioner, its combination beside Y's scatter), and a point's WA runs
+// beside its transforms: they only meet in the gradient's combination.
+//
+// A launch for one placement alone runs double blocks (SETS = 2): the first
+// half A runs the phases' main line, the second half B the WA work, so that
+// the WA's latency hides behind the transforms'; phases whose items need no
+// order are split over both. Batched launches run single blocks (SETS = 1)
+// that do the same work one after the other: there other instances' blocks
+// hide the latency.
 //
 // Every wait is bounded: a barrier that does not complete within its spin
 // budget sets an error word, and the instance's blocks then leave the kernel
@@ -111,19 +128,72 @@ union FoldValue {
   long long l;
 };
 constexpr int kMaxFoldJobs = 3 * kMaxFields + 3;
-template <typename T, typename Op>
-__device__ __forceinline__ T warp_fold(const T* a, int n, T init, Op op) {
+// The partials a warp folds, loaded ahead of the fold itself (five a lane:
+// an instance has at most one virtual block a multiprocessor; more are read
+// when they are folded).
+constexpr int kFoldAhead = 5;
+struct FoldAhead {
+  unsigned long long v[kFoldAhead];
+};
+__device__ __forceinline__ FoldAhead fold_load(const void* a, int n) {
+  FoldAhead f;
   const int lane = threadIdx.x & 31;
-  T v = lane < n ? a[lane] : init;
-#pragma unroll 4
-  for (int i = lane + 32; i < n; i += 32) v = op(v, a[i]);
+#pragma unroll
+  for (int u = 0; u < kFoldAhead; ++u) {
+    const int i = lane + 32 * u;
+    f.v[u] = i < n ? reinterpret_cast<const unsigned long long*>(a)[i] : 0ull;
+  }
+  return f;
+}
+template <typename T, typename Op>
+__device__ __forceinline__ T fold_loaded(const FoldAhead& f, const T* a, int n, T init, Op op) {
+  const int lane = threadIdx.x & 31;
+  auto as = [](unsigned long long x) {
+    T t;
+    memcpy(&t, &x, sizeof(T));
+    return t;
+  };
+  T v = lane < n ? as(f.v[0]) : init;
+#pragma unroll
+  for (int u = 1; u < kFoldAhead; ++u)
+    if (lane + 32 * u < n) v = op(v, as(f.v[u]));
+  for (int i = lane + 32 * kFoldAhead; i < n; i += 32) v = op(v, a[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
+template <typename T, typename Op>
+__device__ __forceinline__ T warp_fold(const T* a, int n, T init, Op op) {
+  return fold_loaded(fold_load(a, n), a, n, init, op);
+}
+__device__ __forceinline__ FoldValue fold_job(const FoldAhead& f, const FoldJob& jb, int n) {
+  FoldValue out;
+  switch (jb.op) {
+    case FOLD_DSUM: out.d = fold_loaded(f, (const double*)jb.a, n, 0.0, OpAdd()); break;
+    case FOLD_ISUM: out.l = fold_loaded(f, (const long long*)jb.a, n, 0ll, OpAdd()); break;
+    case FOLD_IMIN: out.l = fold_loaded(f, (const long long*)jb.a, n, 0x7fffffffffffffffll, OpMin()); break;
+    case FOLD_DMAX: out.d = fold_loaded(f, (const double*)jb.a, n, 0.0, OpMax()); break;
+    default: out.d = fold_loaded(f, (const double*)jb.a, n, (double)INFINITY, OpMin()); break;
+  }
+  return out;
+}
 
-template <bool LARGE>
+// Block-level scratch of the loop's own reductions.
+template <int SETS>
+struct LoopShared {
+  Shared a;                                   // half A's (the block's) folds
+  double pair[2 * (kThreads + 4)];            // two FP64 sums at once (half A)
+  double wa[SETS == 2 ? kThreads + 4 : 1];    // half B's WA value
+  long long tot[kMaxFields][SETS * kThreads / 32];
+  unsigned u[3][SETS * kThreads / 32];
+};
+
+template <bool LARGE, int SETS>
 struct Ctx {
+  static constexpr int kBlock = SETS * kThreads;
+  static constexpr int kWarps = kBlock / 32;
+  using GA = Group<SETS == 2 ? 1 : 0>;
+  using GB = Group<SETS == 2 ? 2 : 0>;
   const Dev& d;
   const Reduce& r;
   const Buffers& B;
@@ -132,32 +202,55 @@ struct Ctx {
   unsigned* gen;
   int* gen_failed;     // shared: the barrier's error word as thread 0 last read it
   GemmShared& gsm;
-  Shared& sh;
-  double* rd;         // reduction scratch (shared)
-  long long* rl;
+  LoopShared<SETS>& sh;
   double* coef;       // shared [kMaxFields]
+  float* coef32;      // shared [kMaxFields]
   FoldValue* fv;      // shared [kMaxFoldJobs] results of fold()
   long long* fmean;   // shared [kMaxFields] fixed-point density means
   int pb, np;         // physical block of the instance, physical block count
   int V;              // virtual blocks of the instance
   unsigned long long nbar;
   unsigned long long* clock;   // shared [8] phase accumulators, [8] last mark, [9] barrier wait
-
   bool tables;                 // the FFT tables stay in the work buffer
 
-  unsigned ph = 0;             // barriers passed, counted by every thread
+  unsigned ws = 0;             // phases that wrote an alternating partial set, counted by every thread
 
-  __device__ bool sync() {
-    ++ph;
-    return grid_sync(bar, (unsigned)np, gen, &nbar, pb == 0 ? clock + 9 : nullptr, gen_failed);
+  __device__ bool in_a() const { return SETS == 1 || threadIdx.x < kThreads; }
+  __device__ bool in_b() const { return SETS == 1 || threadIdx.x >= kThreads; }
+  __device__ GA half_a() const { return GA{(int)threadIdx.x & (kThreads - 1)}; }
+  __device__ GB half_b() const { return GB{(int)threadIdx.x & (kThreads - 1)}; }
+
+  __device__ void meet() {   // thread 0's part of a grid barrier
+    const unsigned long long t0 = pb == 0 ? now_ns() : 0ull;
+    *gen_failed = !grid_arrive_wait(bar, (unsigned)np, gen, kSpinLimit);
+    ++nbar;
+    if (pb == 0) clock[9] += now_ns() - t0;
   }
-  // Partials of the loop's back-to-back phases (extrapolate, candidate,
-  // stationary check) alternate between two sets: a block that leaves a
-  // barrier early and writes the next phase's partials must not overwrite
-  // the ones a slower block of the instance is still reducing. wset() is
-  // written by the current phase, rset() holds the phase that just ended.
-  __device__ Partials wset() const { return (ph & 1u) ? r.q : r.p; }
-  __device__ Partials rset() const { return (ph & 1u) ? r.p : r.q; }
+  // Grid barrier, every thread of the block.
+  __device__ bool sync() {
+    __syncthreads();
+    if (threadIdx.x == 0) meet();
+    __syncthreads();
+    return *gen_failed == 0;   // one read of the error word per block, so all its threads agree
+  }
+  // Grid barrier of half A alone, while half B works on. It orders what the
+  // whole block wrote before its last block barrier, and half A since. After
+  // a failure half A goes on to the next whole-block barrier, which fails at
+  // once, so half B never waits for it.
+  __device__ bool sync_a(const GA& g) {
+    g.sync();
+    if (threadIdx.x == 0) meet();
+    g.sync();
+    return *gen_failed == 0;
+  }
+  // Partials of phases that may follow one another directly (extrapolation,
+  // candidates, stationary check) alternate between two sets: a block that
+  // leaves a barrier early and writes the next phase's partials must not
+  // overwrite the ones a slower block of the instance is still reducing.
+  // Every other slot is written again only after a barrier that its readers
+  // have reached.
+  __device__ Partials set() const { return (ws & 1u) ? r.q : r.p; }
+
   // Charges the time since the previous mark to phase category `cat` (block 0).
   __device__ void mark(int cat) {
     if (pb == 0 && threadIdx.x == 0) {
@@ -166,31 +259,20 @@ struct Ctx {
       clock[8] = t;
     }
   }
-  // Several reductions of partials at once: job j is folded by warp j (mod
-  // the warp count), so the loads of all jobs are in flight together (one
-  // L2 round trip for partials that other SMs wrote, often on the other
-  // die) and the FP64 folds of different jobs run on different SM
-  // sub-partitions. Every thread reads the results in fv after the final
-  // block barrier.
-  __device__ void fold(const FoldJob* jobs, int n) {
-    __syncthreads();   // earlier readers of fv are done
-    const int nw = (int)(blockDim.x >> 5);
-    for (int j = threadIdx.x >> 5; j < n; j += nw) {
-      const FoldJob jb = jobs[j];
-      FoldValue out;
-      switch (jb.op) {
-        case FOLD_DSUM: out.d = warp_fold((const double*)jb.a, V, 0.0, OpAdd()); break;
-        case FOLD_ISUM: out.l = warp_fold((const long long*)jb.a, V, 0ll, OpAdd()); break;
-        case FOLD_IMIN: out.l = warp_fold((const long long*)jb.a, V, 0x7fffffffffffffffll, OpMin()); break;
-        case FOLD_DMAX: out.d = warp_fold((const double*)jb.a, V, 0.0, OpMax()); break;
-        default: out.d = warp_fold((const double*)jb.a, V, (double)INFINITY, OpMin()); break;
-      }
+  // Several reductions of partials at once, right after a grid barrier: job j
+  // is folded by warp j (mod the warp count), so the loads of all jobs are in
+  // flight together (one L2 round trip for partials that other SMs wrote,
+  // often on the other die) and the FP64 folds of different jobs run on
+  // different SM sub-partitions. Every thread reads the results in fv after
+  // the final block barrier.
+  template <class Job>
+  __device__ void fold(int n, Job job) {
+    for (int j = threadIdx.x >> 5; j < n; j += kWarps) {
+      const FoldJob jb = job(j);
+      const FoldValue out = fold_job(fold_load(jb.a, V), jb, V);
       if ((threadIdx.x & 31) == 0) fv[j] = out;
     }
     __syncthreads();
-  }
-  __device__ long long risum_prev(int slot) {
-    return block_reduce_array(islot(rset(), slot), V, 0ll, OpAdd(), rl);
   }
   __device__ float2* X() const { return B.pos[S.ix]; }
   __device__ float2* Xp() const { return B.pos[S.ixp]; }
@@ -201,131 +283,486 @@ struct Ctx {
   __device__ float2* gC() const { return B.grad[S.igc]; }
 
   __device__ void copy(float2* dst, const float2* src, int n) {
-    for (int i = pb * blockDim.x + threadIdx.x; i < n; i += np * blockDim.x) dst[i] = src[i];
+    for (int i = pb * kBlock + threadIdx.x; i < n; i += np * kBlock) dst[i] = src[i];
+  }
+
+  // ---- the phases' work on one virtual block ------------------------------
+
+  // Resets of the accumulators by the calling threads (all or one half).
+  __device__ void init(int v, bool grids, bool wa) {
+    if (grids) {
+      const int n = d.K * d.B, stride = V * kThreads;
+      for (int i = v * kThreads + (threadIdx.x & (kThreads - 1)); i < n; i += stride) {
+        d.phys[i] = -d.capfix[i];
+        d.fill[i] = 0;
+      }
+    }
+    if (wa)
+      for (int i = v * kThreads + (threadIdx.x & (kThreads - 1)); i < 2 * d.U; i += V * kThreads) d.wa_fix[i] = 0ull;
+  }
+
+  // Density scatter by the whole block, with the per-field tap total.
+  __device__ void scatter(const float2* pos, int v) {
+    long long tot[kMaxFields];
+    scatter_items(d, pos, v * kBlock + (int)threadIdx.x, V * kBlock, tot);
+    if (v != pb) __syncthreads();   // the previous virtual block's totals have been read
+#pragma unroll
+    for (int f = 0; f < kMaxFields; ++f)
+      if (f < d.K) {
+        const long long t = warp_sum(tot[f]);
+        if ((threadIdx.x & 31) == 0) sh.tot[f][threadIdx.x >> 5] = t;
+      }
+    __syncthreads();
+    if ((int)threadIdx.x < d.K) {
+      long long t = 0;
+      for (int w = 0; w < kWarps; ++w) t += sh.tot[threadIdx.x][w];
+      islot(r.p, IS_GRID_SUM + threadIdx.x)[v] = t;
+    }
+  }
+
+  // WA by half B (the whole single block).
+  __device__ void wa(const float2* pos, double gam) {
+    const GB g = half_b();
+    for (int v = pb; v < V; v += np) {
+      if constexpr (SETS == 2)
+        stage_wa(g, d, pos, gam, r.p, v, V, sh.wa);
+      else
+        stage_wa(g, d, pos, gam, r.p, v, V, sh.a.d);
+    }
+  }
+
+  // Field gradients of object o (gathered, or with `full` false the ones kept
+  // from the last density evaluation) and the combined gradient; the WA
+  // accumulators are cleared for the next evaluation as they are read. The
+  // KKT residual and the first non-finite index need no order, so the
+  // objects are dealt to all threads of the block. (The L1 norms and the
+  // density force, which only the two evaluations before the first iteration
+  // use, come from stage_gather / stage_combine there.)
+  struct Raw {
+    float2 f[kMaxFields];
+  };
+  __device__ __forceinline__ Raw field_gradient(const float2* pos, int o, bool full) {
+    Raw a;
+#pragma unroll
+    for (int f = 0; f < kMaxFields; ++f) a.f[f] = make_float2(0.f, 0.f);
+    if (o >= d.nobj) return a;
+    if (!full) {
+      if (o < d.U) {
+#pragma unroll
+        for (int f = 0; f < kMaxFields; ++f)
+          if (f < d.K) a.f[f] = d.graw[(size_t)f * d.nobj + o];
+      } else {
+        a.f[0] = d.graw[(size_t)d.fil_field[o - d.U] * d.nobj + o];
+      }
+      return a;
+    }
+    if (o < d.U) {
+      const int m0 = d.unit_mem_ptr[o], m1 = d.unit_mem_ptr[o + 1];
+      const float2 pu = pos[o];
+      for (int m = m0; m < m1; ++m) {
+        const int f = d.mem_field[m];
+        const float2 off = d.mem_off[m];
+        const float q = d.mem_q[m];
+        const float2 s = sample_grad(d, d.phi + (size_t)f * d.B, __fadd_rn(pu.x, off.x), __fadd_rn(pu.y, off.y));
+#pragma unroll
+        for (int ff = 0; ff < kMaxFields; ++ff)
+          if (ff == f) {
+            a.f[ff].x += q * s.x;
+            a.f[ff].y += q * s.y;
+          }
+      }
+#pragma unroll
+      for (int f = 0; f < kMaxFields; ++f)
+        if (f < d.K) d.graw[(size_t)f * d.nobj + o] = a.f[f];
+    } else {
+      const int j = o - d.U;
+      const int f = d.fil_field[j];
+      const float q = d.fil_q[j];
+      const float2 pf = pos[o];
+      const float2 s = sample_grad(d, d.phi + (size_t)f * d.B, pf.x, pf.y);
+      a.f[0] = make_float2(q * s.x, q * s.y);   // a filler's one field
+      d.graw[(size_t)f * d.nobj + o] = a.f[0];
+    }
+    return a;
+  }
+  __device__ __forceinline__ void combine_object(const Raw& a, int o, const float2* pos, float2* g, float& kkt,
+                                                 unsigned& bad) {
+    if (o >= d.nobj) return;
+    const float2 at = pos[o], lo = d.lo[o], hi = d.hi[o];
+    const float P = d.P[o];
+    float gx = 0.f, gy = 0.f;
+    if (o < d.U) {
+      ulonglong2* w = reinterpret_cast<ulonglong2*>(d.wa_fix) + o;
+      const ulonglong2 q = *w;
+      *w = make_ulonglong2(0ull, 0ull);
+      gx = __ll2float_rn((long long)q.x) * kInvFixF;
+      gy = __ll2float_rn((long long)q.y) * kInvFixF;
+#pragma unroll
+      for (int f = 0; f < kMaxFields; ++f)
+        if (f < d.K) {
+          const float c = coef32[f];
+          gx = fmaf(c, a.f[f].x, gx);
+          gy = fmaf(c, a.f[f].y, gy);
+        }
+    } else {
+      const float c = coef32[d.fil_field[o - d.U]];
+      gx = c * a.f[0].x;
+      gy = c * a.f[0].y;
+    }
+    if (!isfinite(gx)) bad = min(bad, 2u * (unsigned)o);
+    else if (!isfinite(gy)) bad = min(bad, 2u * (unsigned)o + 1u);
+    g[o] = make_float2(gx, gy);
+    const float s = rsqrtf(P);
+    kkt = fmaxf(kkt, kkt_comp(gx, at.x, lo.x, hi.x) * s);
+    kkt = fmaxf(kkt, kkt_comp(gy, at.y, lo.y, hi.y) * s);
+  }
+  // The block's KKT maximum and least bad index as partials of block v: the
+  // residuals are not negative, so their bits order as integers.
+  __device__ void write_kkt(float kkt, unsigned bad, int v) {
+    const unsigned k = __reduce_max_sync(0xffffffffu, __float_as_uint(kkt));
+    const unsigned b = __reduce_min_sync(0xffffffffu, bad);
+    if (v != pb) __syncthreads();   // the previous virtual block's values have been read
+    if ((threadIdx.x & 31) == 0) {
+      sh.u[0][threadIdx.x >> 5] = k;
+      sh.u[1][threadIdx.x >> 5] = b;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned km = 0u, bm = 0xffffffffu;
+      for (int w = 0; w < kWarps; ++w) {
+        km = max(km, sh.u[0][w]);
+        bm = min(bm, sh.u[1][w]);
+      }
+      mslot(r.p, MS_KKT)[v] = (double)__uint_as_float(km);
+      islot(r.p, IS_BAD)[v] = bm == 0xffffffffu ? 0x7fffffffffffffffll : (long long)bm;
+    }
+  }
+  // combine(X): the gradient at pos from the kept field gradients.
+  __device__ void combine_kept(const float2* pos, float2* g, int v) {
+    float kkt = 0.f;
+    unsigned bad = 0xffffffffu;
+    for (int o = v * kBlock + (int)threadIdx.x; o < d.nobj; o += V * kBlock)
+      combine_object(field_gradient(pos, o, false), o, pos, g, kkt, bad);
+    write_kkt(kkt, bad, v);
+  }
+  __device__ FoldJob kkt_job(int j) const {
+    return j == 0 ? FoldJob{mslot(r.p, MS_KKT), FOLD_DMAX} : FoldJob{islot(r.p, IS_BAD), FOLD_IMIN};
   }
 
   // fixed-point density mean per field (DC mode), from the scatter's grid sums
-  __device__ void fold_means() {
-    FoldJob jobs[kMaxFields];
-    for (int f = 0; f < d.K; ++f) jobs[f] = FoldJob{islot(r.p, IS_GRID_SUM + f), FOLD_ISUM};
-    fold(jobs, d.K);
-    if (threadIdx.x == 0)
-      for (int f = 0; f < d.K; ++f) fmean[f] = (fv[f].l - d.capsum[f]) / d.B;
-    __syncthreads();
+  __device__ void fold_means(const GA& g) {
+    const int w = g.tid >> 5;
+    if (w < d.K) {
+      const FoldJob jb{islot(r.p, IS_GRID_SUM + w), FOLD_ISUM};
+      const FoldValue s = fold_job(fold_load(jb.a, V), jb, V);
+      if ((g.tid & 31) == 0) fmean[w] = (s.l - d.capsum[w]) / d.B;
+    }
+    g.sync();
   }
 
-  // Objective evaluation at pos after an init phase and its barrier
-  // (ContinuousProblem::evaluate + combined_objective, eplace.rs:137-205, 1022-1044).
-  __device__ bool eval_tail(const float2* pos, float2* g, double gam, bool full, const float2* kkt_pos, ERec& out) {
-    if (full)
-      for (int v = pb; v < V; v += np) stage_scatter(d, pos, r.p, v, V, sh);
-    for (int v = pb; v < V; v += np) stage_wa(d, pos, gam, r.p, v, V, sh);
-    if (!sync()) return false;
-    mark(PC_SCATTER_WA);
-    if (full) {
-      if (d.fft) {
-        // FFT form: rows (with the density preparation folded in), columns, rows
-        fold_means();
-        fft::Smem& fs = *reinterpret_cast<fft::Smem*>(gsm.fft);
-        for (int v = pb; v < V; v += np) fft::pass_rows_fwd(whole_block(), d, r.p, v, V, fs, sh, fmean, tables);
-        if (!sync()) return false;
-        for (int v = pb; v < V; v += np) fft::pass_cols(whole_block(), d, v, V, fs, tables);
-        if (!sync()) return false;
-        for (int v = pb; v < V; v += np) fft::pass_rows_inv(whole_block(), d, r.p, v, V, fs, sh, tables);
-        if (!sync()) return false;
+  // Half A's side of a density evaluation once the grids are complete: phi
+  // and the overflow and energy partials.
+  __device__ bool transforms() {
+    const GA g = half_a();
+    if (d.fft) {
+      // FFT form: rows (with the density preparation folded in), columns, rows
+      fold_means(g);
+      fft::Smem& fs = *reinterpret_cast<fft::Smem*>(gsm.fft);
+      for (int v = pb; v < V; v += np) fft::pass_rows_fwd(g, d, r.p, v, V, fs, sh.a, fmean, tables);
+      if (!sync_a(g)) return false;
+      for (int v = pb; v < V; v += np) fft::pass_cols(g, d, v, V, fs, tables);
+      if (!sync_a(g)) return false;
+      for (int v = pb; v < V; v += np) fft::pass_rows_inv(g, d, r.p, v, V, fs, sh.a, tables);
+    } else {
+      int st0 = 0;
+      if (LARGE) {
+        for (int v = pb; v < V; v += np) stage_prep(g, d, r.p, V, v, V, sh.a);
+        if (!sync_a(g)) return false;
+        mark(PC_PREP);
       } else {
-        int st0 = 0;
-        if (LARGE) {
-          for (int v = pb; v < V; v += np) stage_prep(d, r.p, V, v, V, sh);
-          if (!sync()) return false;
-          mark(PC_PREP);
-        } else {
-          // density preparation folded into the first transform (one phase less)
-          fold_means();
-          for (int v = pb; v < V; v += np) stage_prep_dct0(d, fmean, r.p, v, V, gsm, sh);
-          if (!sync()) return false;
-          st0 = 1;
-        }
-        for (int st = st0; st < 4; ++st) {
-          for (int v = pb; v < V; v += np) stage_dct_t<LARGE>(d, st, r.p, v, V, gsm, sh);
-          if (!sync()) return false;
-        }
+        // density preparation folded into the first transform (one phase less)
+        fold_means(g);
+        for (int v = pb; v < V; v += np) stage_prep_dct0(g, d, fmean, r.p, v, V, gsm, sh.a);
+        if (!sync_a(g)) return false;
+        st0 = 1;
       }
-      mark(PC_DCT);
-    }
-    {
-      // energies, overflow and overflowed bins per field (density side
-      // rebuilt), and the WA value: one fold
-      FoldJob jobs[kMaxFoldJobs];
-      int nj = 0;
-      if (full)
-        for (int f = 0; f < d.K; ++f) {
-          jobs[nj++] = FoldJob{pslot(r.p, SLOT_ENERGY + f), FOLD_DSUM};
-          jobs[nj++] = FoldJob{islot(r.p, IS_OVERFLOW + f), FOLD_ISUM};
-          jobs[nj++] = FoldJob{islot(r.p, IS_OVER_BINS + f), FOLD_ISUM};
-        }
-      jobs[nj++] = FoldJob{pslot(r.p, SLOT_WA_VALUE), FOLD_DSUM};
-      fold(jobs, nj);
-    }
-    if (threadIdx.x == 0) {
-      for (int f = 0; f < d.K; ++f) {
-        if (full) {
-          const long long ov = fv[3 * f + 1].l;
-          out.energy[f] = 0.5 * fv[3 * f].d;
-          out.ovfix[f] = ov;
-          out.bins[f] = fv[3 * f + 2].l;
-          out.overflow[f] = ((double)ov * kInvFix) * S.inv_real_area[f];
-        } else {
-          out.energy[f] = S.cur_energy[f];
-          out.overflow[f] = S.cur_overflow[f];
-          out.ovfix[f] = S.cur_overflow_fixed[f];
-          out.bins[f] = 0;
-        }
+      for (int st = st0; st < 4; ++st) {
+        for (int v = pb; v < V; v += np) stage_dct_t<LARGE>(g, d, st, r.p, v, V, gsm, sh.a);
+        if (st < 3 && !sync_a(g)) return false;
       }
-      const double wa = fv[full ? 3 * d.K : 0].d;
-      out.wa = wa;
-      double value = wa;
-      for (int f = 0; f < d.K; ++f) {
-        const double ne = out.energy[f] * S.inv_e0[f];
-        value += S.lambda[f] * S.e0[f] * (ne + 0.5 * S.beta * ne * ne);
-        coef[f] = S.lambda[f] * (1.0 + S.beta * ne);
-      }
-      out.value = value;
     }
+    return true;
+  }
+
+  // Energies, overflow and WA value of the last evaluation (density side
+  // rebuilt), or the WA value alone, from the folded jobs.
+  __device__ FoldJob eval_job(int j, bool full) const {
+    if (!full || j == 3 * d.K) return FoldJob{pslot(r.p, SLOT_WA_VALUE), FOLD_DSUM};
+    const int f = j / 3, k = j % 3;
+    return k == 0   ? FoldJob{pslot(r.p, SLOT_ENERGY + f), FOLD_DSUM}
+           : k == 1 ? FoldJob{islot(r.p, IS_OVERFLOW + f), FOLD_ISUM}
+                    : FoldJob{islot(r.p, IS_OVER_BINS + f), FOLD_ISUM};
+  }
+  __device__ int eval_jobs(bool full) const { return full ? 3 * d.K + 1 : 1; }
+  // thread 0: the objective and the fields' coefficients from the jobs at fv[at...]
+  __device__ void eval_scalars(ERec& out, bool full, int at = 0) {
+    for (int f = 0; f < d.K; ++f) {
+      if (full) {
+        const long long ov = fv[at + 3 * f + 1].l;
+        out.energy[f] = 0.5 * fv[at + 3 * f].d;
+        out.ovfix[f] = ov;
+        out.bins[f] = fv[at + 3 * f + 2].l;
+        out.overflow[f] = ((double)ov * kInvFix) * S.inv_real_area[f];
+      } else {
+        out.energy[f] = S.cur_energy[f];
+        out.overflow[f] = S.cur_overflow[f];
+        out.ovfix[f] = S.cur_overflow_fixed[f];
+        out.bins[f] = 0;
+      }
+    }
+    const double wa = fv[at + (full ? 3 * d.K : 0)].d;
+    out.wa = wa;
+    double value = wa;
+    for (int f = 0; f < d.K; ++f) {
+      const double ne = out.energy[f] * S.inv_e0[f];
+      value += S.lambda[f] * S.e0[f] * (ne + 0.5 * S.beta * ne * ne);
+      coef[f] = S.lambda[f] * (1.0 + S.beta * ne);
+      coef32[f] = (float)coef[f];
+    }
+    out.value = value;
+  }
+
+  // Objective evaluation with the sums only the initial probes use, after a
+  // barrier that left the accumulators reset (ContinuousProblem::evaluate +
+  // combined_objective, eplace.rs:137-205, 1022-1044).
+  __device__ bool eval_initial(const float2* pos, float2* g, double gam, bool full, ERec& out) {
+    if (full) {
+      for (int v = pb; v < V; v += np) scatter(pos, v);
+      if (!sync()) return false;
+      if (in_a()) transforms();
+      __syncthreads();
+    }
+    if (in_b()) wa(pos, gam);
+    if (!sync()) return false;
+    mark(full ? PC_DCT : PC_SCATTER_WA);
+    fold(eval_jobs(full), [&](int j) { return eval_job(j, full); });
+    if (threadIdx.x == 0) eval_scalars(out, full);
     __syncthreads();
-    // gather and combine of one virtual block run back to back: the same
-    // thread produces and consumes each object's raw field gradient
-    for (int v = pb; v < V; v += np) {
-      if (full) stage_gather(d, pos, r.p, v, V, sh);
-      stage_combine(d, coef, g, r.p, v, V, sh, kkt_pos);
+    if (in_a()) {
+      const GA ga = half_a();
+      for (int v = pb; v < V; v += np) {
+        if (full) stage_gather(ga, d, pos, r.p, v, V, sh.a);
+        stage_combine(ga, d, coef, g, r.p, v, V, sh.a);
+      }
     }
     if (!sync()) return false;
     mark(PC_GATHER);
-    {
-      FoldJob jobs[kMaxFoldJobs];
-      int nj = 0;
-      for (int f = 0; f < d.K; ++f) {
-        jobs[nj++] = FoldJob{pslot(r.p, SLOT_RAWL1 + f), FOLD_DSUM};
-        jobs[nj++] = FoldJob{pslot(r.p, SLOT_FORCE + f), FOLD_DSUM};
-      }
-      jobs[nj++] = FoldJob{pslot(r.p, SLOT_WAL1), FOLD_DSUM};
-      jobs[nj++] = FoldJob{islot(r.p, IS_BAD), FOLD_IMIN};
-      if (kkt_pos) jobs[nj++] = FoldJob{mslot(r.p, MS_KKT), FOLD_DMAX};
-      fold(jobs, nj);
-    }
+    fold(2 * d.K + 2, [&](int j) {
+      return j < d.K       ? FoldJob{pslot(r.p, SLOT_RAWL1 + j), FOLD_DSUM}
+             : j < 2 * d.K ? FoldJob{pslot(r.p, SLOT_FORCE + j - d.K), FOLD_DSUM}
+             : j == 2 * d.K ? FoldJob{pslot(r.p, SLOT_WAL1), FOLD_DSUM}
+                            : FoldJob{islot(r.p, IS_BAD), FOLD_IMIN};
+    });
     if (threadIdx.x == 0) {
       for (int f = 0; f < d.K; ++f) {
-        out.rawl1[f] = fv[2 * f].d;
-        out.force[f] = fv[2 * f + 1].d;
+        out.rawl1[f] = fv[f].d;
+        out.force[f] = fv[d.K + f].d;
       }
       out.wal1 = fv[2 * d.K].d;
       out.bad = fv[2 * d.K + 1].l;
-      out.kkt = kkt_pos ? fv[2 * d.K + 2].d : 0.0;
+      out.kkt = 0.0;
       S.evaluations++;
       if (full) S.density_evaluations++;
     }
     __syncthreads();
     return true;
+  }
+
+  // The loop's evaluation at pos, its positions scattered: the transforms by
+  // half A, WA by half B. With lead the scatter has just ended and half A
+  // waits for the other blocks' first. Returns after a barrier of all.
+  __device__ bool density_and_wa(const float2* pos, double gam, bool lead) {
+    if (SETS == 1 || !in_a()) wa(pos, gam);
+    if (in_a()) {
+      const bool ready = !lead || sync_a(half_a());
+      if (ready) transforms();
+    }
+    const bool k = sync();
+    mark(PC_DCT);
+    return k;
+  }
+  // The rest of it: the scalars, the gathered field gradients and the
+  // combined gradient with its KKT residual. A double block gathers while
+  // the partials are on their way and folded, and needs the coefficients
+  // only to combine.
+  __device__ bool gradient(const float2* pos, float2* g, ERec& out) {
+    const int n = eval_jobs(true), stride = V * kBlock;
+    float kkt = 0.f;
+    unsigned bad = 0xffffffffu;
+    int v = pb;
+    if constexpr (SETS == 2) {
+      const int w = threadIdx.x >> 5;
+      FoldJob jb{nullptr, FOLD_DSUM};
+      FoldAhead fa;
+      if (w < n) {
+        jb = eval_job(w, true);
+        fa = fold_load(jb.a, V);
+      }
+      int o = v * kBlock + (int)threadIdx.x;
+      const Raw a0 = field_gradient(pos, o, true), a1 = field_gradient(pos, o + stride, true);
+      if (w < n) {
+        const FoldValue q = fold_job(fa, jb, V);
+        if ((threadIdx.x & 31) == 0) fv[w] = q;
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) eval_scalars(out, true);
+      __syncthreads();
+      combine_object(a0, o, pos, g, kkt, bad);
+      combine_object(a1, o + stride, pos, g, kkt, bad);
+      for (o += 2 * stride; o < d.nobj; o += stride) combine_object(field_gradient(pos, o, true), o, pos, g, kkt, bad);
+      write_kkt(kkt, bad, v);
+      v += np;
+    } else {
+      fold(n, [&](int j) { return eval_job(j, true); });
+      if (threadIdx.x == 0) eval_scalars(out, true);
+      __syncthreads();
+    }
+    for (; v < V; v += np) {
+      kkt = 0.f;
+      bad = 0xffffffffu;
+      for (int o = v * kBlock + (int)threadIdx.x; o < d.nobj; o += stride)
+        combine_object(field_gradient(pos, o, true), o, pos, g, kkt, bad);
+      write_kkt(kkt, bad, v);
+    }
+    if (!sync()) return false;
+    mark(PC_GATHER);
+    fold(2, [&](int j) { return kkt_job(j); });
+    if (threadIdx.x == 0) {
+      out.kkt = fv[0].d;
+      out.bad = fv[1].l;
+      S.evaluations++;
+      S.density_evaluations++;
+    }
+    __syncthreads();
+    return true;
+  }
+
+  // Half A, before an iteration's evaluations: the preconditioner
+  // (diagonal_preconditioner, eplace.rs:1046-1100) and y = clamp(x + e (x -
+  // xp)) with the count of coordinates that moved.
+  __device__ void precondition(const float* lam, const float2* x, const float2* xp, float e, float2* y, int v) {
+    const GA g = half_a();
+    float lambda[kMaxFields];
+#pragma unroll
+    for (int f = 0; f < kMaxFields; ++f) lambda[f] = f < d.K ? lam[f] : 0.f;
+    float pmin = INFINITY, pmax = 0.f;
+    unsigned diff = 0;
+    bool badp = false;
+    const int stride = V * kThreads;
+    for (int o = v * kThreads + g.tid; o < d.nobj; o += stride) {
+      float q[kMaxFields];
+      float m = d.pre_static[o];
+#pragma unroll
+      for (int f = 0; f < kMaxFields; ++f) q[f] = f < d.K ? d.pre_q[(size_t)f * d.nobj + o] : 0.f;
+      const float2 a = x[o], b = xp[o], lo = d.lo[o], hi = d.hi[o];
+      float2 t;
+      t.x = fclamp(a.x + e * (a.x - b.x), lo.x, hi.x);
+      t.y = fclamp(a.y + e * (a.y - b.y), lo.y, hi.y);
+      diff += (t.x != a.x) + (t.y != a.y);
+      y[o] = t;
+#pragma unroll
+      for (int f = 0; f < kMaxFields; ++f)
+        if (q[f] != 0.f) m = fmaf(lambda[f], q[f], m);
+      if (!isfinite(m) || m < 0.f) badp = true;
+      m = fmaxf(m, 1.f);
+      d.P[o] = m;
+      pmin = fminf(pmin, m);
+      pmax = fmaxf(pmax, m);
+    }
+    // not negative, so the bits order as integers
+    const unsigned lo = __reduce_min_sync(0xffffffffu, __float_as_uint(pmin));
+    const unsigned hi = __reduce_max_sync(0xffffffffu, __float_as_uint(pmax));
+    const unsigned c = __reduce_add_sync(0xffffffffu, diff) | (__any_sync(0xffffffffu, badp) ? 0x80000000u : 0u);
+    g.sync();   // earlier readers of the scratch are done
+    if ((g.tid & 31) == 0) {
+      sh.u[0][g.tid >> 5] = lo;
+      sh.u[1][g.tid >> 5] = hi;
+      sh.u[2][g.tid >> 5] = c;
+    }
+    g.sync();
+    if (g.tid == 0) {
+      unsigned a = 0x7f800000u, b = 0u, bad = 0u;
+      long long n = 0;
+      for (int w = 0; w < kThreads / 32; ++w) {
+        a = min(a, sh.u[0][w]);
+        b = max(b, sh.u[1][w]);
+        bad |= sh.u[2][w] >> 31;
+        n += sh.u[2][w] & 0x7fffffffu;
+      }
+      mslot(r.p, MS_PMIN)[v] = (double)__uint_as_float(a);
+      mslot(r.p, MS_PMAX)[v] = (double)__uint_as_float(b);
+      islot(r.p, IS_PBAD)[v] = bad;
+      islot(set(), IS_DIFF)[v] = n;
+    }
+  }
+
+  // Half A: c = clamp(y - g / (L P)); changed count, <g, c - y>, sum P (c -
+  // y)^2. Each thread's objects and the order of its sums are those of the
+  // 256-thread stage (the sums are FP32), two objects' loads in flight.
+  __device__ void candidate(const float2* y, const float2* gy, float invL, float2* c, int v) {
+    const GA g = half_a();
+    unsigned diff = 0;
+    float dot = 0.f, msn = 0.f;
+    struct In {
+      float2 a, gr, lo, hi;
+      float m;
+    };
+    auto load = [&](int o) { return In{y[o], gy[o], d.lo[o], d.hi[o], d.P[o]}; };
+    auto step = [&](const In& i, int o) {
+      const float s = invL / i.m;
+      float2 t;
+      t.x = fclamp(i.a.x - i.gr.x * s, i.lo.x, i.hi.x);
+      t.y = fclamp(i.a.y - i.gr.y * s, i.lo.y, i.hi.y);
+      diff += (t.x != i.a.x) + (t.y != i.a.y);
+      const float dx = t.x - i.a.x, dy = t.y - i.a.y;
+      dot = fmaf(i.gr.x, dx, fmaf(i.gr.y, dy, dot));
+      msn = fmaf(i.m * dx, dx, fmaf(i.m * dy, dy, msn));
+      c[o] = t;
+    };
+    const int stride = V * kThreads;
+    for (int o = v * kThreads + g.tid; o < d.nobj; o += 2 * stride) {
+      const In i0 = load(o);
+      const bool two = o + stride < d.nobj;
+      const In i1 = two ? load(o + stride) : i0;
+      step(i0, o);
+      if (two) step(i1, o + stride);
+    }
+    // both FP64 sums at once, each in block_fold_fp64's order
+    double *b0 = sh.pair, *b1 = sh.pair + kThreads + 4;
+    const unsigned n = __reduce_add_sync(0xffffffffu, diff);
+    g.sync();   // earlier readers of the scratch are done
+    b0[g.tid] = (double)dot;
+    b1[g.tid] = (double)msn;
+    if ((g.tid & 31) == 0) sh.u[0][g.tid >> 5] = n;
+    g.sync();
+    {
+      const int w = g.tid >> 5, at = (w & 3) * 32 + (g.tid & 31);
+      double* b = w < 4 ? b0 : b1;
+      double t = b[at] + b[at + 128];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, o);
+      if ((g.tid & 31) == 0) b[kThreads + (w & 3)] = t;
+    }
+    g.sync();
+    if (g.tid == 0 || g.tid == 32) {
+      const double* b = (g.tid == 0 ? b0 : b1) + kThreads;
+      pslot(set(), g.tid == 0 ? SLOT_DOT : SLOT_MSN)[v] = ((b[0] + b[1]) + b[2]) + b[3];
+    }
+    if (g.tid == 64) {
+      long long t = 0;
+      for (int w = 0; w < kThreads / 32; ++w) t += sh.u[0][w];
+      islot(set(), IS_DIFF)[v] = t;
+    }
   }
 };
 
@@ -440,6 +877,11 @@ static __device__ int update_multipliers_dev(DevRun& S) {
   S.mstep *= growth;
   return (isfinite(S.mstep) && S.mstep > 0.0) ? TEXO_GP_OK : TEXO_GP_ERR_INVALID_NORMALIZATION;
 }
+// f64::midpoint(1, sqrt(1 + 4 m^2))
+__device__ __forceinline__ double next_momentum_dev(double m) {
+  const double s = sqrt(1.0 + 4.0 * m * m);
+  return fabs(s) <= 8.0e307 ? (1.0 + s) / 2.0 : 0.5 + s / 2.0;
+}
 __device__ __forceinline__ double half_nonzero_dev(double v) {
   const double h = v * 0.5;
   return h == 0.0 ? v : h;
@@ -451,15 +893,15 @@ static __device__ void adopt_density(DevRun& S, const ERec& e) {
   for (int f = 0; f < S.K; ++f) {
     S.cur_overflow[f] = e.overflow[f];
     S.cur_energy[f] = e.energy[f];
-    S.cur_force[f] = e.force[f];
     S.cur_overflow_fixed[f] = e.ovfix[f];
   }
 }
 
 // Shared-memory step bookkeeping that every thread reads after a barrier.
 struct StepVars {
-  int restart, y_is_origin, may_reduce, has_wL, action, stationary;
+  int restart, y_is_origin, may_reduce, has_wL, action, stationary, fresh;
   double wL, tL, f_y, y_stat, next_m, pmin, pmax;
+  float extrapolation, lambda[kMaxFields];
   unsigned trials;
   int pending_best, pending_prev;
 };
@@ -474,18 +916,18 @@ __device__ __forceinline__ void copy_words(T* dst, const T* src) {
     reinterpret_cast<unsigned long long*>(dst)[i] = reinterpret_cast<const unsigned long long*>(src)[i];
 }
 
-// The placement loop of one instance, run by its np physical blocks.
-template <bool LARGE>
+// The placement loop of one instance, run by its np physical blocks of SETS *
+// kThreads threads.
+template <bool LARGE, int SETS>
 static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B, DevRun* run, GridBarrier* bar, int pb,
                          int np, int Vn) {
   __shared__ DevRun S;
   __shared__ ERec eo, ey, ec;
   __shared__ StepVars V;
   __shared__ GemmShared gsm;
-  __shared__ Shared sh;
-  __shared__ double rd[kThreads / 32];
-  __shared__ long long rl[kThreads / 32];
+  __shared__ LoopShared<SETS> sh;
   __shared__ double coef[kMaxFields];
+  __shared__ float coef32[kMaxFields];
   __shared__ FoldValue fvals[kMaxFoldJobs];
   __shared__ long long fmean[kMaxFields];
   __shared__ unsigned gen;
@@ -500,8 +942,10 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
   }
   copy_words(&S, run);
   __syncthreads();
-  Ctx<LARGE> c{d, r, B, S, bar, &gen, &bar_failed, gsm, sh, rd, rl, coef, fvals, fmean, pb, np, Vn, 0ull, clock, fft::tables_stay(d)};
-  if (c.tables) fft::stage_tables(whole_block(), fft::axis_x(d), reinterpret_cast<fft::Smem*>(gsm.fft)->buf, false);
+  Ctx<LARGE, SETS> c{d,  r,  B,  S,   bar,   &gen, &bar_failed, gsm, sh, coef, coef32,
+                     fvals, fmean, pb, np, Vn, 0ull, clock, fft::tables_stay(d)};
+  if (c.tables && c.in_a())
+    fft::stage_tables(c.half_a(), fft::axis_x(d), reinterpret_cast<fft::Smem*>(gsm.fft)->buf, false);
   const int n = d.nobj;
   unsigned done = 0;
   bool ok = true;
@@ -513,11 +957,13 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
   __syncthreads();    \
   if (threadIdx.x == 0)
 #define VLOOP for (int v = c.pb; v < c.V; v += c.np)
+#define LEAVE   \
+  {             \
+    ok = false; \
+    goto out;   \
+  }
 #define SYNC_OR_EXIT(cat) \
-  if (!c.sync()) {        \
-    ok = false;           \
-    goto out;             \
-  }                       \
+  if (!c.sync()) LEAVE    \
   c.mark(cat);
 #define FAIL(code)            \
   {                           \
@@ -533,12 +979,9 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
   if (S.phase == 0) {
     // initial probe at the ePlace gamma base, then at the adaptive gamma with
     // the density side reused (same coordinates), eplace.rs:455-471
-    VLOOP stage_init(d, v, c.V, true, true);
+    if (c.in_a()) VLOOP c.init(v, true, true);
     SYNC_OR_EXIT(PC_PRECOND)
-    if (!c.eval_tail(c.X(), c.gX(), S.gamma_base, true, nullptr, eo)) {
-      ok = false;
-      goto out;
-    }
+    if (!c.eval_initial(c.X(), c.gX(), S.gamma_base, true, eo)) LEAVE
     {
       T0 {
         double g0 = 0.0;
@@ -551,12 +994,9 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
       __syncthreads();
       if (S.status) FAIL(S.status)
     }
-    VLOOP stage_init(d, v, c.V, false, true);
+    if (c.in_a()) VLOOP c.init(v, false, true);
     SYNC_OR_EXIT(PC_PRECOND)
-    if (!c.eval_tail(c.X(), c.gX(), S.gamma, false, nullptr, eo)) {
-      ok = false;
-      goto out;
-    }
+    if (!c.eval_initial(c.X(), c.gX(), S.gamma, false, eo)) LEAVE
     T0 {
       int st = validate_initial_dev(S, eo);
       for (int f = 0; f < S.K; ++f) {
@@ -591,6 +1031,10 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
     if (S.status) FAIL(S.status)
     if (S.phase == 2) goto out;
   }
+  // the loop's combinations clear the WA accumulators they read; whatever ran
+  // before this launch may have left them dirty
+  if (c.in_a()) VLOOP c.init(v, false, true);
+  SYNC_OR_EXIT(PC_PRECOND)
 
   // ---- outer loop -------------------------------------------------------
   for (;;) {
@@ -622,82 +1066,98 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
           S.status = TEXO_GP_ERR_INVALID_LIPSCHITZ_ESTIMATE;
           S.phase = 2;
         }
+        V.next_m = next_momentum_dev(S.a);
+        V.restart = 0;
+        V.has_wL = S.has_L;
+        V.wL = S.L;
+        V.trials = 0;
+        V.fresh = !S.density_at_x;
+        V.extrapolation = (float)((S.a - 1.0) / V.next_m);
+        for (int f = 0; f < S.K; ++f) V.lambda[f] = (float)S.lambda[f];
       }
     }
     __syncthreads();
     if (S.phase == 2 || V.action == ACT_CONTINUE) break;
     ++done;
 
-    // Phase 1: preconditioner (eplace.rs:1046-1100), pending copies, and the
-    // origin evaluation's init. The origin is re-evaluated (eplace's closure
-    // changes with gamma and the multipliers); its density side is reused
-    // when the device already holds it for these coordinates.
+    // Phase 1: the preconditioner (eplace.rs:1046-1100), the extrapolated
+    // point (it needs the positions and the momentum alone), pending copies,
+    // the grids' reset and the origin's WA. The origin is re-evaluated
+    // (eplace's closure changes with gamma and the multipliers); its density
+    // side is reused when the device already holds it for these coordinates.
     {
-      const bool full = !S.density_at_x;
-      VLOOP {
-        stage_precond(d, S.lambda, r.p, v, c.V, sh);
-        stage_init(d, v, c.V, full, true);
+      const bool fresh = V.fresh != 0;
+      if (c.in_a()) {
+        VLOOP {
+          c.precondition(V.lambda, c.X(), V.pending_prev ? c.X() : c.Xp(), V.extrapolation, c.Y(), v);
+          c.init(v, true, false);
+        }
       }
       if (V.pending_best) c.copy(B.best, c.X(), d.U);
       if (V.pending_prev) c.copy(c.Xp(), c.X(), n);
+      if (!fresh && c.in_b()) c.wa(c.X(), S.gamma);
       SYNC_OR_EXIT(PC_PRECOND)
-      {
-        const FoldJob jobs[3] = {{mslot(r.p, MS_PMIN), FOLD_DMIN}, {mslot(r.p, MS_PMAX), FOLD_DMAX},
-                                 {islot(r.p, IS_PBAD), FOLD_ISUM}};
-        c.fold(jobs, 3);
-      }
-      const double pmin = c.fv[0].d, pmax = c.fv[1].d;
-      const long long pbad = c.fv[2].l;
-      T0 {
-        V.pmin = pmin;
-        V.pmax = pmax;
+      const Partials q = c.set();
+      c.fold(fresh ? 4 : 5, [&](int j) {
+        return j == 0   ? FoldJob{mslot(r.p, MS_PMIN), FOLD_DMIN}
+               : j == 1 ? FoldJob{mslot(r.p, MS_PMAX), FOLD_DMAX}
+               : j == 2 ? FoldJob{islot(r.p, IS_PBAD), FOLD_ISUM}
+               : j == 3 ? FoldJob{islot(q, IS_DIFF), FOLD_ISUM}
+                        : FoldJob{pslot(r.p, SLOT_WA_VALUE), FOLD_DSUM};
+      });
+      ++c.ws;
+      if (threadIdx.x == 0) {
+        V.pmin = fvals[0].d;
+        V.pmax = fvals[1].d;
+        V.y_is_origin = fvals[3].l == 0;
         V.pending_best = 0;
         V.pending_prev = 0;
-        if (pbad) S.status = TEXO_GP_ERR_INVALID_NORMALIZATION;
+        if (fvals[2].l) S.status = TEXO_GP_ERR_INVALID_NORMALIZATION;
+        else if (!fresh) c.eval_scalars(eo, false, 4);
       }
       __syncthreads();
       if (S.status) FAIL(S.status)
-      if (!c.eval_tail(c.X(), c.gX(), S.gamma, full, c.X(), eo)) {
-        ok = false;
-        goto out;
+      if (fresh) {
+        VLOOP c.scatter(c.X(), v);
+        if (!c.density_and_wa(c.X(), S.gamma, true)) LEAVE
+        if (!c.gradient(c.X(), c.gX(), eo)) LEAVE
+        if (!V.y_is_origin) {
+          if (c.in_a()) VLOOP c.init(v, true, false);
+          SYNC_OR_EXIT(PC_EXTRAP)
+        }
       }
+      // Phase 2: the origin's gradient, beside the scatter of y
+      if (!V.y_is_origin) VLOOP c.scatter(c.Y(), v);
+      if (!fresh) VLOOP c.combine_kept(c.X(), c.gX(), v);
+      if (!fresh || !V.y_is_origin) {
+        SYNC_OR_EXIT(PC_SCATTER_WA)
+      }
+      if (!fresh) c.fold(2, [&](int j) { return c.kkt_job(j); });
       T0 {
+        if (!fresh) {
+          eo.kkt = fvals[0].d;
+          eo.bad = fvals[1].l;
+          S.evaluations++;
+        }
         S.status = checked_dev(eo);
-        if (full) adopt_density(S, eo);
+        if (fresh) adopt_density(S, eo);
         S.density_at_x = 1;
-        V.restart = 0;
-        V.has_wL = S.has_L;
-        V.wL = S.L;
-        V.trials = 0;
       }
       __syncthreads();
       if (S.status) FAIL(S.status)
     }
 
-    // Phase 2: the dynamic Nesterov step (global_placement.rs:152-335)
+    // Phase 3: the dynamic Nesterov step (global_placement.rs:152-335)
     for (;;) {  // 'step
       T0 {
-        const double m = V.restart ? 1.0 : S.a;
-        const double s = sqrt(1.0 + 4.0 * m * m);
-        V.next_m = fabs(s) <= 8.0e307 ? (1.0 + s) / 2.0 : 0.5 + s / 2.0;   // f64::midpoint(1, s)
+        if (V.restart) {
+          V.next_m = next_momentum_dev(1.0);
+          V.y_is_origin = 1;
+        }
         if (!isfinite(V.next_m)) S.status = TEXO_GP_ERR_ITERATION_OVERFLOW;
       }
       __syncthreads();
       if (S.status) FAIL(S.status)
-      if (!V.restart) {
-        const float e = (float)((S.a - 1.0) / V.next_m);
-        VLOOP {
-          stage_extrapolate(d, c.X(), c.Xp(), e, c.Y(), c.wset(), v, c.V, sh);
-          stage_init(d, v, c.V, true, true);
-        }
-        SYNC_OR_EXIT(PC_EXTRAP)
-        const long long diff = c.risum_prev(IS_DIFF);
-        T0 V.y_is_origin = diff == 0;
-        __syncthreads();
-      } else {
-        T0 V.y_is_origin = 1;
-        __syncthreads();
-      }
       if (V.y_is_origin) {
         T0 {
           V.f_y = eo.value;
@@ -705,10 +1165,8 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
         }
         __syncthreads();
       } else {
-        if (!c.eval_tail(c.Y(), c.gY(), S.gamma, true, c.Y(), ey)) {
-          ok = false;
-          goto out;
-        }
+        if (!c.density_and_wa(c.Y(), S.gamma, false)) LEAVE
+        if (!c.gradient(c.Y(), c.gY(), ey)) LEAVE
         T0 {
           S.density_at_x = 0;
           S.status = checked_dev(ey);
@@ -757,16 +1215,17 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
           // 1/L saturates at FLT_MAX: a huge step clamps to the box as it
           // does in FP64, where an infinite one would turn 0 * inf into NaN
           const float invL = (float)fmin(1.0 / V.tL, 3.0e38);
-          VLOOP {
-            stage_candidate(d, ybuf, gy, invL, c.C(), c.wset(), v, c.V, sh, c.X());
-            stage_init(d, v, c.V, true, true);
-          }
+          if (c.in_a()) VLOOP c.candidate(ybuf, gy, invL, c.C(), v);
+          if (SETS == 1 || !c.in_a()) VLOOP c.init(v, true, false);
           SYNC_OR_EXIT(PC_CANDIDATE)
           {
-            const Partials q = c.rset();
-            const FoldJob jobs[3] = {{islot(q, IS_DIFF), FOLD_ISUM}, {pslot(q, SLOT_DOT), FOLD_DSUM},
-                                     {pslot(q, SLOT_MSN), FOLD_DSUM}};
-            c.fold(jobs, 3);
+            const Partials q = c.set();
+            c.fold(3, [&](int j) {
+              return j == 0   ? FoldJob{islot(q, IS_DIFF), FOLD_ISUM}
+                     : j == 1 ? FoldJob{pslot(q, SLOT_DOT), FOLD_DSUM}
+                              : FoldJob{pslot(q, SLOT_MSN), FOLD_DSUM};
+            });
+            ++c.ws;
           }
           const long long changed = c.fv[0].l;
           const double dot = c.fv[1].d, msn = c.fv[2].d;
@@ -792,10 +1251,9 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
           __syncthreads();
           if (V.action == ACT_CONTINUE) continue;
           if (V.action != ACT_NONE) break;
-          if (!c.eval_tail(c.C(), c.gC(), S.gamma, true, c.C(), ec)) {
-            ok = false;
-            goto out;
-          }
+          VLOOP c.scatter(c.C(), v);
+          if (!c.density_and_wa(c.C(), S.gamma, true)) LEAVE
+          if (!c.gradient(c.C(), c.gC(), ec)) LEAVE
           T0 {
             S.density_at_x = 0;
             S.status = checked_dev(ec);
@@ -854,7 +1312,7 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
       break;
     }
 
-    // Phase 3: checkpoint, stop rules, multipliers (eplace.rs:550-573)
+    // Phase 4: checkpoint, stop rules, multipliers (eplace.rs:550-573)
     T0 {
       double mx, tot;
       excess_dev(S, S.cur_overflow, mx, tot);
@@ -875,9 +1333,10 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
     if (V.stationary) {
       // stationary_target_is_fixed (eplace.rs:973-985): compare rounded targets
       const float2* x = c.X();
-      VLOOP {
+      if (c.in_a()) VLOOP {
+        const auto g = c.half_a();
         long long mism = 0;
-        for (int u = v * blockDim.x + threadIdx.x; u < d.U; u += c.V * blockDim.x) {
+        for (int u = v * kThreads + g.tid; u < d.U; u += c.V * kThreads) {
           const float2 a = x[u];
           const uint32_t tx = (uint32_t)fminf(fmaxf(roundf(a.x), 0.f), (float)(S.W - 1));
           const uint32_t ty = (uint32_t)fminf(fmaxf(roundf(a.y), 0.f), (float)(S.H - 1));
@@ -885,10 +1344,13 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
           B.prev_targets[2 * u] = tx;
           B.prev_targets[2 * u + 1] = ty;
         }
-        write_partial(mism, islot(c.wset(), IS_DIFF), v, sh.l);
+        write_partial(g, mism, islot(c.set(), IS_DIFF), v, sh.a.l);
       }
       SYNC_OR_EXIT(PC_OTHER)
-      const long long total = c.risum_prev(IS_DIFF);
+      const Partials q = c.set();
+      c.fold(1, [&](int) { return FoldJob{islot(q, IS_DIFF), FOLD_ISUM}; });
+      ++c.ws;
+      const long long total = fvals[0].l;
       T0 {
         const bool fixed = S.have_prev_stationary && total == 0;
         S.have_prev_stationary = 1;
@@ -933,6 +1395,7 @@ out:
 #undef T0
 #undef VLOOP
 #undef SYNC_OR_EXIT
+#undef LEAVE
 #undef FAIL
 }
 

@@ -4,9 +4,9 @@
 
 namespace tgp {
 
-__global__ void __launch_bounds__(kThreads, kBlocksPerSm)
+__global__ void __launch_bounds__(2 * kThreads, kBlocksPerSm)
     k_persistent_small(Dev d, Reduce r, Buffers B, DevRun* run, GridBarrier* bar, int V) {
-  run_body<false>(d, r, B, run, bar, (int)blockIdx.x, (int)gridDim.x, V);
+  run_body<false, 2>(d, r, B, run, bar, (int)blockIdx.x, (int)gridDim.x, V);
 }
 
 const void* persistent_kernel_small() { return (const void*)k_persistent_small; }

@@ -34,27 +34,31 @@ __device__ __forceinline__ double* pslot(const Partials& p, int s) { return p.su
 __device__ __forceinline__ long long* islot(const Partials& p, int s) { return p.isum + (size_t)s * kMaxPartials; }
 __device__ __forceinline__ double* mslot(const Partials& p, int s) { return p.mx + (size_t)s * kMaxPartials; }
 
-// Fixed-order reduction of n partials by the whole block; every thread gets
+// Fixed-order reduction of n partials by the whole group; every thread gets
 // the result. Identical in every block that calls it. Warps 0-3 (one per SM
 // sub-partition) fold interleaved quarters with an xor tree and thread 0
 // folds the four: FP64 folds then cost a few warp instructions per
 // sub-partition instead of a tree in every warp. `sh` needs 5 slots.
-template <typename T, typename Op>
-__device__ __forceinline__ T block_reduce_array(const T* a, int n, T init, Op op, T* sh) {
-  const int w = threadIdx.x >> 5;
+template <class G, typename T, typename Op>
+__device__ __forceinline__ T block_reduce_array(const G& g, const T* a, int n, T init, Op op, T* sh) {
+  const int w = g.tid >> 5;
   if (w < 4) {
-    T v = (int)threadIdx.x < n ? a[threadIdx.x] : init;
-    for (int i = threadIdx.x + 128; i < n; i += 128) v = op(v, a[i]);
+    T v = g.tid < n ? a[g.tid] : init;
+    for (int i = g.tid + 128; i < n; i += 128) v = op(v, a[i]);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((threadIdx.x & 31) == 0) sh[w] = v;
+    if ((g.tid & 31) == 0) sh[w] = v;
   }
-  __syncthreads();
-  if (threadIdx.x == 0) sh[4] = op(op(op(sh[0], sh[1]), sh[2]), sh[3]);
-  __syncthreads();
+  g.sync();
+  if (g.tid == 0) sh[4] = op(op(op(sh[0], sh[1]), sh[2]), sh[3]);
+  g.sync();
   const T r = sh[4];
-  __syncthreads();
+  g.sync();
   return r;
+}
+template <typename T, typename Op>
+__device__ __forceinline__ T block_reduce_array(const T* a, int n, T init, Op op, T* sh) {
+  return block_reduce_array(whole_block(), a, n, init, op, sh);
 }
 struct OpAdd {
   template <typename T> __device__ T operator()(T a, T b) const { return a + b; }
@@ -77,26 +81,21 @@ template <typename T>
 __device__ __forceinline__ void write_partial(T v, T* slot, int vb, T* sh) {
   write_partial(whole_block(), v, slot, vb, sh);
 }
-struct FoldMax {
-  __device__ double operator()(double a, double b) const { return fmax(a, b); }
-};
-struct FoldMin {
-  __device__ double operator()(double a, double b) const { return fmin(a, b); }
-};
 // Block max (or min) of per-thread FP32 values, written as FP64 partial vb:
 // folding in FP32 and widening once gives the same value as widening first.
-__device__ __forceinline__ void write_partial_max(float v, double* slot, int vb, float* sh, bool is_min) {
+template <class G>
+__device__ __forceinline__ void write_partial_max(const G& g, float v, double* slot, int vb, float* sh, bool is_min) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float w = __shfl_xor_sync(0xffffffffu, v, o);
     v = is_min ? fminf(v, w) : fmaxf(v, w);
   }
-  __syncthreads();   // earlier readers of sh are done
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
+  g.sync();   // earlier readers of sh are done
+  if ((g.tid & 31) == 0) sh[g.tid >> 5] = v;
+  g.sync();
+  if (g.tid == 0) {
     float r = sh[0];
-    for (int i = 1; i < (int)(blockDim.x >> 5); ++i) r = is_min ? fminf(r, sh[i]) : fmaxf(r, sh[i]);
+    for (int i = 1; i < kThreads / 32; ++i) r = is_min ? fminf(r, sh[i]) : fmaxf(r, sh[i]);
     slot[vb] = (double)r;
   }
 }
@@ -117,9 +116,10 @@ __device__ __forceinline__ AxisTaps taps_y(const Dev& d, float s) {
 // ---------------------------------------------------------------------------
 // S1: reset the accumulation grids.
 // ---------------------------------------------------------------------------
-static __device__ void stage_init(const Dev& d, int vb, int nvb, bool grids, bool wa) {
-  const int stride = nvb * blockDim.x;
-  const int t0 = vb * blockDim.x + threadIdx.x;
+template <class G>
+static __device__ void stage_init(const G& g, const Dev& d, int vb, int nvb, bool grids, bool wa) {
+  const int stride = nvb * kThreads;
+  const int t0 = vb * kThreads + g.tid;
   if (grids) {
     const int n = d.K * d.B;
     for (int i = t0; i < n; i += stride) {
@@ -137,51 +137,72 @@ static __device__ void stage_init(const Dev& d, int vb, int nvb, bool grids, boo
 // exact in any order. The per-field tap total is a partial for the mean.
 // (deposit_quadratic_bspline + the field loop, electrostatic_placement.rs:296-332)
 // ---------------------------------------------------------------------------
-static __device__ void stage_scatter(const Dev& d, const float2* pos, Partials p, int vb, int nvb,
-                                     Shared& sh) {
-  long long tot[kMaxFields];
+struct Deposit {
+  float x, y, q;
+  int f;
+  unsigned long long* grid;
+};
+// Member i, or filler i - Mm.
+__device__ __forceinline__ Deposit deposit_of(const Dev& d, const float2* pos, int i) {
+  Deposit t;
+  if (i < d.Mm) {
+    const int u = d.mem_unit[i];
+    const float2 o = d.mem_off[i];
+    t.q = d.mem_q[i];
+    t.f = d.mem_field[i];
+    const float2 pu = pos[u];
+    t.x = __fadd_rn(pu.x, o.x);
+    t.y = __fadd_rn(pu.y, o.y);
+    t.grid = (unsigned long long*)(d.phys + (size_t)t.f * d.B);
+  } else {
+    const int j = i - d.Mm;
+    const float2 pf = pos[d.U + j];
+    t.x = pf.x;
+    t.y = pf.y;
+    t.q = d.fil_q[j];
+    t.f = d.fil_field[j];
+    t.grid = (unsigned long long*)(d.fill + (size_t)t.f * d.B);
+  }
+  return t;
+}
+// Objects first, first + stride, ...: the tap totals per field in tot. Two
+// objects' loads are in flight before either's atomics (which the compiler
+// will not move loads across).
+__device__ __forceinline__ void scatter_items(const Dev& d, const float2* pos, int first, int stride,
+                                              long long (&tot)[kMaxFields]) {
 #pragma unroll
   for (int f = 0; f < kMaxFields; ++f) tot[f] = 0;
-  const int stride = nvb * blockDim.x;
   const int items = d.Mm + d.F;
-  for (int i = vb * blockDim.x + threadIdx.x; i < items; i += stride) {
-    float sxp, syp, q;
-    int f;
-    unsigned long long* grid;
-    if (i < d.Mm) {
-      const int u = d.mem_unit[i];
-      const float2 o = d.mem_off[i];
-      const float2 pu = pos[u];
-      sxp = __fadd_rn(pu.x, o.x);
-      syp = __fadd_rn(pu.y, o.y);
-      q = d.mem_q[i];
-      f = d.mem_field[i];
-      grid = (unsigned long long*)(d.phys + (size_t)f * d.B);
-    } else {
-      const int j = i - d.Mm;
-      const float2 pf = pos[d.U + j];
-      sxp = pf.x;
-      syp = pf.y;
-      q = d.fil_q[j];
-      f = d.fil_field[j];
-      grid = (unsigned long long*)(d.fill + (size_t)f * d.B);
-    }
-    const AxisTaps ax = taps_x(d, sxp);
-    const AxisTaps ay = taps_y(d, syp);
+  auto put = [&](const Deposit& t, const AxisTaps& ax, const AxisTaps& ay) {
     long long s = 0;
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const long long v = tap_fixed(q, ax.w[c], ay.w[r]);
+        const long long v = tap_fixed(t.q, ax.w[c], ay.w[r]);
         s += v;
-        atomicAdd(grid + (size_t)ay.idx[r] * d.g.Wb + ax.idx[c], (unsigned long long)v);
+        atomicAdd(t.grid + (size_t)ay.idx[r] * d.g.Wb + ax.idx[c], (unsigned long long)v);
       }
 #pragma unroll
     for (int ff = 0; ff < kMaxFields; ++ff)
-      if (ff == f) tot[ff] += s;
+      if (ff == t.f) tot[ff] += s;
+  };
+  for (int i = first; i < items; i += 2 * stride) {
+    const bool two = i + stride < items;
+    const Deposit a = deposit_of(d, pos, i), b = two ? deposit_of(d, pos, i + stride) : a;
+    const AxisTaps ax = taps_x(d, a.x), ay = taps_y(d, a.y), bx = taps_x(d, b.x), by = taps_y(d, b.y);
+    put(a, ax, ay);
+    if (two) put(b, bx, by);
   }
-  for (int f = 0; f < d.K; ++f) write_partial(tot[f], islot(p, IS_GRID_SUM + f), vb, sh.l);
+}
+template <class G>
+static __device__ void stage_scatter(const G& g, const Dev& d, const float2* pos, Partials p, int vb, int nvb,
+                                     Shared& sh) {
+  long long tot[kMaxFields];
+  scatter_items(d, pos, vb * kThreads + g.tid, nvb * kThreads, tot);
+#pragma unroll
+  for (int f = 0; f < kMaxFields; ++f)
+    if (f < d.K) write_partial(g, tot[f], islot(p, IS_GRID_SUM + f), vb, sh.l);
 }
 
 // ---------------------------------------------------------------------------
@@ -313,11 +334,12 @@ __device__ __forceinline__ void wa_class(const Dev& d, const float2* pos, float 
   acc += (double)vacc;
 }
 
-static __device__ void stage_wa(const Dev& d, const float2* pos, double gamma, Partials p, int vb,
-                                int nvb, Shared& sh) {
+template <class G>
+static __device__ void stage_wa(const G& g, const Dev& d, const float2* pos, double gamma, Partials p, int vb,
+                                int nvb, double* sh) {
   double acc = 0.0;
   const float ig = (float)(1.0 / gamma);
-  const int gl = vb * blockDim.x + threadIdx.x;
+  const int gl = vb * kThreads + g.tid;
   int c = 0;
   while (c < d.n_classes && gl >= d.class_lane[c + 1]) ++c;
   if (c < d.n_classes) {
@@ -333,31 +355,32 @@ static __device__ void stage_wa(const Dev& d, const float2* pos, double gamma, P
       }
     }
   }
-  write_partial(acc, pslot(p, SLOT_WA_VALUE), vb, sh.d);
+  write_partial(g, acc, pslot(p, SLOT_WA_VALUE), vb, sh);
 }
 
 // ---------------------------------------------------------------------------
 // S4: density grid -> FP32 mean-free charge, physical overflow partials
 // (the pre-filler positive overflow, electrostatic_placement.rs:317-318).
 // ---------------------------------------------------------------------------
-static __device__ void stage_prep(const Dev& d, Partials p, int nvb_scatter, int vb, int nvb, Shared& sh) {
+template <class G>
+static __device__ void stage_prep(const G& g, const Dev& d, Partials p, int nvb_scatter, int vb, int nvb, Shared& sh) {
   __shared__ long long s_mean[kMaxFields];
   __shared__ long long red[kThreads / 32];
   for (int f = 0; f < d.K; ++f) {
-    long long tot = block_reduce_array(islot(p, IS_GRID_SUM + f), nvb_scatter, 0ll, OpAdd(), red);
-    if (threadIdx.x == 0) s_mean[f] = (tot - d.capsum[f]) / d.B;   // fixed-point mean (DC mode only)
+    long long tot = block_reduce_array(g, islot(p, IS_GRID_SUM + f), nvb_scatter, 0ll, OpAdd(), red);
+    if (g.tid == 0) s_mean[f] = (tot - d.capsum[f]) / d.B;   // fixed-point mean (DC mode only)
   }
-  __syncthreads();
+  g.sync();
   long long ov[kMaxFields], cnt[kMaxFields];
 #pragma unroll
   for (int f = 0; f < kMaxFields; ++f) ov[f] = cnt[f] = 0;
-  const int stride = nvb * blockDim.x;
+  const int stride = nvb * kThreads;
   for (int f = 0; f < d.K; ++f) {
     const long long mean = s_mean[f];
     const long long* ph = d.phys + (size_t)f * d.B;
     const long long* fl = d.fill + (size_t)f * d.B;
     float* rho = d.rho + (size_t)f * d.B;
-    for (int i = vb * blockDim.x + threadIdx.x; i < d.B; i += stride) {
+    for (int i = vb * kThreads + g.tid; i < d.B; i += stride) {
       const long long a = ph[i];
       if (a > 0) {
         ov[f] += a;
@@ -367,8 +390,8 @@ static __device__ void stage_prep(const Dev& d, Partials p, int nvb_scatter, int
     }
   }
   for (int f = 0; f < d.K; ++f) {
-    write_partial(ov[f], islot(p, IS_OVERFLOW + f), vb, sh.l);
-    write_partial(cnt[f], islot(p, IS_OVER_BINS + f), vb, sh.l);
+    write_partial(g, ov[f], islot(p, IS_OVERFLOW + f), vb, sh.l);
+    write_partial(g, cnt[f], islot(p, IS_OVER_BINS + f), vb, sh.l);
   }
 }
 
@@ -400,15 +423,15 @@ __device__ __forceinline__ void two_sum_acc(float& s, float& c, float part) {
   c = __fadd_rn(c, e);
 }
 
-template <int TM, int TN, int TK, int RM, int RN>
-__device__ void gemm_tiles(const float* A, long sa, const float* Bm, long sb, float* Cm, long sc, int M, int N,
+template <int TM, int TN, int TK, int RM, int RN, class G>
+__device__ void gemm_tiles(const G& g, const float* A, long sa, const float* Bm, long sb, float* Cm, long sc, int M, int N,
                            int Kd, int nf, int epi, const float* inv_eig, const float* rho, double* energy_acc,
                            int vb, int nvb, GemmSmem<TM, TN, TK, RM, RN>& sm) {
   static_assert((TM / RM) * (TN / RN) == kThreads, "tile / thread mismatch");
   static_assert(TK % kChunk == 0, "k slab must hold whole chunks");
   constexpr int TX = TN / RN;
   constexpr int LA = TM * TK / kThreads, LB = TK * TN / kThreads;  // loads per thread per slab
-  const int tx = threadIdx.x % TX, ty = threadIdx.x / TX;
+  const int tx = g.tid % TX, ty = g.tid / TX;
   const int tiles_m = (M + TM - 1) / TM, tiles_n = (N + TN - 1) / TN;
   const int tiles = tiles_m * tiles_n * nf;
   for (int t = vb; t < tiles; t += nvb) {
@@ -427,14 +450,14 @@ __device__ void gemm_tiles(const float* A, long sa, const float* Bm, long sb, fl
     auto fetch = [&](int k0) {
 #pragma unroll
       for (int q = 0; q < LA; ++q) {
-        const int e = threadIdx.x + q * kThreads;
+        const int e = g.tid + q * kThreads;
         const int mm = e / TK, kk = e % TK;
         const int gm = m0 + mm, gk = k0 + kk;
         ra[q] = (gm < M && gk < Kd) ? Af[(size_t)gm * Kd + gk] : 0.f;
       }
 #pragma unroll
       for (int q = 0; q < LB; ++q) {
-        const int e = threadIdx.x + q * kThreads;
+        const int e = g.tid + q * kThreads;
         const int kk = e / TN, nn = e % TN;
         const int gk = k0 + kk, gn = n0 + nn;
         rb[q] = (gk < Kd && gn < N) ? Bf[(size_t)gk * N + gn] : 0.f;
@@ -442,18 +465,18 @@ __device__ void gemm_tiles(const float* A, long sa, const float* Bm, long sb, fl
     };
     fetch(0);
     for (int k0 = 0; k0 < Kd; k0 += TK) {
-      __syncthreads();
+      g.sync();
 #pragma unroll
       for (int q = 0; q < LA; ++q) {
-        const int e = threadIdx.x + q * kThreads;
+        const int e = g.tid + q * kThreads;
         sm.a[e % TK][e / TK] = ra[q];
       }
 #pragma unroll
       for (int q = 0; q < LB; ++q) {
-        const int e = threadIdx.x + q * kThreads;
+        const int e = g.tid + q * kThreads;
         sm.b[e / TN][e % TN] = rb[q];
       }
-      __syncthreads();
+      g.sync();
       if (k0 + TK < Kd) fetch(k0 + TK);
 #pragma unroll
       for (int kc = 0; kc < TK; kc += kChunk) {
@@ -497,7 +520,7 @@ __device__ void gemm_tiles(const float* A, long sa, const float* Bm, long sb, fl
       }
     if (epi == 2) energy_acc[f] += (double)eacc;
   }
-  __syncthreads();
+  g.sync();
 }
 
 // Small grids: 16x16 output tiles, one output per thread, K in slabs of
@@ -520,16 +543,16 @@ struct PrepFold {
   long long ov[kMaxFields], cnt[kMaxFields];
 };
 
-template <bool FOLD = false>
-static __device__ void gemm16(const float* A, long sa, const float* Bm, long sb, float* Cm, long sc, int M, int N,
+template <bool FOLD = false, class G>
+static __device__ void gemm16(const G& g, const float* A, long sa, const float* Bm, long sb, float* Cm, long sc, int M, int N,
                               int Kd, int nf, int epi, const float* inv_eig, const float* rho, double* energy_acc,
                               int vb, int nvb, Smem16& sm, const Dev* dp = nullptr, PrepFold* pf = nullptr) {
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int tx = g.tid & 15, ty = g.tid >> 4;
   const int tiles_m = (M + 15) / 16, tiles_n = (N + 15) / 16;
   const int tiles = tiles_m * tiles_n * nf;
   // slab-load roles: A element (row ra + 2j, column ca), B element (row rb + 16j, column cb)
-  const int ca = threadIdx.x & (kT16Slab - 1), ra = threadIdx.x / kT16Slab;
-  const int cb = threadIdx.x & 15, rb = threadIdx.x >> 4;
+  const int ca = g.tid & (kT16Slab - 1), ra = g.tid / kT16Slab;
+  const int cb = g.tid & 15, rb = g.tid >> 4;
   for (int t = vb; t < tiles; t += nvb) {
     const int f = t / (tiles_m * tiles_n);
     const int r = t % (tiles_m * tiles_n);
@@ -572,13 +595,13 @@ static __device__ void gemm16(const float* A, long sa, const float* Bm, long sb,
     };
     fetch(0);
     for (int k0 = 0; k0 < Kd; k0 += kT16Slab) {
-      __syncthreads();
+      g.sync();
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         sm.a[ra + 2 * j][ca] = va[j];
         sm.bt[cb][rb + 16 * j] = vbv[j];
       }
-      __syncthreads();
+      g.sync();
       if (k0 + kT16Slab < Kd) fetch(k0 + kT16Slab);
       const float4* a4 = reinterpret_cast<const float4*>(sm.a[ty]);
       const float4* b4 = reinterpret_cast<const float4*>(sm.bt[tx]);
@@ -605,7 +628,7 @@ static __device__ void gemm16(const float* A, long sa, const float* Bm, long sb,
       if (epi == 2) energy_acc[f] += (double)(rho[(size_t)f * M * N + idx] * v);
     }
   }
-  __syncthreads();
+  g.sync();
 }
 
 // Large-grid tile shape (register-blocked) and the small-grid one.
@@ -616,38 +639,39 @@ union alignas(16) GemmShared {
   float4 fft[2048];   // work buffer of the FFT form (fft::Smem: double-float complex)
 };
 
-template <bool LARGE>
-__device__ __forceinline__ void gemm_any(const float* A, long sa, const float* Bm, long sb, float* Cm, long sc, int M,
+template <bool LARGE, class G>
+__device__ __forceinline__ void gemm_any(const G& g, const float* A, long sa, const float* Bm, long sb, float* Cm, long sc, int M,
                                          int N, int Kd, int nf, int epi, const float* inv_eig, const float* rho,
                                          double* eacc, int vb, int nvb, GemmShared& sm) {
   if (LARGE)
-    gemm_tiles<64, 64, 16, 4, 4>(A, sa, Bm, sb, Cm, sc, M, N, Kd, nf, epi, inv_eig, rho, eacc, vb, nvb, sm.l);
+    gemm_tiles<64, 64, 16, 4, 4>(g, A, sa, Bm, sb, Cm, sc, M, N, Kd, nf, epi, inv_eig, rho, eacc, vb, nvb, sm.l);
   else
-    gemm16(A, sa, Bm, sb, Cm, sc, M, N, Kd, nf, epi, inv_eig, rho, eacc, vb, nvb, sm.s);
+    gemm16(g, A, sa, Bm, sb, Cm, sc, M, N, Kd, nf, epi, inv_eig, rho, eacc, vb, nvb, sm.s);
 }
 
 // The four transforms of the spectral solve (Poisson2d::solve,
 // electrostatic_placement.rs:725-776) as dense GEMMs:
 //   t1 = rho Cx^T ; t2 = (Cy t1) o inv_eig ; t1 = Cy^T t2 ; phi = t1 Cx.
 // `step` selects one of the four (a grid barrier separates them).
-template <bool LARGE>
-static __device__ void stage_dct_t(const Dev& d, int step, Partials p, int vb, int nvb, GemmShared& sm, Shared& sh) {
+template <bool LARGE, class G>
+static __device__ void stage_dct_t(const G& g, const Dev& d, int step, Partials p, int vb, int nvb, GemmShared& sm, Shared& sh) {
   const int W = d.g.Wb, H = d.g.Hb;
   const long sg = d.B;
   double eacc[kMaxFields] = {0.0, 0.0, 0.0, 0.0};
   switch (step) {
-    case 0: gemm_any<LARGE>(d.rho, sg, d.CxT, 0, d.t1, sg, H, W, W, d.K, 0, nullptr, nullptr, eacc, vb, nvb, sm); break;
-    case 1: gemm_any<LARGE>(d.Cy, 0, d.t1, sg, d.t2, sg, H, W, H, d.K, 1, d.inv_eig, nullptr, eacc, vb, nvb, sm); break;
-    case 2: gemm_any<LARGE>(d.CyT, 0, d.t2, sg, d.t1, sg, H, W, H, d.K, 0, nullptr, nullptr, eacc, vb, nvb, sm); break;
-    default: gemm_any<LARGE>(d.t1, sg, d.Cx, 0, d.phi, sg, H, W, W, d.K, 2, nullptr, d.rho, eacc, vb, nvb, sm); break;
+    case 0: gemm_any<LARGE>(g, d.rho, sg, d.CxT, 0, d.t1, sg, H, W, W, d.K, 0, nullptr, nullptr, eacc, vb, nvb, sm); break;
+    case 1: gemm_any<LARGE>(g, d.Cy, 0, d.t1, sg, d.t2, sg, H, W, H, d.K, 1, d.inv_eig, nullptr, eacc, vb, nvb, sm); break;
+    case 2: gemm_any<LARGE>(g, d.CyT, 0, d.t2, sg, d.t1, sg, H, W, H, d.K, 0, nullptr, nullptr, eacc, vb, nvb, sm); break;
+    default: gemm_any<LARGE>(g, d.t1, sg, d.Cx, 0, d.phi, sg, H, W, W, d.K, 2, nullptr, d.rho, eacc, vb, nvb, sm); break;
   }
   if (step == 3)
-    for (int f = 0; f < d.K; ++f) write_partial(eacc[f], pslot(p, SLOT_ENERGY + f), vb, sh.d);
+    for (int f = 0; f < d.K; ++f) write_partial(g, eacc[f], pslot(p, SLOT_ENERGY + f), vb, sh.d);
 }
 // stage_prep + pass 0 of stage_dct_t<false> in one phase (small tiles only):
 // the same rho, overflow sums and t1 as the two phases, bit for bit.
 // `mean` holds the fixed-point mean of each field (from the scatter totals).
-static __device__ void stage_prep_dct0(const Dev& d, const long long* mean, Partials p, int vb, int nvb,
+template <class G>
+static __device__ void stage_prep_dct0(const G& g, const Dev& d, const long long* mean, Partials p, int vb, int nvb,
                                        GemmShared& sm, Shared& sh) {
   const int W = d.g.Wb, H = d.g.Hb;
   const long sg = d.B;
@@ -656,18 +680,11 @@ static __device__ void stage_prep_dct0(const Dev& d, const long long* mean, Part
 #pragma unroll
   for (int f = 0; f < kMaxFields; ++f) pf.ov[f] = pf.cnt[f] = 0;
   double eacc[kMaxFields] = {0.0, 0.0, 0.0, 0.0};
-  gemm16<true>(nullptr, sg, d.CxT, 0, d.t1, sg, H, W, W, d.K, 0, nullptr, nullptr, eacc, vb, nvb, sm.s, &d, &pf);
+  gemm16<true>(g, nullptr, sg, d.CxT, 0, d.t1, sg, H, W, W, d.K, 0, nullptr, nullptr, eacc, vb, nvb, sm.s, &d, &pf);
   for (int f = 0; f < d.K; ++f) {
-    write_partial(pf.ov[f], islot(p, IS_OVERFLOW + f), vb, sh.l);
-    write_partial(pf.cnt[f], islot(p, IS_OVER_BINS + f), vb, sh.l);
+    write_partial(g, pf.ov[f], islot(p, IS_OVERFLOW + f), vb, sh.l);
+    write_partial(g, pf.cnt[f], islot(p, IS_OVER_BINS + f), vb, sh.l);
   }
-}
-__device__ __forceinline__ void stage_dct(const Dev& d, int step, bool large, Partials p, int vb, int nvb,
-                                          GemmShared& sm, Shared& sh) {
-  if (large)
-    stage_dct_t<true>(d, step, p, vb, nvb, sm, sh);
-  else
-    stage_dct_t<false>(d, step, p, vb, nvb, sm, sh);
 }
 
 // ---------------------------------------------------------------------------
@@ -702,11 +719,12 @@ __device__ __forceinline__ float2 sample_grad(const Dev& d, const float* phi, fl
   return make_float2(gx, gy);
 }
 
-static __device__ void stage_gather(const Dev& d, const float2* pos, Partials p, int vb, int nvb,
+template <class G>
+static __device__ void stage_gather(const G& g, const Dev& d, const float2* pos, Partials p, int vb, int nvb,
                                     Shared& sh) {
   float force[kMaxFields] = {0.f, 0.f, 0.f, 0.f};
-  const int stride = nvb * blockDim.x;
-  for (int o = vb * blockDim.x + threadIdx.x; o < d.nobj; o += stride) {
+  const int stride = nvb * kThreads;
+  for (int o = vb * kThreads + g.tid; o < d.nobj; o += stride) {
     if (o < d.U) {
       float2 acc[kMaxFields];
 #pragma unroll
@@ -717,13 +735,13 @@ static __device__ void stage_gather(const Dev& d, const float2* pos, Partials p,
         const int f = d.mem_field[m];
         const float2 off = d.mem_off[m];
         const float q = d.mem_q[m];
-        const float2 g = sample_grad(d, d.phi + (size_t)f * d.B, __fadd_rn(pu.x, off.x), __fadd_rn(pu.y, off.y));
+        const float2 gr = sample_grad(d, d.phi + (size_t)f * d.B, __fadd_rn(pu.x, off.x), __fadd_rn(pu.y, off.y));
 #pragma unroll
         for (int ff = 0; ff < kMaxFields; ++ff)
           if (ff == f) {
-            acc[ff].x += q * g.x;
-            acc[ff].y += q * g.y;
-            force[ff] += q * (fabsf(g.x) + fabsf(g.y));
+            acc[ff].x += q * gr.x;
+            acc[ff].y += q * gr.y;
+            force[ff] += q * (fabsf(gr.x) + fabsf(gr.y));
           }
       }
       for (int f = 0; f < d.K; ++f) d.graw[(size_t)f * d.nobj + o] = acc[f];
@@ -732,14 +750,14 @@ static __device__ void stage_gather(const Dev& d, const float2* pos, Partials p,
       const int f = d.fil_field[j];
       const float q = d.fil_q[j];
       const float2 pf = pos[o];
-      const float2 g = sample_grad(d, d.phi + (size_t)f * d.B, pf.x, pf.y);
-      d.graw[(size_t)f * d.nobj + o] = make_float2(q * g.x, q * g.y);
+      const float2 gr = sample_grad(d, d.phi + (size_t)f * d.B, pf.x, pf.y);
+      d.graw[(size_t)f * d.nobj + o] = make_float2(q * gr.x, q * gr.y);
 #pragma unroll
       for (int ff = 0; ff < kMaxFields; ++ff)
-        if (ff == f) force[ff] += q * (fabsf(g.x) + fabsf(g.y));
+        if (ff == f) force[ff] += q * (fabsf(gr.x) + fabsf(gr.y));
     }
   }
-  for (int f = 0; f < d.K; ++f) write_partial((double)force[f], pslot(p, SLOT_FORCE + f), vb, sh.d);
+  for (int f = 0; f < d.K; ++f) write_partial(g, (double)force[f], pslot(p, SLOT_FORCE + f), vb, sh.d);
 }
 
 // ---------------------------------------------------------------------------
@@ -754,7 +772,8 @@ __device__ __forceinline__ float kkt_comp(float g, float x, float lo, float hi) 
 
 // With kkt_pos, the box-metric KKT residual of the new gradient at kkt_pos is
 // reduced in the same pass (box_metric_kkt_residual, global_placement.rs:648-663).
-static __device__ void stage_combine(const Dev& d, const double* coef_d, float2* gout, Partials p,
+template <class G>
+static __device__ void stage_combine(const G& g, const Dev& d, const double* coef_d, float2* gout, Partials p,
                                      int vb, int nvb, Shared& sh, const float2* kkt_pos = nullptr) {
   float coef[kMaxFields];
 #pragma unroll
@@ -762,8 +781,8 @@ static __device__ void stage_combine(const Dev& d, const double* coef_d, float2*
   float rawl1[kMaxFields] = {0.f, 0.f, 0.f, 0.f};
   float wal1 = 0.f, kkt = 0.f;
   long long bad = 0x7fffffffffffffffll;
-  const int stride = nvb * blockDim.x;
-  for (int o = vb * blockDim.x + threadIdx.x; o < d.nobj; o += stride) {
+  const int stride = nvb * kThreads;
+  for (int o = vb * kThreads + g.tid; o < d.nobj; o += stride) {
     float gx = 0.f, gy = 0.f;
     if (o < d.U) {
       gx = __ll2float_rn((long long)d.wa_fix[2 * o]) * kInvFixF;
@@ -796,9 +815,9 @@ static __device__ void stage_combine(const Dev& d, const double* coef_d, float2*
       kkt = fmaxf(kkt, kkt_comp(gy, a.y, lo.y, hi.y) * s);
     }
   }
-  for (int f = 0; f < d.K; ++f) write_partial((double)rawl1[f], pslot(p, SLOT_RAWL1 + f), vb, sh.d);
-  write_partial((double)wal1, pslot(p, SLOT_WAL1), vb, sh.d);
-  if (kkt_pos) write_partial_max(kkt, mslot(p, MS_KKT), vb, sh.f, false);
+  for (int f = 0; f < d.K; ++f) write_partial(g, (double)rawl1[f], pslot(p, SLOT_RAWL1 + f), vb, sh.d);
+  write_partial(g, (double)wal1, pslot(p, SLOT_WAL1), vb, sh.d);
+  if (kkt_pos) write_partial_max(g, kkt, mslot(p, MS_KKT), vb, sh.f, false);
   {
     long long v = bad;
 #pragma unroll
@@ -806,12 +825,12 @@ static __device__ void stage_combine(const Dev& d, const double* coef_d, float2*
       long long w = __shfl_xor_sync(0xffffffffu, v, o);
       v = w < v ? w : v;
     }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) sh.l[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    g.sync();
+    if ((g.tid & 31) == 0) sh.l[g.tid >> 5] = v;
+    g.sync();
+    if (g.tid == 0) {
       long long r = sh.l[0];
-      for (int i = 1; i < (int)(blockDim.x >> 5); ++i) r = sh.l[i] < r ? sh.l[i] : r;
+      for (int i = 1; i < kThreads / 32; ++i) r = sh.l[i] < r ? sh.l[i] : r;
       islot(p, IS_BAD)[vb] = r;
     }
   }
@@ -823,11 +842,12 @@ static __device__ void stage_combine(const Dev& d, const double* coef_d, float2*
 __device__ __forceinline__ float fclamp(float v, float lo, float hi) { return v < lo ? lo : (v > hi ? hi : v); }
 
 // y = clamp(x + e (x - prev)); counts coordinates where y != x.
-static __device__ void stage_extrapolate(const Dev& d, const float2* x, const float2* xp,
+template <class G>
+static __device__ void stage_extrapolate(const G& g, const Dev& d, const float2* x, const float2* xp,
                                          float e, float2* y, Partials p, int vb, int nvb, Shared& sh) {
   long long diff = 0;
-  const int stride = nvb * blockDim.x;
-  for (int o = vb * blockDim.x + threadIdx.x; o < d.nobj; o += stride) {
+  const int stride = nvb * kThreads;
+  for (int o = vb * kThreads + g.tid; o < d.nobj; o += stride) {
     const float2 a = x[o], b = xp[o], lo = d.lo[o], hi = d.hi[o];
     float2 r;
     r.x = fclamp(a.x + e * (a.x - b.x), lo.x, hi.x);
@@ -835,27 +855,28 @@ static __device__ void stage_extrapolate(const Dev& d, const float2* x, const fl
     diff += (r.x != a.x) + (r.y != a.y);
     y[o] = r;
   }
-  write_partial(diff, islot(p, IS_DIFF), vb, sh.l);
+  write_partial(g, diff, islot(p, IS_DIFF), vb, sh.l);
 }
 
 // c = clamp(y - g / (L P)); changed count, <g, c - y>, sum P (c - y)^2.
 // With origin, also the max coordinate change |c - origin|.
-static __device__ void stage_candidate(const Dev& d, const float2* y, const float2* gy,
+template <class G>
+static __device__ void stage_candidate(const G& g, const Dev& d, const float2* y, const float2* gy,
                                        float invL, float2* c, Partials p, int vb, int nvb, Shared& sh,
                                        const float2* origin = nullptr) {
   long long diff = 0;
   float dot = 0.f, msn = 0.f, ch = 0.f;
-  const int stride = nvb * blockDim.x;
-  for (int o = vb * blockDim.x + threadIdx.x; o < d.nobj; o += stride) {
-    const float2 a = y[o], g = gy[o], lo = d.lo[o], hi = d.hi[o];
+  const int stride = nvb * kThreads;
+  for (int o = vb * kThreads + g.tid; o < d.nobj; o += stride) {
+    const float2 a = y[o], gr = gy[o], lo = d.lo[o], hi = d.hi[o];
     const float m = d.P[o];
     const float s = invL / m;
     float2 r;
-    r.x = fclamp(a.x - g.x * s, lo.x, hi.x);
-    r.y = fclamp(a.y - g.y * s, lo.y, hi.y);
+    r.x = fclamp(a.x - gr.x * s, lo.x, hi.x);
+    r.y = fclamp(a.y - gr.y * s, lo.y, hi.y);
     diff += (r.x != a.x) + (r.y != a.y);
     const float dx = r.x - a.x, dy = r.y - a.y;
-    dot = fmaf(g.x, dx, fmaf(g.y, dy, dot));
+    dot = fmaf(gr.x, dx, fmaf(gr.y, dy, dot));
     msn = fmaf(m * dx, dx, fmaf(m * dy, dy, msn));
     c[o] = r;
     if (origin) {
@@ -863,20 +884,21 @@ static __device__ void stage_candidate(const Dev& d, const float2* y, const floa
       ch = fmaxf(ch, fmaxf(fabsf(r.x - b.x), fabsf(r.y - b.y)));
     }
   }
-  write_partial(diff, islot(p, IS_DIFF), vb, sh.l);
-  write_partial((double)dot, pslot(p, SLOT_DOT), vb, sh.d);
-  write_partial((double)msn, pslot(p, SLOT_MSN), vb, sh.d);
-  if (origin) write_partial_max(ch, mslot(p, MS_CHANGE), vb, sh.f, false);
+  write_partial(g, diff, islot(p, IS_DIFF), vb, sh.l);
+  write_partial(g, (double)dot, pslot(p, SLOT_DOT), vb, sh.d);
+  write_partial(g, (double)msn, pslot(p, SLOT_MSN), vb, sh.d);
+  if (origin) write_partial_max(g, ch, mslot(p, MS_CHANGE), vb, sh.f, false);
 }
 
 // box_metric_kkt_residual (global_placement.rs:648-663) and, optionally, the
 // max coordinate change against `ref`.
-static __device__ void stage_kkt(const Dev& d, const float2* x, const float2* g,
+template <class G>
+static __device__ void stage_kkt(const G& g, const Dev& d, const float2* x, const float2* grad,
                                  const float2* ref, Partials p, int vb, int nvb, Shared& sh) {
   float r = 0.f, ch = 0.f;
-  const int stride = nvb * blockDim.x;
-  for (int o = vb * blockDim.x + threadIdx.x; o < d.nobj; o += stride) {
-    const float2 a = x[o], gg = g[o], lo = d.lo[o], hi = d.hi[o];
+  const int stride = nvb * kThreads;
+  for (int o = vb * kThreads + g.tid; o < d.nobj; o += stride) {
+    const float2 a = x[o], gg = grad[o], lo = d.lo[o], hi = d.hi[o];
     const float s = rsqrtf(d.P[o]);
     r = fmaxf(r, kkt_comp(gg.x, a.x, lo.x, hi.x) * s);
     r = fmaxf(r, kkt_comp(gg.y, a.y, lo.y, hi.y) * s);
@@ -886,19 +908,20 @@ static __device__ void stage_kkt(const Dev& d, const float2* x, const float2* g,
       ch = fmaxf(ch, fabsf(a.y - b.y));
     }
   }
-  write_partial_max(r, mslot(p, MS_KKT), vb, sh.f, false);
-  if (ref) write_partial_max(ch, mslot(p, MS_CHANGE), vb, sh.f, false);
+  write_partial_max(g, r, mslot(p, MS_KKT), vb, sh.f, false);
+  if (ref) write_partial_max(g, ch, mslot(p, MS_CHANGE), vb, sh.f, false);
 }
 
 // diagonal_preconditioner (eplace.rs:1046-1100).
-static __device__ void stage_precond(const Dev& d, const double* lambda_d, Partials p, int vb, int nvb, Shared& sh) {
+template <class G>
+static __device__ void stage_precond(const G& g, const Dev& d, const double* lambda_d, Partials p, int vb, int nvb, Shared& sh) {
   float lambda[kMaxFields];
 #pragma unroll
   for (int f = 0; f < kMaxFields; ++f) lambda[f] = f < d.K ? (float)lambda_d[f] : 0.f;
   float pmin = INFINITY, pmax = 0.f;
   long long badp = 0;
-  const int stride = nvb * blockDim.x;
-  for (int o = vb * blockDim.x + threadIdx.x; o < d.nobj; o += stride) {
+  const int stride = nvb * kThreads;
+  for (int o = vb * kThreads + g.tid; o < d.nobj; o += stride) {
     float v = d.pre_static[o];
     for (int f = 0; f < d.K; ++f) {
       const float q = d.pre_q[(size_t)f * d.nobj + o];
@@ -911,9 +934,9 @@ static __device__ void stage_precond(const Dev& d, const double* lambda_d, Parti
     pmin = fminf(pmin, v);
     pmax = fmaxf(pmax, v);
   }
-  write_partial_max(pmin, mslot(p, MS_PMIN), vb, sh.f, true);
-  write_partial_max(pmax, mslot(p, MS_PMAX), vb, sh.f, false);
-  write_partial(badp, islot(p, IS_PBAD), vb, sh.l);
+  write_partial_max(g, pmin, mslot(p, MS_PMIN), vb, sh.f, true);
+  write_partial_max(g, pmax, mslot(p, MS_PMAX), vb, sh.f, false);
+  write_partial(g, badp, islot(p, IS_PBAD), vb, sh.l);
 }
 
 // HPWL over the baseline hypernets at `pos` (per-net FP32 spans, FP64 sum).
