@@ -2,20 +2,38 @@
 // (defined in persistent_{solo,batch}_{small,large}.cu over run_body).
 #include "persistent.cuh"
 
+#include <atomic>
 #include <cstring>
 
 namespace tgp {
 
+size_t persistent_shared();   // dynamic shared memory of the persistent kernels
 const void* persistent_kernel_small();
 const void* persistent_kernel_large();
 const void* batch_kernel_small();
 const void* batch_kernel_large();
 
+// The persistent kernels' shared-memory limit, raised once on each device.
+static bool raise_shared_limit() {
+  static std::atomic<unsigned long long> raised{0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (raised.load(std::memory_order_acquire) & bit) return true;
+  for (const void* k : {persistent_kernel_small(), persistent_kernel_large()})
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)persistent_shared()) != cudaSuccess)
+      return false;
+  raised.fetch_or(bit, std::memory_order_release);
+  return true;
+}
+
 int persistent_blocks_per_sm() {
   int a = 0, b = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, persistent_kernel_small(), 2 * kThreads, 0) != cudaSuccess)
+  const int bytes = (int)persistent_shared();
+  if (!raise_shared_limit()) return 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, persistent_kernel_small(), 2 * kThreads, bytes) != cudaSuccess)
     return 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, persistent_kernel_large(), 2 * kThreads, 0) != cudaSuccess)
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, persistent_kernel_large(), 2 * kThreads, bytes) != cudaSuccess)
     return 0;
   return a < b ? a : b;
 }
@@ -38,7 +56,8 @@ int32_t enqueue_persistent(const Dev& d, const Reduce& r, const Buffers& b, RunB
   GridBarrier* bar = &dev->bar;
   void* args[] = {&dd, &rr, &bb, &run, &bar, &V};
   const void* fn = large_tiles(d) ? persistent_kernel_large() : persistent_kernel_small();
-  if (cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(2 * kThreads), args, 0, s) != cudaSuccess) return TEXO_GP_ERR_CUDA;
+  if (!raise_shared_limit()) return TEXO_GP_ERR_CUDA;
+  if (cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(2 * kThreads), args, persistent_shared(), s) != cudaSuccess) return TEXO_GP_ERR_CUDA;
   if (cudaMemcpyAsync(host, dev, sizeof(RunBlock), cudaMemcpyDeviceToHost, s) != cudaSuccess) return TEXO_GP_ERR_CUDA;
   return TEXO_GP_OK;
 }

@@ -9,7 +9,7 @@ __global__ void __launch_bounds__(kThreads, kBatchBlocksPerSm) k_batch_small(con
   const int4 m = map[blockIdx.x];
   copy_words(&sd, descs + m.x);
   __syncthreads();
-  run_body<false, 1>(sd.d, sd.r, sd.B, sd.run, sd.bar, m.y, m.z, sd.V);
+  run_body<false, 1>(sd.d, sd.r, sd.B, sd.run, sd.bar, m.y, m.z, sd.V, nullptr);
 }
 
 const void* batch_kernel_small() { return (const void*)k_batch_small; }

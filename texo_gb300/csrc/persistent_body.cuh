@@ -14,20 +14,27 @@
 // on every SM or shares one launch with other instances (batched serving).
 //
 // One iteration, with the usual origin whose density is known (X the origin,
-// Y the extrapolated point, C a candidate; "|" a grid barrier):
-//   preconditioner, Y, reset of the grids; WA(X) | scatter(Y), combine(X) |
-//   transforms(Y) | | ; WA(Y) | gather + combine(Y) |
-//   candidate C, reset of the grids | scatter(C) | transforms(C) | | ; WA(C) |
-//   gather + combine(C) |
-// The origin's gradient costs no phase of its own (its WA runs beside the
-// preconditioner, its combination beside Y's scatter), and a point's WA runs
-// beside its transforms: they only meet in the gradient's combination.
+// Y the extrapolated point, C a candidate; "|" a grid barrier; A and B run
+// side by side):
+//   A: preconditioner, Y, scatter(Y)            B: WA(X) |
+//   A: rows(Y)                                  B: combine(X) |
+//   A: columns(Y) |a rows inverse(Y)            B: WA(Y) |
+//   gather(Y), combine(Y), reset of the grids |
+//   A: candidate C, scatter(C) |
+//   A: rows(C) |a columns(C) |a rows inverse(C) B: WA(C) |
+//   gather(C), combine(C), reset of the grids |
+// A point is scattered by the thread that formed it, so it needs no barrier
+// of its own; a point's WA runs beside its transforms, and they only meet in
+// the gradient's combination.
 //
-// A launch for one placement alone runs double blocks (SETS = 2): the first
-// half A runs the phases' main line, the second half B the WA work, so that
-// the WA's latency hides behind the transforms'; phases whose items need no
-// order are split over both. Batched launches run single blocks (SETS = 1)
-// that do the same work one after the other: there other instances' blocks
+// A launch for one placement alone runs double blocks (SETS = 2): A is the
+// first half of the block, B the second (|a is a barrier of the halves A
+// alone). What an object's owner reads in every phase and never changes (its
+// density member, its box, the tile-to-bin map) and the point being evaluated
+// stay in the block's shared memory: behind each grid barrier L1 is cold, and
+// a phase's time was the length of its chain of dependent L2 trips. Batched
+// launches run single blocks (SETS = 1) that do A's and B's work one after
+// the other and read everything from memory: there other instances' blocks
 // hide the latency.
 //
 // Every wait is bounded: a barrier that does not complete within its spin
@@ -127,7 +134,7 @@ union FoldValue {
   double d;
   long long l;
 };
-constexpr int kMaxFoldJobs = 3 * kMaxFields + 3;
+constexpr int kMaxFoldJobs = 3 * kMaxFields + 3;   // the largest fold (energies, overflows, WA, the origin's KKT)
 // The partials a warp folds, loaded ahead of the fold itself (five a lane:
 // an instance has at most one virtual block a multiprocessor; more are read
 // when they are folded).
@@ -184,9 +191,22 @@ struct LoopShared {
   Shared a;                                   // half A's (the block's) folds
   double pair[2 * (kThreads + 4)];            // two FP64 sums at once (half A)
   double wa[SETS == 2 ? kThreads + 4 : 1];    // half B's WA value
-  long long tot[kMaxFields][SETS * kThreads / 32];
+  long long tot[kMaxFields][kThreads / 32];
   unsigned u[3][SETS * kThreads / 32];
+  unsigned x[2][kThreads / 32];               // half B's combination
 };
+
+// What stays in a double block's shared memory (dynamic): the first kResident
+// objects of the block, in the order (k, thread) of its threads' objects.
+constexpr int kResident = 1536;     // 6 a thread: 233 k objects on 152 SMs; further ones are read from memory
+constexpr int kResidentMap = 512;   // tiles a side the resident map covers
+struct Resident {
+  float2 pos[kResident];     // the point being evaluated
+  float4 mem[kResident];     // (offset x, offset y, charge, field bits): kNoMember, kManyMembers or a field
+  float4 box[kResident];     // (lo.x, lo.y, hi.x, hi.y)
+  float2 mapx[kResidentMap], mapy[kResidentMap];
+};
+constexpr int kNoMember = -1, kManyMembers = -2;
 
 template <bool LARGE, int SETS>
 struct Ctx {
@@ -203,10 +223,13 @@ struct Ctx {
   int* gen_failed;     // shared: the barrier's error word as thread 0 last read it
   GemmShared& gsm;
   LoopShared<SETS>& sh;
+  Resident* res;      // null: nothing is resident
+  const float2 *mapx, *mapy;   // tile-to-bin maps (resident, or d's)
   double* coef;       // shared [kMaxFields]
   float* coef32;      // shared [kMaxFields]
   FoldValue* fv;      // shared [kMaxFoldJobs] results of fold()
   long long* fmean;   // shared [kMaxFields] fixed-point density means
+  const long long* capsum;     // shared [kMaxFields] copy of d.capsum
   int pb, np;         // physical block of the instance, physical block count
   int V;              // virtual blocks of the instance
   unsigned long long nbar;
@@ -286,38 +309,118 @@ struct Ctx {
     for (int i = pb * kBlock + threadIdx.x; i < n; i += np * kBlock) dst[i] = src[i];
   }
 
-  // ---- the phases' work on one virtual block ------------------------------
-
-  // Resets of the accumulators by the calling threads (all or one half).
-  __device__ void init(int v, bool grids, bool wa) {
-    if (grids) {
-      const int n = d.K * d.B, stride = V * kThreads;
-      for (int i = v * kThreads + (threadIdx.x & (kThreads - 1)); i < n; i += stride) {
-        d.phys[i] = -d.capfix[i];
-        d.fill[i] = 0;
+  // ---- objects ----------------------------------------------------------------
+  // Virtual block v owns the objects v * kThreads + t + k * V * kThreads of its
+  // threads t; `j` = k * kThreads + t numbers them inside the block.
+  __device__ __forceinline__ int object(int v, int j) const {
+    return v * kThreads + (j & (kThreads - 1)) + (j / kThreads) * V * kThreads;
+  }
+  __device__ __forceinline__ bool resident(int j) const { return SETS == 2 && res && j < kResident; }
+  // an object's one density member, or kNoMember / kManyMembers
+  __device__ __forceinline__ float4 member(int j, int o) const {
+    return resident(j) ? res->mem[j] : member_from_memory(o);
+  }
+  __device__ __forceinline__ float4 member_from_memory(int o) const {
+    if (o >= d.U) return make_float4(0.f, 0.f, d.fil_q[o - d.U], __int_as_float(d.fil_field[o - d.U]));
+    const int m = d.unit_mem_ptr[o], n = d.unit_mem_ptr[o + 1] - m;
+    if (n != 1) return make_float4(0.f, 0.f, 0.f, __int_as_float(n == 0 ? kNoMember : kManyMembers));
+    const float2 off = d.mem_off[m];
+    return make_float4(off.x, off.y, d.mem_q[m], __int_as_float(d.mem_field[m]));
+  }
+  __device__ __forceinline__ float4 box(int j, int o) const {
+    if (resident(j)) return res->box[j];
+    const float2 lo = d.lo[o], hi = d.hi[o];
+    return make_float4(lo.x, lo.y, hi.x, hi.y);
+  }
+  __device__ void make_resident() {
+    if constexpr (SETS == 2) {
+      if (!res) return;
+      for (int j = threadIdx.x; j < kResident; j += kBlock) {
+        const int o = object(pb, j);
+        if (o >= d.nobj) break;
+        const float2 lo = d.lo[o], hi = d.hi[o];
+        res->mem[j] = member_from_memory(o);
+        res->box[j] = make_float4(lo.x, lo.y, hi.x, hi.y);
+      }
+      if (mapx != d.binmap_x) {
+        for (int i = threadIdx.x; i < d.g.W; i += kBlock) res->mapx[i] = d.binmap_x[i];
+        for (int i = threadIdx.x; i < d.g.H; i += kBlock) res->mapy[i] = d.binmap_y[i];
       }
     }
-    if (wa)
-      for (int i = v * kThreads + (threadIdx.x & (kThreads - 1)); i < 2 * d.U; i += V * kThreads) d.wa_fix[i] = 0ull;
+  }
+  __device__ __forceinline__ AxisTaps tx(float s) const {
+    return axis_taps(d.g.Wb, s, mapx, d.g.sx, d.g.identity, d.g.W);
+  }
+  __device__ __forceinline__ AxisTaps ty(float s) const {
+    return axis_taps(d.g.Hb, s, mapy, d.g.sy, d.g.identity, d.g.H);
   }
 
-  // Density scatter by the whole block, with the per-field tap total.
-  __device__ void scatter(const float2* pos, int v) {
-    long long tot[kMaxFields];
-    scatter_items(d, pos, v * kBlock + (int)threadIdx.x, V * kBlock, tot);
-    if (v != pb) __syncthreads();   // the previous virtual block's totals have been read
+  // ---- the phases' work on one virtual block ------------------------------
+
+  // Resets of the accumulators, dealt to all threads of the block.
+  __device__ void reset_grids(int v, int from = 0) {
+    const int n = d.K * d.B, stride = V * kBlock;
+    for (int i = from + v * kBlock + (int)threadIdx.x; i < n; i += stride) {
+      d.phys[i] = -d.capfix[i];
+      d.fill[i] = 0;
+    }
+  }
+  __device__ void reset_wa(int v) {
+    for (int i = v * kBlock + (int)threadIdx.x; i < 2 * d.U; i += V * kBlock) d.wa_fix[i] = 0ull;
+  }
+
+  // Scatters object o at p, into the totals per field.
+  __device__ __forceinline__ void deposit(const float4& m, int o, float2 p, long long (&tot)[kMaxFields]) {
+    const int f = __float_as_int(m.w);
+    auto put = [&](float x, float y, float q, int field, long long* grids) {
+      const long long s = deposit_taps(d, (unsigned long long*)(grids + (size_t)field * d.B), q, tx(x), ty(y));
+#pragma unroll
+      for (int ff = 0; ff < kMaxFields; ++ff)
+        if (ff == field) tot[ff] += s;
+    };
+    if (f >= 0) {
+      if (o < d.U)
+        put(__fadd_rn(p.x, m.x), __fadd_rn(p.y, m.y), m.z, f, d.phys);
+      else
+        put(p.x, p.y, m.z, f, d.fill);
+    } else if (f == kManyMembers) {
+      for (int i = d.unit_mem_ptr[o], e = d.unit_mem_ptr[o + 1]; i < e; ++i) {
+        const float2 off = d.mem_off[i];
+        put(__fadd_rn(p.x, off.x), __fadd_rn(p.y, off.y), d.mem_q[i], d.mem_field[i], d.phys);
+      }
+    }
+  }
+  // half A: its warps' totals, then (after the group's barrier) partial v
+  __device__ __forceinline__ void stage_totals(const GA& g, const long long (&tot)[kMaxFields]) {
 #pragma unroll
     for (int f = 0; f < kMaxFields; ++f)
       if (f < d.K) {
         const long long t = warp_sum(tot[f]);
-        if ((threadIdx.x & 31) == 0) sh.tot[f][threadIdx.x >> 5] = t;
+        if ((g.tid & 31) == 0) sh.tot[f][g.tid >> 5] = t;
       }
-    __syncthreads();
-    if ((int)threadIdx.x < d.K) {
+  }
+  __device__ __forceinline__ void write_totals(const GA& g, int v) {
+    const int f = g.tid - 128;
+    if (f >= 0 && f < d.K) {
       long long t = 0;
-      for (int w = 0; w < kWarps; ++w) t += sh.tot[threadIdx.x][w];
-      islot(r.p, IS_GRID_SUM + threadIdx.x)[v] = t;
+#pragma unroll
+      for (int w = 0; w < kThreads / 32; ++w) t += sh.tot[f][w];
+      islot(r.p, IS_GRID_SUM + f)[v] = t;
     }
+  }
+  // Half A: the scatter of a point that is in memory.
+  __device__ void scatter(const float2* pos, int v) {
+    const GA g = half_a();
+    long long tot[kMaxFields] = {0, 0, 0, 0};
+    for (int j = g.tid, o; (o = object(v, j)) < d.nobj; j += kThreads) {
+      const float2 p = pos[o];
+      if (resident(j)) res->pos[j] = p;
+      deposit(member(j, o), o, p, tot);
+    }
+    g.sync();   // earlier readers of the scratch are done
+    stage_totals(g, tot);
+    g.sync();
+    write_totals(g, v);
   }
 
   // WA by half B (the whole single block).
@@ -331,72 +434,86 @@ struct Ctx {
     }
   }
 
-  // Field gradients of object o (gathered, or with `full` false the ones kept
-  // from the last density evaluation) and the combined gradient; the WA
-  // accumulators are cleared for the next evaluation as they are read. The
-  // KKT residual and the first non-finite index need no order, so the
-  // objects are dealt to all threads of the block. (The L1 norms and the
-  // density force, which only the two evaluations before the first iteration
-  // use, come from stage_gather / stage_combine there.)
+  // Raw field gradients of an object and what its combination reads besides,
+  // all loaded together. (The L1 norms and the density force, which only the
+  // two evaluations before the first iteration use, come from stage_gather /
+  // stage_combine there.)
   struct Raw {
     float2 f[kMaxFields];
+    float2 at;
+    ulonglong2 wa;
+    float P;
   };
-  __device__ __forceinline__ Raw field_gradient(const float2* pos, int o, bool full) {
+  __device__ __forceinline__ void operands(Raw& a, int o) {
+    a.P = d.P[o];
+    a.wa = o < d.U ? reinterpret_cast<const ulonglong2*>(d.wa_fix)[o] : make_ulonglong2(0ull, 0ull);
+  }
+  // gathered at pos (sample_quadratic_bspline_with_gradient and the member and
+  // filler loops, electrostatic_placement.rs:338-374, 919-941), and kept
+  __device__ __forceinline__ Raw gathered(const float2* pos, int j, int o) {
     Raw a;
 #pragma unroll
     for (int f = 0; f < kMaxFields; ++f) a.f[f] = make_float2(0.f, 0.f);
     if (o >= d.nobj) return a;
-    if (!full) {
-      if (o < d.U) {
+    operands(a, o);
+    a.at = resident(j) ? res->pos[j] : pos[o];
+    const float4 m = member(j, o);
+    const int f = __float_as_int(m.w);
+    auto add = [&](float x, float y, float q, int field) {
+      const float2 s = sample_grad(d, d.phi + (size_t)field * d.B, tx(x), ty(y));
 #pragma unroll
-        for (int f = 0; f < kMaxFields; ++f)
-          if (f < d.K) a.f[f] = d.graw[(size_t)f * d.nobj + o];
-      } else {
-        a.f[0] = d.graw[(size_t)d.fil_field[o - d.U] * d.nobj + o];
-      }
+      for (int ff = 0; ff < kMaxFields; ++ff)
+        if (ff == field) {
+          a.f[ff].x += q * s.x;
+          a.f[ff].y += q * s.y;
+        }
+    };
+    if (o >= d.U) {
+      const float2 s = sample_grad(d, d.phi + (size_t)f * d.B, tx(a.at.x), ty(a.at.y));
+      a.f[0] = make_float2(m.z * s.x, m.z * s.y);   // a filler's one field
+      d.graw[(size_t)f * d.nobj + o] = a.f[0];
       return a;
     }
-    if (o < d.U) {
-      const int m0 = d.unit_mem_ptr[o], m1 = d.unit_mem_ptr[o + 1];
-      const float2 pu = pos[o];
-      for (int m = m0; m < m1; ++m) {
-        const int f = d.mem_field[m];
-        const float2 off = d.mem_off[m];
-        const float q = d.mem_q[m];
-        const float2 s = sample_grad(d, d.phi + (size_t)f * d.B, __fadd_rn(pu.x, off.x), __fadd_rn(pu.y, off.y));
-#pragma unroll
-        for (int ff = 0; ff < kMaxFields; ++ff)
-          if (ff == f) {
-            a.f[ff].x += q * s.x;
-            a.f[ff].y += q * s.y;
-          }
+    if (f >= 0) {
+      add(__fadd_rn(a.at.x, m.x), __fadd_rn(a.at.y, m.y), m.z, f);
+    } else if (f == kManyMembers) {
+      for (int i = d.unit_mem_ptr[o], e = d.unit_mem_ptr[o + 1]; i < e; ++i) {
+        const float2 off = d.mem_off[i];
+        add(__fadd_rn(a.at.x, off.x), __fadd_rn(a.at.y, off.y), d.mem_q[i], d.mem_field[i]);
       }
+    }
+#pragma unroll
+    for (int ff = 0; ff < kMaxFields; ++ff)
+      if (ff < d.K) d.graw[(size_t)ff * d.nobj + o] = a.f[ff];
+    return a;
+  }
+  // the ones kept from the last density evaluation
+  __device__ __forceinline__ Raw kept(const float2* pos, int o) {
+    Raw a;
+    operands(a, o);
+    a.at = pos[o];
+#pragma unroll
+    for (int f = 0; f < kMaxFields; ++f) a.f[f] = make_float2(0.f, 0.f);
+    if (o < d.U) {
 #pragma unroll
       for (int f = 0; f < kMaxFields; ++f)
-        if (f < d.K) d.graw[(size_t)f * d.nobj + o] = a.f[f];
+        if (f < d.K) a.f[f] = d.graw[(size_t)f * d.nobj + o];
     } else {
-      const int j = o - d.U;
-      const int f = d.fil_field[j];
-      const float q = d.fil_q[j];
-      const float2 pf = pos[o];
-      const float2 s = sample_grad(d, d.phi + (size_t)f * d.B, pf.x, pf.y);
-      a.f[0] = make_float2(q * s.x, q * s.y);   // a filler's one field
-      d.graw[(size_t)f * d.nobj + o] = a.f[0];
+      a.f[0] = d.graw[(size_t)d.fil_field[o - d.U] * d.nobj + o];
     }
     return a;
   }
-  __device__ __forceinline__ void combine_object(const Raw& a, int o, const float2* pos, float2* g, float& kkt,
-                                                 unsigned& bad) {
+  // The combined gradient of an object (combined_objective, eplace.rs:1022-
+  // 1044); the WA accumulators it has read are cleared for the next evaluation.
+  // The KKT residual and the first non-finite index need no order.
+  __device__ __forceinline__ void combine(const Raw& a, int j, int o, float2* g, float& kkt, unsigned& bad) {
     if (o >= d.nobj) return;
-    const float2 at = pos[o], lo = d.lo[o], hi = d.hi[o];
-    const float P = d.P[o];
+    const float4 bx = box(j, o);
     float gx = 0.f, gy = 0.f;
     if (o < d.U) {
-      ulonglong2* w = reinterpret_cast<ulonglong2*>(d.wa_fix) + o;
-      const ulonglong2 q = *w;
-      *w = make_ulonglong2(0ull, 0ull);
-      gx = __ll2float_rn((long long)q.x) * kInvFixF;
-      gy = __ll2float_rn((long long)q.y) * kInvFixF;
+      reinterpret_cast<ulonglong2*>(d.wa_fix)[o] = make_ulonglong2(0ull, 0ull);
+      gx = __ll2float_rn((long long)a.wa.x) * kInvFixF;
+      gy = __ll2float_rn((long long)a.wa.y) * kInvFixF;
 #pragma unroll
       for (int f = 0; f < kMaxFields; ++f)
         if (f < d.K) {
@@ -405,88 +522,95 @@ struct Ctx {
           gy = fmaf(c, a.f[f].y, gy);
         }
     } else {
-      const float c = coef32[d.fil_field[o - d.U]];
+      const float c = coef32[d.K == 1 ? 0 : d.fil_field[o - d.U]];
       gx = c * a.f[0].x;
       gy = c * a.f[0].y;
     }
     if (!isfinite(gx)) bad = min(bad, 2u * (unsigned)o);
     else if (!isfinite(gy)) bad = min(bad, 2u * (unsigned)o + 1u);
     g[o] = make_float2(gx, gy);
-    const float s = rsqrtf(P);
-    kkt = fmaxf(kkt, kkt_comp(gx, at.x, lo.x, hi.x) * s);
-    kkt = fmaxf(kkt, kkt_comp(gy, at.y, lo.y, hi.y) * s);
+    const float s = rsqrtf(a.P);
+    kkt = fmaxf(kkt, kkt_comp(gx, a.at.x, bx.x, bx.z) * s);
+    kkt = fmaxf(kkt, kkt_comp(gy, a.at.y, bx.y, bx.w) * s);
   }
-  // The block's KKT maximum and least bad index as partials of block v: the
-  // residuals are not negative, so their bits order as integers.
-  __device__ void write_kkt(float kkt, unsigned bad, int v) {
+  // Warp results of a KKT maximum and a least bad index: the residuals are not
+  // negative, so their bits order as integers.
+  __device__ __forceinline__ void stage_kkt_warp(float kkt, unsigned bad, unsigned* ks, unsigned* bs, int w) {
     const unsigned k = __reduce_max_sync(0xffffffffu, __float_as_uint(kkt));
     const unsigned b = __reduce_min_sync(0xffffffffu, bad);
-    if (v != pb) __syncthreads();   // the previous virtual block's values have been read
     if ((threadIdx.x & 31) == 0) {
-      sh.u[0][threadIdx.x >> 5] = k;
-      sh.u[1][threadIdx.x >> 5] = b;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned km = 0u, bm = 0xffffffffu;
-      for (int w = 0; w < kWarps; ++w) {
-        km = max(km, sh.u[0][w]);
-        bm = min(bm, sh.u[1][w]);
-      }
-      mslot(r.p, MS_KKT)[v] = (double)__uint_as_float(km);
-      islot(r.p, IS_BAD)[v] = bm == 0xffffffffu ? 0x7fffffffffffffffll : (long long)bm;
+      ks[w] = k;
+      bs[w] = b;
     }
   }
-  // combine(X): the gradient at pos from the kept field gradients.
+  __device__ __forceinline__ void write_kkt(const Partials& p, const unsigned* ks, const unsigned* bs, int n, int v) {
+    unsigned k = 0u, b = 0xffffffffu;
+    for (int w = 0; w < n; ++w) {
+      k = max(k, ks[w]);
+      b = min(b, bs[w]);
+    }
+    mslot(p, MS_KKT)[v] = (double)__uint_as_float(k);
+    islot(p, IS_BAD)[v] = b == 0xffffffffu ? 0x7fffffffffffffffll : (long long)b;
+  }
+  // Half B: the origin's combined gradient from the kept field gradients; its
+  // partials go to the second set (the first holds the evaluated points').
   __device__ void combine_kept(const float2* pos, float2* g, int v) {
+    const GB gb = half_b();
     float kkt = 0.f;
     unsigned bad = 0xffffffffu;
-    for (int o = v * kBlock + (int)threadIdx.x; o < d.nobj; o += V * kBlock)
-      combine_object(field_gradient(pos, o, false), o, pos, g, kkt, bad);
-    write_kkt(kkt, bad, v);
-  }
-  __device__ FoldJob kkt_job(int j) const {
-    return j == 0 ? FoldJob{mslot(r.p, MS_KKT), FOLD_DMAX} : FoldJob{islot(r.p, IS_BAD), FOLD_IMIN};
-  }
-
-  // fixed-point density mean per field (DC mode), from the scatter's grid sums
-  __device__ void fold_means(const GA& g) {
-    const int w = g.tid >> 5;
-    if (w < d.K) {
-      const FoldJob jb{islot(r.p, IS_GRID_SUM + w), FOLD_ISUM};
-      const FoldValue s = fold_job(fold_load(jb.a, V), jb, V);
-      if ((g.tid & 31) == 0) fmean[w] = (s.l - d.capsum[w]) / d.B;
+    for (int j = gb.tid, o; (o = object(v, j)) < d.nobj; j += 2 * kThreads) {   // two objects' loads in flight
+      const int o2 = object(v, j + kThreads);
+      const bool two = o2 < d.nobj;
+      const Raw a = kept(pos, o), b = two ? kept(pos, o2) : a;
+      combine(a, j, o, g, kkt, bad);
+      if (two) combine(b, j + kThreads, o2, g, kkt, bad);
     }
-    g.sync();
+    gb.sync();   // earlier readers of the scratch are done
+    stage_kkt_warp(kkt, bad, sh.x[0], sh.x[1], gb.tid >> 5);
+    gb.sync();
+    if (gb.tid == 0) write_kkt(r.q, sh.x[0], sh.x[1], kThreads / 32, v);
+  }
+  __device__ FoldJob kkt_job(const Partials& p, int j) const {
+    return j == 0 ? FoldJob{mslot(p, MS_KKT), FOLD_DMAX} : FoldJob{islot(p, IS_BAD), FOLD_IMIN};
   }
 
-  // Half A's side of a density evaluation once the grids are complete: phi
-  // and the overflow and energy partials.
-  __device__ bool transforms() {
+  // fixed-point density mean (DC mode) of field f, from its folded grid sum;
+  // truncated division, a shift for the power-of-two grids
+  __device__ void set_mean(int f, long long sum) {
+    const long long t = sum - capsum[f];
+    const int B_ = d.B;
+    fmean[f] = (B_ & (B_ - 1)) == 0 ? (t + (long long)((unsigned long long)(t >> 63) & (unsigned long long)(B_ - 1))) >> (31 - __clz(B_))
+                                    : t / B_;
+  }
+  __device__ FoldJob sum_job(int f) const { return FoldJob{islot(r.p, IS_GRID_SUM + f), FOLD_ISUM}; }
+
+  // Half A's side of a density evaluation once the grids are complete, in two
+  // parts around the first barrier: the density preparation with the first
+  // transform, and the rest to phi and the overflow and energy partials.
+  __device__ bool transform_first() {
     const GA g = half_a();
     if (d.fft) {
-      // FFT form: rows (with the density preparation folded in), columns, rows
-      fold_means(g);
-      fft::Smem& fs = *reinterpret_cast<fft::Smem*>(gsm.fft);
-      for (int v = pb; v < V; v += np) fft::pass_rows_fwd(g, d, r.p, v, V, fs, sh.a, fmean, tables);
+      for (int v = pb; v < V; v += np)
+        fft::pass_rows_fwd(g, d, r.p, v, V, *reinterpret_cast<fft::Smem*>(gsm.fft), sh.a, fmean, tables);
+    } else if (LARGE) {
+      for (int v = pb; v < V; v += np) stage_prep(g, d, r.p, V, v, V, sh.a);
       if (!sync_a(g)) return false;
+      mark(PC_PREP);
+      for (int v = pb; v < V; v += np) stage_dct_t<LARGE>(g, d, 0, r.p, v, V, gsm, sh.a);
+    } else {
+      for (int v = pb; v < V; v += np) stage_prep_dct0(g, d, fmean, r.p, v, V, gsm, sh.a);
+    }
+    return true;
+  }
+  __device__ bool transform_rest() {
+    const GA g = half_a();
+    if (d.fft) {
+      fft::Smem& fs = *reinterpret_cast<fft::Smem*>(gsm.fft);
       for (int v = pb; v < V; v += np) fft::pass_cols(g, d, v, V, fs, tables);
       if (!sync_a(g)) return false;
       for (int v = pb; v < V; v += np) fft::pass_rows_inv(g, d, r.p, v, V, fs, sh.a, tables);
     } else {
-      int st0 = 0;
-      if (LARGE) {
-        for (int v = pb; v < V; v += np) stage_prep(g, d, r.p, V, v, V, sh.a);
-        if (!sync_a(g)) return false;
-        mark(PC_PREP);
-      } else {
-        // density preparation folded into the first transform (one phase less)
-        fold_means(g);
-        for (int v = pb; v < V; v += np) stage_prep_dct0(g, d, fmean, r.p, v, V, gsm, sh.a);
-        if (!sync_a(g)) return false;
-        st0 = 1;
-      }
-      for (int st = st0; st < 4; ++st) {
+      for (int st = 1; st < 4; ++st) {
         for (int v = pb; v < V; v += np) stage_dct_t<LARGE>(g, d, st, r.p, v, V, gsm, sh.a);
         if (st < 3 && !sync_a(g)) return false;
       }
@@ -504,8 +628,19 @@ struct Ctx {
                     : FoldJob{islot(r.p, IS_OVER_BINS + f), FOLD_ISUM};
   }
   __device__ int eval_jobs(bool full) const { return full ? 3 * d.K + 1 : 1; }
-  // thread 0: the objective and the fields' coefficients from the jobs at fv[at...]
-  __device__ void eval_scalars(ERec& out, bool full, int at = 0) {
+  // one thread: the fields' coefficients from the jobs at fv[at...]
+  __device__ void eval_coefficients(bool full, int at = 0) {
+    for (int f = 0; f < d.K; ++f) {
+      const double ne = (full ? 0.5 * fv[at + 3 * f].d : S.cur_energy[f]) * S.inv_e0[f];
+      coef[f] = S.lambda[f] * (1.0 + S.beta * ne);
+      coef32[f] = (float)coef[f];
+    }
+  }
+  // one thread: the objective
+  __device__ void eval_value(ERec& out, bool full, int at = 0) {
+    const double wa = fv[at + (full ? 3 * d.K : 0)].d;
+    out.wa = wa;
+    double value = wa;
     for (int f = 0; f < d.K; ++f) {
       if (full) {
         const long long ov = fv[at + 3 * f + 1].l;
@@ -519,15 +654,8 @@ struct Ctx {
         out.ovfix[f] = S.cur_overflow_fixed[f];
         out.bins[f] = 0;
       }
-    }
-    const double wa = fv[at + (full ? 3 * d.K : 0)].d;
-    out.wa = wa;
-    double value = wa;
-    for (int f = 0; f < d.K; ++f) {
       const double ne = out.energy[f] * S.inv_e0[f];
       value += S.lambda[f] * S.e0[f] * (ne + 0.5 * S.beta * ne * ne);
-      coef[f] = S.lambda[f] * (1.0 + S.beta * ne);
-      coef32[f] = (float)coef[f];
     }
     out.value = value;
   }
@@ -537,16 +665,25 @@ struct Ctx {
   // combined_objective, eplace.rs:137-205, 1022-1044).
   __device__ bool eval_initial(const float2* pos, float2* g, double gam, bool full, ERec& out) {
     if (full) {
-      for (int v = pb; v < V; v += np) scatter(pos, v);
+      if (in_a())
+        for (int v = pb; v < V; v += np) scatter(pos, v);
       if (!sync()) return false;
-      if (in_a()) transforms();
+      fold(d.K, [&](int j) { return sum_job(j); });
+      if ((int)threadIdx.x < d.K) set_mean(threadIdx.x, fv[threadIdx.x].l);
+      __syncthreads();
+      if (in_a()) {
+        if (transform_first() && sync_a(half_a())) transform_rest();
+      }
       __syncthreads();
     }
     if (in_b()) wa(pos, gam);
     if (!sync()) return false;
     mark(full ? PC_DCT : PC_SCATTER_WA);
     fold(eval_jobs(full), [&](int j) { return eval_job(j, full); });
-    if (threadIdx.x == 0) eval_scalars(out, full);
+    if (threadIdx.x == 0) {
+      eval_coefficients(full);
+      eval_value(out, full);
+    }
     __syncthreads();
     if (in_a()) {
       const GA ga = half_a();
@@ -578,25 +715,45 @@ struct Ctx {
     return true;
   }
 
-  // The loop's evaluation at pos, its positions scattered: the transforms by
-  // half A, WA by half B. With lead the scatter has just ended and half A
-  // waits for the other blocks' first. Returns after a barrier of all.
-  __device__ bool density_and_wa(const float2* pos, double gam, bool lead) {
-    if (SETS == 1 || !in_a()) wa(pos, gam);
+  // The loop's evaluation at pos, scattered and the means known. With
+  // origin_g, half B first combines the origin's gradient, and WA(pos) starts
+  // once every block has read the origin's WA accumulators.
+  __device__ bool density_and_wa(const float2* pos, double gam, const float2* origin, float2* origin_g) {
+    bool ready = true;
+    if (SETS == 1 && !origin_g) wa(pos, gam);
+    if (in_a()) ready = transform_first();
+    if (origin_g) {
+      if (in_b())
+        for (int v = pb; v < V; v += np) combine_kept(origin, origin_g, v);
+      ready = sync();
+      if (SETS == 1 && ready) wa(pos, gam);
+    }
     if (in_a()) {
-      const bool ready = !lead || sync_a(half_a());
-      if (ready) transforms();
+      if (!origin_g && ready) ready = sync_a(half_a());
+      if (ready) transform_rest();
+    } else {
+      if (ready) wa(pos, gam);
     }
     const bool k = sync();
     mark(PC_DCT);
     return k;
   }
   // The rest of it: the scalars, the gathered field gradients and the
-  // combined gradient with its KKT residual. A double block gathers while
-  // the partials are on their way and folded, and needs the coefficients
-  // only to combine.
-  __device__ bool gradient(const float2* pos, float2* g, ERec& out) {
-    const int n = eval_jobs(true), stride = V * kBlock;
+  // combined gradient with its KKT residual, and the grids reset for the next
+  // scatter. A double block gathers while the partials are on their way and
+  // folded, and needs the coefficients only to combine; the objective's value
+  // is formed by a warp of its own meanwhile. With `origin` the origin's
+  // deferred KKT residual and index check are folded too.
+  __device__ bool gradient(const float2* pos, float2* g, ERec& out, ERec* origin) {
+    const int ne = eval_jobs(true), n = ne + (origin ? 2 : 0);
+    auto job = [&](int j) { return j < ne ? eval_job(j, true) : kkt_job(r.q, j - ne); };
+    auto scalars = [&]() {
+      eval_value(out, true);
+      if (origin) {
+        origin->kkt = fv[ne].d;
+        origin->bad = fv[ne + 1].l;
+      }
+    };
     float kkt = 0.f;
     unsigned bad = 0xffffffffu;
     int v = pb;
@@ -605,38 +762,60 @@ struct Ctx {
       FoldJob jb{nullptr, FOLD_DSUM};
       FoldAhead fa;
       if (w < n) {
-        jb = eval_job(w, true);
+        jb = job(w);
         fa = fold_load(jb.a, V);
       }
-      int o = v * kBlock + (int)threadIdx.x;
-      const Raw a0 = field_gradient(pos, o, true), a1 = field_gradient(pos, o + stride, true);
+      int j = threadIdx.x;
+      const int o0 = object(v, j), o1 = object(v, j + kBlock);
+      const int bin = v * kBlock + j;   // the first bin this thread resets
+      const long long cap = bin < d.K * d.B ? d.capfix[bin] : 0;
+      const Raw a0 = gathered(pos, j, o0), a1 = gathered(pos, j + kBlock, o1);
       if (w < n) {
         const FoldValue q = fold_job(fa, jb, V);
         if ((threadIdx.x & 31) == 0) fv[w] = q;
       }
       __syncthreads();
-      if (threadIdx.x == 0) eval_scalars(out, true);
+      if (threadIdx.x == 0) eval_coefficients(true);
       __syncthreads();
-      combine_object(a0, o, pos, g, kkt, bad);
-      combine_object(a1, o + stride, pos, g, kkt, bad);
-      for (o += 2 * stride; o < d.nobj; o += stride) combine_object(field_gradient(pos, o, true), o, pos, g, kkt, bad);
-      write_kkt(kkt, bad, v);
+      if (threadIdx.x == kBlock - 32) scalars();
+      combine(a0, j, o0, g, kkt, bad);
+      combine(a1, j + kBlock, o1, g, kkt, bad);
+      for (j += 2 * kBlock;; j += kBlock) {
+        const int o = object(v, j);
+        if (o >= d.nobj) break;
+        combine(gathered(pos, j, o), j, o, g, kkt, bad);
+      }
+      if (bin < d.K * d.B) {
+        d.phys[bin] = -cap;
+        d.fill[bin] = 0;
+      }
+      reset_grids(v, V * kBlock);
+      stage_kkt_warp(kkt, bad, sh.u[0], sh.u[1], w);
+      __syncthreads();
+      if (threadIdx.x == 0) write_kkt(r.p, sh.u[0], sh.u[1], kWarps, v);
       v += np;
     } else {
-      fold(n, [&](int j) { return eval_job(j, true); });
-      if (threadIdx.x == 0) eval_scalars(out, true);
+      fold(n, job);
+      if (threadIdx.x == 0) {
+        eval_coefficients(true);
+        scalars();
+      }
       __syncthreads();
     }
     for (; v < V; v += np) {
       kkt = 0.f;
       bad = 0xffffffffu;
-      for (int o = v * kBlock + (int)threadIdx.x; o < d.nobj; o += stride)
-        combine_object(field_gradient(pos, o, true), o, pos, g, kkt, bad);
-      write_kkt(kkt, bad, v);
+      for (int j = threadIdx.x, o; (o = object(v, j)) < d.nobj; j += kBlock)
+        combine(gathered(pos, j, o), j, o, g, kkt, bad);
+      reset_grids(v);
+      __syncthreads();   // earlier readers of the scratch are done
+      stage_kkt_warp(kkt, bad, sh.u[0], sh.u[1], threadIdx.x >> 5);
+      __syncthreads();
+      if (threadIdx.x == 0) write_kkt(r.p, sh.u[0], sh.u[1], kWarps, v);
     }
     if (!sync()) return false;
     mark(PC_GATHER);
-    fold(2, [&](int j) { return kkt_job(j); });
+    fold(2, [&](int j) { return kkt_job(r.p, j); });
     if (threadIdx.x == 0) {
       out.kkt = fv[0].d;
       out.bad = fv[1].l;
@@ -649,8 +828,10 @@ struct Ctx {
 
   // Half A, before an iteration's evaluations: the preconditioner
   // (diagonal_preconditioner, eplace.rs:1046-1100) and y = clamp(x + e (x -
-  // xp)) with the count of coordinates that moved.
-  __device__ void precondition(const float* lam, const float2* x, const float2* xp, float e, float2* y, int v) {
+  // xp)) with the count of coordinates that moved; y is scattered with
+  // `deposits`. Two objects' loads are in flight.
+  __device__ void precondition(const float* lam, const float2* x, const float2* xp, float e, float2* y, bool deposits,
+                               int v) {
     const GA g = half_a();
     float lambda[kMaxFields];
 #pragma unroll
@@ -658,32 +839,58 @@ struct Ctx {
     float pmin = INFINITY, pmax = 0.f;
     unsigned diff = 0;
     bool badp = false;
-    const int stride = V * kThreads;
-    for (int o = v * kThreads + g.tid; o < d.nobj; o += stride) {
-      float q[kMaxFields];
-      float m = d.pre_static[o];
+    long long tot[kMaxFields] = {0, 0, 0, 0};
+    struct In {
+      float2 a, b;
+      float4 bx, mem;
+      float m, q[kMaxFields];
+    };
+    auto load = [&](int j, int o) {
+      In i;
+      i.a = x[o];
+      i.b = xp[o];
+      i.m = d.pre_static[o];
 #pragma unroll
-      for (int f = 0; f < kMaxFields; ++f) q[f] = f < d.K ? d.pre_q[(size_t)f * d.nobj + o] : 0.f;
-      const float2 a = x[o], b = xp[o], lo = d.lo[o], hi = d.hi[o];
+      for (int f = 0; f < kMaxFields; ++f) i.q[f] = f < d.K ? d.pre_q[(size_t)f * d.nobj + o] : 0.f;
+      i.bx = box(j, o);
+      i.mem = member(j, o);
+      return i;
+    };
+    auto step = [&](const In& i, int j, int o) {
       float2 t;
-      t.x = fclamp(a.x + e * (a.x - b.x), lo.x, hi.x);
-      t.y = fclamp(a.y + e * (a.y - b.y), lo.y, hi.y);
-      diff += (t.x != a.x) + (t.y != a.y);
+      t.x = fclamp(i.a.x + e * (i.a.x - i.b.x), i.bx.x, i.bx.z);
+      t.y = fclamp(i.a.y + e * (i.a.y - i.b.y), i.bx.y, i.bx.w);
+      diff += (t.x != i.a.x) + (t.y != i.a.y);
       y[o] = t;
+      if (resident(j)) res->pos[j] = t;
+      float m = i.m;
 #pragma unroll
       for (int f = 0; f < kMaxFields; ++f)
-        if (q[f] != 0.f) m = fmaf(lambda[f], q[f], m);
+        if (i.q[f] != 0.f) m = fmaf(lambda[f], i.q[f], m);
       if (!isfinite(m) || m < 0.f) badp = true;
       m = fmaxf(m, 1.f);
       d.P[o] = m;
       pmin = fminf(pmin, m);
       pmax = fmaxf(pmax, m);
+      return t;
+    };
+    for (int j = g.tid, o; (o = object(v, j)) < d.nobj; j += 2 * kThreads) {
+      const int o2 = object(v, j + kThreads);
+      const bool two = o2 < d.nobj;
+      const In i0 = load(j, o), i1 = two ? load(j + kThreads, o2) : i0;
+      const float2 t0 = step(i0, j, o);
+      const float2 t1 = two ? step(i1, j + kThreads, o2) : t0;
+      if (deposits) {
+        deposit(i0.mem, o, t0, tot);
+        if (two) deposit(i1.mem, o2, t1, tot);
+      }
     }
     // not negative, so the bits order as integers
     const unsigned lo = __reduce_min_sync(0xffffffffu, __float_as_uint(pmin));
     const unsigned hi = __reduce_max_sync(0xffffffffu, __float_as_uint(pmax));
     const unsigned c = __reduce_add_sync(0xffffffffu, diff) | (__any_sync(0xffffffffu, badp) ? 0x80000000u : 0u);
     g.sync();   // earlier readers of the scratch are done
+    stage_totals(g, tot);
     if ((g.tid & 31) == 0) {
       sh.u[0][g.tid >> 5] = lo;
       sh.u[1][g.tid >> 5] = hi;
@@ -704,47 +911,61 @@ struct Ctx {
       islot(r.p, IS_PBAD)[v] = bad;
       islot(set(), IS_DIFF)[v] = n;
     }
+    if (deposits) write_totals(g, v);
   }
 
-  // Half A: c = clamp(y - g / (L P)); changed count, <g, c - y>, sum P (c -
-  // y)^2. Each thread's objects and the order of its sums are those of the
-  // 256-thread stage (the sums are FP32), two objects' loads in flight.
+  // Half A: c = clamp(y - g / (L P)), scattered as it is formed; changed
+  // count, <g, c - y>, sum P (c - y)^2. Each thread's objects and the order of
+  // its sums are those of the 256-thread stage (the sums are FP32), two
+  // objects' loads in flight.
   __device__ void candidate(const float2* y, const float2* gy, float invL, float2* c, int v) {
     const GA g = half_a();
     unsigned diff = 0;
     float dot = 0.f, msn = 0.f;
+    long long tot[kMaxFields] = {0, 0, 0, 0};
     struct In {
-      float2 a, gr, lo, hi;
+      float2 a, gr;
+      float4 bx, mem;
       float m;
     };
-    auto load = [&](int o) { return In{y[o], gy[o], d.lo[o], d.hi[o], d.P[o]}; };
-    auto step = [&](const In& i, int o) {
+    auto load = [&](int j, int o) { return In{y[o], gy[o], box(j, o), member(j, o), d.P[o]}; };
+    auto step = [&](const In& i, int j, int o) {
       const float s = invL / i.m;
       float2 t;
-      t.x = fclamp(i.a.x - i.gr.x * s, i.lo.x, i.hi.x);
-      t.y = fclamp(i.a.y - i.gr.y * s, i.lo.y, i.hi.y);
+      t.x = fclamp(i.a.x - i.gr.x * s, i.bx.x, i.bx.z);
+      t.y = fclamp(i.a.y - i.gr.y * s, i.bx.y, i.bx.w);
       diff += (t.x != i.a.x) + (t.y != i.a.y);
       const float dx = t.x - i.a.x, dy = t.y - i.a.y;
       dot = fmaf(i.gr.x, dx, fmaf(i.gr.y, dy, dot));
       msn = fmaf(i.m * dx, dx, fmaf(i.m * dy, dy, msn));
       c[o] = t;
+      if (resident(j)) res->pos[j] = t;
+      return t;
     };
-    const int stride = V * kThreads;
-    for (int o = v * kThreads + g.tid; o < d.nobj; o += 2 * stride) {
-      const In i0 = load(o);
-      const bool two = o + stride < d.nobj;
-      const In i1 = two ? load(o + stride) : i0;
-      step(i0, o);
-      if (two) step(i1, o + stride);
+    for (int j = g.tid, o; (o = object(v, j)) < d.nobj; j += 2 * kThreads) {
+      const int o2 = object(v, j + kThreads);
+      const bool two = o2 < d.nobj;
+      const In i0 = load(j, o), i1 = two ? load(j + kThreads, o2) : i0;
+      const float2 t0 = step(i0, j, o);
+      const float2 t1 = two ? step(i1, j + kThreads, o2) : t0;
+      deposit(i0.mem, o, t0, tot);
+      if (two) deposit(i1.mem, o2, t1, tot);
     }
     // both FP64 sums at once, each in block_fold_fp64's order
     double *b0 = sh.pair, *b1 = sh.pair + kThreads + 4;
     const unsigned n = __reduce_add_sync(0xffffffffu, diff);
     g.sync();   // earlier readers of the scratch are done
+    stage_totals(g, tot);
     b0[g.tid] = (double)dot;
     b1[g.tid] = (double)msn;
     if ((g.tid & 31) == 0) sh.u[0][g.tid >> 5] = n;
     g.sync();
+    if (g.tid == 64) {
+      long long t = 0;
+      for (int w = 0; w < kThreads / 32; ++w) t += sh.u[0][w];
+      islot(set(), IS_DIFF)[v] = t;
+    }
+    write_totals(g, v);
     {
       const int w = g.tid >> 5, at = (w & 3) * 32 + (g.tid & 31);
       double* b = w < 4 ? b0 : b1;
@@ -757,11 +978,6 @@ struct Ctx {
     if (g.tid == 0 || g.tid == 32) {
       const double* b = (g.tid == 0 ? b0 : b1) + kThreads;
       pslot(set(), g.tid == 0 ? SLOT_DOT : SLOT_MSN)[v] = ((b[0] + b[1]) + b[2]) + b[3];
-    }
-    if (g.tid == 64) {
-      long long t = 0;
-      for (int w = 0; w < kThreads / 32; ++w) t += sh.u[0][w];
-      islot(set(), IS_DIFF)[v] = t;
     }
   }
 };
@@ -846,25 +1062,34 @@ static __device__ int checked_dev(const ERec& e) {
   if (e.bad != 0x7fffffffffffffffll) return TEXO_GP_ERR_NONFINITE_GRADIENT;
   return TEXO_GP_OK;
 }
-// update_density_multipliers + next_multiplier_step (eplace.rs:1234-1298)
+// update_density_multipliers (eplace.rs:1234-1260), with the step of this
+// iteration; growth_dev gives the next step's factor (next_multiplier_step,
+// :1261-1298), which depends on the energies alone
 static __device__ int update_multipliers_dev(DevRun& S) {
   for (int f = 0; f < S.K; ++f)
     if (!isfinite(S.cur_energy[f]) || !(S.e0[f] > 0.0)) return TEXO_GP_ERR_DENSITY_FIELD_CHANGED;
   double sg[kMaxFields], nn = 0.0;
-  for (int f = 0; f < S.K; ++f) {
-    const double ne = S.cur_energy[f] * S.inv_e0[f];
-    sg[f] = ne + 0.5 * S.beta * ne * ne;
-    if (!isfinite(sg[f]) || sg[f] < 0.0) return TEXO_GP_ERR_INVALID_NORMALIZATION;
-    nn += sg[f] * sg[f];
-  }
+#pragma unroll
+  for (int f = 0; f < kMaxFields; ++f)
+    if (f < S.K) {
+      const double ne = S.cur_energy[f] * S.inv_e0[f];
+      sg[f] = ne + 0.5 * S.beta * ne * ne;
+      if (!isfinite(sg[f]) || sg[f] < 0.0) return TEXO_GP_ERR_INVALID_NORMALIZATION;
+      nn += sg[f] * sg[f];
+    }
   const double norm = sqrt(nn);
   if (norm != 0.0) {
     if (!isfinite(norm) || !isfinite(S.mstep) || S.mstep <= 0.0) return TEXO_GP_ERR_INVALID_NORMALIZATION;
-    for (int f = 0; f < S.K; ++f) {
-      S.lambda[f] += S.mstep * sg[f] / norm;
-      if (!isfinite(S.lambda[f]) || S.lambda[f] < 0.0) return TEXO_GP_ERR_INVALID_NORMALIZATION;
-    }
+#pragma unroll
+    for (int f = 0; f < kMaxFields; ++f)
+      if (f < S.K) {
+        S.lambda[f] += S.mstep * sg[f] / norm;
+        if (!isfinite(S.lambda[f]) || S.lambda[f] < 0.0) return TEXO_GP_ERR_INVALID_NORMALIZATION;
+      }
   }
+  return TEXO_GP_OK;
+}
+static __device__ int growth_dev(const DevRun& S, double& growth) {
   double en = 0.0;
   for (int f = 0; f < S.K; ++f) {
     const double ne = S.cur_energy[f] * S.inv_e0[f];
@@ -872,10 +1097,8 @@ static __device__ int update_multipliers_dev(DevRun& S) {
   }
   const double lg = log(S.beta * sqrt(en) + 1.0);
   if (!isfinite(lg) || lg < 0.0) return TEXO_GP_ERR_INVALID_NORMALIZATION;
-  const double growth = S.alpha_low + (1.0 - 1.0 / (1.0 + lg)) * (S.alpha_high - S.alpha_low);
-  if (!(growth >= S.alpha_low && growth <= S.alpha_high)) return TEXO_GP_ERR_INVALID_NORMALIZATION;
-  S.mstep *= growth;
-  return (isfinite(S.mstep) && S.mstep > 0.0) ? TEXO_GP_OK : TEXO_GP_ERR_INVALID_NORMALIZATION;
+  growth = S.alpha_low + (1.0 - 1.0 / (1.0 + lg)) * (S.alpha_high - S.alpha_low);
+  return (growth >= S.alpha_low && growth <= S.alpha_high) ? TEXO_GP_OK : TEXO_GP_ERR_INVALID_NORMALIZATION;
 }
 // f64::midpoint(1, sqrt(1 + 4 m^2))
 __device__ __forceinline__ double next_momentum_dev(double m) {
@@ -899,9 +1122,11 @@ static __device__ void adopt_density(DevRun& S, const ERec& e) {
 
 // Shared-memory step bookkeeping that every thread reads after a barrier.
 struct StepVars {
-  int restart, y_is_origin, may_reduce, has_wL, action, stationary, fresh;
+  int restart, y_is_origin, may_reduce, has_wL, action, stationary, fresh, deposited, dirty;
   double wL, tL, f_y, y_stat, next_m, pmin, pmax;
-  float extrapolation, lambda[kMaxFields];
+  double gamma, growth;                       // of the next iteration
+  int st_multipliers, st_growth, st_gamma;
+  float extrapolation, lambda[kMaxFields], inv_L;
   unsigned trials;
   int pending_best, pending_prev;
 };
@@ -917,10 +1142,10 @@ __device__ __forceinline__ void copy_words(T* dst, const T* src) {
 }
 
 // The placement loop of one instance, run by its np physical blocks of SETS *
-// kThreads threads.
+// kThreads threads; `resident` is a double block's dynamic shared memory.
 template <bool LARGE, int SETS>
 static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B, DevRun* run, GridBarrier* bar, int pb,
-                         int np, int Vn) {
+                         int np, int Vn, Resident* resident) {
   __shared__ DevRun S;
   __shared__ ERec eo, ey, ec;
   __shared__ StepVars V;
@@ -929,7 +1154,7 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
   __shared__ double coef[kMaxFields];
   __shared__ float coef32[kMaxFields];
   __shared__ FoldValue fvals[kMaxFoldJobs];
-  __shared__ long long fmean[kMaxFields];
+  __shared__ long long fmean[kMaxFields], capsum[kMaxFields];
   __shared__ unsigned gen;
   __shared__ int bar_failed;
   __shared__ unsigned long long clock[10];
@@ -939,11 +1164,18 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
     gen = 0;   // the barrier is cleared with the state copy before every launch
     V.pending_best = 0;
     V.pending_prev = 0;
+    V.dirty = 0;
   }
+  if ((int)threadIdx.x < d.K) capsum[threadIdx.x] = d.capsum[threadIdx.x];
   copy_words(&S, run);
+  // one virtual block a physical one: its objects can stay in shared memory
+  Resident* const res = SETS == 2 && np == Vn ? resident : nullptr;
+  const bool maps = res && !d.g.identity && d.g.W <= kResidentMap && d.g.H <= kResidentMap;
+  Ctx<LARGE, SETS> c{d,   r,    B,      S,      bar,   &gen,  &bar_failed, gsm,  sh,    res,
+                     maps ? res->mapx : d.binmap_x, maps ? res->mapy : d.binmap_y, coef, coef32,
+                     fvals, fmean, capsum, pb, np, Vn, 0ull, clock, fft::tables_stay(d)};
+  c.make_resident();
   __syncthreads();
-  Ctx<LARGE, SETS> c{d,  r,  B,  S,   bar,   &gen, &bar_failed, gsm, sh, coef, coef32,
-                     fvals, fmean, pb, np, Vn, 0ull, clock, fft::tables_stay(d)};
   if (c.tables && c.in_a())
     fft::stage_tables(c.half_a(), fft::axis_x(d), reinterpret_cast<fft::Smem*>(gsm.fft)->buf, false);
   const int n = d.nobj;
@@ -979,7 +1211,10 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
   if (S.phase == 0) {
     // initial probe at the ePlace gamma base, then at the adaptive gamma with
     // the density side reused (same coordinates), eplace.rs:455-471
-    if (c.in_a()) VLOOP c.init(v, true, true);
+    VLOOP {
+      c.reset_grids(v);
+      c.reset_wa(v);
+    }
     SYNC_OR_EXIT(PC_PRECOND)
     if (!c.eval_initial(c.X(), c.gX(), S.gamma_base, true, eo)) LEAVE
     {
@@ -994,7 +1229,7 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
       __syncthreads();
       if (S.status) FAIL(S.status)
     }
-    if (c.in_a()) VLOOP c.init(v, false, true);
+    VLOOP c.reset_wa(v);
     SYNC_OR_EXIT(PC_PRECOND)
     if (!c.eval_initial(c.X(), c.gX(), S.gamma, false, eo)) LEAVE
     T0 {
@@ -1031,16 +1266,53 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
     if (S.status) FAIL(S.status)
     if (S.phase == 2) goto out;
   }
-  // the loop's combinations clear the WA accumulators they read; whatever ran
-  // before this launch may have left them dirty
-  if (c.in_a()) VLOOP c.init(v, false, true);
+  // the loop's evaluations leave the accumulators reset; whatever ran before
+  // this launch, or the probes above, may have left them dirty
+  VLOOP {
+    c.reset_grids(v);
+    c.reset_wa(v);
+  }
   SYNC_OR_EXIT(PC_PRECOND)
 
   // ---- outer loop -------------------------------------------------------
-  for (;;) {
+  for (bool update = false;; update = true) {
+    // The scalar rules between two iterations (FP64 functions of a thousand
+    // cycles and more each on this part) are independent of one another: the
+    // multipliers, their step's growth, gamma and the momentum run in a warp
+    // each.
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+      switch (threadIdx.x >> 5) {
+        case 0:
+          if (update) V.st_multipliers = update_multipliers_dev(S);
+          break;
+        case 1:
+          if (update) V.st_growth = growth_dev(S, V.growth);
+          break;
+        case 2: V.st_gamma = adaptive_gamma_dev(S, S.cur_overflow, V.gamma); break;
+        case 3:
+          V.next_m = next_momentum_dev(S.a);
+          V.extrapolation = (float)((S.a - 1.0) / V.next_m);
+          break;
+        default: break;
+      }
+    }
     T0 {
       V.action = ACT_NONE;
-      if (stop_dev(S, S.cur_overflow)) {
+      if (update) {
+        int st = V.st_multipliers;
+        if (!st) st = V.st_growth;
+        if (!st) {
+          S.mstep *= V.growth;
+          if (!(isfinite(S.mstep) && S.mstep > 0.0)) st = TEXO_GP_ERR_INVALID_NORMALIZATION;
+        }
+        if (st) {
+          S.status = st;
+          S.phase = 2;
+        }
+      }
+      if (S.phase == 2) {
+      } else if (stop_dev(S, S.cur_overflow)) {
         S.converged = 1;
         S.phase = 2;
       } else if (S.completed >= S.max_iterations) {
@@ -1050,13 +1322,11 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
       } else if (S.budget && done >= S.budget) {
         V.action = ACT_CONTINUE;   // leave with the loop still running
       } else {
-        double gam = 0.0;
-        const int st = adaptive_gamma_dev(S, S.cur_overflow, gam);
-        if (st) {
-          S.status = st;
+        if (V.st_gamma) {
+          S.status = V.st_gamma;
           S.phase = 2;
         }
-        S.gamma = gam;
+        S.gamma = V.gamma;
         S.completed++;
         if (!isfinite(S.a) || S.a < 1.0) {
           S.status = TEXO_GP_ERR_INVALID_MOMENTUM_PARAMETER;
@@ -1066,13 +1336,12 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
           S.status = TEXO_GP_ERR_INVALID_LIPSCHITZ_ESTIMATE;
           S.phase = 2;
         }
-        V.next_m = next_momentum_dev(S.a);
         V.restart = 0;
         V.has_wL = S.has_L;
         V.wL = S.L;
         V.trials = 0;
         V.fresh = !S.density_at_x;
-        V.extrapolation = (float)((S.a - 1.0) / V.next_m);
+        V.deposited = !V.fresh && V.extrapolation != 0.f;   // without momentum y is the origin
         for (int f = 0; f < S.K; ++f) V.lambda[f] = (float)S.lambda[f];
       }
     }
@@ -1081,73 +1350,91 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
     ++done;
 
     // Phase 1: the preconditioner (eplace.rs:1046-1100), the extrapolated
-    // point (it needs the positions and the momentum alone), pending copies,
-    // the grids' reset and the origin's WA. The origin is re-evaluated
+    // point (it needs the positions and the momentum alone) and its scatter,
+    // pending copies, and the origin's WA. The origin is re-evaluated
     // (eplace's closure changes with gamma and the multipliers); its density
     // side is reused when the device already holds it for these coordinates.
+    const bool fresh = V.fresh != 0, deposited = V.deposited != 0;
     {
-      const bool fresh = V.fresh != 0;
-      if (c.in_a()) {
-        VLOOP {
-          c.precondition(V.lambda, c.X(), V.pending_prev ? c.X() : c.Xp(), V.extrapolation, c.Y(), v);
-          c.init(v, true, false);
-        }
-      }
+      if (c.in_a())
+        VLOOP c.precondition(V.lambda, c.X(), V.pending_prev ? c.X() : c.Xp(), V.extrapolation, c.Y(), deposited, v);
       if (V.pending_best) c.copy(B.best, c.X(), d.U);
       if (V.pending_prev) c.copy(c.Xp(), c.X(), n);
       if (!fresh && c.in_b()) c.wa(c.X(), S.gamma);
       SYNC_OR_EXIT(PC_PRECOND)
       const Partials q = c.set();
-      c.fold(fresh ? 4 : 5, [&](int j) {
+      const int nj = (fresh ? 4 : 5), ns = deposited ? d.K : 0;
+      c.fold(nj + ns, [&](int j) {
         return j == 0   ? FoldJob{mslot(r.p, MS_PMIN), FOLD_DMIN}
                : j == 1 ? FoldJob{mslot(r.p, MS_PMAX), FOLD_DMAX}
                : j == 2 ? FoldJob{islot(r.p, IS_PBAD), FOLD_ISUM}
                : j == 3 ? FoldJob{islot(q, IS_DIFF), FOLD_ISUM}
-                        : FoldJob{pslot(r.p, SLOT_WA_VALUE), FOLD_DSUM};
+               : j < nj ? FoldJob{pslot(r.p, SLOT_WA_VALUE), FOLD_DSUM}
+                        : c.sum_job(j - nj);
       });
       ++c.ws;
       if (threadIdx.x == 0) {
         V.pmin = fvals[0].d;
         V.pmax = fvals[1].d;
         V.y_is_origin = fvals[3].l == 0;
+        V.dirty = deposited && fvals[3].l == 0;
         V.pending_best = 0;
         V.pending_prev = 0;
         if (fvals[2].l) S.status = TEXO_GP_ERR_INVALID_NORMALIZATION;
-        else if (!fresh) c.eval_scalars(eo, false, 4);
+        else if (!fresh) c.eval_coefficients(false);
+      }
+      if (threadIdx.x == 32 && !fresh) c.eval_value(eo, false, 4);
+      if ((int)threadIdx.x >= 64 && (int)threadIdx.x < 64 + ns) c.set_mean(threadIdx.x - 64, fvals[nj + threadIdx.x - 64].l);
+      __syncthreads();
+      if (S.status) FAIL(S.status)
+      if (!fresh) {
+        T0 {
+          S.evaluations++;
+          if (!isfinite(eo.value)) S.status = TEXO_GP_ERR_INVALID_OBJECTIVE;
+        }
+        __syncthreads();
+        if (S.status) FAIL(S.status)
+      }
+    }
+    if (fresh) {
+      if (c.in_a()) VLOOP c.scatter(c.X(), v);
+      SYNC_OR_EXIT(PC_SCATTER_WA)
+      c.fold(d.K, [&](int j) { return c.sum_job(j); });
+      if ((int)threadIdx.x < d.K) c.set_mean(threadIdx.x, fvals[threadIdx.x].l);
+      __syncthreads();
+      if (!c.density_and_wa(c.X(), S.gamma, nullptr, nullptr)) LEAVE
+      if (!c.gradient(c.X(), c.gX(), eo, nullptr)) LEAVE
+      T0 {
+        S.status = checked_dev(eo);
+        adopt_density(S, eo);
+        S.density_at_x = 1;
       }
       __syncthreads();
       if (S.status) FAIL(S.status)
-      if (fresh) {
-        VLOOP c.scatter(c.X(), v);
-        if (!c.density_and_wa(c.X(), S.gamma, true)) LEAVE
-        if (!c.gradient(c.X(), c.gX(), eo)) LEAVE
-        if (!V.y_is_origin) {
-          if (c.in_a()) VLOOP c.init(v, true, false);
-          SYNC_OR_EXIT(PC_EXTRAP)
-        }
+      if (!V.y_is_origin) {
+        if (c.in_a()) VLOOP c.scatter(c.Y(), v);
+        SYNC_OR_EXIT(PC_EXTRAP)
+        c.fold(d.K, [&](int j) { return c.sum_job(j); });
+        if ((int)threadIdx.x < d.K) c.set_mean(threadIdx.x, fvals[threadIdx.x].l);
+        __syncthreads();
       }
-      // Phase 2: the origin's gradient, beside the scatter of y
-      if (!V.y_is_origin) VLOOP c.scatter(c.Y(), v);
-      if (!fresh) VLOOP c.combine_kept(c.X(), c.gX(), v);
-      if (!fresh || !V.y_is_origin) {
-        SYNC_OR_EXIT(PC_SCATTER_WA)
-      }
-      if (!fresh) c.fold(2, [&](int j) { return c.kkt_job(j); });
+    } else if (V.y_is_origin) {
+      // the origin's gradient in a phase of its own
+      if (c.in_b()) VLOOP c.combine_kept(c.X(), c.gX(), v);
+      if (V.dirty) VLOOP c.reset_grids(v);
+      SYNC_OR_EXIT(PC_SCATTER_WA)
+      c.fold(2, [&](int j) { return c.kkt_job(r.q, j); });
       T0 {
-        if (!fresh) {
-          eo.kkt = fvals[0].d;
-          eo.bad = fvals[1].l;
-          S.evaluations++;
-        }
+        eo.kkt = fvals[0].d;
+        eo.bad = fvals[1].l;
+        V.dirty = 0;
         S.status = checked_dev(eo);
-        if (fresh) adopt_density(S, eo);
-        S.density_at_x = 1;
       }
       __syncthreads();
       if (S.status) FAIL(S.status)
     }
 
-    // Phase 3: the dynamic Nesterov step (global_placement.rs:152-335)
+    // Phase 2: the dynamic Nesterov step (global_placement.rs:152-335)
     for (;;) {  // 'step
       T0 {
         if (V.restart) {
@@ -1155,30 +1442,28 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
           V.y_is_origin = 1;
         }
         if (!isfinite(V.next_m)) S.status = TEXO_GP_ERR_ITERATION_OVERFLOW;
+        V.f_y = eo.value;
+        V.y_stat = eo.kkt;
       }
       __syncthreads();
       if (S.status) FAIL(S.status)
-      if (V.y_is_origin) {
-        T0 {
-          V.f_y = eo.value;
-          V.y_stat = eo.kkt;
-        }
-        __syncthreads();
-      } else {
-        if (!c.density_and_wa(c.Y(), S.gamma, false)) LEAVE
-        if (!c.gradient(c.Y(), c.gY(), ey)) LEAVE
-        T0 {
-          S.density_at_x = 0;
-          S.status = checked_dev(ey);
+      if (!V.y_is_origin) {
+        if (!c.density_and_wa(c.Y(), S.gamma, fresh ? nullptr : c.X(), fresh ? nullptr : c.gX())) LEAVE
+        if (!c.gradient(c.Y(), c.gY(), ey, fresh ? nullptr : &eo)) LEAVE
+      }
+      T0 {
+        if (!V.y_is_origin) {
+          if (!fresh) S.status = checked_dev(eo);   // the origin's own check, folded with y's
+          if (!S.status) {
+            S.density_at_x = 0;
+            S.status = checked_dev(ey);
+          }
           V.f_y = ey.value;
           V.y_stat = ey.kkt;
         }
-        __syncthreads();
-        if (S.status) FAIL(S.status)
-      }
-      T0 {
         V.action = ACT_NONE;
-        if (!isfinite(V.y_stat)) {
+        if (S.status) {
+        } else if (!isfinite(V.y_stat)) {
           S.status = TEXO_GP_ERR_LINE_SEARCH_OVERFLOW;
         } else if (V.y_stat == 0.0) {
           V.action = V.y_is_origin ? ACT_STATIONARY : ACT_RESTART;
@@ -1207,30 +1492,37 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
               V.may_reduce = 0;
               if (!isfinite(V.tL)) S.status = TEXO_GP_ERR_LINE_SEARCH_OVERFLOW;
               V.action = ACT_CONTINUE;
+            } else {
+              // 1/L saturates at FLT_MAX: a huge step clamps to the box as it
+              // does in FP64, where an infinite one would turn 0 * inf into NaN
+              V.inv_L = (float)fmin(1.0 / V.tL, 3.0e38);
             }
           }
           __syncthreads();
           if (S.status) FAIL(S.status)
           if (V.action == ACT_CONTINUE) continue;
-          // 1/L saturates at FLT_MAX: a huge step clamps to the box as it
-          // does in FP64, where an infinite one would turn 0 * inf into NaN
-          const float invL = (float)fmin(1.0 / V.tL, 3.0e38);
-          if (c.in_a()) VLOOP c.candidate(ybuf, gy, invL, c.C(), v);
-          if (SETS == 1 || !c.in_a()) VLOOP c.init(v, true, false);
+          if (V.dirty) {   // a rejected scatter is in the grids
+            VLOOP c.reset_grids(v);
+            SYNC_OR_EXIT(PC_EXTRAP)
+          }
+          if (c.in_a()) VLOOP c.candidate(ybuf, gy, V.inv_L, c.C(), v);
           SYNC_OR_EXIT(PC_CANDIDATE)
           {
             const Partials q = c.set();
-            c.fold(3, [&](int j) {
+            c.fold(3 + d.K, [&](int j) {
               return j == 0   ? FoldJob{islot(q, IS_DIFF), FOLD_ISUM}
                      : j == 1 ? FoldJob{pslot(q, SLOT_DOT), FOLD_DSUM}
-                              : FoldJob{pslot(q, SLOT_MSN), FOLD_DSUM};
+                     : j == 2 ? FoldJob{pslot(q, SLOT_MSN), FOLD_DSUM}
+                              : c.sum_job(j - 3);
             });
             ++c.ws;
           }
-          const long long changed = c.fv[0].l;
-          const double dot = c.fv[1].d, msn = c.fv[2].d;
+          const long long changed = fvals[0].l;
+          const double dot = fvals[1].d, msn = fvals[2].d;
+          if ((int)threadIdx.x >= 64 && (int)threadIdx.x < 64 + d.K) c.set_mean(threadIdx.x - 64, fvals[3 + threadIdx.x - 64].l);
           T0 {
             V.action = ACT_NONE;
+            V.dirty = changed == 0;
             if (changed == 0) {
               const double smaller = half_nonzero_dev(V.tL);
               if (V.may_reduce && smaller < V.tL) {
@@ -1251,9 +1543,8 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
           __syncthreads();
           if (V.action == ACT_CONTINUE) continue;
           if (V.action != ACT_NONE) break;
-          VLOOP c.scatter(c.C(), v);
-          if (!c.density_and_wa(c.C(), S.gamma, true)) LEAVE
-          if (!c.gradient(c.C(), c.gC(), ec)) LEAVE
+          if (!c.density_and_wa(c.C(), S.gamma, nullptr, nullptr)) LEAVE
+          if (!c.gradient(c.C(), c.gC(), ec, nullptr)) LEAVE
           T0 {
             S.density_at_x = 0;
             S.status = checked_dev(ec);
@@ -1283,7 +1574,8 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
         }
       }
       if (V.action == ACT_RESTART) continue;
-      // leave the step: accepted or numerically stationary
+      // leave the step: accepted or numerically stationary; then the
+      // checkpoint and the stop rules (eplace.rs:550-573)
       T0 {
         S.trials += V.trials;
         if (V.action == ACT_ACCEPT) {
@@ -1307,28 +1599,23 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
           V.pending_prev = 1;
           V.stationary = 1;
         }
+        double mx, tot;
+        excess_dev(S, S.cur_overflow, mx, tot);
+        if (mx < S.best_max || (mx == S.best_max && tot < S.best_tot)) {
+          S.best_max = mx;
+          S.best_tot = tot;
+          V.pending_best = 1;
+        }
+        if (stop_dev(S, S.cur_overflow)) {
+          S.converged = 1;
+          S.phase = 2;
+        } else if (!V.stationary) {
+          S.have_prev_stationary = 0;
+        }
       }
       __syncthreads();
       break;
     }
-
-    // Phase 4: checkpoint, stop rules, multipliers (eplace.rs:550-573)
-    T0 {
-      double mx, tot;
-      excess_dev(S, S.cur_overflow, mx, tot);
-      if (mx < S.best_max || (mx == S.best_max && tot < S.best_tot)) {
-        S.best_max = mx;
-        S.best_tot = tot;
-        V.pending_best = 1;
-      }
-      if (stop_dev(S, S.cur_overflow)) {
-        S.converged = 1;
-        S.phase = 2;
-      } else if (!V.stationary) {
-        S.have_prev_stationary = 0;
-      }
-    }
-    __syncthreads();
     if (S.phase == 2) break;
     if (V.stationary) {
       // stationary_target_is_fixed (eplace.rs:973-985): compare rounded targets
@@ -1346,6 +1633,7 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
         }
         write_partial(g, mism, islot(c.set(), IS_DIFF), v, sh.a.l);
       }
+      if (V.dirty) VLOOP c.reset_grids(v);   // the next iteration scatters at once
       SYNC_OR_EXIT(PC_OTHER)
       const Partials q = c.set();
       c.fold(1, [&](int) { return FoldJob{islot(q, IS_DIFF), FOLD_ISUM}; });
@@ -1354,6 +1642,7 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
       T0 {
         const bool fixed = S.have_prev_stationary && total == 0;
         S.have_prev_stationary = 1;
+        V.dirty = 0;
         if (fixed) {
           S.exhausted = 1;
           S.phase = 2;
@@ -1363,15 +1652,6 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
       __syncthreads();
       if (S.phase == 2) break;
     }
-    T0 {
-      const int st = update_multipliers_dev(S);
-      if (st) {
-        S.status = st;
-        S.phase = 2;
-      }
-    }
-    __syncthreads();
-    if (S.phase == 2) break;
   }
 
 out:

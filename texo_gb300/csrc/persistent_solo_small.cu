@@ -6,9 +6,12 @@ namespace tgp {
 
 __global__ void __launch_bounds__(2 * kThreads, kBlocksPerSm)
     k_persistent_small(Dev d, Reduce r, Buffers B, DevRun* run, GridBarrier* bar, int V) {
-  run_body<false, 2>(d, r, B, run, bar, (int)blockIdx.x, (int)gridDim.x, V);
+  extern __shared__ __align__(16) unsigned char resident[];
+  run_body<false, 2>(d, r, B, run, bar, (int)blockIdx.x, (int)gridDim.x, V,
+                     reinterpret_cast<Resident*>(resident));
 }
 
+size_t persistent_shared() { return sizeof(Resident); }
 const void* persistent_kernel_small() { return (const void*)k_persistent_small; }
 
 }  // namespace tgp

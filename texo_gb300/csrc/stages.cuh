@@ -165,6 +165,20 @@ __device__ __forceinline__ Deposit deposit_of(const Dev& d, const float2* pos, i
   }
   return t;
 }
+// The nine taps of one charge into its grid; their fixed-point sum.
+__device__ __forceinline__ long long deposit_taps(const Dev& d, unsigned long long* grid, float q, const AxisTaps& ax,
+                                                  const AxisTaps& ay) {
+  long long s = 0;
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const long long v = tap_fixed(q, ax.w[c], ay.w[r]);
+      s += v;
+      atomicAdd(grid + (size_t)ay.idx[r] * d.g.Wb + ax.idx[c], (unsigned long long)v);
+    }
+  return s;
+}
 // Objects first, first + stride, ...: the tap totals per field in tot. Two
 // objects' loads are in flight before either's atomics (which the compiler
 // will not move loads across).
@@ -174,15 +188,7 @@ __device__ __forceinline__ void scatter_items(const Dev& d, const float2* pos, i
   for (int f = 0; f < kMaxFields; ++f) tot[f] = 0;
   const int items = d.Mm + d.F;
   auto put = [&](const Deposit& t, const AxisTaps& ax, const AxisTaps& ay) {
-    long long s = 0;
-#pragma unroll
-    for (int r = 0; r < 3; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const long long v = tap_fixed(t.q, ax.w[c], ay.w[r]);
-        s += v;
-        atomicAdd(t.grid + (size_t)ay.idx[r] * d.g.Wb + ax.idx[c], (unsigned long long)v);
-      }
+    const long long s = deposit_taps(d, t.grid, t.q, ax, ay);
 #pragma unroll
     for (int ff = 0; ff < kMaxFields; ++ff)
       if (ff == t.f) tot[ff] += s;
@@ -692,9 +698,7 @@ static __device__ void stage_prep_dct0(const G& g, const Dev& d, const long long
 // filler loops, electrostatic_placement.rs:338-374, 919-941): raw per-field
 // gradient q * dphi per optimizer object, and force_l1 partials.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 sample_grad(const Dev& d, const float* phi, float sxp, float syp) {
-  const AxisTaps ax = taps_x(d, sxp);
-  const AxisTaps ay = taps_y(d, syp);
+__device__ __forceinline__ float2 sample_grad(const Dev& d, const float* phi, const AxisTaps& ax, const AxisTaps& ay) {
   const float dx[3] = {ax.o - 0.5f, -2.f * ax.o, ax.o + 0.5f};
   const float dy[3] = {ay.o - 0.5f, -2.f * ay.o, ay.o + 0.5f};
   // The derivative weights of each axis sum to zero, so the centre tap's
@@ -735,7 +739,8 @@ static __device__ void stage_gather(const G& g, const Dev& d, const float2* pos,
         const int f = d.mem_field[m];
         const float2 off = d.mem_off[m];
         const float q = d.mem_q[m];
-        const float2 gr = sample_grad(d, d.phi + (size_t)f * d.B, __fadd_rn(pu.x, off.x), __fadd_rn(pu.y, off.y));
+        const float2 gr = sample_grad(d, d.phi + (size_t)f * d.B, taps_x(d, __fadd_rn(pu.x, off.x)),
+                                      taps_y(d, __fadd_rn(pu.y, off.y)));
 #pragma unroll
         for (int ff = 0; ff < kMaxFields; ++ff)
           if (ff == f) {
@@ -750,7 +755,7 @@ static __device__ void stage_gather(const G& g, const Dev& d, const float2* pos,
       const int f = d.fil_field[j];
       const float q = d.fil_q[j];
       const float2 pf = pos[o];
-      const float2 gr = sample_grad(d, d.phi + (size_t)f * d.B, pf.x, pf.y);
+      const float2 gr = sample_grad(d, d.phi + (size_t)f * d.B, taps_x(d, pf.x), taps_y(d, pf.y));
       d.graw[(size_t)f * d.nobj + o] = make_float2(q * gr.x, q * gr.y);
 #pragma unroll
       for (int ff = 0; ff < kMaxFields; ++ff)
