@@ -127,6 +127,7 @@ __device__ __forceinline__ Axis stage_tables(const G& g, const Axis& a, float4* 
   float2* inv_s = reinterpret_cast<float2*>(pre + a.n);
   if (!there) {
     g.sync();   // earlier readers of the buffer are done
+#pragma unroll 1
     for (int i = g.tid; i < a.n; i += kThreads) {
       if (i < (a.n >> 1)) tw[i] = a.tw[i];
       post[i] = a.post[i];
@@ -250,6 +251,7 @@ __device__ __forceinline__ void exchange(const G& g, const Place<NB>& at, int s,
 template <int NB, class G>
 __device__ __forceinline__ void stages(const G& g, const Place<NB>& at, int from, Pair (&x)[NB], const Axis& a,
                                        float4* exch) {
+#pragma unroll 1
   for (int s = from; s < at.L; ++s) {
     exchange(g, at, s, x, exch);
 #pragma unroll
@@ -353,7 +355,7 @@ __device__ __forceinline__ float2* stage_out(float4* buf) {
 // the physical overflow is counted into the IS_OVERFLOW / IS_OVER_BINS
 // partials.
 template <int NB, class G>
-static __device__ __forceinline__ void rows_fwd(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
+static __device__ __noinline__ void rows_fwd(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
                                                 Shared& sh, const long long* mean, bool tables) {
   const int W = d.g.Wb, H = d.g.Hb, L = d.logW, GV = min(group_size(L), H), per = GV << L;
   const int gpf = (H + GV - 1) / GV, groups = gpf * d.K;
@@ -364,6 +366,7 @@ static __device__ __forceinline__ void rows_fwd(const G& g, const Dev& d, Partia
   long long ov[kMaxFields], cnt[kMaxFields];
 #pragma unroll
   for (int f = 0; f < kMaxFields; ++f) ov[f] = cnt[f] = 0;
+#pragma unroll 1
   for (int t = vb; t < groups; t += nvb) {
     const int f = t / gpf, y0 = (t % gpf) * GV;
     const size_t base = (size_t)f * d.B + (size_t)y0 * W;
@@ -428,7 +431,7 @@ static __device__ __forceinline__ void rows_fwd(const G& g, const Dev& d, Partia
 // Pass 2: t2 = cols-IDCT(cols-DCT(t1) * inv_eig), whole columns per group;
 // the scaled coefficients stay double-floats between the two transforms.
 template <int NB, class G>
-static __device__ __forceinline__ void cols(const G& g, const Dev& d, int vb, int nvb, float4* buf, bool tables) {
+static __device__ __noinline__ void cols(const G& g, const Dev& d, int vb, int nvb, float4* buf, bool tables) {
   const int W = d.g.Wb, H = d.g.Hb, L = d.logH, GV = min(group_size(L), W), per = GV << L;
   const int gpf = (W + GV - 1) / GV, groups = gpf * d.K;
   const Axis a = vb < groups ? stage_tables(g, axis_y(d), buf, tables) : axis_y(d);
@@ -436,6 +439,7 @@ static __device__ __forceinline__ void cols(const G& g, const Dev& d, int vb, in
   const int stride = pad_k(H), logG = 31 - __clz(GV);
   float2 *in = stage_in<NB>(buf), *mid = stage_out<NB>(buf);
   const float inv_n = 1.0f / (float)H;
+#pragma unroll 1
   for (int t = vb; t < groups; t += nvb) {
     const int f = t / gpf, x0 = (t % gpf) * GV;
     const size_t base = (size_t)f * d.B + x0;
@@ -490,7 +494,7 @@ static __device__ __forceinline__ void cols(const G& g, const Dev& d, int vb, in
 
 // Pass 3: phi = rows-IDCT(t2) and the energy partials <rho, phi>.
 template <int NB, class G>
-static __device__ __forceinline__ void rows_inv(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
+static __device__ __noinline__ void rows_inv(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
                                                 Shared& sh, bool tables) {
   const int W = d.g.Wb, H = d.g.Hb, L = d.logW, GV = min(group_size(L), H), per = GV << L;
   const int gpf = (H + GV - 1) / GV, groups = gpf * d.K;
@@ -501,6 +505,7 @@ static __device__ __forceinline__ void rows_inv(const G& g, const Dev& d, Partia
   float* out = reinterpret_cast<float*>(stage_out<NB>(buf));
   const float inv_n = 1.0f / (float)W;
   double eacc[kMaxFields] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 1
   for (int t = vb; t < groups; t += nvb) {
     const int f = t / gpf, y0 = (t % gpf) * GV;
     const size_t base = (size_t)f * d.B + (size_t)y0 * W;

@@ -49,12 +49,15 @@ static bool large_tiles(const Dev& d) { return d.dct_large != 0; }
 int32_t enqueue_persistent(const Dev& d, const Reduce& r, const Buffers& b, RunBlock* dev, RunBlock* host,
                            int blocks, int V, cudaStream_t s) {
   if (cudaMemcpyAsync(dev, host, sizeof(RunBlock), cudaMemcpyHostToDevice, s) != cudaSuccess) return TEXO_GP_ERR_CUDA;
-  Dev dd = d;
-  Reduce rr = r;
-  Buffers bb = b;
-  DevRun* run = &dev->run;
-  GridBarrier* bar = &dev->bar;
-  void* args[] = {&dd, &rr, &bb, &run, &bar, &V};
+  InstDesc desc;
+  desc.d = d;
+  desc.r = r;
+  desc.B = b;
+  desc.run = &dev->run;
+  desc.bar = &dev->bar;
+  desc.V = V;
+  desc.pad = 0;
+  void* args[] = {&desc};
   const void* fn = large_tiles(d) ? persistent_kernel_large() : persistent_kernel_small();
   if (!raise_shared_limit()) return TEXO_GP_ERR_CUDA;
   if (cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(2 * kThreads), args, persistent_shared(), s) != cudaSuccess) return TEXO_GP_ERR_CUDA;

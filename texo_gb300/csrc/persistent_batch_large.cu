@@ -5,11 +5,10 @@
 namespace tgp {
 
 __global__ void __launch_bounds__(kThreads, kBatchBlocksPerSm) k_batch_large(const InstDesc* descs, const int4* map) {
-  __shared__ InstDesc sd;
   const int4 m = map[blockIdx.x];
-  copy_words(&sd, descs + m.x);
+  copy_words(&loop_state<1>().inst, descs + m.x);
   __syncthreads();
-  run_body<true, 1>(sd.d, sd.r, sd.B, sd.run, sd.bar, m.y, m.z, sd.V, nullptr);
+  run_body<true, 1>(m.y, m.z, nullptr);
 }
 
 const void* batch_kernel_large() { return (const void*)k_batch_large; }

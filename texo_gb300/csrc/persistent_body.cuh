@@ -173,16 +173,24 @@ template <typename T, typename Op>
 __device__ __forceinline__ T warp_fold(const T* a, int n, T init, Op op) {
   return fold_loaded(fold_load(a, n), a, n, init, op);
 }
-__device__ __forceinline__ FoldValue fold_job(const FoldAhead& f, const FoldJob& jb, int n) {
+// One copy for all folds (the values in registers).
+static __device__ __noinline__ FoldValue fold_values(unsigned long long v0, unsigned long long v1,
+                                                     unsigned long long v2, unsigned long long v3,
+                                                     unsigned long long v4, const void* a, int op, int n) {
+  const FoldAhead f{{v0, v1, v2, v3, v4}};
   FoldValue out;
-  switch (jb.op) {
-    case FOLD_DSUM: out.d = fold_loaded(f, (const double*)jb.a, n, 0.0, OpAdd()); break;
-    case FOLD_ISUM: out.l = fold_loaded(f, (const long long*)jb.a, n, 0ll, OpAdd()); break;
-    case FOLD_IMIN: out.l = fold_loaded(f, (const long long*)jb.a, n, 0x7fffffffffffffffll, OpMin()); break;
-    case FOLD_DMAX: out.d = fold_loaded(f, (const double*)jb.a, n, 0.0, OpMax()); break;
-    default: out.d = fold_loaded(f, (const double*)jb.a, n, (double)INFINITY, OpMin()); break;
+  switch (op) {
+    case FOLD_DSUM: out.d = fold_loaded(f, (const double*)a, n, 0.0, OpAdd()); break;
+    case FOLD_ISUM: out.l = fold_loaded(f, (const long long*)a, n, 0ll, OpAdd()); break;
+    case FOLD_IMIN: out.l = fold_loaded(f, (const long long*)a, n, 0x7fffffffffffffffll, OpMin()); break;
+    case FOLD_DMAX: out.d = fold_loaded(f, (const double*)a, n, 0.0, OpMax()); break;
+    default: out.d = fold_loaded(f, (const double*)a, n, (double)INFINITY, OpMin()); break;
   }
   return out;
+}
+__device__ __forceinline__ FoldValue fold_ahead(const FoldAhead& f, const FoldJob& jb, int n) {
+  static_assert(kFoldAhead == 5, "one argument a value");
+  return fold_values(f.v[0], f.v[1], f.v[2], f.v[3], f.v[4], jb.a, jb.op, n);
 }
 
 // Block-level scratch of the loop's own reductions.
@@ -208,35 +216,88 @@ struct Resident {
 };
 constexpr int kNoMember = -1, kManyMembers = -2;
 
+// Shared-memory step bookkeeping that every thread reads after a barrier.
+struct StepVars {
+  int restart, y_is_origin, may_reduce, has_wL, action, stationary, fresh, deposited, dirty;
+  double wL, tL, f_y, y_stat, next_m, pmin, pmax;
+  double gamma, growth;                       // of the next iteration
+  int st_multipliers, st_growth, st_gamma;
+  unsigned ws;                                // phases that wrote an alternating partial set
+  float extrapolation, lambda[kMaxFields], inv_L;
+  unsigned trials;
+  int pending_best, pending_prev;
+};
+// Everything a block's phases read, in its shared memory: the phases are
+// functions of their own (inlined wherever they are called the loop was two
+// megabytes of code, and its phases, each run once between two grid barriers,
+// were bound by instruction fetches), and what they would otherwise pass on
+// the stack would be an L2 trip behind every grid barrier, which leaves L1
+// cold.
+template <int SETS>
+struct LoopState {
+  InstDesc inst;
+  DevRun S;            // written by thread 0
+  ERec eo, ey, ec;     // the origin's, the extrapolated point's and the candidate's evaluation
+  StepVars V;
+  GemmShared gsm;
+  LoopShared<SETS> sh;
+  double coef[kMaxFields];
+  float coef32[kMaxFields];
+  FoldValue fv[kMaxFoldJobs];        // results of the folds after a barrier
+  long long fmean[kMaxFields];       // fixed-point density means
+  long long capsum[kMaxFields];      // copy of d.capsum
+  unsigned long long nbar, clock[10];   // clock: [8] phase accumulators, [8] last mark, [9] barrier wait
+  Resident* res;                     // null: nothing is resident
+  const float2 *mapx, *mapy;         // tile-to-bin maps (resident, or d's)
+  unsigned gen;
+  int gen_failed;                    // the barrier's error word as thread 0 last read it
+  int pb, np;                        // physical block of the instance, physical block count
+  int tables;                        // the FFT tables stay in the work buffer
+};
+template <int SETS>
+__device__ __forceinline__ LoopState<SETS>& loop_state() {
+  __shared__ LoopState<SETS> state;
+  return state;
+}
+
+template <bool LARGE, int SETS>
+struct Ctx;
+// The phases out of line, one copy each.
+#define OUTLINED(type, name) template <bool LARGE, int SETS> static __device__ __noinline__ type name
+OUTLINED(bool, run_sync)();
+OUTLINED(void, run_wa)(const float2* pos, double gam);
+OUTLINED(void, run_scatter)(const float2* pos);
+OUTLINED(void, run_combine_kept)(const float2* pos, float2* g);
+OUTLINED(bool, run_transform_first)();
+OUTLINED(bool, run_transform_rest)();
+OUTLINED(bool, run_density_and_wa)(const float2* pos, double gam, const float2* origin, float2* origin_g);
+OUTLINED(bool, run_gradient)(const float2* pos, float2* g, ERec* out, ERec* origin);
+OUTLINED(bool, run_eval_initial)(const float2* pos, float2* g, double gam, bool full);
+OUTLINED(void, run_precondition)(bool deposits);
+OUTLINED(void, run_candidate)(const float2* y, const float2* gy, float2* c);
+
 template <bool LARGE, int SETS>
 struct Ctx {
   static constexpr int kBlock = SETS * kThreads;
   static constexpr int kWarps = kBlock / 32;
   using GA = Group<SETS == 2 ? 1 : 0>;
   using GB = Group<SETS == 2 ? 2 : 0>;
+  LoopState<SETS>& L;
   const Dev& d;
   const Reduce& r;
   const Buffers& B;
-  DevRun& S;          // shared memory, written by thread 0
-  GridBarrier* bar;
-  unsigned* gen;
-  int* gen_failed;     // shared: the barrier's error word as thread 0 last read it
+  DevRun& S;
   GemmShared& gsm;
   LoopShared<SETS>& sh;
-  Resident* res;      // null: nothing is resident
-  const float2 *mapx, *mapy;   // tile-to-bin maps (resident, or d's)
-  double* coef;       // shared [kMaxFields]
-  float* coef32;      // shared [kMaxFields]
-  FoldValue* fv;      // shared [kMaxFoldJobs] results of fold()
-  long long* fmean;   // shared [kMaxFields] fixed-point density means
-  const long long* capsum;     // shared [kMaxFields] copy of d.capsum
-  int pb, np;         // physical block of the instance, physical block count
+  FoldValue* fv;
+  Resident* res;
+  const float2 *mapx, *mapy;
+  int pb, np;
   int V;              // virtual blocks of the instance
-  unsigned long long nbar;
-  unsigned long long* clock;   // shared [8] phase accumulators, [8] last mark, [9] barrier wait
-  bool tables;                 // the FFT tables stay in the work buffer
 
-  unsigned ws = 0;             // phases that wrote an alternating partial set, counted by every thread
+  __device__ __forceinline__ explicit Ctx(LoopState<SETS>& l)
+      : L(l), d(l.inst.d), r(l.inst.r), B(l.inst.B), S(l.S), gsm(l.gsm), sh(l.sh), fv(l.fv), res(l.res), mapx(l.mapx),
+        mapy(l.mapy), pb(l.pb), np(l.np), V(l.inst.V) {}
 
   __device__ bool in_a() const { return SETS == 1 || threadIdx.x < kThreads; }
   __device__ bool in_b() const { return SETS == 1 || threadIdx.x >= kThreads; }
@@ -245,16 +306,17 @@ struct Ctx {
 
   __device__ void meet() {   // thread 0's part of a grid barrier
     const unsigned long long t0 = pb == 0 ? now_ns() : 0ull;
-    *gen_failed = !grid_arrive_wait(bar, (unsigned)np, gen, kSpinLimit);
-    ++nbar;
-    if (pb == 0) clock[9] += now_ns() - t0;
+    L.gen_failed = !grid_arrive_wait(L.inst.bar, (unsigned)np, &L.gen, kSpinLimit);
+    ++L.nbar;
+    if (pb == 0) L.clock[9] += now_ns() - t0;
   }
   // Grid barrier, every thread of the block.
-  __device__ bool sync() {
+  __device__ __forceinline__ bool sync() { return run_sync<LARGE, SETS>(); }
+  __device__ __forceinline__ bool sync_body() {
     __syncthreads();
     if (threadIdx.x == 0) meet();
     __syncthreads();
-    return *gen_failed == 0;   // one read of the error word per block, so all its threads agree
+    return L.gen_failed == 0;   // one read of the error word per block, so all its threads agree
   }
   // Grid barrier of half A alone, while half B works on. It orders what the
   // whole block wrote before its last block barrier, and half A since. After
@@ -264,22 +326,22 @@ struct Ctx {
     g.sync();
     if (threadIdx.x == 0) meet();
     g.sync();
-    return *gen_failed == 0;
+    return L.gen_failed == 0;
   }
   // Partials of phases that may follow one another directly (extrapolation,
-  // candidates, stationary check) alternate between two sets: a block that
-  // leaves a barrier early and writes the next phase's partials must not
-  // overwrite the ones a slower block of the instance is still reducing.
-  // Every other slot is written again only after a barrier that its readers
-  // have reached.
-  __device__ Partials set() const { return (ws & 1u) ? r.q : r.p; }
+  // candidates, stationary check) alternate between two sets (V.ws counts
+  // them): a block that leaves a barrier early and writes the next phase's
+  // partials must not overwrite the ones a slower block of the instance is
+  // still reducing. Every other slot is written again only after a barrier
+  // that its readers have reached.
+  __device__ Partials set() const { return (L.V.ws & 1u) ? r.q : r.p; }
 
   // Charges the time since the previous mark to phase category `cat` (block 0).
   __device__ void mark(int cat) {
     if (pb == 0 && threadIdx.x == 0) {
       const unsigned long long t = now_ns();
-      clock[cat] += t - clock[8];
-      clock[8] = t;
+      L.clock[cat] += t - L.clock[8];
+      L.clock[8] = t;
     }
   }
   // Several reductions of partials at once, right after a grid barrier: job j
@@ -289,10 +351,11 @@ struct Ctx {
   // different SM sub-partitions. Every thread reads the results in fv after
   // the final block barrier.
   template <class Job>
-  __device__ void fold(int n, Job job) {
+  __device__ __forceinline__ void fold(int n, Job job) {
+#pragma unroll 1
     for (int j = threadIdx.x >> 5; j < n; j += kWarps) {
       const FoldJob jb = job(j);
-      const FoldValue out = fold_job(fold_load(jb.a, V), jb, V);
+      const FoldValue out = fold_ahead(fold_load(jb.a, V), jb, V);
       if ((threadIdx.x & 31) == 0) fv[j] = out;
     }
     __syncthreads();
@@ -321,9 +384,15 @@ struct Ctx {
     return resident(j) ? res->mem[j] : member_from_memory(o);
   }
   __device__ __forceinline__ float4 member_from_memory(int o) const {
+    // a filler deposits at its position itself (a zero offset changes no bit
+    // of the taps: an offset of +0 leaves every coordinate but -0 as it is,
+    // and the axis clamps -0 like +0)
     if (o >= d.U) return make_float4(0.f, 0.f, d.fil_q[o - d.U], __int_as_float(d.fil_field[o - d.U]));
     const int m = d.unit_mem_ptr[o], n = d.unit_mem_ptr[o + 1] - m;
     if (n != 1) return make_float4(0.f, 0.f, 0.f, __int_as_float(n == 0 ? kNoMember : kManyMembers));
+    return member_at(m);
+  }
+  __device__ __forceinline__ float4 member_at(int m) const {
     const float2 off = d.mem_off[m];
     return make_float4(off.x, off.y, d.mem_q[m], __int_as_float(d.mem_field[m]));
   }
@@ -370,24 +439,27 @@ struct Ctx {
   }
 
   // Scatters object o at p, into the totals per field.
-  __device__ __forceinline__ void deposit(const float4& m, int o, float2 p, long long (&tot)[kMaxFields]) {
-    const int f = __float_as_int(m.w);
-    auto put = [&](float x, float y, float q, int field, long long* grids) {
-      const long long s = deposit_taps(d, (unsigned long long*)(grids + (size_t)field * d.B), q, tx(x), ty(y));
+  __device__ __forceinline__ void deposit(float4 m, int o, float2 p, long long (&tot)[kMaxFields]) {
+    int f = __float_as_int(m.w);
+    if (f == kNoMember) return;
+    int i = 0, left = 1;
+    if (f == kManyMembers) {
+      i = d.unit_mem_ptr[o];
+      left = d.unit_mem_ptr[o + 1] - i;
+      m = member_at(i);
+      f = __float_as_int(m.w);
+    }
+    long long* const grids = o < d.U ? d.phys : d.fill;
+#pragma unroll 1
+    for (;;) {
+      const long long s = deposit_taps(d, (unsigned long long*)(grids + (size_t)f * d.B), m.z, tx(__fadd_rn(p.x, m.x)),
+                                       ty(__fadd_rn(p.y, m.y)));
 #pragma unroll
       for (int ff = 0; ff < kMaxFields; ++ff)
-        if (ff == field) tot[ff] += s;
-    };
-    if (f >= 0) {
-      if (o < d.U)
-        put(__fadd_rn(p.x, m.x), __fadd_rn(p.y, m.y), m.z, f, d.phys);
-      else
-        put(p.x, p.y, m.z, f, d.fill);
-    } else if (f == kManyMembers) {
-      for (int i = d.unit_mem_ptr[o], e = d.unit_mem_ptr[o + 1]; i < e; ++i) {
-        const float2 off = d.mem_off[i];
-        put(__fadd_rn(p.x, off.x), __fadd_rn(p.y, off.y), d.mem_q[i], d.mem_field[i], d.phys);
-      }
+        if (ff == f) tot[ff] += s;
+      if (--left == 0) break;
+      m = member_at(++i);
+      f = __float_as_int(m.w);
     }
   }
   // half A: its warps' totals, then (after the group's barrier) partial v
@@ -450,58 +522,47 @@ struct Ctx {
   }
   // gathered at pos (sample_quadratic_bspline_with_gradient and the member and
   // filler loops, electrostatic_placement.rs:338-374, 919-941), and kept
-  __device__ __forceinline__ Raw gathered(const float2* pos, int j, int o) {
-    Raw a;
+  __device__ __forceinline__ void gathered(Raw& a, const float2* pos, int j, int o) {
 #pragma unroll
     for (int f = 0; f < kMaxFields; ++f) a.f[f] = make_float2(0.f, 0.f);
-    if (o >= d.nobj) return a;
+    if (o >= d.nobj) return;
     operands(a, o);
     a.at = resident(j) ? res->pos[j] : pos[o];
-    const float4 m = member(j, o);
-    const int f = __float_as_int(m.w);
-    auto add = [&](float x, float y, float q, int field) {
-      const float2 s = sample_grad(d, d.phi + (size_t)field * d.B, tx(x), ty(y));
-#pragma unroll
-      for (int ff = 0; ff < kMaxFields; ++ff)
-        if (ff == field) {
-          a.f[ff].x += q * s.x;
-          a.f[ff].y += q * s.y;
-        }
-    };
-    if (o >= d.U) {
-      const float2 s = sample_grad(d, d.phi + (size_t)f * d.B, tx(a.at.x), ty(a.at.y));
-      a.f[0] = make_float2(m.z * s.x, m.z * s.y);   // a filler's one field
-      d.graw[(size_t)f * d.nobj + o] = a.f[0];
-      return a;
+    float4 m = member(j, o);
+    int f = __float_as_int(m.w), i = 0, left = 1;
+    if (f == kManyMembers) {
+      i = d.unit_mem_ptr[o];
+      left = d.unit_mem_ptr[o + 1] - i;
+      m = member_at(i);
+      f = __float_as_int(m.w);
     }
-    if (f >= 0) {
-      add(__fadd_rn(a.at.x, m.x), __fadd_rn(a.at.y, m.y), m.z, f);
-    } else if (f == kManyMembers) {
-      for (int i = d.unit_mem_ptr[o], e = d.unit_mem_ptr[o + 1]; i < e; ++i) {
-        const float2 off = d.mem_off[i];
-        add(__fadd_rn(a.at.x, off.x), __fadd_rn(a.at.y, off.y), d.mem_q[i], d.mem_field[i]);
+    if (f != kNoMember) {
+#pragma unroll 1
+      for (;;) {
+        const float2 s = sample_grad(d, d.phi + (size_t)f * d.B, tx(__fadd_rn(a.at.x, m.x)), ty(__fadd_rn(a.at.y, m.y)));
+#pragma unroll
+        for (int ff = 0; ff < kMaxFields; ++ff)
+          if (ff == f) {
+            a.f[ff].x += m.z * s.x;
+            a.f[ff].y += m.z * s.y;
+          }
+        if (--left == 0) break;
+        m = member_at(++i);
+        f = __float_as_int(m.w);
       }
     }
 #pragma unroll
     for (int ff = 0; ff < kMaxFields; ++ff)
-      if (ff < d.K) d.graw[(size_t)ff * d.nobj + o] = a.f[ff];
-    return a;
+      if (ff < d.K && (o < d.U || ff == f)) d.graw[(size_t)ff * d.nobj + o] = a.f[ff];
   }
   // the ones kept from the last density evaluation
-  __device__ __forceinline__ Raw kept(const float2* pos, int o) {
-    Raw a;
+  __device__ __forceinline__ void kept(Raw& a, const float2* pos, int o) {
     operands(a, o);
     a.at = pos[o];
+    const int only = o < d.U || d.K == 1 ? -1 : d.fil_field[o - d.U];
 #pragma unroll
-    for (int f = 0; f < kMaxFields; ++f) a.f[f] = make_float2(0.f, 0.f);
-    if (o < d.U) {
-#pragma unroll
-      for (int f = 0; f < kMaxFields; ++f)
-        if (f < d.K) a.f[f] = d.graw[(size_t)f * d.nobj + o];
-    } else {
-      a.f[0] = d.graw[(size_t)d.fil_field[o - d.U] * d.nobj + o];
-    }
-    return a;
+    for (int f = 0; f < kMaxFields; ++f)
+      a.f[f] = f < d.K && (only < 0 || only == f) ? d.graw[(size_t)f * d.nobj + o] : make_float2(0.f, 0.f);
   }
   // The combined gradient of an object (combined_objective, eplace.rs:1022-
   // 1044); the WA accumulators it has read are cleared for the next evaluation.
@@ -514,18 +575,15 @@ struct Ctx {
       reinterpret_cast<ulonglong2*>(d.wa_fix)[o] = make_ulonglong2(0ull, 0ull);
       gx = __ll2float_rn((long long)a.wa.x) * kInvFixF;
       gy = __ll2float_rn((long long)a.wa.y) * kInvFixF;
-#pragma unroll
-      for (int f = 0; f < kMaxFields; ++f)
-        if (f < d.K) {
-          const float c = coef32[f];
-          gx = fmaf(c, a.f[f].x, gx);
-          gy = fmaf(c, a.f[f].y, gy);
-        }
-    } else {
-      const float c = coef32[d.K == 1 ? 0 : d.fil_field[o - d.U]];
-      gx = c * a.f[0].x;
-      gy = c * a.f[0].y;
     }
+    // a filler has one field: the others' gradients are zero and add nothing
+#pragma unroll
+    for (int f = 0; f < kMaxFields; ++f)
+      if (f < d.K) {
+        const float c = L.coef32[f];
+        gx = fmaf(c, a.f[f].x, gx);
+        gy = fmaf(c, a.f[f].y, gy);
+      }
     if (!isfinite(gx)) bad = min(bad, 2u * (unsigned)o);
     else if (!isfinite(gy)) bad = min(bad, 2u * (unsigned)o + 1u);
     g[o] = make_float2(gx, gy);
@@ -558,12 +616,17 @@ struct Ctx {
     const GB gb = half_b();
     float kkt = 0.f;
     unsigned bad = 0xffffffffu;
-    for (int j = gb.tid, o; (o = object(v, j)) < d.nobj; j += 2 * kThreads) {   // two objects' loads in flight
+    Raw a, b;
+    int j = gb.tid, o = object(v, j);
+    if (o < d.nobj) kept(a, pos, o);
+#pragma unroll 1
+    while (o < d.nobj) {   // the next object's loads in flight
       const int o2 = object(v, j + kThreads);
-      const bool two = o2 < d.nobj;
-      const Raw a = kept(pos, o), b = two ? kept(pos, o2) : a;
+      if (o2 < d.nobj) kept(b, pos, o2);
       combine(a, j, o, g, kkt, bad);
-      if (two) combine(b, j + kThreads, o2, g, kkt, bad);
+      a = b;
+      o = o2;
+      j += kThreads;
     }
     gb.sync();   // earlier readers of the scratch are done
     stage_kkt_warp(kkt, bad, sh.x[0], sh.x[1], gb.tid >> 5);
@@ -577,9 +640,9 @@ struct Ctx {
   // fixed-point density mean (DC mode) of field f, from its folded grid sum;
   // truncated division, a shift for the power-of-two grids
   __device__ void set_mean(int f, long long sum) {
-    const long long t = sum - capsum[f];
+    const long long t = sum - L.capsum[f];
     const int B_ = d.B;
-    fmean[f] = (B_ & (B_ - 1)) == 0 ? (t + (long long)((unsigned long long)(t >> 63) & (unsigned long long)(B_ - 1))) >> (31 - __clz(B_))
+    L.fmean[f] = (B_ & (B_ - 1)) == 0 ? (t + (long long)((unsigned long long)(t >> 63) & (unsigned long long)(B_ - 1))) >> (31 - __clz(B_))
                                     : t / B_;
   }
   __device__ FoldJob sum_job(int f) const { return FoldJob{islot(r.p, IS_GRID_SUM + f), FOLD_ISUM}; }
@@ -591,14 +654,14 @@ struct Ctx {
     const GA g = half_a();
     if (d.fft) {
       for (int v = pb; v < V; v += np)
-        fft::pass_rows_fwd(g, d, r.p, v, V, *reinterpret_cast<fft::Smem*>(gsm.fft), sh.a, fmean, tables);
+        fft::pass_rows_fwd(g, d, r.p, v, V, *reinterpret_cast<fft::Smem*>(gsm.fft), sh.a, L.fmean, L.tables);
     } else if (LARGE) {
       for (int v = pb; v < V; v += np) stage_prep(g, d, r.p, V, v, V, sh.a);
       if (!sync_a(g)) return false;
       mark(PC_PREP);
       for (int v = pb; v < V; v += np) stage_dct_t<LARGE>(g, d, 0, r.p, v, V, gsm, sh.a);
     } else {
-      for (int v = pb; v < V; v += np) stage_prep_dct0(g, d, fmean, r.p, v, V, gsm, sh.a);
+      for (int v = pb; v < V; v += np) stage_prep_dct0(g, d, L.fmean, r.p, v, V, gsm, sh.a);
     }
     return true;
   }
@@ -606,9 +669,9 @@ struct Ctx {
     const GA g = half_a();
     if (d.fft) {
       fft::Smem& fs = *reinterpret_cast<fft::Smem*>(gsm.fft);
-      for (int v = pb; v < V; v += np) fft::pass_cols(g, d, v, V, fs, tables);
+      for (int v = pb; v < V; v += np) fft::pass_cols(g, d, v, V, fs, L.tables);
       if (!sync_a(g)) return false;
-      for (int v = pb; v < V; v += np) fft::pass_rows_inv(g, d, r.p, v, V, fs, sh.a, tables);
+      for (int v = pb; v < V; v += np) fft::pass_rows_inv(g, d, r.p, v, V, fs, sh.a, L.tables);
     } else {
       for (int st = 1; st < 4; ++st) {
         for (int v = pb; v < V; v += np) stage_dct_t<LARGE>(g, d, st, r.p, v, V, gsm, sh.a);
@@ -632,8 +695,8 @@ struct Ctx {
   __device__ void eval_coefficients(bool full, int at = 0) {
     for (int f = 0; f < d.K; ++f) {
       const double ne = (full ? 0.5 * fv[at + 3 * f].d : S.cur_energy[f]) * S.inv_e0[f];
-      coef[f] = S.lambda[f] * (1.0 + S.beta * ne);
-      coef32[f] = (float)coef[f];
+      L.coef[f] = S.lambda[f] * (1.0 + S.beta * ne);
+      L.coef32[f] = (float)L.coef[f];
     }
   }
   // one thread: the objective
@@ -665,18 +728,17 @@ struct Ctx {
   // combined_objective, eplace.rs:137-205, 1022-1044).
   __device__ bool eval_initial(const float2* pos, float2* g, double gam, bool full, ERec& out) {
     if (full) {
-      if (in_a())
-        for (int v = pb; v < V; v += np) scatter(pos, v);
+      if (in_a()) run_scatter<LARGE, SETS>(pos);
       if (!sync()) return false;
       fold(d.K, [&](int j) { return sum_job(j); });
       if ((int)threadIdx.x < d.K) set_mean(threadIdx.x, fv[threadIdx.x].l);
       __syncthreads();
       if (in_a()) {
-        if (transform_first() && sync_a(half_a())) transform_rest();
+        if (run_transform_first<LARGE, SETS>() && sync_a(half_a())) run_transform_rest<LARGE, SETS>();
       }
       __syncthreads();
     }
-    if (in_b()) wa(pos, gam);
+    if (in_b()) run_wa<LARGE, SETS>(pos, gam);
     if (!sync()) return false;
     mark(full ? PC_DCT : PC_SCATTER_WA);
     fold(eval_jobs(full), [&](int j) { return eval_job(j, full); });
@@ -689,7 +751,7 @@ struct Ctx {
       const GA ga = half_a();
       for (int v = pb; v < V; v += np) {
         if (full) stage_gather(ga, d, pos, r.p, v, V, sh.a);
-        stage_combine(ga, d, coef, g, r.p, v, V, sh.a);
+        stage_combine(ga, d, L.coef, g, r.p, v, V, sh.a);
       }
     }
     if (!sync()) return false;
@@ -720,19 +782,18 @@ struct Ctx {
   // once every block has read the origin's WA accumulators.
   __device__ bool density_and_wa(const float2* pos, double gam, const float2* origin, float2* origin_g) {
     bool ready = true;
-    if (SETS == 1 && !origin_g) wa(pos, gam);
-    if (in_a()) ready = transform_first();
+    if (SETS == 1 && !origin_g) run_wa<LARGE, SETS>(pos, gam);
+    if (in_a()) ready = run_transform_first<LARGE, SETS>();
     if (origin_g) {
-      if (in_b())
-        for (int v = pb; v < V; v += np) combine_kept(origin, origin_g, v);
+      if (in_b()) run_combine_kept<LARGE, SETS>(origin, origin_g);
       ready = sync();
-      if (SETS == 1 && ready) wa(pos, gam);
+      if (SETS == 1 && ready) run_wa<LARGE, SETS>(pos, gam);
     }
     if (in_a()) {
       if (!origin_g && ready) ready = sync_a(half_a());
-      if (ready) transform_rest();
+      if (ready) run_transform_rest<LARGE, SETS>();
     } else {
-      if (ready) wa(pos, gam);
+      if (ready) run_wa<LARGE, SETS>(pos, gam);
     }
     const bool k = sync();
     mark(PC_DCT);
@@ -765,25 +826,25 @@ struct Ctx {
         jb = job(w);
         fa = fold_load(jb.a, V);
       }
-      int j = threadIdx.x;
-      const int o0 = object(v, j), o1 = object(v, j + kBlock);
+      int j = threadIdx.x, o = object(v, j);
       const int bin = v * kBlock + j;   // the first bin this thread resets
       const long long cap = bin < d.K * d.B ? d.capfix[bin] : 0;
-      const Raw a0 = gathered(pos, j, o0), a1 = gathered(pos, j + kBlock, o1);
+      Raw a;
+      gathered(a, pos, j, o);
       if (w < n) {
-        const FoldValue q = fold_job(fa, jb, V);
+        const FoldValue q = fold_ahead(fa, jb, V);
         if ((threadIdx.x & 31) == 0) fv[w] = q;
       }
       __syncthreads();
       if (threadIdx.x == 0) eval_coefficients(true);
       __syncthreads();
       if (threadIdx.x == kBlock - 32) scalars();
-      combine(a0, j, o0, g, kkt, bad);
-      combine(a1, j + kBlock, o1, g, kkt, bad);
-      for (j += 2 * kBlock;; j += kBlock) {
-        const int o = object(v, j);
-        if (o >= d.nobj) break;
-        combine(gathered(pos, j, o), j, o, g, kkt, bad);
+#pragma unroll 1
+      while (o < d.nobj) {
+        combine(a, j, o, g, kkt, bad);
+        j += kBlock;
+        o = object(v, j);
+        gathered(a, pos, j, o);
       }
       if (bin < d.K * d.B) {
         d.phys[bin] = -cap;
@@ -805,8 +866,12 @@ struct Ctx {
     for (; v < V; v += np) {
       kkt = 0.f;
       bad = 0xffffffffu;
-      for (int j = threadIdx.x, o; (o = object(v, j)) < d.nobj; j += kBlock)
-        combine(gathered(pos, j, o), j, o, g, kkt, bad);
+      Raw a;
+#pragma unroll 1
+      for (int j = threadIdx.x, o; (o = object(v, j)) < d.nobj; j += kBlock) {
+        gathered(a, pos, j, o);
+        combine(a, j, o, g, kkt, bad);
+      }
       reset_grids(v);
       __syncthreads();   // earlier readers of the scratch are done
       stage_kkt_warp(kkt, bad, sh.u[0], sh.u[1], threadIdx.x >> 5);
@@ -829,7 +894,7 @@ struct Ctx {
   // Half A, before an iteration's evaluations: the preconditioner
   // (diagonal_preconditioner, eplace.rs:1046-1100) and y = clamp(x + e (x -
   // xp)) with the count of coordinates that moved; y is scattered with
-  // `deposits`. Two objects' loads are in flight.
+  // `deposits`. The next object's loads are in flight.
   __device__ void precondition(const float* lam, const float2* x, const float2* xp, float e, float2* y, bool deposits,
                                int v) {
     const GA g = half_a();
@@ -874,16 +939,18 @@ struct Ctx {
       pmax = fmaxf(pmax, m);
       return t;
     };
-    for (int j = g.tid, o; (o = object(v, j)) < d.nobj; j += 2 * kThreads) {
+    int j = g.tid, o = object(v, j);
+    In cur, next;
+    if (o < d.nobj) cur = load(j, o);
+#pragma unroll 1
+    while (o < d.nobj) {
       const int o2 = object(v, j + kThreads);
-      const bool two = o2 < d.nobj;
-      const In i0 = load(j, o), i1 = two ? load(j + kThreads, o2) : i0;
-      const float2 t0 = step(i0, j, o);
-      const float2 t1 = two ? step(i1, j + kThreads, o2) : t0;
-      if (deposits) {
-        deposit(i0.mem, o, t0, tot);
-        if (two) deposit(i1.mem, o2, t1, tot);
-      }
+      if (o2 < d.nobj) next = load(j + kThreads, o2);
+      const float2 t = step(cur, j, o);
+      if (deposits) deposit(cur.mem, o, t, tot);
+      cur = next;
+      j += kThreads;
+      o = o2;
     }
     // not negative, so the bits order as integers
     const unsigned lo = __reduce_min_sync(0xffffffffu, __float_as_uint(pmin));
@@ -916,8 +983,8 @@ struct Ctx {
 
   // Half A: c = clamp(y - g / (L P)), scattered as it is formed; changed
   // count, <g, c - y>, sum P (c - y)^2. Each thread's objects and the order of
-  // its sums are those of the 256-thread stage (the sums are FP32), two
-  // objects' loads in flight.
+  // its sums are those of the 256-thread stage (the sums are FP32), the next
+  // object's loads in flight.
   __device__ void candidate(const float2* y, const float2* gy, float invL, float2* c, int v) {
     const GA g = half_a();
     unsigned diff = 0;
@@ -942,14 +1009,18 @@ struct Ctx {
       if (resident(j)) res->pos[j] = t;
       return t;
     };
-    for (int j = g.tid, o; (o = object(v, j)) < d.nobj; j += 2 * kThreads) {
+    int j = g.tid, o = object(v, j);
+    In cur, next;
+    if (o < d.nobj) cur = load(j, o);
+#pragma unroll 1
+    while (o < d.nobj) {
       const int o2 = object(v, j + kThreads);
-      const bool two = o2 < d.nobj;
-      const In i0 = load(j, o), i1 = two ? load(j + kThreads, o2) : i0;
-      const float2 t0 = step(i0, j, o);
-      const float2 t1 = two ? step(i1, j + kThreads, o2) : t0;
-      deposit(i0.mem, o, t0, tot);
-      if (two) deposit(i1.mem, o2, t1, tot);
+      if (o2 < d.nobj) next = load(j + kThreads, o2);
+      const float2 t = step(cur, j, o);
+      deposit(cur.mem, o, t, tot);
+      cur = next;
+      j += kThreads;
+      o = o2;
     }
     // both FP64 sums at once, each in block_fold_fp64's order
     double *b0 = sh.pair, *b1 = sh.pair + kThreads + 4;
@@ -981,6 +1052,44 @@ struct Ctx {
     }
   }
 };
+
+OUTLINED(bool, run_sync)() { return Ctx<LARGE, SETS>(loop_state<SETS>()).sync_body(); }
+OUTLINED(void, run_wa)(const float2* pos, double gam) { Ctx<LARGE, SETS>(loop_state<SETS>()).wa(pos, gam); }
+OUTLINED(void, run_scatter)(const float2* pos) {
+  Ctx<LARGE, SETS> c(loop_state<SETS>());
+#pragma unroll 1
+  for (int v = c.pb; v < c.V; v += c.np) c.scatter(pos, v);
+}
+OUTLINED(void, run_combine_kept)(const float2* pos, float2* g) {
+  Ctx<LARGE, SETS> c(loop_state<SETS>());
+#pragma unroll 1
+  for (int v = c.pb; v < c.V; v += c.np) c.combine_kept(pos, g, v);
+}
+OUTLINED(bool, run_transform_first)() { return Ctx<LARGE, SETS>(loop_state<SETS>()).transform_first(); }
+OUTLINED(bool, run_transform_rest)() { return Ctx<LARGE, SETS>(loop_state<SETS>()).transform_rest(); }
+OUTLINED(bool, run_density_and_wa)(const float2* pos, double gam, const float2* origin, float2* origin_g) {
+  return Ctx<LARGE, SETS>(loop_state<SETS>()).density_and_wa(pos, gam, origin, origin_g);
+}
+OUTLINED(bool, run_gradient)(const float2* pos, float2* g, ERec* out, ERec* origin) {
+  return Ctx<LARGE, SETS>(loop_state<SETS>()).gradient(pos, g, *out, origin);
+}
+OUTLINED(bool, run_eval_initial)(const float2* pos, float2* g, double gam, bool full) {
+  Ctx<LARGE, SETS> c(loop_state<SETS>());
+  return c.eval_initial(pos, g, gam, full, c.L.eo);
+}
+OUTLINED(void, run_precondition)(bool deposits) {
+  Ctx<LARGE, SETS> c(loop_state<SETS>());
+  const StepVars& V = c.L.V;
+#pragma unroll 1
+  for (int v = c.pb; v < c.V; v += c.np)
+    c.precondition(V.lambda, c.X(), V.pending_prev ? c.X() : c.Xp(), V.extrapolation, c.Y(), deposits, v);
+}
+OUTLINED(void, run_candidate)(const float2* y, const float2* gy, float2* to) {
+  Ctx<LARGE, SETS> c(loop_state<SETS>());
+#pragma unroll 1
+  for (int v = c.pb; v < c.V; v += c.np) c.candidate(y, gy, c.L.V.inv_L, to, v);
+}
+#undef OUTLINED
 
 // ---- scalar rules (eplace.rs:1300-1415), evaluated by thread 0 ------------
 static __device__ int field_gamma_dev(double overflow, double target, double slope, double base, double& g) {
@@ -1120,16 +1229,6 @@ static __device__ void adopt_density(DevRun& S, const ERec& e) {
   }
 }
 
-// Shared-memory step bookkeeping that every thread reads after a barrier.
-struct StepVars {
-  int restart, y_is_origin, may_reduce, has_wL, action, stationary, fresh, deposited, dirty;
-  double wL, tL, f_y, y_stat, next_m, pmin, pmax;
-  double gamma, growth;                       // of the next iteration
-  int st_multipliers, st_growth, st_gamma;
-  float extrapolation, lambda[kMaxFields], inv_L;
-  unsigned trials;
-  int pending_best, pending_prev;
-};
 enum { ACT_NONE = 0, ACT_RESTART, ACT_CONTINUE, ACT_ACCEPT, ACT_STATIONARY };
 
 // Copies *src to *dst one 8-byte word per thread of the block (a struct copy
@@ -1142,42 +1241,45 @@ __device__ __forceinline__ void copy_words(T* dst, const T* src) {
 }
 
 // The placement loop of one instance, run by its np physical blocks of SETS *
-// kThreads threads; `resident` is a double block's dynamic shared memory.
+// kThreads threads; the caller has the instance's descriptor in
+// loop_state<SETS>().inst. `resident` is a double block's dynamic shared
+// memory.
 template <bool LARGE, int SETS>
-static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B, DevRun* run, GridBarrier* bar, int pb,
-                         int np, int Vn, Resident* resident) {
-  __shared__ DevRun S;
-  __shared__ ERec eo, ey, ec;
-  __shared__ StepVars V;
-  __shared__ GemmShared gsm;
-  __shared__ LoopShared<SETS> sh;
-  __shared__ double coef[kMaxFields];
-  __shared__ float coef32[kMaxFields];
-  __shared__ FoldValue fvals[kMaxFoldJobs];
-  __shared__ long long fmean[kMaxFields], capsum[kMaxFields];
-  __shared__ unsigned gen;
-  __shared__ int bar_failed;
-  __shared__ unsigned long long clock[10];
+static __device__ void run_body(int pb, int np, Resident* resident) {
+  LoopState<SETS>& L = loop_state<SETS>();
+  DevRun& S = L.S;
+  ERec &eo = L.eo, &ey = L.ey, &ec = L.ec;
+  StepVars& V = L.V;
+  FoldValue* const fvals = L.fv;
+  const Dev& d = L.inst.d;
   if (threadIdx.x == 0) {
-    for (int i = 0; i < 10; ++i) clock[i] = 0;
-    clock[8] = now_ns();
-    gen = 0;   // the barrier is cleared with the state copy before every launch
+    for (int i = 0; i < 10; ++i) L.clock[i] = 0;
+    L.clock[8] = now_ns();
+    L.nbar = 0;
+    L.gen = 0;   // the barrier is cleared with the state copy before every launch
+    L.pb = pb;
+    L.np = np;
+    // one virtual block a physical one: its objects can stay in shared memory
+    L.res = SETS == 2 && np == L.inst.V ? resident : nullptr;
+    const bool maps = L.res && !d.g.identity && d.g.W <= kResidentMap && d.g.H <= kResidentMap;
+    L.mapx = maps ? L.res->mapx : d.binmap_x;
+    L.mapy = maps ? L.res->mapy : d.binmap_y;
+    L.tables = fft::tables_stay(d);
+    V.ws = 0;
     V.pending_best = 0;
     V.pending_prev = 0;
     V.dirty = 0;
   }
-  if ((int)threadIdx.x < d.K) capsum[threadIdx.x] = d.capsum[threadIdx.x];
-  copy_words(&S, run);
-  // one virtual block a physical one: its objects can stay in shared memory
-  Resident* const res = SETS == 2 && np == Vn ? resident : nullptr;
-  const bool maps = res && !d.g.identity && d.g.W <= kResidentMap && d.g.H <= kResidentMap;
-  Ctx<LARGE, SETS> c{d,   r,    B,      S,      bar,   &gen,  &bar_failed, gsm,  sh,    res,
-                     maps ? res->mapx : d.binmap_x, maps ? res->mapy : d.binmap_y, coef, coef32,
-                     fvals, fmean, capsum, pb, np, Vn, 0ull, clock, fft::tables_stay(d)};
+  if ((int)threadIdx.x < d.K) L.capsum[threadIdx.x] = d.capsum[threadIdx.x];
+  copy_words(&S, L.inst.run);
+  __syncthreads();
+  Ctx<LARGE, SETS> c(L);
+  const Reduce& r = c.r;
+  const Buffers& B = c.B;
   c.make_resident();
   __syncthreads();
-  if (c.tables && c.in_a())
-    fft::stage_tables(c.half_a(), fft::axis_x(d), reinterpret_cast<fft::Smem*>(gsm.fft)->buf, false);
+  if (L.tables && c.in_a())
+    fft::stage_tables(c.half_a(), fft::axis_x(d), reinterpret_cast<fft::Smem*>(L.gsm.fft)->buf, false);
   const int n = d.nobj;
   unsigned done = 0;
   bool ok = true;
@@ -1188,7 +1290,7 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
 #define T0            \
   __syncthreads();    \
   if (threadIdx.x == 0)
-#define VLOOP for (int v = c.pb; v < c.V; v += c.np)
+#define VLOOP _Pragma("unroll 1") for (int v = c.pb; v < c.V; v += c.np)
 #define LEAVE   \
   {             \
     ok = false; \
@@ -1216,7 +1318,7 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
       c.reset_wa(v);
     }
     SYNC_OR_EXIT(PC_PRECOND)
-    if (!c.eval_initial(c.X(), c.gX(), S.gamma_base, true, eo)) LEAVE
+    if (!run_eval_initial<LARGE, SETS>(c.X(), c.gX(), S.gamma_base, true)) LEAVE
     {
       T0 {
         double g0 = 0.0;
@@ -1231,7 +1333,7 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
     }
     VLOOP c.reset_wa(v);
     SYNC_OR_EXIT(PC_PRECOND)
-    if (!c.eval_initial(c.X(), c.gX(), S.gamma, false, eo)) LEAVE
+    if (!run_eval_initial<LARGE, SETS>(c.X(), c.gX(), S.gamma, false)) LEAVE
     T0 {
       int st = validate_initial_dev(S, eo);
       for (int f = 0; f < S.K; ++f) {
@@ -1356,11 +1458,10 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
     // side is reused when the device already holds it for these coordinates.
     const bool fresh = V.fresh != 0, deposited = V.deposited != 0;
     {
-      if (c.in_a())
-        VLOOP c.precondition(V.lambda, c.X(), V.pending_prev ? c.X() : c.Xp(), V.extrapolation, c.Y(), deposited, v);
+      if (c.in_a()) run_precondition<LARGE, SETS>(deposited);
       if (V.pending_best) c.copy(B.best, c.X(), d.U);
       if (V.pending_prev) c.copy(c.Xp(), c.X(), n);
-      if (!fresh && c.in_b()) c.wa(c.X(), S.gamma);
+      if (!fresh && c.in_b()) run_wa<LARGE, SETS>(c.X(), S.gamma);
       SYNC_OR_EXIT(PC_PRECOND)
       const Partials q = c.set();
       const int nj = (fresh ? 4 : 5), ns = deposited ? d.K : 0;
@@ -1372,8 +1473,8 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
                : j < nj ? FoldJob{pslot(r.p, SLOT_WA_VALUE), FOLD_DSUM}
                         : c.sum_job(j - nj);
       });
-      ++c.ws;
       if (threadIdx.x == 0) {
+        ++V.ws;
         V.pmin = fvals[0].d;
         V.pmax = fvals[1].d;
         V.y_is_origin = fvals[3].l == 0;
@@ -1397,13 +1498,13 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
       }
     }
     if (fresh) {
-      if (c.in_a()) VLOOP c.scatter(c.X(), v);
+      if (c.in_a()) run_scatter<LARGE, SETS>(c.X());
       SYNC_OR_EXIT(PC_SCATTER_WA)
       c.fold(d.K, [&](int j) { return c.sum_job(j); });
       if ((int)threadIdx.x < d.K) c.set_mean(threadIdx.x, fvals[threadIdx.x].l);
       __syncthreads();
-      if (!c.density_and_wa(c.X(), S.gamma, nullptr, nullptr)) LEAVE
-      if (!c.gradient(c.X(), c.gX(), eo, nullptr)) LEAVE
+      if (!run_density_and_wa<LARGE, SETS>(c.X(), S.gamma, nullptr, nullptr)) LEAVE
+      if (!run_gradient<LARGE, SETS>(c.X(), c.gX(), &eo, nullptr)) LEAVE
       T0 {
         S.status = checked_dev(eo);
         adopt_density(S, eo);
@@ -1412,7 +1513,7 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
       __syncthreads();
       if (S.status) FAIL(S.status)
       if (!V.y_is_origin) {
-        if (c.in_a()) VLOOP c.scatter(c.Y(), v);
+        if (c.in_a()) run_scatter<LARGE, SETS>(c.Y());
         SYNC_OR_EXIT(PC_EXTRAP)
         c.fold(d.K, [&](int j) { return c.sum_job(j); });
         if ((int)threadIdx.x < d.K) c.set_mean(threadIdx.x, fvals[threadIdx.x].l);
@@ -1420,7 +1521,7 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
       }
     } else if (V.y_is_origin) {
       // the origin's gradient in a phase of its own
-      if (c.in_b()) VLOOP c.combine_kept(c.X(), c.gX(), v);
+      if (c.in_b()) run_combine_kept<LARGE, SETS>(c.X(), c.gX());
       if (V.dirty) VLOOP c.reset_grids(v);
       SYNC_OR_EXIT(PC_SCATTER_WA)
       c.fold(2, [&](int j) { return c.kkt_job(r.q, j); });
@@ -1448,8 +1549,8 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
       __syncthreads();
       if (S.status) FAIL(S.status)
       if (!V.y_is_origin) {
-        if (!c.density_and_wa(c.Y(), S.gamma, fresh ? nullptr : c.X(), fresh ? nullptr : c.gX())) LEAVE
-        if (!c.gradient(c.Y(), c.gY(), ey, fresh ? nullptr : &eo)) LEAVE
+        if (!run_density_and_wa<LARGE, SETS>(c.Y(), S.gamma, fresh ? nullptr : c.X(), fresh ? nullptr : c.gX())) LEAVE
+        if (!run_gradient<LARGE, SETS>(c.Y(), c.gY(), &ey, fresh ? nullptr : &eo)) LEAVE
       }
       T0 {
         if (!V.y_is_origin) {
@@ -1505,7 +1606,7 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
             VLOOP c.reset_grids(v);
             SYNC_OR_EXIT(PC_EXTRAP)
           }
-          if (c.in_a()) VLOOP c.candidate(ybuf, gy, V.inv_L, c.C(), v);
+          if (c.in_a()) run_candidate<LARGE, SETS>(ybuf, gy, c.C());
           SYNC_OR_EXIT(PC_CANDIDATE)
           {
             const Partials q = c.set();
@@ -1515,12 +1616,12 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
                      : j == 2 ? FoldJob{pslot(q, SLOT_MSN), FOLD_DSUM}
                               : c.sum_job(j - 3);
             });
-            ++c.ws;
           }
           const long long changed = fvals[0].l;
           const double dot = fvals[1].d, msn = fvals[2].d;
           if ((int)threadIdx.x >= 64 && (int)threadIdx.x < 64 + d.K) c.set_mean(threadIdx.x - 64, fvals[3 + threadIdx.x - 64].l);
           T0 {
+            ++V.ws;
             V.action = ACT_NONE;
             V.dirty = changed == 0;
             if (changed == 0) {
@@ -1543,8 +1644,8 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
           __syncthreads();
           if (V.action == ACT_CONTINUE) continue;
           if (V.action != ACT_NONE) break;
-          if (!c.density_and_wa(c.C(), S.gamma, nullptr, nullptr)) LEAVE
-          if (!c.gradient(c.C(), c.gC(), ec, nullptr)) LEAVE
+          if (!run_density_and_wa<LARGE, SETS>(c.C(), S.gamma, nullptr, nullptr)) LEAVE
+          if (!run_gradient<LARGE, SETS>(c.C(), c.gC(), &ec, nullptr)) LEAVE
           T0 {
             S.density_at_x = 0;
             S.status = checked_dev(ec);
@@ -1631,15 +1732,15 @@ static __device__ void run_body(const Dev& d, const Reduce& r, const Buffers& B,
           B.prev_targets[2 * u] = tx;
           B.prev_targets[2 * u + 1] = ty;
         }
-        write_partial(g, mism, islot(c.set(), IS_DIFF), v, sh.a.l);
+        write_partial(g, mism, islot(c.set(), IS_DIFF), v, L.sh.a.l);
       }
       if (V.dirty) VLOOP c.reset_grids(v);   // the next iteration scatters at once
       SYNC_OR_EXIT(PC_OTHER)
       const Partials q = c.set();
       c.fold(1, [&](int) { return FoldJob{islot(q, IS_DIFF), FOLD_ISUM}; });
-      ++c.ws;
       const long long total = fvals[0].l;
       T0 {
+        ++V.ws;
         const bool fixed = S.have_prev_stationary && total == 0;
         S.have_prev_stationary = 1;
         V.dirty = 0;
@@ -1665,12 +1766,12 @@ out:
   __syncthreads();
   if (pb == 0) {
     if (threadIdx.x == 0) {
-      S.barriers += c.nbar;
-      for (int i = 0; i < 8; ++i) S.phase_ns[i] += clock[i];
-      S.barrier_wait_ns += clock[9];
+      S.barriers += L.nbar;
+      for (int i = 0; i < 8; ++i) S.phase_ns[i] += L.clock[i];
+      S.barrier_wait_ns += L.clock[9];
     }
     __syncthreads();
-    copy_words(run, &S);
+    copy_words(L.inst.run, &S);
   }
 #undef T0
 #undef VLOOP

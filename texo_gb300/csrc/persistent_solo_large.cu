@@ -4,11 +4,11 @@
 
 namespace tgp {
 
-__global__ void __launch_bounds__(2 * kThreads, kBlocksPerSm)
-    k_persistent_large(Dev d, Reduce r, Buffers B, DevRun* run, GridBarrier* bar, int V) {
+__global__ void __launch_bounds__(2 * kThreads, kBlocksPerSm) k_persistent_large(const __grid_constant__ InstDesc desc) {
   extern __shared__ __align__(16) unsigned char resident[];
-  run_body<true, 2>(d, r, B, run, bar, (int)blockIdx.x, (int)gridDim.x, V,
-                     reinterpret_cast<Resident*>(resident));
+  copy_words(&loop_state<2>().inst, &desc);
+  __syncthreads();
+  run_body<true, 2>((int)blockIdx.x, (int)gridDim.x, reinterpret_cast<Resident*>(resident));
 }
 
 const void* persistent_kernel_large() { return (const void*)k_persistent_large; }
