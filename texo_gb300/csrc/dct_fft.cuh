@@ -355,7 +355,7 @@ __device__ __forceinline__ float2* stage_out(float4* buf) {
 // the physical overflow is counted into the IS_OVERFLOW / IS_OVER_BINS
 // partials.
 template <int NB, class G>
-static __device__ __noinline__ void rows_fwd(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
+static __device__ __forceinline__ void rows_fwd(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
                                                 Shared& sh, const long long* mean, bool tables) {
   const int W = d.g.Wb, H = d.g.Hb, L = d.logW, GV = min(group_size(L), H), per = GV << L;
   const int gpf = (H + GV - 1) / GV, groups = gpf * d.K;
@@ -431,7 +431,7 @@ static __device__ __noinline__ void rows_fwd(const G& g, const Dev& d, Partials 
 // Pass 2: t2 = cols-IDCT(cols-DCT(t1) * inv_eig), whole columns per group;
 // the scaled coefficients stay double-floats between the two transforms.
 template <int NB, class G>
-static __device__ __noinline__ void cols(const G& g, const Dev& d, int vb, int nvb, float4* buf, bool tables) {
+static __device__ __forceinline__ void cols(const G& g, const Dev& d, int vb, int nvb, float4* buf, bool tables) {
   const int W = d.g.Wb, H = d.g.Hb, L = d.logH, GV = min(group_size(L), W), per = GV << L;
   const int gpf = (W + GV - 1) / GV, groups = gpf * d.K;
   const Axis a = vb < groups ? stage_tables(g, axis_y(d), buf, tables) : axis_y(d);
@@ -494,7 +494,7 @@ static __device__ __noinline__ void cols(const G& g, const Dev& d, int vb, int n
 
 // Pass 3: phi = rows-IDCT(t2) and the energy partials <rho, phi>.
 template <int NB, class G>
-static __device__ __noinline__ void rows_inv(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
+static __device__ __forceinline__ void rows_inv(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
                                                 Shared& sh, bool tables) {
   const int W = d.g.Wb, H = d.g.Hb, L = d.logW, GV = min(group_size(L), H), per = GV << L;
   const int gpf = (H + GV - 1) / GV, groups = gpf * d.K;
@@ -551,30 +551,6 @@ static __device__ __noinline__ void rows_inv(const G& g, const Dev& d, Partials 
 #pragma unroll
   for (int f = 0; f < kMaxFields; ++f)
     if (f < d.K) write_partial(g, eacc[f], pslot(p, SLOT_ENERGY + f), vb, sh.d);
-}
-
-template <class G>
-static __device__ void pass_rows_fwd(const G& g, const Dev& d, Partials p, int vb, int nvb, Smem& sm, Shared& sh,
-                                     const long long* mean, bool tables) {
-  if (d.logW == 10)
-    rows_fwd<2>(g, d, p, vb, nvb, sm.buf, sh, mean, tables);
-  else
-    rows_fwd<1>(g, d, p, vb, nvb, sm.buf, sh, mean, tables);
-}
-template <class G>
-static __device__ void pass_cols(const G& g, const Dev& d, int vb, int nvb, Smem& sm, bool tables) {
-  if (d.logH == 10)
-    cols<2>(g, d, vb, nvb, sm.buf, tables);
-  else
-    cols<1>(g, d, vb, nvb, sm.buf, tables);
-}
-template <class G>
-static __device__ void pass_rows_inv(const G& g, const Dev& d, Partials p, int vb, int nvb, Smem& sm, Shared& sh,
-                                     bool tables) {
-  if (d.logW == 10)
-    rows_inv<2>(g, d, p, vb, nvb, sm.buf, sh, tables);
-  else
-    rows_inv<1>(g, d, p, vb, nvb, sm.buf, sh, tables);
 }
 
 }  // namespace fft

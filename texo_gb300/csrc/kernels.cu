@@ -6,20 +6,25 @@
 
 namespace tgp {
 
-// The FFT form's three passes (dct_fft.cuh).
-__global__ void __launch_bounds__(kThreads) k_fft_rows_fwd(Dev d, Partials p) {
+// The FFT form's three passes (dct_fft.cuh), NB = 2 for 1024 points. Four blocks
+// an SM for the row passes (1024^2 rows inverse: 39 us with 118 registers and
+// two blocks, 33 with 64 and four).
+template <int NB>
+__global__ void __launch_bounds__(kThreads, 4) k_fft_rows_fwd(Dev d, Partials p) {
   __shared__ fft::Smem sm;
   __shared__ Shared sh;
-  fft::pass_rows_fwd(whole_block(), d, p, blockIdx.x, gridDim.x, sm, sh, nullptr, false);
+  fft::rows_fwd<NB>(whole_block(), d, p, blockIdx.x, gridDim.x, sm.buf, sh, nullptr, false);
 }
+template <int NB>
 __global__ void __launch_bounds__(kThreads) k_fft_cols(Dev d) {
   __shared__ fft::Smem sm;
-  fft::pass_cols(whole_block(), d, blockIdx.x, gridDim.x, sm, false);
+  fft::cols<NB>(whole_block(), d, blockIdx.x, gridDim.x, sm.buf, false);
 }
-__global__ void __launch_bounds__(kThreads) k_fft_rows_inv(Dev d, Partials p) {
+template <int NB>
+__global__ void __launch_bounds__(kThreads, 4) k_fft_rows_inv(Dev d, Partials p) {
   __shared__ fft::Smem sm;
   __shared__ Shared sh;
-  fft::pass_rows_inv(whole_block(), d, p, blockIdx.x, gridDim.x, sm, sh, false);
+  fft::rows_inv<NB>(whole_block(), d, p, blockIdx.x, gridDim.x, sm.buf, sh, false);
 }
 
 // The slice phase before tensor-core pass `step` (memory-bound, every block).
@@ -89,7 +94,8 @@ __global__ void __launch_bounds__(kThreads) k_spread_positions(Dev d, float2* ou
     out[o] = make_float2(fmaf(hi.x - lo.x, fx, lo.x), fmaf(hi.y - lo.y, fy, lo.y));
   }
 }
-__global__ void __launch_bounds__(kThreads) k_wa(Dev d, Partials p, const float2* pos, double gamma) {
+// 4 blocks an SM: the stage waits on memory (72 registers and 3 blocks: 85 us at 1M cells, 79 with 64)
+__global__ void __launch_bounds__(kThreads, 4) k_wa(Dev d, Partials p, const float2* pos, double gamma) {
   __shared__ Shared sh;
   stage_wa(whole_block(), d, pos, gamma, p, blockIdx.x, gridDim.x, sh.d);
 }
@@ -284,11 +290,11 @@ void launch_dct(const Dev& d, const Reduce& r, int step, int nvb, cudaStream_t s
     if (step == 2) return;
     COUNT;
     if (step == 0)
-      k_fft_rows_fwd<<<nvb, kThreads, 0, s>>>(d, r.p);
+      (d.logW == 10 ? k_fft_rows_fwd<2> : k_fft_rows_fwd<1>)<<<nvb, kThreads, 0, s>>>(d, r.p);
     else if (step == 1)
-      k_fft_cols<<<nvb, kThreads, 0, s>>>(d);
+      (d.logH == 10 ? k_fft_cols<2> : k_fft_cols<1>)<<<nvb, kThreads, 0, s>>>(d);
     else
-      k_fft_rows_inv<<<nvb, kThreads, 0, s>>>(d, r.p);
+      (d.logW == 10 ? k_fft_rows_inv<2> : k_fft_rows_inv<1>)<<<nvb, kThreads, 0, s>>>(d, r.p);
     return;
   }
   if (d.tc) {

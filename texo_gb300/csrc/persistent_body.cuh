@@ -164,6 +164,7 @@ __device__ __forceinline__ T fold_loaded(const FoldAhead& f, const T* a, int n, 
 #pragma unroll
   for (int u = 1; u < kFoldAhead; ++u)
     if (lane + 32 * u < n) v = op(v, as(f.v[u]));
+#pragma unroll 1
   for (int i = lane + 32 * kFoldAhead; i < n; i += 32) v = op(v, a[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -264,6 +265,9 @@ template <bool LARGE, int SETS>
 struct Ctx;
 // The phases out of line, one copy each.
 #define OUTLINED(type, name) template <bool LARGE, int SETS> static __device__ __noinline__ type name
+template <int NB, int SETS> static __device__ __noinline__ void run_rows_fwd();
+template <int NB, int SETS> static __device__ __noinline__ void run_cols();
+template <int NB, int SETS> static __device__ __noinline__ void run_rows_inv();
 OUTLINED(bool, run_sync)();
 OUTLINED(void, run_wa)(const float2* pos, double gam);
 OUTLINED(void, run_scatter)(const float2* pos);
@@ -429,12 +433,14 @@ struct Ctx {
   // Resets of the accumulators, dealt to all threads of the block.
   __device__ void reset_grids(int v, int from = 0) {
     const int n = d.K * d.B, stride = V * kBlock;
+#pragma unroll 1
     for (int i = from + v * kBlock + (int)threadIdx.x; i < n; i += stride) {
       d.phys[i] = -d.capfix[i];
       d.fill[i] = 0;
     }
   }
   __device__ void reset_wa(int v) {
+#pragma unroll 1
     for (int i = v * kBlock + (int)threadIdx.x; i < 2 * d.U; i += V * kBlock) d.wa_fix[i] = 0ull;
   }
 
@@ -653,8 +659,7 @@ struct Ctx {
   __device__ bool transform_first() {
     const GA g = half_a();
     if (d.fft) {
-      for (int v = pb; v < V; v += np)
-        fft::pass_rows_fwd(g, d, r.p, v, V, *reinterpret_cast<fft::Smem*>(gsm.fft), sh.a, L.fmean, L.tables);
+      d.logW == 10 ? run_rows_fwd<2, SETS>() : run_rows_fwd<1, SETS>();
     } else if (LARGE) {
       for (int v = pb; v < V; v += np) stage_prep(g, d, r.p, V, v, V, sh.a);
       if (!sync_a(g)) return false;
@@ -668,10 +673,9 @@ struct Ctx {
   __device__ bool transform_rest() {
     const GA g = half_a();
     if (d.fft) {
-      fft::Smem& fs = *reinterpret_cast<fft::Smem*>(gsm.fft);
-      for (int v = pb; v < V; v += np) fft::pass_cols(g, d, v, V, fs, L.tables);
+      d.logH == 10 ? run_cols<2, SETS>() : run_cols<1, SETS>();
       if (!sync_a(g)) return false;
-      for (int v = pb; v < V; v += np) fft::pass_rows_inv(g, d, r.p, v, V, fs, sh.a, L.tables);
+      d.logW == 10 ? run_rows_inv<2, SETS>() : run_rows_inv<1, SETS>();
     } else {
       for (int st = 1; st < 4; ++st) {
         for (int v = pb; v < V; v += np) stage_dct_t<LARGE>(g, d, st, r.p, v, V, gsm, sh.a);
@@ -693,6 +697,7 @@ struct Ctx {
   __device__ int eval_jobs(bool full) const { return full ? 3 * d.K + 1 : 1; }
   // one thread: the fields' coefficients from the jobs at fv[at...]
   __device__ void eval_coefficients(bool full, int at = 0) {
+#pragma unroll 1
     for (int f = 0; f < d.K; ++f) {
       const double ne = (full ? 0.5 * fv[at + 3 * f].d : S.cur_energy[f]) * S.inv_e0[f];
       L.coef[f] = S.lambda[f] * (1.0 + S.beta * ne);
@@ -704,6 +709,7 @@ struct Ctx {
     const double wa = fv[at + (full ? 3 * d.K : 0)].d;
     out.wa = wa;
     double value = wa;
+#pragma unroll 1
     for (int f = 0; f < d.K; ++f) {
       if (full) {
         const long long ov = fv[at + 3 * f + 1].l;
@@ -967,6 +973,7 @@ struct Ctx {
     if (g.tid == 0) {
       unsigned a = 0x7f800000u, b = 0u, bad = 0u;
       long long n = 0;
+  #pragma unroll 1
       for (int w = 0; w < kThreads / 32; ++w) {
         a = min(a, sh.u[0][w]);
         b = max(b, sh.u[1][w]);
@@ -1053,6 +1060,26 @@ struct Ctx {
   }
 };
 
+template <int NB, int SETS>
+static __device__ __noinline__ void run_rows_fwd() {
+  Ctx<false, SETS> c(loop_state<SETS>());
+#pragma unroll 1
+  for (int v = c.pb; v < c.V; v += c.np)
+    fft::rows_fwd<NB>(c.half_a(), c.d, c.r.p, v, c.V, c.gsm.fft, c.sh.a, c.L.fmean, c.L.tables);
+}
+template <int NB, int SETS>
+static __device__ __noinline__ void run_cols() {
+  Ctx<false, SETS> c(loop_state<SETS>());
+#pragma unroll 1
+  for (int v = c.pb; v < c.V; v += c.np) fft::cols<NB>(c.half_a(), c.d, v, c.V, c.gsm.fft, c.L.tables);
+}
+template <int NB, int SETS>
+static __device__ __noinline__ void run_rows_inv() {
+  Ctx<false, SETS> c(loop_state<SETS>());
+#pragma unroll 1
+  for (int v = c.pb; v < c.V; v += c.np)
+    fft::rows_inv<NB>(c.half_a(), c.d, c.r.p, v, c.V, c.gsm.fft, c.sh.a, c.L.tables);
+}
 OUTLINED(bool, run_sync)() { return Ctx<LARGE, SETS>(loop_state<SETS>()).sync_body(); }
 OUTLINED(void, run_wa)(const float2* pos, double gam) { Ctx<LARGE, SETS>(loop_state<SETS>()).wa(pos, gam); }
 OUTLINED(void, run_scatter)(const float2* pos) {

@@ -229,18 +229,25 @@ __device__ __forceinline__ float2 pin_xy(const Dev& d, const float2* pos, int k)
 // lanes (both multiples of 32 at the segment start, so a group never
 // straddles a warp and every lane of a warp makes the same passes). Lane l
 // of a group takes pins p0 + l, p0 + l + G, ...; the first kWaPins of them
-// stay in registers across the three passes (their loads are issued
-// together), any further ones are read again.
+// stay in registers across the three passes with their exponential weights
+// (their loads are issued together), any further ones are read again.
+// One body for every group size G (a power of two up to 32): a copy for each
+// was 139 KB of code, and the warps of a block, each in another class, drove
+// one another out of the instruction cache.
 constexpr int kWaPins = 4;
-template <int G>
-__device__ __forceinline__ void wa_class(const Dev& d, const float2* pos, float inv_gamma, int nb,
-                                         int ne, int slot, int seg, double& acc) {
+__device__ __forceinline__ void wa_nets(const Dev& d, const float2* pos, float inv_gamma, int G, int nb, int ne,
+                                        int slot, int seg, double& acc) {
   const int lane = slot & (G - 1);
-  const int group = slot / G;
-  const int groups = seg / G;
+  const int shift = 31 - __clz(G);
+  const int group = slot >> shift;
+  const int groups = seg >> shift;
   const unsigned mask = 0xffffffffu;
   const int count = ne - nb;
   float vacc = 0.f;
+  struct Weights {
+    float xp, xn, yp, yn;
+  };
+#pragma unroll 1
   for (int base = 0; base < count; base += groups) {
     const int e = nb + base + group;
     const bool active = base + group < count;
@@ -260,6 +267,7 @@ __device__ __forceinline__ void wa_class(const Dev& d, const float2* pos, float 
       pu[j] = k < p1 ? d.pin_unit[k] : -2;   // -2: no pin, -1: fixed pin
       pv[j] = k < p1 ? d.pin_base[k] : make_float2(0.f, 0.f);
     }
+    const int more = p0 + lane + kWaPins * G;   // pins beyond the registers
     float mx = -INFINITY, mnx = INFINITY, my = -INFINITY, mny = INFINITY;
 #pragma unroll
     for (int j = 0; j < kWaPins; ++j) {
@@ -273,41 +281,52 @@ __device__ __forceinline__ void wa_class(const Dev& d, const float2* pos, float 
       my = fmaxf(my, pv[j].y);
       mny = fminf(mny, pv[j].y);
     }
-    for (int k = p0 + lane + kWaPins * G; k < p1; k += G) {
+#pragma unroll 1
+    for (int k = more; k < p1; k += G) {
       const float2 v = pin_xy(d, pos, k);
       mx = fmaxf(mx, v.x);
       mnx = fminf(mnx, v.x);
       my = fmaxf(my, v.y);
       mny = fminf(mny, v.y);
     }
-#pragma unroll
+#pragma unroll 1
     for (int o = G / 2; o > 0; o >>= 1) {
-      mx = fmaxf(mx, __shfl_xor_sync(mask, mx, o, G));
-      mnx = fminf(mnx, __shfl_xor_sync(mask, mnx, o, G));
-      my = fmaxf(my, __shfl_xor_sync(mask, my, o, G));
-      mny = fminf(mny, __shfl_xor_sync(mask, mny, o, G));
+      mx = fmaxf(mx, __shfl_xor_sync(mask, mx, o));
+      mnx = fminf(mnx, __shfl_xor_sync(mask, mnx, o));
+      my = fmaxf(my, __shfl_xor_sync(mask, my, o));
+      mny = fminf(mny, __shfl_xor_sync(mask, mny, o));
     }
     // pass 2: exponential weights (exactly 1 at the extremum) and their sums
     float sw[4] = {0.f, 0.f, 0.f, 0.f}, sd[4] = {0.f, 0.f, 0.f, 0.f};
-    auto weigh = [&](float2 v) {
+    auto weights = [&](float2 v) {
       const float dxp = v.x - mx, dxn = v.x - mnx, dyp = v.y - my, dyn = v.y - mny;
-      const float wxp = expf(dxp * inv_gamma), wxn = expf(-dxn * inv_gamma);
-      const float wyp = expf(dyp * inv_gamma), wyn = expf(-dyn * inv_gamma);
-      sw[0] += wxp; sd[0] = fmaf(wxp, dxp, sd[0]);
-      sw[1] += wxn; sd[1] = fmaf(wxn, dxn, sd[1]);
-      sw[2] += wyp; sd[2] = fmaf(wyp, dyp, sd[2]);
-      sw[3] += wyn; sd[3] = fmaf(wyn, dyn, sd[3]);
+      return Weights{expf(dxp * inv_gamma), expf(-dxn * inv_gamma), expf(dyp * inv_gamma), expf(-dyn * inv_gamma)};
     };
+    auto weigh = [&](float2 v, const Weights& q) {
+      const float dxp = v.x - mx, dxn = v.x - mnx, dyp = v.y - my, dyn = v.y - mny;
+      sw[0] += q.xp; sd[0] = fmaf(q.xp, dxp, sd[0]);
+      sw[1] += q.xn; sd[1] = fmaf(q.xn, dxn, sd[1]);
+      sw[2] += q.yp; sd[2] = fmaf(q.yp, dyp, sd[2]);
+      sw[3] += q.yn; sd[3] = fmaf(q.yn, dyn, sd[3]);
+    };
+    Weights wt[kWaPins];
 #pragma unroll
     for (int j = 0; j < kWaPins; ++j)
-      if (pu[j] != -2) weigh(pv[j]);
-    for (int k = p0 + lane + kWaPins * G; k < p1; k += G) weigh(pin_xy(d, pos, k));
-#pragma unroll
+      if (pu[j] != -2) {
+        wt[j] = weights(pv[j]);
+        weigh(pv[j], wt[j]);
+      }
+#pragma unroll 1
+    for (int k = more; k < p1; k += G) {
+      const float2 v = pin_xy(d, pos, k);
+      weigh(v, weights(v));
+    }
+#pragma unroll 1
     for (int o = G / 2; o > 0; o >>= 1)
 #pragma unroll
       for (int a = 0; a < 4; ++a) {
-        sw[a] += __shfl_xor_sync(mask, sw[a], o, G);
-        sd[a] += __shfl_xor_sync(mask, sd[a], o, G);
+        sw[a] += __shfl_xor_sync(mask, sw[a], o);
+        sd[a] += __shfl_xor_sync(mask, sd[a], o);
       }
     if (!active) continue;
     float mean[4], inv[4];
@@ -317,23 +336,25 @@ __device__ __forceinline__ void wa_class(const Dev& d, const float2* pos, float 
       mean[a] = sd[a] * inv[a];
     }
     // pass 3: per-pin derivative into the fixed-point unit gradient
-    auto derive = [&](int u, float2 v) {
+    auto derive = [&](int u, float2 v, const Weights& q) {
       const float dxp = v.x - mx, dxn = v.x - mnx, dyp = v.y - my, dyn = v.y - mny;
-      const float wxp = expf(dxp * inv_gamma), wxn = expf(-dxn * inv_gamma);
-      const float wyp = expf(dyp * inv_gamma), wyn = expf(-dyn * inv_gamma);
-      const float gx = wxp * inv[0] * (1.f + (dxp - mean[0]) * inv_gamma) -
-                       wxn * inv[1] * (1.f - (dxn - mean[1]) * inv_gamma);
-      const float gy = wyp * inv[2] * (1.f + (dyp - mean[2]) * inv_gamma) -
-                       wyn * inv[3] * (1.f - (dyn - mean[3]) * inv_gamma);
+      const float gx = q.xp * inv[0] * (1.f + (dxp - mean[0]) * inv_gamma) -
+                       q.xn * inv[1] * (1.f - (dxn - mean[1]) * inv_gamma);
+      const float gy = q.yp * inv[2] * (1.f + (dyp - mean[2]) * inv_gamma) -
+                       q.yn * inv[3] * (1.f - (dyn - mean[3]) * inv_gamma);
       atomicAdd(d.wa_fix + 2 * u, (unsigned long long)__float2ll_rn(w * gx * kFixF));
       atomicAdd(d.wa_fix + 2 * u + 1, (unsigned long long)__float2ll_rn(w * gy * kFixF));
     };
 #pragma unroll
     for (int j = 0; j < kWaPins; ++j)
-      if (pu[j] >= 0) derive(pu[j], pv[j]);
-    for (int k = p0 + lane + kWaPins * G; k < p1; k += G) {
+      if (pu[j] >= 0) derive(pu[j], pv[j], wt[j]);
+#pragma unroll 1
+    for (int k = more; k < p1; k += G) {
       const int u = d.pin_unit[k];
-      if (u >= 0) derive(u, pin_xy(d, pos, k));
+      if (u >= 0) {
+        const float2 v = pin_xy(d, pos, k);
+        derive(u, v, weights(v));
+      }
     }
     if (lane == 0) vacc += w * (((mx - mnx) + mean[0] - mean[1]) + ((my - mny) + mean[2] - mean[3]));
   }
@@ -351,15 +372,7 @@ static __device__ void stage_wa(const G& g, const Dev& d, const float2* pos, dou
   if (c < d.n_classes) {
     const int nb = d.class_begin[c], ne = d.class_begin[c + 1];
     const int slot = gl - d.class_lane[c], seg = d.class_lane[c + 1] - d.class_lane[c];
-    if (ne > nb && seg > 0) {
-      switch (d.class_group[c]) {
-        case 1: wa_class<1>(d, pos, ig, nb, ne, slot, seg, acc); break;
-        case 2: wa_class<2>(d, pos, ig, nb, ne, slot, seg, acc); break;
-        case 4: wa_class<4>(d, pos, ig, nb, ne, slot, seg, acc); break;
-        case 8: wa_class<8>(d, pos, ig, nb, ne, slot, seg, acc); break;
-        default: wa_class<32>(d, pos, ig, nb, ne, slot, seg, acc); break;
-      }
-    }
+    if (ne > nb && seg > 0) wa_nets(d, pos, ig, d.class_group[c], nb, ne, slot, seg, acc);
   }
   write_partial(g, acc, pslot(p, SLOT_WA_VALUE), vb, sh);
 }
