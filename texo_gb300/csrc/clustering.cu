@@ -10,16 +10,32 @@
 // enable) on the host, so a clock enable's sum runs in input order and the
 // per-enable totals in ascending enable order, as in the reference's
 // BTreeMaps. Sums and soft ceilings use explicitly rounded FP64 operations
-// (no fused multiply-add, which the reference never uses); erf is CUDA's.
-// A pair whose windows lie more than 8 sigma sqrt(2) apart on an axis
-// contributes an exact zero (erf saturates), so it is skipped, after a
-// conservative FP32 test. Threads take the registers of a control set in
-// tile order, so the lanes of a warp agree on which pairs are far (FP64
-// runs at a low rate on this part: a warp whose lanes disagree pays for the
-// slowest lane's erf work on every pair).
+// (no fused multiply-add, which the reference never uses).
+//
+// The window probability of a register at distance x from the focal one,
+// (erf((x + w) / s) - erf((x - w) / s)) / 2 with w = 2.5 sigma and
+// s = sigma sqrt(2), depends on u = |x| / s alone, so it is one even function
+// of u for every call. It is evaluated as a Taylor polynomial of degree 8 on
+// intervals of 1/32 (Window), whose remainder stays below 1e-18: 13 FP64
+// operations an axis in place of two divisions and two erfs. FP64 runs at a
+// sixty-fourth of the FP32 rate here and bounded the kernel (pipe 85 % busy):
+// 42,000 registers in 8 control sets, device time with the copies, 10.8 ms
+// with the erfs and 0.90 ms with the table; the areas are 3e-16 off the exact
+// ones where those were 1.8e-15 off (the window's edges x + w were rounded at
+// the coordinates' magnitude). Beyond u = w / s + 6 the two erfs are both one
+// and the probability is an exact zero; such pairs are skipped after a
+// conservative FP32 test.
+//
+// Threads take the registers of a control set in blocks of about 32 near one
+// another, so a warp's focal registers agree on which others are far: the
+// warp tests 32 of them at a time against its bounding box and visits only
+// the ones inside, in order (a register that is far from all the warp's adds
+// an exact zero to sums and ceilings alike).
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -31,65 +47,160 @@ namespace {
 
 constexpr int kClusterThreads = 128;
 
-// soft_division_ceiling (register_clustering.rs:89-97)
-__device__ __forceinline__ double soft_ceiling(double value, double divisor) {
-  const double quotient = __ddiv_rn(value, divisor);
+// Taylor coefficients of the window probability about the middles of the
+// intervals [k / 32, (k + 1) / 32) of u, and the middles.
+constexpr int kTerms = 9;
+constexpr int kPerUnit = 32;
+constexpr double kHalfWindow = 1.7677669529663688;   // 2.5 / sqrt(2)
+constexpr double kReach = kHalfWindow + 6.0;         // erf(6) rounds to one
+constexpr int kIntervals = (int)(kReach * kPerUnit) + 1;
+struct Window {
+  double middle, c[kTerms];
+};
+
+// The table, formed once in extended precision (erf' = 2 / sqrt(pi)
+// exp(-x^2), and its n-th derivative times (-1)^n H_n(x), the Hermite
+// polynomials' three-term recurrence) and kept on each device.
+cudaError_t window_table(int device, const Window** out) {
+  static std::mutex mu;
+  static std::map<int, Window*> cache;
+  std::lock_guard<std::mutex> lk(mu);
+  auto it = cache.find(device);
+  if (it == cache.end()) {
+    std::vector<Window> t(kIntervals);
+    const long double h = 2.5L / sqrtl(2.0L), two_over_sqrt_pi = 2.0L / sqrtl(3.14159265358979323846264338327950288L);
+    for (int k = 0; k < kIntervals; ++k) {
+      const long double m = (k + 0.5L) / kPerUnit;
+      t[k].middle = (double)m;
+      long double c[kTerms] = {0.5L * (erfcl(m - h) - erfcl(m + h))};
+      for (int side = 0; side < 2; ++side) {
+        const long double x = side ? m - h : m + h, e = (side ? -0.5L : 0.5L) * two_over_sqrt_pi * expl(-x * x);
+        long double h0 = 1.0L, h1 = 2.0L * x, sign = 1.0L, factorial = 1.0L;
+        for (int n = 0; n + 1 < kTerms; ++n) {   // c[n + 1]: the n-th derivative of erf' over (n + 1)!
+          factorial *= n + 1;
+          c[n + 1] += sign * h0 * e / factorial;
+          const long double h2 = 2.0L * x * h1 - 2.0L * (n + 1) * h0;
+          h0 = h1;
+          h1 = h2;
+          sign = -sign;
+        }
+      }
+      for (int n = 0; n < kTerms; ++n) t[k].c[n] = (double)c[n];
+    }
+    Window* d = nullptr;
+    cudaError_t e = cudaMalloc(&d, t.size() * sizeof(Window));
+    if (e == cudaSuccess) e = cudaMemcpy(d, t.data(), t.size() * sizeof(Window), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return e;
+    it = cache.emplace(device, d).first;
+  }
+  *out = it->second;
+  return cudaSuccess;
+}
+
+// soft_division_ceiling (register_clustering.rs:89-97); the divisors are
+// powers of two, so the quotients are exact products
+__device__ __forceinline__ double soft_ceiling(double value, double divisor, double inverse) {
+  const double quotient = __dmul_rn(value, inverse);
   const double fl = floor(quotient);
-  if (__dsub_rn(quotient, fl) < __ddiv_rn(1.0, divisor)) return __dadd_rn(value, __dmul_rn(1.0 - divisor, fl));
+  if (__dsub_rn(quotient, fl) < inverse) return __dadd_rn(value, __dmul_rn(1.0 - divisor, fl));
   return ceil(quotient);
 }
 
-// gaussian_interval_probability (register_clustering.rs:84-87)
-__device__ __forceinline__ double window_probability(double low, double high, double mean, double scale) {
-  const double p = __dmul_rn(0.5, __dsub_rn(erf(__ddiv_rn(__dsub_rn(high, mean), scale)),
-                                           erf(__ddiv_rn(__dsub_rn(low, mean), scale))));
-  return fmin(fmax(p, 0.0), 1.0);
+// gaussian_interval_probability (register_clustering.rs:84-87) at distance x
+__device__ __forceinline__ double window_probability(double x, double inv_scale, const Window* table) {
+  const double u = __dmul_rn(fabs(x), inv_scale);
+  const int k = min((int)(__double2float_rn(u) * (float)kPerUnit), kIntervals - 1);   // a neighbour's interval serves too
+  const Window& w = table[k];
+  const double t = __dsub_rn(u, w.middle);
+  double p = w.c[kTerms - 1];
+#pragma unroll
+  for (int n = kTerms - 2; n >= 0; --n) p = __fma_rn(p, t, w.c[n]);
+  return fmax(p, 0.0);   // a NaN distance counts zero
 }
 
 struct ClusterDev {
   unsigned n;
-  const double *x, *y;                 // sorted by (clock, lsr, ce), stable
+  const double2* xy;                   // sorted by (clock, lsr, ce), stable
   const float2* xy32;                  // the same positions in FP32, for the far-pair test
   const unsigned long long* ce;
   const unsigned* focal;               // thread -> sorted position: near registers share a warp
   const unsigned *group_begin, *group_end;   // per sorted register: its control set's range
   const unsigned* order;               // sorted position -> input index
-  double half_window, scale, cutoff;
+  const Window* table;
+  double inv_scale, cutoff;
   float cutoff32;                      // cutoff plus a margin that covers the FP32 rounding
   double* areas;                       // by input index
   int* bad;
 };
 
 __global__ void __launch_bounds__(kClusterThreads) k_clustering(ClusterDev d) {
-  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.n) return;
-  const unsigned p = __ldg(d.focal + t);
-  const float2 fi = __ldg(d.xy32 + p);
-  const unsigned b = __ldg(d.group_begin + p), e = __ldg(d.group_end + p);
-  const double xi = __ldg(d.x + p), yi = __ldg(d.y + p);
-  const unsigned long long focal_ce = __ldg(d.ce + p);
-  const double xlo = __dsub_rn(xi, d.half_window), xhi = __dadd_rn(xi, d.half_window);
-  const double ylo = __dsub_rn(yi, d.half_window), yhi = __dadd_rn(yi, d.half_window);
-  double total = 0.0, focal = 0.0, sum = 0.0;
-  unsigned long long cur = __ldg(d.ce + b);
-  for (unsigned j = b; j < e; ++j) {
-    const unsigned long long cj = __ldg(d.ce + j);
-    if (cj != cur) {   // one clock enable's expectation is complete
-      total = __dadd_rn(total, soft_ceiling(sum, 2.0));
-      if (cur == focal_ce) focal = sum;
-      sum = 0.0;
-      cur = cj;
-    }
-    // far in FP32 (with margin) implies far in FP64: skip without FP64 work
-    const float2 fj = __ldg(d.xy32 + j);
-    if (fabsf(fi.x - fj.x) > d.cutoff32 || fabsf(fi.y - fj.y) > d.cutoff32) continue;
-    const double xj = __ldg(d.x + j), yj = __ldg(d.y + j);
-    if (fabs(__dsub_rn(xi, xj)) > d.cutoff || fabs(__dsub_rn(yi, yj)) > d.cutoff) continue;
-    const double px = window_probability(xlo, xhi, xj, d.scale);
-    const double py = window_probability(ylo, yhi, yj, d.scale);
-    sum = __dadd_rn(sum, __dmul_rn(px, py));
+  __shared__ Window table[kIntervals];
+  {
+    const double* src = reinterpret_cast<const double*>(d.table);
+    double* dst = reinterpret_cast<double*>(table);
+    for (int i = threadIdx.x; i < (int)(sizeof(table) / 8); i += kClusterThreads) dst[i] = __ldg(src + i);
   }
-  total = __dadd_rn(total, soft_ceiling(sum, 2.0));
+  __syncthreads();
+  const unsigned all = 0xffffffffu;
+  const unsigned t = blockIdx.x * kClusterThreads + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  const bool active = t < d.n;
+  const unsigned p = __ldg(d.focal + (active ? t : d.n - 1));
+  const float2 fi = __ldg(d.xy32 + p);
+  const unsigned gb = __ldg(d.group_begin + p), ge = __ldg(d.group_end + p);
+  const double2 at = __ldg(d.xy + p);
+  const unsigned long long focal_ce = __ldg(d.ce + p);
+  double total = 0.0, focal = 0.0, sum = 0.0;
+  unsigned long long cur = 0;
+  // the warp's control sets in turn (one but where two meet)
+  for (unsigned todo = __ballot_sync(all, active); todo;) {
+    const int lead = __ffs(todo) - 1;
+    const unsigned b = __shfl_sync(all, gb, lead), e = __shfl_sync(all, ge, lead);
+    const bool mine = active && gb == b;
+    todo &= ~__ballot_sync(all, mine);
+    // the box within which a register may be near one of the warp's
+    float x0 = mine ? fi.x : INFINITY, x1 = mine ? fi.x : -INFINITY, y0 = mine ? fi.y : INFINITY,
+          y1 = mine ? fi.y : -INFINITY;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      x0 = fminf(x0, __shfl_xor_sync(all, x0, o));
+      x1 = fmaxf(x1, __shfl_xor_sync(all, x1, o));
+      y0 = fminf(y0, __shfl_xor_sync(all, y0, o));
+      y1 = fmaxf(y1, __shfl_xor_sync(all, y1, o));
+    }
+    if (mine) {
+      cur = __ldg(d.ce + b);
+    }
+    float2 fj = b + lane < e ? __ldg(d.xy32 + b + lane) : make_float2(NAN, NAN);
+    for (unsigned j0 = b; j0 < e; j0 += 32) {
+      const float2 f = fj;
+      if (j0 + 32 + lane < e) fj = __ldg(d.xy32 + j0 + 32 + lane);
+      const bool in = j0 + lane < e && f.x - x1 <= d.cutoff32 && x0 - f.x <= d.cutoff32 && f.y - y1 <= d.cutoff32 &&
+                      y0 - f.y <= d.cutoff32;
+      for (unsigned m = __ballot_sync(all, in); m; m &= m - 1) {
+        const int q = __ffs(m) - 1;
+        const float2 g = make_float2(__shfl_sync(all, f.x, q), __shfl_sync(all, f.y, q));
+        if (!mine) continue;
+        // far in FP32 (with margin) implies far in FP64: skip without FP64 work
+        const bool near = !(fabsf(fi.x - g.x) > d.cutoff32 || fabsf(fi.y - g.y) > d.cutoff32);
+        const unsigned long long cj = __ldg(d.ce + j0 + q);
+        if (cj != cur) {   // one clock enable's expectation is complete
+          total = __dadd_rn(total, soft_ceiling(sum, 2.0, 0.5));
+          if (cur == focal_ce) focal = sum;
+          sum = 0.0;
+          cur = cj;
+        }
+        if (!near) continue;
+        const double2 c = __ldg(d.xy + j0 + q);
+        const double dx = __dsub_rn(at.x, c.x), dy = __dsub_rn(at.y, c.y);
+        if (fabs(dx) > d.cutoff || fabs(dy) > d.cutoff) continue;
+        const double px = window_probability(dx, d.inv_scale, table), py = window_probability(dy, d.inv_scale, table);
+        sum = __dadd_rn(sum, __dmul_rn(px, py));
+      }
+    }
+  }
+  if (!active) return;
+  total = __dadd_rn(total, soft_ceiling(sum, 2.0, 0.5));
   if (cur == focal_ce) focal = sum;
   const unsigned out = __ldg(d.order + p);
   if (!(isfinite(focal) && focal > 0.0)) {
@@ -98,8 +209,9 @@ __global__ void __launch_bounds__(kClusterThreads) k_clustering(ClusterDev d) {
     return;
   }
   // 8 / E_focal * ceil2(E_focal) / total * ceil4(total), left to right
-  const double area = __dmul_rn(__ddiv_rn(__dmul_rn(__ddiv_rn(8.0, focal), soft_ceiling(focal, 2.0)), total),
-                                soft_ceiling(total, 4.0));
+  const double area =
+      __dmul_rn(__ddiv_rn(__dmul_rn(__ddiv_rn(8.0, focal), soft_ceiling(focal, 2.0, 0.5)), total),
+                soft_ceiling(total, 4.0, 0.25));
   if (!(isfinite(area) && area >= 0.0)) atomicExch(d.bad, 1);
   d.areas[out] = area;
 }
@@ -131,7 +243,7 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
   const double sigma = std::sqrt(1.0e-5 * (double)(uint32_t)movable_instance_count);
   if (!std::isfinite(sigma) || sigma <= 0.0) return TEXO_GP_ERR_INVALID_NORMALIZATION;
   const double half_window = 2.5 * sigma, scale = sigma * 1.4142135623730951;   // sigma sqrt(2)
-  const double cutoff = half_window + 8.0 * scale;
+  const double cutoff = half_window + 6.0 * scale;   // kReach in units of scale
 
   // sort by (clock, lsr, ce), stable: input order within a clock enable
   std::vector<uint32_t> order(n);
@@ -142,19 +254,19 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
       return clock_lsr[2 * (size_t)a + 1] < clock_lsr[2 * (size_t)b + 1];
     return ce[a] < ce[b];
   });
-  std::vector<double> sx(n), sy(n);
+  std::vector<double> sxy(2 * n);
   std::vector<float> s32(2 * n);
   std::vector<unsigned long long> sce(n);
   std::vector<uint32_t> gb(n), ge(n), focal(n);
   double extent = 0.0;
   for (uint64_t p = 0; p < n; ++p) {
-    sx[p] = xy[2 * (size_t)order[p]];
-    sy[p] = xy[2 * (size_t)order[p] + 1];
-    s32[2 * p] = (float)sx[p];
-    s32[2 * p + 1] = (float)sy[p];
+    for (int k = 0; k < 2; ++k) {
+      const double v = xy[2 * (size_t)order[p] + k];
+      sxy[2 * p + k] = v;
+      s32[2 * p + k] = (float)v;
+      if (std::isfinite(v)) extent = std::max(extent, std::fabs(v));
+    }
     sce[p] = ce[order[p]];
-    if (std::isfinite(sx[p])) extent = std::max(extent, std::fabs(sx[p]));
-    if (std::isfinite(sy[p])) extent = std::max(extent, std::fabs(sy[p]));
   }
   for (uint64_t p = 0; p < n;) {
     uint64_t q = p + 1;
@@ -166,14 +278,25 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
       gb[r] = (uint32_t)p;
       ge[r] = (uint32_t)q;
     }
-    // the threads of a control set take its registers in tile order (rows
-    // of 8-tile blocks), so a warp's registers are near one another and
-    // agree on which pairs are far
+    // the threads of a control set take its registers block by block, the
+    // blocks of a size that holds about a warp's 32 of them
     std::iota(focal.begin() + p, focal.begin() + q, (uint32_t)p);
+    double lo[2] = {1e300, 1e300}, hi[2] = {-1e300, -1e300};
+    for (uint64_t r = p; r < q; ++r)
+      for (int k = 0; k < 2; ++k)
+        if (std::isfinite(sxy[2 * r + k])) {
+          lo[k] = std::min(lo[k], sxy[2 * r + k]);
+          hi[k] = std::max(hi[k], sxy[2 * r + k]);
+        }
+    const double side = std::max(1.0, std::sqrt(32.0 * std::max(hi[0] - lo[0], 1.0) * std::max(hi[1] - lo[1], 1.0) /
+                                                (double)(q - p)));
     auto block_of = [&](uint32_t r) -> uint64_t {
-      const double bx = std::isfinite(sx[r]) ? std::floor(sx[r] / 8.0) : 0.0;
-      const double by = std::isfinite(sy[r]) ? std::floor(sy[r] / 8.0) : 0.0;
-      return ((uint64_t)(int64_t)(by + 1.0e6) << 32) | (uint64_t)(uint32_t)(int64_t)(bx + 1.0e6);
+      uint64_t at[2];
+      for (int k = 0; k < 2; ++k) {
+        const double v = sxy[2 * (size_t)r + k];
+        at[k] = std::isfinite(v) ? (uint64_t)std::min(std::floor((v - lo[k]) / side), 1.0e9) : 0;
+      }
+      return at[1] << 32 | at[0];
     };
     std::stable_sort(focal.begin() + p, focal.begin() + q,
                      [&](uint32_t a, uint32_t b) { return block_of(a) < block_of(b); });
@@ -195,11 +318,9 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
   }
   ClusterDev d{};
   d.n = (unsigned)n;
-  d.half_window = half_window;
-  d.scale = scale;
+  d.inv_scale = 1.0 / scale;
   d.cutoff = cutoff;
-  double* dx = (double*)base;
-  double* dy = (double*)(base + s8);
+  double2* dxy = (double2*)base;
   unsigned long long* dce = (unsigned long long*)(base + 2 * s8);
   d.areas = (double*)(base + 3 * s8);
   unsigned* dgb = (unsigned*)(base + 4 * s8);
@@ -211,8 +332,7 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
   d.xy32 = d32;
   d.focal = dfoc;
   d.cutoff32 = cutoff32;
-  d.x = dx;
-  d.y = dy;
+  d.xy = dxy;
   d.ce = dce;
   d.group_begin = dgb;
   d.group_end = dge;
@@ -221,8 +341,8 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
   cudaEventCreate(&e0);
   cudaEventCreate(&e1);
   cudaEventRecord(e0, s);
-  bool ok = cudaMemcpyAsync(dx, sx.data(), n * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
-            cudaMemcpyAsync(dy, sy.data(), n * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+  bool ok = window_table(device, &d.table) == cudaSuccess &&
+            cudaMemcpyAsync(dxy, sxy.data(), n * 16, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(dce, sce.data(), n * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(dgb, gb.data(), n * 4, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(dge, ge.data(), n * 4, cudaMemcpyHostToDevice, s) == cudaSuccess &&
