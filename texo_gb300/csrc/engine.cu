@@ -81,12 +81,28 @@ cudaError_t keep_pool(int device) {
   if (e == cudaSuccess) done.push_back(device);
   return e;
 }
-// Host FP64 coordinates -> device FP32 optimizer buffer.
-int32_t upload_coords(Instance& I, float2* dst, const double* src, size_t nobj) {
-  std::vector<float> tmp(2 * nobj);
-  for (size_t i = 0; i < 2 * nobj; ++i) tmp[i] = (float)src[i];
-  CU(cudaMemcpyAsync(dst, tmp.data(), nobj * sizeof(float2), cudaMemcpyHostToDevice, I.stream));
-  CU(cudaStreamSynchronize(I.stream));
+// Device memory for one call's FP64 arrays, from the stream-ordered pool and
+// back to it when the call's work on the stream is done: nothing is added to
+// an instance's footprint.
+struct Staged {
+  cudaStream_t s;
+  char* p = nullptr;
+  explicit Staged(cudaStream_t stream) : s(stream) {}
+  Staged(const Staged&) = delete;
+  ~Staged() {
+    if (p) cudaFreeAsync(p, s);
+  }
+  cudaError_t get(size_t n) { return cudaMallocAsync((void**)&p, std::max<size_t>(n, 16), s); }
+};
+// Host FP64 coordinates -> device FP32 optimizer buffer, on the instance's
+// stream; `src` is read until the caller synchronizes.
+// With a `mark` (growing from call to call) SI_NONFINITE becomes it when a
+// coordinate is not finite.
+int32_t upload_coords(Instance& I, float2* dst, const double* src, size_t nobj, long long mark = 0) {
+  Staged buf(I.stream);
+  CU(buf.get(2 * nobj * sizeof(double)));
+  CU(cudaMemcpyAsync(buf.p, src, 2 * nobj * sizeof(double), cudaMemcpyHostToDevice, I.stream));
+  launch_narrow((const double*)buf.p, (float*)dst, 2 * nobj, mark ? I.r.iscal + SI_NONFINITE : nullptr, mark, I.stream);
   return TEXO_GP_OK;
 }
 std::vector<double> dct_basis(uint32_t n) {
@@ -739,8 +755,14 @@ struct Controller {
   std::vector<double> fixed_scales;
   uint64_t iter_offset = 0;
 
-  explicit Controller(Instance& i) : I(i), hr(i.h_run->run) { std::memset(&hr, 0, sizeof(hr)); }
+  explicit Controller(Instance& i) : I(i), coordinate_calls(i.coordinate_calls), hr(i.h_run->run) { std::memset(&hr, 0, sizeof(hr)); }
+  // texo_gp_evaluate's coordinate check: the event behind its flag, and the
+  // calls made (a flag equal to the call's number is this call's)
+  cudaEvent_t check_ev = nullptr;
+  long long& coordinate_calls;
+
   ~Controller() {
+    if (check_ev) cudaEventDestroy(check_ev);
     if (step_exec) cudaGraphExecDestroy(step_exec);
     for (cudaEvent_t e : step_ev)
       if (e) cudaEventDestroy(e);
@@ -1673,24 +1695,30 @@ uint32_t round_coord(double v, uint32_t extent) {
 int32_t handle_targets(texo_gp_handle h, uint32_t* out, double* coords, texo_gp_stats* st, int32_t status) {
   Instance& I = *h->inst;
   Controller& C = *h->ctl;
-  const size_t nobj = (size_t)I.d.nobj;
-  std::vector<float> best32(2 * (size_t)I.m.U), cur32(2 * nobj);
-  std::vector<double> best(2 * (size_t)I.m.U), cur(2 * nobj);
-  if (I.m.has_density)
-    CU(cudaMemcpyAsync(best32.data(), I.best, best32.size() * sizeof(float), cudaMemcpyDeviceToHost, I.stream));
-  CU(cudaMemcpyAsync(cur32.data(), I.bufX, cur32.size() * sizeof(float), cudaMemcpyDeviceToHost, I.stream));
+  const size_t nobj = (size_t)I.d.nobj, U = I.m.U;
   launch_hpwl(I.d, I.r, I.bufX, I.nvb, I.stream);
   launch_finalize(I.d, I.r, I.nvb, FIN_HPWL, I.stream);
   CU(cudaMemcpyAsync(I.h_scal + SC_HPWL, I.r.scal + SC_HPWL, sizeof(double), cudaMemcpyDeviceToHost, I.stream));
-  CU(cudaStreamSynchronize(I.stream));
-  for (size_t i = 0; i < best.size(); ++i) best[i] = I.m.has_density ? (double)best32[i] : I.m.init[i];
-  for (size_t i = 0; i < cur.size(); ++i) cur[i] = cur32[i];
-  if (out)
-    for (uint32_t u = 0; u < I.m.U; ++u) {
-      out[2 * (size_t)u] = round_coord(best[2 * (size_t)u], I.m.W);
-      out[2 * (size_t)u + 1] = round_coord(best[2 * (size_t)u + 1], I.m.H);
+  {
+    Staged buf(I.stream);
+    const bool rounded = out && I.m.has_density && U;   // without a density field the checkpoint is the initial point
+    const size_t cb = coords ? 2 * nobj * sizeof(double) : 0, tb = rounded ? 2 * U * sizeof(uint32_t) : 0;
+    if (cb + tb) {
+      CU(buf.get(cb + tb));
+      double* c = cb ? (double*)buf.p : nullptr;
+      uint32_t* t = tb ? (uint32_t*)(buf.p + cb) : nullptr;
+      launch_widen_point(I.d, I.best, I.bufX, t, c, I.stream);
+      if (cb) CU(cudaMemcpyAsync(coords, c, cb, cudaMemcpyDeviceToHost, I.stream));
+      if (tb) CU(cudaMemcpyAsync(out, t, tb, cudaMemcpyDeviceToHost, I.stream));
     }
-  if (coords) std::memcpy(coords, cur.data(), cur.size() * sizeof(double));
+    CU(cudaStreamSynchronize(I.stream));
+    CU(cudaGetLastError());
+    if (out && !rounded)
+      for (size_t u = 0; u < U; ++u) {
+        out[2 * u] = round_coord(I.m.init[2 * u], I.m.W);
+        out[2 * u + 1] = round_coord(I.m.init[2 * u + 1], I.m.H);
+      }
+  }
   if (st) {
     st->status = status;
     st->iterations = C.completed;
@@ -1863,12 +1891,54 @@ int32_t texo_gp_evaluate(texo_gp_handle h, const double* coordinates, double gam
   Instance& I = *h->inst;
   Controller& C = *h->ctl;
   const size_t nobj = (size_t)I.d.nobj, B = I.m.bins(), K = I.m.K;
-  for (size_t i = 0; i < 2 * nobj; ++i)
-    if (!std::isfinite(coordinates[i])) return TEXO_GP_ERR_NONFINITE_UNIT_COORDINATE;
-  TRY(upload_coords(I, I.bufY, coordinates, nobj));
-  EvalRec e;
-  TRY(C.evaluate(I.bufY, I.gY, gamma, false, e));
+  // The coordinates' finiteness is checked while they are narrowed; the
+  // evaluation is queued behind (a non-finite coordinate lands on the grid's
+  // edge there), and while it runs the host reads the check: nothing is given
+  // out unless it has passed.
+  const long long mark = ++C.coordinate_calls;
+  if (!C.check_ev) CU(cudaEventCreateWithFlags(&C.check_ev, cudaEventDisableTiming));
+  TRY(upload_coords(I, I.bufY, coordinates, nobj, mark));
+  CU(cudaMemcpyAsync(I.h_iscal + SI_NONFINITE, I.r.iscal + SI_NONFINITE, sizeof(long long), cudaMemcpyDeviceToHost,
+                     I.stream));
+  CU(cudaEventRecord(C.check_ev, I.stream));
   C.density_at_x = false;
+  C.enqueue_eval(I.bufY, I.gY, gamma, false);
+  Staged buf(I.stream);
+  const size_t counts[4] = {wa_gradient ? 2 * (size_t)I.m.U : 0, field_gradient ? K * 2 * nobj : 0,
+                            density ? K * B : 0, potential ? K * B : 0};
+  double* const host[4] = {wa_gradient, field_gradient, density, potential};
+  double* dev[4] = {nullptr, nullptr, nullptr, nullptr};
+  size_t total = 0;
+  for (size_t c : counts) total += (c + 1) & ~(size_t)1;   // each array starts on 16 bytes
+  if (total) {
+    CU(buf.get(total * sizeof(double)));
+    double* at = (double*)buf.p;
+    for (int i = 0; i < 4; ++i)
+      if (counts[i]) {
+        dev[i] = at;
+        at += (counts[i] + 1) & ~(size_t)1;
+      }
+    launch_widen_eval(I.d, dev[0], dev[1], dev[2], dev[3], I.stream);
+  }
+  CU(cudaEventSynchronize(C.check_ev));
+  if (I.h_iscal[SI_NONFINITE] == mark) {
+    CU(cudaStreamSynchronize(I.stream));
+    return TEXO_GP_ERR_NONFINITE_UNIT_COORDINATE;
+  }
+  CU(cudaMemcpyAsync(I.h_iscal, I.r.iscal, kIScalars * sizeof(long long), cudaMemcpyDeviceToHost, I.stream));
+  CU(cudaMemcpyAsync(I.h_scal, I.r.scal, kScalars * sizeof(double), cudaMemcpyDeviceToHost, I.stream));
+  for (int i = 0; i < 4; ++i)
+    if (counts[i])
+      CU(cudaMemcpyAsync(host[i], dev[i], counts[i] * sizeof(double), cudaMemcpyDeviceToHost, I.stream));
+  CU(cudaStreamSynchronize(I.stream));
+  CU(cudaGetLastError());
+  if (I.h_iscal[SI_TC_FAIL]) {
+    set_last_error("tensor-core DCT: an mbarrier wait ran out");
+    return TEXO_GP_ERR_DEVICE_TIMEOUT;
+  }
+  EvalRec e;
+  C.read_eval(e);
+  C.evaluations++;
   if (out) {
     out->wirelength = e.wa;
     out->num_fields = (uint32_t)K;
@@ -1884,37 +1954,6 @@ int32_t texo_gp_evaluate(texo_gp_handle h, const double* coordinates, double gam
       out->fields[f].overflow_fixed = e.overflow_fixed[f];
       out->fields[f].overflow_bins = (uint64_t)e.overflow_bins[f];
     }
-  }
-  if (wa_gradient) {
-    std::vector<long long> fix(2 * (size_t)I.m.U);
-    CU(cudaMemcpyAsync(fix.data(), I.d.wa_fix, fix.size() * 8, cudaMemcpyDeviceToHost, I.stream));
-    CU(cudaStreamSynchronize(I.stream));
-    for (size_t i = 0; i < fix.size(); ++i) wa_gradient[i] = (double)fix[i] * kInvFix;
-  }
-  if (field_gradient) {
-    std::vector<float2> g(K * nobj);
-    CU(cudaMemcpyAsync(g.data(), I.d.graw, g.size() * sizeof(float2), cudaMemcpyDeviceToHost, I.stream));
-    CU(cudaStreamSynchronize(I.stream));
-    for (size_t f = 0; f < K; ++f)
-      for (size_t o = 0; o < nobj; ++o) {
-        bool valid = o < I.m.U || (size_t)I.m.fil_field[o - I.m.U] == f;
-        const float2 v = valid ? g[f * nobj + o] : make_float2(0.f, 0.f);
-        field_gradient[f * 2 * nobj + 2 * o] = v.x;
-        field_gradient[f * 2 * nobj + 2 * o + 1] = v.y;
-      }
-  }
-  if (density) {
-    std::vector<long long> a(K * B), b(K * B);
-    CU(cudaMemcpyAsync(a.data(), I.d.phys, a.size() * 8, cudaMemcpyDeviceToHost, I.stream));
-    CU(cudaMemcpyAsync(b.data(), I.d.fill, b.size() * 8, cudaMemcpyDeviceToHost, I.stream));
-    CU(cudaStreamSynchronize(I.stream));
-    for (size_t i = 0; i < K * B; ++i) density[i] = (double)(a[i] + b[i]) * kInvFix;
-  }
-  if (potential) {
-    std::vector<float> p(K * B);
-    CU(cudaMemcpyAsync(p.data(), I.d.phi, p.size() * 4, cudaMemcpyDeviceToHost, I.stream));
-    CU(cudaStreamSynchronize(I.stream));
-    for (size_t i = 0; i < K * B; ++i) potential[i] = p[i];
   }
   return TEXO_GP_OK;
 }

@@ -143,97 +143,179 @@ __global__ void __launch_bounds__(kThreads) k_hpwl(Dev d, Partials p, const floa
 
 // Reduces the partials selected by `mask` in a fixed order and derives the
 // objective scalars (combined_objective / augmented_density_value_and_coefficient,
-// eplace.rs:1022-1044, 1111-1124).
-__global__ void __launch_bounds__(kThreads) k_finalize(Dev d, Reduce r, int nvb, int mask) {
-  __shared__ double shd[kThreads / 32];
-  __shared__ long long shl[kThreads / 32];
+// eplace.rs:1022-1044, 1111-1124). Each slot is folded by 128 threads (four
+// warps, one per SM sub-partition) in block_reduce_array's order, eight slots
+// side by side: a slot is a round trip to memory and a chain of FP64 adds of
+// 64 cycles each; the nine slots of an evaluation took 14.6 us one after
+// another at 1M cells and take 9.3 this way (two rounds of eight).
+constexpr int kFinThreads = 1024;
+constexpr int kMaxFinJobs = 6 * kMaxFields + 16;
+struct FinJob {
+  const void* a;
+  int op;    // 0 FP64 sum, 1 integer sum, 2 integer minimum, 3 FP64 maximum, 4 FP64 minimum
+};
+__device__ __forceinline__ unsigned long long fin_fold(const FinJob& j, int n, unsigned long long* warps, int t) {
+  auto fold = [&](auto zero, auto op) {
+    using T = decltype(zero);
+    const T* a = reinterpret_cast<const T*>(j.a);
+    T v = t < n ? a[t] : zero;
+#pragma unroll 4
+    for (int i = t + 128; i < n; i += 128) v = op(v, a[i]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+    T* w = reinterpret_cast<T*>(warps);
+    if ((t & 31) == 0) w[t >> 5] = v;
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + (int)(threadIdx.x >> 7)) : "memory");
+    const T r = op(op(op(w[0], w[1]), w[2]), w[3]);
+    asm volatile("bar.sync %0, 128;" ::"r"(1 + (int)(threadIdx.x >> 7)) : "memory");
+    unsigned long long bits;
+    memcpy(&bits, &r, 8);
+    return bits;
+  };
+  switch (j.op) {
+    case 0: return fold(0.0, OpAdd());
+    case 1: return fold(0ll, OpAdd());
+    case 2: return fold(0x7fffffffffffffffll, OpMin());
+    case 3: return fold(0.0, OpMax());
+    default: return fold((double)INFINITY, OpMin());
+  }
+}
+__global__ void __launch_bounds__(kFinThreads) k_finalize(Dev d, Reduce r, int nvb, int mask) {
+  __shared__ FinJob jobs[kMaxFinJobs];
+  __shared__ int to[kMaxFinJobs];               // output: scalar slot, or kScalars + integer slot
+  __shared__ int count;
+  __shared__ unsigned long long warps[kFinThreads / 128][4];
+  __shared__ double sc[kScalars];
   const Partials& p = r.p;
-  double* sc = r.scal;
-  long long* si = r.iscal;
-  if (mask & (FIN_ENERGY | FIN_WA)) {
-    const double wa = block_reduce_array(pslot(p, SLOT_WA_VALUE), nvb, 0.0, OpAdd(), shd);
-    if (threadIdx.x == 0) sc[SC_WA] = wa;
-  }
-  if (mask & FIN_ENERGY) {
-    for (int f = 0; f < d.K; ++f) {
-      const double e = block_reduce_array(pslot(p, SLOT_ENERGY + f), nvb, 0.0, OpAdd(), shd);
-      const long long ov = block_reduce_array(islot(p, IS_OVERFLOW + f), nvb, 0ll, OpAdd(), shl);
-      const long long bins = block_reduce_array(islot(p, IS_OVER_BINS + f), nvb, 0ll, OpAdd(), shl);
-      const long long gs = block_reduce_array(islot(p, IS_GRID_SUM + f), nvb, 0ll, OpAdd(), shl);
-      if (threadIdx.x == 0) {
-        sc[SC_ENERGY + f] = 0.5 * e;
-        si[SI_OVERFLOW_FIXED + f] = ov;
-        si[SI_OVER_BINS + f] = bins;
-        si[SI_GRID_SUM + f] = gs;
-        sc[SC_OVERFLOW + f] = ((double)ov * kInvFix) / sc[SC_REAL_AREA + f];
-        sc[SC_MEAN + f] = (double)(gs - d.capsum[f]) * kInvFix;
-      }
-    }
-  }
-  if (mask & (FIN_ENERGY | FIN_WA)) {
-    if (threadIdx.x == 0) {
-      double value = sc[SC_WA];
-      const double beta = sc[SC_BETA];
+  if (threadIdx.x < kScalars) sc[threadIdx.x] = r.scal[threadIdx.x];
+  if (threadIdx.x == 0) {
+    int n = 0;
+    auto add = [&](const void* a, int op, int out) {
+      jobs[n] = FinJob{a, op};
+      to[n++] = out;
+    };
+    if (mask & (FIN_ENERGY | FIN_WA)) add(pslot(p, SLOT_WA_VALUE), 0, SC_WA);
+    if (mask & FIN_ENERGY)
       for (int f = 0; f < d.K; ++f) {
-        const double e0 = sc[SC_E0 + f], lam = sc[SC_LAMBDA + f];
-        const double ne = sc[SC_ENERGY + f] / e0;
-        value += lam * e0 * (ne + 0.5 * beta * ne * ne);
-        sc[SC_COEF + f] = lam * (1.0 + beta * ne);
+        add(pslot(p, SLOT_ENERGY + f), 0, SC_ENERGY + f);
+        add(islot(p, IS_OVERFLOW + f), 1, kScalars + SI_OVERFLOW_FIXED + f);
+        add(islot(p, IS_OVER_BINS + f), 1, kScalars + SI_OVER_BINS + f);
+        add(islot(p, IS_GRID_SUM + f), 1, kScalars + SI_GRID_SUM + f);
       }
-      sc[SC_VALUE] = value;
+    if (mask & FIN_COMBINE) {
+      for (int f = 0; f < d.K; ++f) {
+        add(pslot(p, SLOT_RAWL1 + f), 0, SC_RAWL1 + f);
+        add(pslot(p, SLOT_FORCE + f), 0, SC_FORCE + f);
+      }
+      add(pslot(p, SLOT_WAL1), 0, SC_WAL1);
+      add(islot(p, IS_BAD), 2, kScalars + SI_BAD);
     }
-    __syncthreads();
+    if (mask & (FIN_CAND | FIN_DIFF)) add(islot(p, IS_DIFF), 1, kScalars + SI_DIFF);
+    if (mask & FIN_CAND) {
+      add(pslot(p, SLOT_DOT), 0, SC_DOT);
+      add(pslot(p, SLOT_MSN), 0, SC_MSN);
+    }
+    if (mask & FIN_KKT) {
+      add(mslot(p, MS_KKT), 3, SC_KKT);
+      add(mslot(p, MS_CHANGE), 3, SC_CHANGE);
+    }
+    if (mask & FIN_PRECOND) {
+      add(mslot(p, MS_PMIN), 4, SC_PMIN);
+      add(mslot(p, MS_PMAX), 3, SC_PMAX);
+      add(islot(p, IS_PBAD), 1, kScalars + SI_PBAD);
+    }
+    if (mask & FIN_HPWL) add(pslot(p, SLOT_HPWL), 0, SC_HPWL);
+    count = n;
   }
-  if (mask & FIN_COMBINE) {
+  __syncthreads();
+  const int g = threadIdx.x >> 7, t = threadIdx.x & 127;
+  for (int j = g; j < count; j += kFinThreads / 128) {
+    const unsigned long long v = fin_fold(jobs[j], nvb, warps[g], t);
+    if (t == 0) {
+      const int o = to[j];
+      if (o >= kScalars) {
+        r.iscal[o - kScalars] = (long long)v;
+        // the derived values of an integer sum, by the thread that has it
+        const int s = o - kScalars;
+        if (s >= SI_OVERFLOW_FIXED && s < SI_OVERFLOW_FIXED + kMaxFields) {
+          const int f = s - SI_OVERFLOW_FIXED;
+          r.scal[SC_OVERFLOW + f] = ((double)(long long)v * kInvFix) / sc[SC_REAL_AREA + f];
+        } else if (s >= SI_GRID_SUM && s < SI_GRID_SUM + kMaxFields) {
+          const int f = s - SI_GRID_SUM;
+          r.scal[SC_MEAN + f] = (double)((long long)v - d.capsum[f]) * kInvFix;
+        }
+      } else {
+        double x;
+        memcpy(&x, &v, 8);
+        if (o >= SC_ENERGY && o < SC_ENERGY + kMaxFields) x *= 0.5;
+        sc[o] = x;
+        r.scal[o] = x;
+      }
+    }
+  }
+  if (!(mask & (FIN_ENERGY | FIN_WA))) return;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double value = sc[SC_WA];
+    const double beta = sc[SC_BETA];
     for (int f = 0; f < d.K; ++f) {
-      const double a = block_reduce_array(pslot(p, SLOT_RAWL1 + f), nvb, 0.0, OpAdd(), shd);
-      const double b = block_reduce_array(pslot(p, SLOT_FORCE + f), nvb, 0.0, OpAdd(), shd);
-      if (threadIdx.x == 0) {
-        sc[SC_RAWL1 + f] = a;
-        sc[SC_FORCE + f] = b;
+      const double e0 = sc[SC_E0 + f], lam = sc[SC_LAMBDA + f];
+      const double ne = sc[SC_ENERGY + f] / e0;
+      value += lam * e0 * (ne + 0.5 * beta * ne * ne);
+      r.scal[SC_COEF + f] = lam * (1.0 + beta * ne);
+    }
+    r.scal[SC_VALUE] = value;
+  }
+}
+
+// The API's FP64 arrays on the device: the host arrays are copied as they are
+// (on this machine a copy from or to pageable memory runs at the pinned rate)
+// and narrowed or widened here. On one host core the conversions of a
+// million-cell call took 6.5 ms of its 15.
+__global__ void __launch_bounds__(kThreads) k_narrow(const double* __restrict__ src, float* __restrict__ dst, size_t n,
+                                                     long long* nonfinite, long long mark) {
+  bool bad = false;
+  for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += (size_t)gridDim.x * kThreads) {
+    const double v = src[i];
+    dst[i] = __double2float_rn(v);
+    bad = bad || !isfinite(v);
+  }
+  if (nonfinite && bad) atomicMax(nonfinite, mark);
+}
+// rounded_targets_from_coordinates (eplace.rs:954-971) of the checkpoint, and
+// the current coordinates; either output may be null.
+__global__ void __launch_bounds__(kThreads) k_widen_point(Dev d, const float2* best, const float2* x,
+                                                          uint2* __restrict__ targets, double2* __restrict__ coords) {
+  const float top_x = (float)(d.g.W - 1), top_y = (float)(d.g.H - 1);
+  for (int o = blockIdx.x * kThreads + threadIdx.x; o < d.nobj; o += gridDim.x * kThreads) {
+    if (targets && o < d.U) {
+      const float2 b = best[o];
+      targets[o] = make_uint2((uint32_t)fminf(fmaxf(roundf(b.x), 0.f), top_x),
+                              (uint32_t)fminf(fmaxf(roundf(b.y), 0.f), top_y));
+    }
+    if (coords) {
+      const float2 a = x[o];
+      coords[o] = make_double2((double)a.x, (double)a.y);
+    }
+  }
+}
+// texo_gp_evaluate's arrays; each may be null.
+__global__ void __launch_bounds__(kThreads) k_widen_eval(Dev d, double* __restrict__ wa, double2* __restrict__ field,
+                                                         double* __restrict__ density, double* __restrict__ potential) {
+  const int first = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
+  if (wa)
+    for (int i = first; i < 2 * d.U; i += stride) wa[i] = (double)(long long)d.wa_fix[i] * kInvFix;
+  if (field)
+    for (int f = 0; f < d.K; ++f)
+      for (int o = first; o < d.nobj; o += stride) {
+        const bool valid = o < d.U || d.fil_field[o - d.U] == f;
+        const float2 v = valid ? d.graw[(size_t)f * d.nobj + o] : make_float2(0.f, 0.f);
+        field[(size_t)f * d.nobj + o] = make_double2((double)v.x, (double)v.y);
       }
-    }
-    const double w = block_reduce_array(pslot(p, SLOT_WAL1), nvb, 0.0, OpAdd(), shd);
-    const long long bad = block_reduce_array(islot(p, IS_BAD), nvb, 0x7fffffffffffffffll, OpMin(), shl);
-    if (threadIdx.x == 0) {
-      sc[SC_WAL1] = w;
-      si[SI_BAD] = bad;
-    }
-  }
-  if (mask & (FIN_CAND | FIN_DIFF)) {
-    const long long diff = block_reduce_array(islot(p, IS_DIFF), nvb, 0ll, OpAdd(), shl);
-    if (threadIdx.x == 0) si[SI_DIFF] = diff;
-  }
-  if (mask & FIN_CAND) {
-    const double a = block_reduce_array(pslot(p, SLOT_DOT), nvb, 0.0, OpAdd(), shd);
-    const double b = block_reduce_array(pslot(p, SLOT_MSN), nvb, 0.0, OpAdd(), shd);
-    if (threadIdx.x == 0) {
-      sc[SC_DOT] = a;
-      sc[SC_MSN] = b;
-    }
-  }
-  if (mask & FIN_KKT) {
-    const double a = block_reduce_array(mslot(p, MS_KKT), nvb, 0.0, OpMax(), shd);
-    const double b = block_reduce_array(mslot(p, MS_CHANGE), nvb, 0.0, OpMax(), shd);
-    if (threadIdx.x == 0) {
-      sc[SC_KKT] = a;
-      sc[SC_CHANGE] = b;
-    }
-  }
-  if (mask & FIN_PRECOND) {
-    const double a = block_reduce_array(mslot(p, MS_PMIN), nvb, (double)INFINITY, OpMin(), shd);
-    const double b = block_reduce_array(mslot(p, MS_PMAX), nvb, 0.0, OpMax(), shd);
-    const long long c = block_reduce_array(islot(p, IS_PBAD), nvb, 0ll, OpAdd(), shl);
-    if (threadIdx.x == 0) {
-      sc[SC_PMIN] = a;
-      sc[SC_PMAX] = b;
-      si[SI_PBAD] = c;
-    }
-  }
-  if (mask & FIN_HPWL) {
-    const double a = block_reduce_array(pslot(p, SLOT_HPWL), nvb, 0.0, OpAdd(), shd);
-    if (threadIdx.x == 0) sc[SC_HPWL] = a;
-  }
+  if (density)
+    for (int i = first; i < d.K * d.B; i += stride) density[i] = (double)(d.phys[i] + d.fill[i]) * kInvFix;
+  if (potential)
+    for (int i = first; i < d.K * d.B; i += stride) potential[i] = (double)d.phi[i];
 }
 
 // rounded_targets_from_coordinates (eplace.rs:954-971) compared with the
@@ -356,7 +438,24 @@ void launch_hpwl(const Dev& d, const Reduce& r, const float2* pos, int nvb, cuda
 }
 void launch_finalize(const Dev& d, const Reduce& r, int nvb, int mask, cudaStream_t s) {
   COUNT;
-  k_finalize<<<1, kThreads, 0, s>>>(d, r, nvb, mask);
+  k_finalize<<<1, kFinThreads, 0, s>>>(d, r, nvb, mask);
+}
+static inline int wide_blocks(size_t n) { return (int)std::min<size_t>((n + kThreads - 1) / kThreads, 2048); }
+void launch_narrow(const double* src, float* dst, size_t n, long long* nonfinite, long long mark, cudaStream_t s) {
+  if (!n) return;
+  COUNT;
+  k_narrow<<<wide_blocks(n), kThreads, 0, s>>>(src, dst, n, nonfinite, mark);
+}
+void launch_widen_point(const Dev& d, const float2* best, const float2* x, uint32_t* targets, double* coords,
+                        cudaStream_t s) {
+  if (!d.nobj) return;
+  COUNT;
+  k_widen_point<<<wide_blocks((size_t)d.nobj), kThreads, 0, s>>>(d, best, x, (uint2*)targets, (double2*)coords);
+}
+void launch_widen_eval(const Dev& d, double* wa, double* field, double* density, double* potential, cudaStream_t s) {
+  COUNT;
+  k_widen_eval<<<wide_blocks(std::max<size_t>((size_t)d.nobj, (size_t)d.B)), kThreads, 0, s>>>(d, wa, (double2*)field,
+                                                                                             density, potential);
 }
 void launch_round_compare(const Dev& d, const float2* x, uint32_t* prev, int W, int H, unsigned long long* mismatch,
                           int nvb, cudaStream_t s) {
