@@ -351,10 +351,10 @@ __device__ __forceinline__ float2* stage_out(float4* buf) {
 
 // Pass 1: t1 = rows-DCT(rho). With `mean` (fixed-point mean per field) the
 // density preparation is folded in: rho = (phys + fill - mean) 2^-32 enters
-// the transform exactly (as a double-float), is stored rounded to FP32, and
-// the physical overflow is counted into the IS_OVERFLOW / IS_OVER_BINS
-// partials.
-template <int NB, class G>
+// the transform exactly (EXACT, as a double-float) or as the FP32 value that
+// is stored, and the physical overflow is counted into the IS_OVERFLOW /
+// IS_OVER_BINS partials.
+template <int NB, bool EXACT, class G>
 static __device__ __forceinline__ void rows_fwd(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
                                                 Shared& sh, const long long* mean, bool tables) {
   const int W = d.g.Wb, H = d.g.Hb, L = d.logW, GV = min(group_size(L), H), per = GV << L;
@@ -382,12 +382,13 @@ static __device__ __forceinline__ void rows_fwd(const G& g, const Dev& d, Partia
         } else {
           const long long ph = d.phys[base + e];
           const long long v = ph + d.fill[base + e] - mean[f];
-          d.rho[base + e] = __ll2float_rn(v) * kInvFixF;
+          const float rho = __ll2float_rn(v) * kInvFixF;
+          d.rho[base + e] = rho;
           if (ph > 0) {
             o += ph;
             c += 1;
           }
-          x = df_scale(df_from_ll(v), kInvFixF);
+          x = EXACT ? df_scale(df_from_ll(v), kInvFixF) : DF{rho, 0.f};
         }
         in[(e & ~(W - 1)) + mak(e & (W - 1), W)] = make_float2(x.hi, x.lo);
       }

@@ -282,11 +282,11 @@ cudaError_t shared_inv_eig(int device, uint32_t Wb, uint32_t Hb, float** out) {
 }  // namespace
 
 // Pinned host mirrors of the controller state, grid barrier and reduction
-// scalars of one instance, carved from shared slabs: page-locking memory per
+// scalars (two copies of these) of one instance, carved from shared slabs: page-locking memory per
 // instance would dominate admitting small jobs.
 namespace {
 constexpr size_t kMirrorBytes =
-    sizeof(RunBlock) + (((kScalars * sizeof(double) + kIScalars * sizeof(long long)) + 255) & ~(size_t)255);
+    sizeof(RunBlock) + ((2 * (kScalars * sizeof(double) + kIScalars * sizeof(long long)) + 255) & ~(size_t)255);
 static_assert(sizeof(RunBlock) % 256 == 0, "RunBlock keeps the scalars 256-byte aligned");
 std::mutex g_mirror_mu;
 std::vector<char*> g_mirror_free;
@@ -304,7 +304,7 @@ int32_t acquire_mirror(RunBlock** run, double** scal, long long** iscal) {
   std::memset(b, 0, kMirrorBytes);
   *run = (RunBlock*)b;
   *scal = (double*)(b + sizeof(RunBlock));
-  *iscal = (long long*)(b + sizeof(RunBlock) + kScalars * sizeof(double));
+  *iscal = (long long*)(b + sizeof(RunBlock) + 2 * kScalars * sizeof(double));
   return TEXO_GP_OK;
 }
 void release_mirror(RunBlock* run) {
@@ -761,7 +761,17 @@ struct Controller {
   cudaEvent_t check_ev = nullptr;
   long long& coordinate_calls;
 
+  // WA's stream and the events around it (the host engine's evaluations)
+  cudaStream_t side = nullptr;
+  cudaEvent_t side_ev[2] = {nullptr, nullptr};
+
   ~Controller() {
+    if (side) {
+      cudaStreamSynchronize(side);
+      cudaStreamDestroy(side);
+    }
+    for (cudaEvent_t e : side_ev)
+      if (e) cudaEventDestroy(e);
     if (check_ev) cudaEventDestroy(check_ev);
     if (step_exec) cudaGraphExecDestroy(step_exec);
     for (cudaEvent_t e : step_ev)
@@ -801,30 +811,49 @@ struct Controller {
   // Enqueues one objective evaluation (ContinuousProblem::evaluate +
   // combined_objective). With reuse, the density side of `pos` is the one
   // already on the device (same coordinates), and only WA and the
-  // combination are recomputed.
-  void enqueue_eval(const float2* pos, float2* g, double gam, bool reuse) {
+  // combination are recomputed. `cleared`: the launch that formed pos has
+  // reset the accumulators. `fin`: partials of earlier launches to finalize
+  // besides. `kkt`: the KKT residual of the gradient at pos with it.
+  //
+  // WA reads the positions alone and meets the density side only in the
+  // combination, so it runs on a second stream beside scatter, transforms and
+  // gather (at 512^2 the tensor-core passes fill 32 of 152 SMs, and an
+  // evaluation of 250k cells took 27 us longer with WA in line).
+  int32_t enqueue_eval(const float2* pos, float2* g, double gam, bool reuse, bool cleared = false, int fin = 0,
+                       bool kkt = false) {
     const Dev& D = I.d;
     cudaStream_t s = I.stream;
     const int nvb = I.nvb;
-    if (!reuse && I.m.has_density) {
-      launch_init(D, true, true, nvb, s);
+    const bool density = !reuse && I.m.has_density;
+    if (!cleared) launch_init(D, density, true, nvb, s);
+    if (density) {
+      if (!side) {
+        CU(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        for (cudaEvent_t& e : side_ev) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      }
+      CU(cudaEventRecord(side_ev[0], s));
+      CU(cudaStreamWaitEvent(side, side_ev[0], 0));
+      launch_wa(D, I.r, pos, gam, nvb, side);
+      CU(cudaEventRecord(side_ev[1], side));
       launch_scatter(D, I.r, pos, nvb, s);
-      launch_prep(D, I.r, nvb, s);
-      for (int st = 0; st < 4; ++st) launch_dct(D, I.r, st, nvb, s, &I.tmaps);
+      if (!D.fft) launch_prep(D, I.r, nvb, s);
+      for (int st = 0; st < 4; ++st) launch_dct(D, I.r, st, nvb, s, &I.tmaps, true);
       launch_gather(D, I.r, pos, nvb, s);
+      CU(cudaStreamWaitEvent(s, side_ev[1], 0));
       density_evaluations++;
     } else {
-      launch_init(D, false, true, nvb, s);
+      launch_wa(D, I.r, pos, gam, nvb, s);
     }
-    launch_wa(D, I.r, pos, gam, nvb, s);
-    launch_finalize(D, I.r, nvb, (reuse || !I.m.has_density) ? FIN_WA : FIN_ENERGY, s);
-    launch_combine(D, I.r, g, nvb, s);
-    launch_finalize(D, I.r, nvb, FIN_COMBINE, s);
+    launch_finalize(D, I.r, nvb, (density ? FIN_ENERGY : FIN_WA) | fin, s);
+    launch_combine(D, I.r, g, nvb, s, kkt ? pos : nullptr);
+    launch_finalize(D, I.r, nvb, FIN_COMBINE | (kkt ? FIN_KKT : 0), s);
     device_evaluations++;
+    return TEXO_GP_OK;
   }
-  void read_eval(EvalRec& e) const {
-    const double* sc = I.h_scal;
-    const long long* si = I.h_iscal;
+  // From the scalars last read (0), or those copied out before them (1).
+  void read_eval(EvalRec& e, int at = 0) const {
+    const double* sc = I.h_scal + at * kScalars;
+    const long long* si = I.h_iscal + at * kIScalars;
     e.value = sc[SC_VALUE];
     e.wa = sc[SC_WA];
     e.wal1 = sc[SC_WAL1];
@@ -840,7 +869,7 @@ struct Controller {
     e.bad = si[SI_BAD];
   }
   int32_t evaluate(const float2* pos, float2* g, double gam, bool reuse, EvalRec& e) {
-    enqueue_eval(pos, g, gam, reuse);
+    TRY(enqueue_eval(pos, g, gam, reuse));
     TRY(sync_read());
     read_eval(e);
     evaluations++;
@@ -978,14 +1007,42 @@ struct Controller {
     const int nvb = I.nvb;
     if (!std::isfinite(a) || a < 1.0) return TEXO_GP_ERR_INVALID_MOMENTUM_PARAMETER;
     if (has_L && (!std::isfinite(L) || L <= 0.0)) return TEXO_GP_ERR_INVALID_LIPSCHITZ_ESTIMATE;
-    // preconditioner range for the denominator checks
+    // One submission: the preconditioner (its range for the denominator
+    // checks), the origin's evaluation, the extrapolated point and its
+    // evaluation. The origin's scalars are copied out before the next
+    // evaluation overwrites them; the checks follow in their order once the
+    // host has waited, once. Without momentum the extrapolated point is the
+    // origin; should it turn out to be otherwise, its evaluation was the
+    // origin's own again and is not counted.
+    const double next = midpoint1(std::sqrt(1.0 + 4.0 * a * a));
+    const double e = std::isfinite(next) ? (a - 1.0) / next : 0.0;
+    const bool ahead = std::isfinite(next) && (float)e != 0.f;
     launch_precond(D, I.r, nvb, s);
-    launch_finalize(D, I.r, nvb, FIN_PRECOND, s);
+    TRY(enqueue_eval(I.bufX, I.gX, gam, density_at_x, false, FIN_PRECOND));
+    if (ahead) {
+      CU(cudaMemcpyAsync(I.h_scal + kScalars, I.r.scal, kScalars * sizeof(double), cudaMemcpyDeviceToHost, s));
+      CU(cudaMemcpyAsync(I.h_iscal + kIScalars, I.r.iscal, kIScalars * sizeof(long long), cudaMemcpyDeviceToHost, s));
+      launch_extrapolate(D, I.r, I.bufX, I.bufXp, e, I.bufY, nvb, s, true);
+      TRY(enqueue_eval(I.bufY, I.gY, gam, false, true, FIN_DIFF, true));
+    } else {
+      launch_kkt(D, I.r, I.bufX, I.gX, nullptr, nvb, s);
+      launch_finalize(D, I.r, nvb, FIN_KKT, s);
+    }
+    TRY(sync_read());
     EvalRec eo;
-    TRY(evaluate(I.bufX, I.gX, gam, density_at_x, eo));
+    read_eval(eo, ahead ? 1 : 0);
+    evaluations++;
     if (I.h_iscal[SI_PBAD]) return fail_norm("preconditioner out of range");
     const double pmin = I.h_scal[SC_PMIN], pmax = I.h_scal[SC_PMAX];
     TRY(checked(eo));
+    bool origin = !ahead || I.h_iscal[SI_DIFF] == 0;   // the extrapolated point is the origin
+    double origin_kkt = I.h_scal[SC_KKT];
+    if (ahead) {
+      if (origin)
+        density_evaluations--;   // the device still describes the origin's coordinates
+      else
+        density_at_x = false;
+    }
     bool restart = false;
     bool has_wL = has_L;
     double wL = L;
@@ -994,32 +1051,23 @@ struct Controller {
       const double momentum = restart ? 1.0 : a;
       const double next_m = midpoint1(std::sqrt(1.0 + 4.0 * momentum * momentum));
       if (!std::isfinite(next_m)) return TEXO_GP_ERR_ITERATION_OVERFLOW;
-      const double extrap = (momentum - 1.0) / next_m;
-      bool y_is_origin = true;
-      if (!restart) {
-        launch_extrapolate(D, I.r, I.bufX, I.bufXp, extrap, I.bufY, nvb, s);
-        launch_finalize(D, I.r, nvb, FIN_DIFF, s);
-        TRY(sync_read());
-        y_is_origin = I.h_iscal[SI_DIFF] == 0;
-      }
+      const bool y_is_origin = restart || origin;
       const float2* ybuf = y_is_origin ? I.bufX : I.bufY;
       const float2* gy = y_is_origin ? I.gX : I.gY;
-      double f_y = eo.value;
-      if (!y_is_origin) {
-        enqueue_eval(I.bufY, I.gY, gam, false);
-        density_at_x = false;
-      }
-      launch_kkt(D, I.r, ybuf, gy, nullptr, nvb, s);
-      launch_finalize(D, I.r, nvb, FIN_KKT, s);
-      TRY(sync_read());
+      double f_y = eo.value, y_stat = origin_kkt;
       if (!y_is_origin) {
         EvalRec ey;
         read_eval(ey);
         evaluations++;
         TRY(checked(ey));
         f_y = ey.value;
+      } else if (restart && !origin) {   // the origin's own residual was not needed so far
+        launch_kkt(D, I.r, I.bufX, I.gX, nullptr, nvb, s);
+        launch_finalize(D, I.r, nvb, FIN_KKT, s);
+        TRY(sync_read());
+        y_stat = origin_kkt = I.h_scal[SC_KKT];
+        origin = true;
       }
-      const double y_stat = I.h_scal[SC_KKT];
       if (!std::isfinite(y_stat)) return TEXO_GP_ERR_LINE_SEARCH_OVERFLOW;
       if (y_stat == 0.0) {
         if (!y_is_origin) {
@@ -1047,11 +1095,10 @@ struct Controller {
           if (!std::isfinite(tL)) return TEXO_GP_ERR_LINE_SEARCH_OVERFLOW;
           continue;
         }
-        launch_candidate(D, I.r, ybuf, gy, (float)std::fmin(1.0 / tL, 3.0e38), I.bufC, nvb, s);
-        launch_finalize(D, I.r, nvb, FIN_CAND, s);
-        // The candidate is evaluated speculatively in the same submission;
-        // it is discarded when the candidate equals y.
-        enqueue_eval(I.bufC, I.gC, gam, false);
+        launch_candidate(D, I.r, ybuf, gy, (float)std::fmin(1.0 / tL, 3.0e38), I.bufC, nvb, s, true);
+        // The candidate is evaluated speculatively in the same submission
+        // (its stationarity with it); it is discarded when it equals y.
+        TRY(enqueue_eval(I.bufC, I.gC, gam, false, true, FIN_CAND, true));
         density_at_x = false;
         TRY(sync_read());
         const long long changed = I.h_iscal[SI_DIFF];
@@ -1101,10 +1148,7 @@ struct Controller {
         if (!std::isfinite(tL)) return TEXO_GP_ERR_LINE_SEARCH_OVERFLOW;
       }
       if (restart_step) continue;
-      // accept: stationarity at the candidate and the coordinate change
-      launch_kkt(D, I.r, I.bufC, I.gC, I.bufX, nvb, s);
-      launch_finalize(D, I.r, nvb, FIN_KKT, s);
-      TRY(sync_read());
+      // accept, with a finite stationarity at the candidate
       if (!std::isfinite(I.h_scal[SC_KKT])) return TEXO_GP_ERR_LINE_SEARCH_OVERFLOW;
       std::swap(I.bufXp, I.bufX);   // previous <- origin
       std::swap(I.bufX, I.bufC);    // origin <- candidate
@@ -1902,7 +1946,7 @@ int32_t texo_gp_evaluate(texo_gp_handle h, const double* coordinates, double gam
                      I.stream));
   CU(cudaEventRecord(C.check_ev, I.stream));
   C.density_at_x = false;
-  C.enqueue_eval(I.bufY, I.gY, gamma, false);
+  TRY(C.enqueue_eval(I.bufY, I.gY, gamma, false));
   Staged buf(I.stream);
   const size_t counts[4] = {wa_gradient ? 2 * (size_t)I.m.U : 0, field_gradient ? K * 2 * nobj : 0,
                             density ? K * B : 0, potential ? K * B : 0};
@@ -2176,7 +2220,7 @@ int32_t texo_gp_stage_times(texo_gp_handle h, uint32_t reps, double* ms, uint32_
   CU(cudaEventCreate(&b));
   const double gam = I.m.gamma_base_tiles();
   // one evaluation first so that every input of every stage is populated
-  h->ctl->enqueue_eval(I.bufX, I.gX, gam, false);
+  TRY(h->ctl->enqueue_eval(I.bufX, I.gX, gam, false));
   launch_precond(D, I.r, nvb, s);
   for (uint32_t st = 0; st < kNumStages && st < capacity; ++st) {
     CU(cudaStreamSynchronize(s));
@@ -2203,7 +2247,7 @@ int32_t texo_gp_stage_times(texo_gp_handle h, uint32_t reps, double* ms, uint32_
     CU(cudaEventElapsedTime(&t, a, b));
     ms[st] = (double)t / reps;
     // restore the accumulation grids that repeated launches disturbed
-    if (st == 1 || st == 2) h->ctl->enqueue_eval(I.bufX, I.gX, gam, false);
+    if (st == 1 || st == 2) TRY(h->ctl->enqueue_eval(I.bufX, I.gX, gam, false));
   }
   CU(cudaStreamSynchronize(s));
   CU(cudaGetLastError());

@@ -9,14 +9,25 @@ namespace tgp {
 // The FFT form's three passes (dct_fft.cuh), NB = 2 for 1024 points. Four blocks
 // an SM for the row passes (1024^2 rows inverse: 39 us with 118 registers and
 // two blocks, 33 with 64 and four).
-template <int NB>
+// PREP: the density preparation folded in (k_prep's rho and overflow sums bit
+// for bit, one pass over the grids less: 11 us of 38 at 1024^2), each block
+// with groups folding the scatter's totals for the means.
+template <int NB, bool PREP>
 __global__ void __launch_bounds__(kThreads, 4) k_fft_rows_fwd(Dev d, Partials p) {
   __shared__ fft::Smem sm;
   __shared__ Shared sh;
-  fft::rows_fwd<NB>(whole_block(), d, p, blockIdx.x, gridDim.x, sm.buf, sh, nullptr, false);
+  __shared__ long long mean[kMaxFields];
+  if (PREP) {
+    for (int f = 0; f < d.K; ++f) {
+      const long long tot = block_reduce_array(islot(p, IS_GRID_SUM + f), (int)gridDim.x, 0ll, OpAdd(), sh.l);
+      if (threadIdx.x == 0) mean[f] = (tot - d.capsum[f]) / d.B;
+    }
+    __syncthreads();
+  }
+  fft::rows_fwd<NB, false>(whole_block(), d, p, blockIdx.x, gridDim.x, sm.buf, sh, PREP ? mean : nullptr, false);
 }
 template <int NB>
-__global__ void __launch_bounds__(kThreads) k_fft_cols(Dev d) {
+__global__ void __launch_bounds__(kThreads, NB == 2 ? 4 : 1) k_fft_cols(Dev d) {
   __shared__ fft::Smem sm;
   fft::cols<NB>(whole_block(), d, blockIdx.x, gridDim.x, sm.buf, false);
 }
@@ -113,19 +124,25 @@ __global__ void __launch_bounds__(kThreads) k_gather(Dev d, Partials p, const fl
   __shared__ Shared sh;
   stage_gather(whole_block(), d, pos, p, blockIdx.x, gridDim.x, sh);
 }
-__global__ void __launch_bounds__(kThreads) k_combine(Dev d, Partials p, const double* coef, float2* gout) {
+__global__ void __launch_bounds__(kThreads) k_combine(Dev d, Partials p, const double* coef, float2* gout,
+                                                     const float2* kkt_pos) {
   __shared__ Shared sh;
-  stage_combine(whole_block(), d, coef, gout, p, blockIdx.x, gridDim.x, sh);
+  __shared__ double buf[(kMaxFields + 1) * (kThreads + 4)];
+  stage_combine(whole_block(), d, coef, gout, p, blockIdx.x, gridDim.x, sh, buf, kMaxFields + 1, kkt_pos);
 }
+// The next point, and (reset) the accumulators cleared for its evaluation.
 __global__ void __launch_bounds__(kThreads) k_extrapolate(Dev d, Partials p, const float2* x, const float2* xp,
-                                                         float e, float2* y) {
+                                                         float e, float2* y, bool reset) {
   __shared__ Shared sh;
+  if (reset) stage_init(whole_block(), d, blockIdx.x, gridDim.x, true, true);
   stage_extrapolate(whole_block(), d, x, xp, e, y, p, blockIdx.x, gridDim.x, sh);
 }
 __global__ void __launch_bounds__(kThreads) k_candidate(Dev d, Partials p, const float2* y, const float2* gy,
-                                                       float invL, float2* c) {
+                                                       float invL, float2* c, bool reset) {
   __shared__ Shared sh;
-  stage_candidate(whole_block(), d, y, gy, invL, c, p, blockIdx.x, gridDim.x, sh);
+  __shared__ double buf[2 * (kThreads + 4)];
+  if (reset) stage_init(whole_block(), d, blockIdx.x, gridDim.x, true, true);
+  stage_candidate(whole_block(), d, y, gy, invL, c, p, blockIdx.x, gridDim.x, sh, buf);
 }
 __global__ void __launch_bounds__(kThreads) k_kkt(Dev d, Partials p, const float2* x, const float2* g,
                                                  const float2* ref) {
@@ -367,12 +384,13 @@ void launch_prep(const Dev& d, const Reduce& r, int nvb, cudaStream_t s) {
   COUNT;
   k_prep<<<nvb, kThreads, 0, s>>>(d, r.p);
 }
-void launch_dct(const Dev& d, const Reduce& r, int step, int nvb, cudaStream_t s, const tc::TcMaps* maps) {
+void launch_dct(const Dev& d, const Reduce& r, int step, int nvb, cudaStream_t s, const tc::TcMaps* maps, bool prep) {
   if (d.fft) {   // rows, columns (forward, scale, inverse), rows: step 2 has no work
     if (step == 2) return;
     COUNT;
     if (step == 0)
-      (d.logW == 10 ? k_fft_rows_fwd<2> : k_fft_rows_fwd<1>)<<<nvb, kThreads, 0, s>>>(d, r.p);
+      (prep ? (d.logW == 10 ? k_fft_rows_fwd<2, true> : k_fft_rows_fwd<1, true>)
+            : (d.logW == 10 ? k_fft_rows_fwd<2, false> : k_fft_rows_fwd<1, false>))<<<nvb, kThreads, 0, s>>>(d, r.p);
     else if (step == 1)
       (d.logH == 10 ? k_fft_cols<2> : k_fft_cols<1>)<<<nvb, kThreads, 0, s>>>(d);
     else
@@ -409,19 +427,19 @@ void launch_gather(const Dev& d, const Reduce& r, const float2* pos, int nvb, cu
   COUNT;
   k_gather<<<nvb, kThreads, 0, s>>>(d, r.p, pos);
 }
-void launch_combine(const Dev& d, const Reduce& r, float2* gout, int nvb, cudaStream_t s) {
+void launch_combine(const Dev& d, const Reduce& r, float2* gout, int nvb, cudaStream_t s, const float2* kkt_pos) {
   COUNT;
-  k_combine<<<nvb, kThreads, 0, s>>>(d, r.p, r.scal + SC_COEF, gout);
+  k_combine<<<nvb, kThreads, 0, s>>>(d, r.p, r.scal + SC_COEF, gout, kkt_pos);
 }
 void launch_extrapolate(const Dev& d, const Reduce& r, const float2* x, const float2* xp, float e, float2* y,
-                        int nvb, cudaStream_t s) {
+                        int nvb, cudaStream_t s, bool reset) {
   COUNT;
-  k_extrapolate<<<nvb, kThreads, 0, s>>>(d, r.p, x, xp, e, y);
+  k_extrapolate<<<nvb, kThreads, 0, s>>>(d, r.p, x, xp, e, y, reset);
 }
 void launch_candidate(const Dev& d, const Reduce& r, const float2* y, const float2* gy, float invL, float2* c,
-                      int nvb, cudaStream_t s) {
+                      int nvb, cudaStream_t s, bool reset) {
   COUNT;
-  k_candidate<<<nvb, kThreads, 0, s>>>(d, r.p, y, gy, invL, c);
+  k_candidate<<<nvb, kThreads, 0, s>>>(d, r.p, y, gy, invL, c, reset);
 }
 void launch_kkt(const Dev& d, const Reduce& r, const float2* x, const float2* g, const float2* ref, int nvb,
                 cudaStream_t s) {

@@ -69,13 +69,14 @@ void launch_spread_positions(const Dev& d, float2* out, int nvb, cudaStream_t s)
 void launch_wa(const Dev& d, const Reduce& r, const float2* pos, double gamma, int nvb, cudaStream_t s);
 void launch_prep(const Dev& d, const Reduce& r, int nvb, cudaStream_t s);
 void launch_dct(const Dev& d, const Reduce& r, int step, int nvb, cudaStream_t s,
-                const tc::TcMaps* maps = nullptr);
+                const tc::TcMaps* maps = nullptr, bool prep = false);   // prep: FFT form, step 0 prepares the density
 void launch_gather(const Dev& d, const Reduce& r, const float2* pos, int nvb, cudaStream_t s);
-void launch_combine(const Dev& d, const Reduce& r, float2* gout, int nvb, cudaStream_t s);
+void launch_combine(const Dev& d, const Reduce& r, float2* gout, int nvb, cudaStream_t s,
+                    const float2* kkt_pos = nullptr);
 void launch_extrapolate(const Dev& d, const Reduce& r, const float2* x, const float2* xp, float e, float2* y,
-                        int nvb, cudaStream_t s);
+                        int nvb, cudaStream_t s, bool reset = false);
 void launch_candidate(const Dev& d, const Reduce& r, const float2* y, const float2* gy, float invL, float2* c,
-                      int nvb, cudaStream_t s);
+                      int nvb, cudaStream_t s, bool reset = false);
 void launch_kkt(const Dev& d, const Reduce& r, const float2* x, const float2* g, const float2* ref, int nvb,
                 cudaStream_t s);
 void launch_precond(const Dev& d, const Reduce& r, int nvb, cudaStream_t s);

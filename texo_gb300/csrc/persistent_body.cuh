@@ -757,7 +757,7 @@ struct Ctx {
       const GA ga = half_a();
       for (int v = pb; v < V; v += np) {
         if (full) stage_gather(ga, d, pos, r.p, v, V, sh.a);
-        stage_combine(ga, d, L.coef, g, r.p, v, V, sh.a);
+        stage_combine(ga, d, L.coef, g, r.p, v, V, sh.a, sh.pair, 2);
       }
     }
     if (!sync()) return false;
@@ -1065,7 +1065,7 @@ static __device__ __noinline__ void run_rows_fwd() {
   Ctx<false, SETS> c(loop_state<SETS>());
 #pragma unroll 1
   for (int v = c.pb; v < c.V; v += c.np)
-    fft::rows_fwd<NB>(c.half_a(), c.d, c.r.p, v, c.V, c.gsm.fft, c.sh.a, c.L.fmean, c.L.tables);
+    fft::rows_fwd<NB, true>(c.half_a(), c.d, c.r.p, v, c.V, c.gsm.fft, c.sh.a, c.L.fmean, c.L.tables);
 }
 template <int NB, int SETS>
 static __device__ __noinline__ void run_cols() {

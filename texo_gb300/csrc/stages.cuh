@@ -81,6 +81,37 @@ template <typename T>
 __device__ __forceinline__ void write_partial(T v, T* slot, int vb, T* sh) {
   write_partial(whole_block(), v, slot, vb, sh);
 }
+// The first n of N FP64 block sums, each in block_fold_fp64's order, `cap` at
+// a time (buf: cap rows of kThreads + 4): their folds run side by side, a
+// quarter of a sum a warp. slot(i) is sum i's partial array.
+template <int N, class G, class Slot>
+__device__ __forceinline__ void write_partials(const G& g, const double (&v)[N], int n, Slot slot, int vb, double* buf,
+                                               int cap) {
+  constexpr int kRow = kThreads + 4;
+#pragma unroll 1
+  for (int c = 0; c < n; c += cap) {
+    const int m = min(cap, n - c);
+    g.sync();   // earlier readers of buf are done
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (i >= c && i < c + m) buf[(i - c) * kRow + g.tid] = v[i];
+    g.sync();
+#pragma unroll 1
+    for (int job = g.tid >> 5; job < 4 * m; job += kThreads / 32) {
+      double* b = buf + (job >> 2) * kRow;
+      const int at = (job & 3) * 32 + (g.tid & 31);
+      double t = b[at] + b[at + 128];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t = t + __shfl_xor_sync(0xffffffffu, t, o);
+      if ((g.tid & 31) == 0) b[kThreads + (job & 3)] = t;
+    }
+    g.sync();
+    if (g.tid < m) {
+      const double* b = buf + g.tid * kRow + kThreads;
+      slot(c + g.tid)[vb] = ((b[0] + b[1]) + b[2]) + b[3];
+    }
+  }
+}
 // Block max (or min) of per-thread FP32 values, written as FP64 partial vb:
 // folding in FP32 and widening once gives the same value as widening first.
 template <class G>
@@ -792,7 +823,7 @@ __device__ __forceinline__ float kkt_comp(float g, float x, float lo, float hi) 
 // reduced in the same pass (box_metric_kkt_residual, global_placement.rs:648-663).
 template <class G>
 static __device__ void stage_combine(const G& g, const Dev& d, const double* coef_d, float2* gout, Partials p,
-                                     int vb, int nvb, Shared& sh, const float2* kkt_pos = nullptr) {
+                                     int vb, int nvb, Shared& sh, double* buf, int cap, const float2* kkt_pos = nullptr) {
   float coef[kMaxFields];
 #pragma unroll
   for (int f = 0; f < kMaxFields; ++f) coef[f] = f < d.K ? (float)coef_d[f] : 0.f;
@@ -833,8 +864,10 @@ static __device__ void stage_combine(const G& g, const Dev& d, const double* coe
       kkt = fmaxf(kkt, kkt_comp(gy, a.y, lo.y, hi.y) * s);
     }
   }
-  for (int f = 0; f < d.K; ++f) write_partial(g, (double)rawl1[f], pslot(p, SLOT_RAWL1 + f), vb, sh.d);
-  write_partial(g, (double)wal1, pslot(p, SLOT_WAL1), vb, sh.d);
+  const double sums[kMaxFields + 1] = {(double)wal1, (double)rawl1[0], (double)rawl1[1], (double)rawl1[2],
+                                       (double)rawl1[3]};
+  write_partials(g, sums, d.K + 1, [&](int i) { return pslot(p, i == 0 ? SLOT_WAL1 : SLOT_RAWL1 + i - 1); }, vb, buf,
+                 cap);
   if (kkt_pos) write_partial_max(g, kkt, mslot(p, MS_KKT), vb, sh.f, false);
   {
     long long v = bad;
@@ -876,14 +909,14 @@ static __device__ void stage_extrapolate(const G& g, const Dev& d, const float2*
   write_partial(g, diff, islot(p, IS_DIFF), vb, sh.l);
 }
 
-// c = clamp(y - g / (L P)); changed count, <g, c - y>, sum P (c - y)^2.
-// With origin, also the max coordinate change |c - origin|.
+// c = clamp(y - g / (L P)); changed count, <g, c - y>, sum P (c - y)^2 (buf
+// holds two folds).
 template <class G>
 static __device__ void stage_candidate(const G& g, const Dev& d, const float2* y, const float2* gy,
                                        float invL, float2* c, Partials p, int vb, int nvb, Shared& sh,
-                                       const float2* origin = nullptr) {
+                                       double* buf) {
   long long diff = 0;
-  float dot = 0.f, msn = 0.f, ch = 0.f;
+  float dot = 0.f, msn = 0.f;
   const int stride = nvb * kThreads;
   for (int o = vb * kThreads + g.tid; o < d.nobj; o += stride) {
     const float2 a = y[o], gr = gy[o], lo = d.lo[o], hi = d.hi[o];
@@ -897,15 +930,10 @@ static __device__ void stage_candidate(const G& g, const Dev& d, const float2* y
     dot = fmaf(gr.x, dx, fmaf(gr.y, dy, dot));
     msn = fmaf(m * dx, dx, fmaf(m * dy, dy, msn));
     c[o] = r;
-    if (origin) {
-      const float2 b = origin[o];
-      ch = fmaxf(ch, fmaxf(fabsf(r.x - b.x), fabsf(r.y - b.y)));
-    }
   }
   write_partial(g, diff, islot(p, IS_DIFF), vb, sh.l);
-  write_partial(g, (double)dot, pslot(p, SLOT_DOT), vb, sh.d);
-  write_partial(g, (double)msn, pslot(p, SLOT_MSN), vb, sh.d);
-  if (origin) write_partial_max(g, ch, mslot(p, MS_CHANGE), vb, sh.f, false);
+  const double sums[2] = {(double)dot, (double)msn};
+  write_partials(g, sums, 2, [&](int i) { return pslot(p, i == 0 ? SLOT_DOT : SLOT_MSN); }, vb, buf, 2);
 }
 
 // box_metric_kkt_residual (global_placement.rs:648-663) and, optionally, the
