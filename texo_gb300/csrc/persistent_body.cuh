@@ -458,7 +458,7 @@ struct Ctx {
     long long* const grids = o < d.U ? d.phys : d.fill;
 #pragma unroll 1
     for (;;) {
-      const long long s = deposit_taps(d, (unsigned long long*)(grids + (size_t)f * d.B), m.z, tx(__fadd_rn(p.x, m.x)),
+      const long long s = deposit_taps<kSharedBinLoop>(d, (unsigned long long*)(grids + (size_t)f * d.B), m.z, tx(__fadd_rn(p.x, m.x)),
                                        ty(__fadd_rn(p.y, m.y)));
 #pragma unroll
       for (int ff = 0; ff < kMaxFields; ++ff)

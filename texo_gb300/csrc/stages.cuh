@@ -196,10 +196,43 @@ __device__ __forceinline__ Deposit deposit_of(const Dev& d, const float2* pos, i
   }
   return t;
 }
-// The nine taps of one charge into its grid; their fixed-point sum.
+// The nine taps of one charge into its grid; their fixed-point sum. Lanes of
+// a warp whose charges share the centre bin share all nine addresses: where
+// at least kSharedBin of them do, one lane deposits their sum (integers: the
+// grids do not change). Spread objects pay the match alone; but the line
+// search's first steps throw most objects into the corners of their box,
+// where every lane of every warp met the same few words (the slowest scatter
+// of a 1M-cell line search 925 -> 344 us, a spread one 47.3 -> 49.3). SHARED
+// is 3 in the standalone kernel (thresholds 2 / 3 / 4 / 8: three iterations at
+// 1M cells 6.8 / 6.9 / 7.0 / 8.5 ms) and 8 in the persistent loop, where a
+// small instance's few blocks hardly contend (4 / 8: device time of a 2k
+// placement 6.60 / 6.23 ms, of a 42k one 12.74 / 12.87).
+constexpr int kSharedBin = 3, kSharedBinLoop = 8;
+template <int SHARED>
 __device__ __forceinline__ long long deposit_taps(const Dev& d, unsigned long long* grid, float q, const AxisTaps& ax,
                                                   const AxisTaps& ay) {
+  const unsigned long long centre =
+      reinterpret_cast<unsigned long long>(grid + (size_t)ay.idx[1] * d.g.Wb + ax.idx[1]);
+  const unsigned same = __match_any_sync(__activemask(), centre);
   long long s = 0;
+  // a tap's high part (above 24 bits) sums in 32 bits over a warp while the
+  // charges stay below 2^17
+  if (__popc(same) >= SHARED && __all_sync(same, q < 131072.0f)) {
+    const bool first = (threadIdx.x & 31) == __ffs(same) - 1;
+#pragma unroll 1
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        const long long v = tap_fixed(q, ax.w[c], r == 0 ? ay.w[0] : r == 1 ? ay.w[1] : ay.w[2]);
+        s += v;
+        const unsigned hi = __reduce_add_sync(same, (unsigned)(v >> 24));
+        const unsigned lo = __reduce_add_sync(same, (unsigned)v & 0xffffffu);
+        if (first)
+          atomicAdd(grid + (size_t)(r == 0 ? ay.idx[0] : r == 1 ? ay.idx[1] : ay.idx[2]) * d.g.Wb + ax.idx[c],
+                    ((unsigned long long)hi << 24) + lo);
+      }
+    return s;
+  }
 #pragma unroll
   for (int r = 0; r < 3; ++r)
 #pragma unroll
@@ -219,7 +252,7 @@ __device__ __forceinline__ void scatter_items(const Dev& d, const float2* pos, i
   for (int f = 0; f < kMaxFields; ++f) tot[f] = 0;
   const int items = d.Mm + d.F;
   auto put = [&](const Deposit& t, const AxisTaps& ax, const AxisTaps& ay) {
-    const long long s = deposit_taps(d, t.grid, t.q, ax, ay);
+    const long long s = deposit_taps<kSharedBin>(d, t.grid, t.q, ax, ay);
 #pragma unroll
     for (int ff = 0; ff < kMaxFields; ++ff)
       if (ff == t.f) tot[ff] += s;
