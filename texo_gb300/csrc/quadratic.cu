@@ -2,25 +2,41 @@
 // Jacobi-preconditioned conjugate gradients for (D - W) x = b
 // (`solve_quadratic`, crates/texo-pnr/src/lib.rs:4586-4752), FP64.
 //
-// One cooperative persistent kernel runs the whole solve. Each block owns
-// rows strided over the grid; the products of a row (`multiply_quadratic`,
-// lib.rs:4767-4782: diagonal * v[i], then minus weight * v[j] in adjacency
-// order) and the vector updates use the reference's operations in its order
-// without contraction into FMAs, so a row's value is the reference's bit for
-// bit given the same inputs. The dot products fold per-block partials in a
-// fixed order (one warp per reduction), so the solve is deterministic, but
-// their rounding differs from the reference's left-to-right sums: the
-// iterates agree to rounding, not bit for bit.
+// One cooperative persistent kernel runs the whole solve, two grid barriers a
+// CG step:
+//   product: p = z + beta p_old and q = (D - W) p (`multiply_quadratic`,
+//     lib.rs:4767-4782) with the partial of <p, q>. The new direction is formed
+//     where it is read, from the pair (z, p_old) that one 16-byte load brings,
+//     by one fused operation that gives every reader the same bits;
+//   update: x += alpha p, r -= alpha q, z = r / D with the partials of <r, r>
+//     and <r, z>, and the pairs (z, p) of the next product, into the other of
+//     two buffers.
 //
-// A CG step takes three grid barriers: the product q = A p with the partial
-// <p, q>; the updates of x and r with <r, r>, z = r / D and <r, z>; the new
-// direction p = z + beta p. Partials alternate between two sets so a block
-// that leaves a barrier early never overwrites a set another block still
+// FP64 issue bounds it: two lanes a cycle on a multiprocessor, whether or not
+// a warp's lanes are all at work. So the matrix is laid out once, by each
+// block for the rows it owns, so that a warp's lanes stay busy: rows are cut
+// into segments of at most 16 entries, a thread takes a segment, and the
+// segments of a tile (the rows of up to 512 of them) are dealt to the warps in
+// order of length, entry k of a warp's 32 segments side by side. That is two
+// FP64 instructions a 32 entries, where eight lanes a row, the rows as they
+// come, spend 18 on four rows. At 42,000 unknowns and 565,000 entries (31
+// steps, about half of whose 14 us is the two barriers with their reductions):
+// 0.43 ms; eight lanes a row 1.00 ms; one thread a row, with a third barrier
+// for the direction, 1.2 ms. Segments of 8 entries took 0.07 ms more, eight
+// entries' loads in flight instead of four the same, a direct divide by the
+// diagonal 0.04 ms more, two blocks of half the registers (which spilled)
+// 0.04 ms more.
+//
+// Sums run in fixed orders (segments, trees, one warp per partial), so the
+// solve is deterministic; against the reference's left-to-right sums they
+// agree to rounding, not bit for bit. Partials alternate between two sets so a
+// block that leaves a barrier early never overwrites a set another block still
 // reads. Every wait is the bounded grid barrier of the placement engine.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <vector>
 
 #include "engine.h"
 #include "persistent_body.cuh"
@@ -39,209 +55,411 @@ struct PcgResult {
   double initial_rr, target, final_rr;
 };
 
+// A tile: the rows of one pass of a block, cut into at most kPcgThreads
+// segments of at most `segment` entries (kSegment, or what makes a longer row
+// fit); `base`: where its entries start in the dealt arrays.
+constexpr int kPcgThreads = 512;
+constexpr unsigned kSegment = 16;
+constexpr int kPcgWarps = kPcgThreads / 32;
+constexpr unsigned kAhead = 4;   // entries whose loads are in flight together
+struct PcgTile {
+  unsigned row0, rows, segment;
+  unsigned long long base;
+};
+
 struct PcgDev {
-  int n;
+  int n, tiles;
   const double *diag, *w, *b;
   const unsigned *ptr, *idx;
-  double *x, *r, *z, *p, *q;
-  double* part;          // [2 sets][kPcgSlots][kMaxPcgBlocks]
+  const PcgTile* tile;
+  double* dealt_w;           // a tile's warps in turn: entry k of its 32 segments side by side
+  unsigned* dealt_i;
+  uint2* warp;               // [tiles][kPcgWarps] where a warp's entries start in its tile, and how many a lane
+  unsigned short* place;     // [tiles][kPcgThreads] a thread's segment, by position in row order
+  unsigned* row_segments;    // [n] a row's first segment in its tile | their count << 16
+  double *x, *r, *p, *q, *inv;
+  double2* zp[2];            // (z, p) of the last update
+  double* part;              // [2 sets][kPcgSlots][kMaxPcgBlocks]
   GridBarrier* bar;
   PcgResult* out;
 };
 
-__device__ __forceinline__ double row_product(const PcgDev& d, const double* v, int i) {
-  double s = __dmul_rn(d.diag[i], v[i]);
-  for (unsigned k = d.ptr[i]; k < d.ptr[i + 1]; ++k) s = __dsub_rn(s, __dmul_rn(d.w[k], v[d.idx[k]]));
-  return s;
+struct PcgShared {
+  union {
+    struct {                       // while the tiles are laid out
+      unsigned first[kPcgThreads];       // a segment's first entry, from the tile's first
+      unsigned length[kPcgThreads];
+      unsigned short seg[kPcgThreads];   // by place
+      unsigned total[kPcgWarps];
+    } lay;
+    double sums[2][kPcgThreads];   // the segments' sums, of alternate tiles
+  };
+  double part[2][kPcgThreads];
+  double quarter[8];
+  FoldValue fv[kPcgSlots];
+  unsigned gen;
+  int failed;
+  // controller state, identical in every block (thread 0 writes it)
+  double rr, rho, alpha, beta, target;
+  unsigned iterations, restarts;
+  int stop, action;
+};
+
+// a / b from b's rounded reciprocal and one correction by the remainder
+// (Markstein 1990): three operations for the divide's nine, the result the
+// same but for the rarest ties. A diagonal near the ends of the range of
+// exponents has no such reciprocal (zero) and is divided by.
+__device__ __forceinline__ double reciprocal(double b) { return b > 1e-200 && b < 1e200 ? __drcp_rn(b) : 0.0; }
+__device__ __forceinline__ double quotient(double a, double b, double inverse) {
+  if (__double2hiint(inverse) == 0) return __ddiv_rn(a, b);
+  const double q = __dmul_rn(a, inverse);
+  return __fma_rn(__fma_rn(-q, b, a), inverse, q);
 }
 
-__global__ void __launch_bounds__(kThreads, 2) k_pcg(PcgDev d) {
-  __shared__ double sh[kThreads + 4];
-  __shared__ FoldValue fv[kPcgSlots];
-  __shared__ unsigned gen;
-  __shared__ int failed;
-  // controller state, identical in every block (thread 0 writes it)
-  __shared__ double rr, rho, alpha, beta, target;
-  __shared__ unsigned iterations, restarts;
-  __shared__ int stop, action;
-  const int pb = blockIdx.x, np = gridDim.x, n = d.n;
-  const int stride = np * blockDim.x;
-  unsigned long long nbar = 0;
-  unsigned phase = 0;
-  if (threadIdx.x == 0) {
-    gen = 0;   // the barrier is cleared before the launch
-    iterations = restarts = 0;
-    stop = 2;
+// Deals a tile's entries to the block's warps.
+__device__ void lay_out(const PcgDev& d, int t, PcgShared& S) {
+  const PcgTile tile = d.tile[t];
+  const unsigned tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const unsigned e0 = d.ptr[tile.row0];
+  unsigned b = 0, len = 0, count = 0;
+  if (tid < tile.rows) {
+    b = d.ptr[tile.row0 + tid];
+    len = d.ptr[tile.row0 + tid + 1] - b;
+    count = len / tile.segment + (len % tile.segment != 0);
+  }
+  unsigned at = count;   // the sum up to this row
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned v = __shfl_up_sync(0xffffffffu, at, o);
+    if (lane >= (unsigned)o) at += v;
+  }
+  if (lane == 31) S.lay.total[warp] = at;
+  __syncthreads();
+  unsigned before = 0, segments = 0;
+  for (int k = 0; k < kPcgWarps; ++k) {
+    if (k < (int)warp) before += S.lay.total[k];
+    segments += S.lay.total[k];
+  }
+  at += before - count;
+  if (tid < tile.rows) {
+    d.row_segments[tile.row0 + tid] = at | count << 16;
+    for (unsigned j = 0; j < count; ++j) {
+      S.lay.first[at + j] = b - e0 + j * tile.segment;
+      S.lay.length[at + j] = min(tile.segment, len - j * tile.segment);
+    }
   }
   __syncthreads();
+  // the longest first, equal ones in row order
+  if (tid < segments) {
+    const unsigned mine = S.lay.length[tid];
+    unsigned rank = 0;
+    for (unsigned j = 0; j < segments; ++j) {
+      const unsigned v = S.lay.length[j];
+      rank += v > mine || (v == mine && j < tid);
+    }
+    S.lay.seg[rank] = (unsigned short)tid;
+  }
+  __syncthreads();
+  // the four schedulers take the warps' loads in turn, then in reverse
+  const unsigned load = (warp & 4) ? warp ^ 3 : warp, place = 32 * load + lane;
+  unsigned start = 0, width = 0;
+  for (unsigned k = 0; k <= load; ++k) {
+    start += 32 * width;
+    width = 32 * k < segments ? S.lay.length[S.lay.seg[32 * k]] : 0;
+  }
+  if (lane == 0) d.warp[(size_t)t * kPcgWarps + warp] = make_uint2(start, width);
+  const bool some = place < segments;
+  const unsigned seg = some ? S.lay.seg[place] : place;   // a thread without one: a place of its own
+  d.place[(size_t)t * kPcgThreads + tid] = (unsigned short)seg;
+  const unsigned have = some ? S.lay.length[seg] : 0;
+  const size_t from = (size_t)e0 + (some ? S.lay.first[seg] : 0), to = tile.base + start + lane;
+  for (unsigned k = 0; k < width; ++k) {   // a lane with fewer entries adds zeros times a row of its tile
+    d.dealt_w[to + 32 * (size_t)k] = k < have ? d.w[from + k] : 0.0;
+    d.dealt_i[to + 32 * (size_t)k] = k < have ? d.idx[from + k] : tile.row0;
+  }
+  __syncthreads();
+}
+
+__global__ void __launch_bounds__(kPcgThreads, 1) k_pcg(PcgDev d) {
+  __shared__ PcgShared S;
+  const int pb = blockIdx.x, np = gridDim.x, n = d.n;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  unsigned long long nbar = 0;
+  unsigned phase = 0;
+  int cur = 0;         // the pair buffer the next product reads
+  int most = 0;        // the most rows of a tile of this block
+  if (tid == 0) {
+    S.gen = 0;   // the barrier is cleared before the launch
+    S.iterations = S.restarts = 0;
+    S.stop = 2;
+    S.beta = 0.0;
+  }
+  for (int t = pb; t < d.tiles; t += np) {
+    lay_out(d, t, S);
+    most = max(most, (int)d.tile[t].rows);
+  }
   auto slot = [&](int s) { return d.part + ((size_t)(phase & 1u) * kPcgSlots + s) * kMaxPcgBlocks; };
-  auto put = [&](int s, double v) {
-    const double t = block_fold_fp64(v, sh, FoldAdd());
-    if (threadIdx.x == 0) slot(s)[pb] = t;
+  // the block's partials of the phase: four warps a sum, a quarter of the
+  // threads' values each
+  auto put = [&](double a, double c, int slots) {
+    S.part[0][tid] = a;
+    if (slots > 1) S.part[1][tid] = c;
+    __syncthreads();
+    if (warp < 4 * slots) {
+      const double* v = S.part[warp >> 2];
+      double s = 0.0;
+      for (int i = (warp & 3) * 32 + lane; i < most; i += 128) s = __dadd_rn(s, v[i]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+      if (lane == 0) S.quarter[warp] = s;
+    }
+    __syncthreads();
+    if (tid < slots) {
+      const double* v = S.quarter + 4 * tid;
+      slot(tid)[pb] = __dadd_rn(__dadd_rn(v[0], v[1]), __dadd_rn(v[2], v[3]));
+    }
   };
   // barrier, then fold the slots of the phase that just ended
   auto sync_fold = [&](int nslots) -> bool {
-    if (!grid_sync(d.bar, (unsigned)np, &gen, &nbar, nullptr, &failed)) return false;
-    const int w = threadIdx.x >> 5;
-    if (w < nslots) {
-      const double* a = slot(w);
-      const double v = warp_fold(a, np, 0.0, OpAdd());
-      if ((threadIdx.x & 31) == 0) fv[w].d = v;
+    if (!grid_sync(d.bar, (unsigned)np, &S.gen, &nbar, nullptr, &S.failed)) return false;
+    if (warp < nslots) {
+      const double v = warp_fold(slot(warp), np, 0.0, OpAdd());
+      if (lane == 0) S.fv[warp].d = v;
     }
     __syncthreads();
     ++phase;
     return true;
   };
-  auto sync_only = [&]() -> bool {
-    if (!grid_sync(d.bar, (unsigned)np, &gen, &nbar, nullptr, &failed)) return false;
-    ++phase;
-    return true;
+  // what this thread needs to know of a tile; the first one's is kept
+  struct Work {
+    unsigned row0, rows, segment, segments, width, j[kAhead];
+    const double* w;
+    const unsigned* idx;
+  };
+  auto work = [&](int t) {
+    const PcgTile tile = d.tile[t];
+    const uint2 mine = d.warp[(size_t)t * kPcgWarps + warp];
+    Work k;
+    k.row0 = tile.row0;
+    k.rows = tile.rows;
+    k.segment = d.place[(size_t)t * kPcgThreads + tid];
+    k.segments = tid < (int)tile.rows ? d.row_segments[tile.row0 + tid] : 0;
+    k.width = mine.y;
+    k.w = d.dealt_w + tile.base + mine.x + lane;
+    k.idx = d.dealt_i + tile.base + mine.x + lane;
+#pragma unroll
+    for (unsigned u = 0; u < kAhead; ++u) k.j[u] = u < k.width ? k.idx[32 * u] : tile.row0;
+    return k;
+  };
+  const Work first = work(pb);
+  // For every row of the block's tiles: the sum of W's row times the vector
+  // that `load` and `value` give, handed to `row`.
+  auto product = [&](auto load, auto value, auto row) {
+    int odd = 0;
+    Work k = first;
+    for (int t = pb; t < d.tiles; t += np, odd ^= 1) {
+      Work next = k;
+      if (t + np < d.tiles) next = work(t + np);
+      double s = 0.0;
+      for (unsigned at = 0; at < k.width; at += kAhead) {
+        decltype(load(0u)) v[kAhead];
+        double w[kAhead];
+#pragma unroll
+        for (unsigned u = 0; u < kAhead; ++u) {
+          v[u] = load(k.j[u]);
+          w[u] = at + u < k.width ? k.w[32 * (size_t)(at + u)] : 0.0;
+        }
+#pragma unroll
+        for (unsigned u = 0; u < kAhead; ++u)
+          if (at + kAhead + u < k.width) k.j[u] = k.idx[32 * (size_t)(at + kAhead + u)];
+#pragma unroll
+        for (unsigned u = 0; u < kAhead; ++u)
+          if (at + u < k.width) s = __fma_rn(w[u], value(v[u]), s);
+      }
+      S.sums[odd][k.segment] = s;
+      __syncthreads();
+      if (tid < (int)k.rows) {
+        double total = 0.0;
+        const unsigned from = k.segments & 0xffffu, count = k.segments >> 16;
+        for (unsigned j = 0; j < count; ++j) total = j ? __dadd_rn(total, S.sums[odd][from + j]) : S.sums[odd][from];
+        row((int)k.row0 + tid, total);
+      }
+      k = next;
+    }
+  };
+  // r = b - (D - W) x with <r, r>; with `pairs` also z = r / D, the pairs
+  // (z, 0) and <r, z>
+  auto residual = [&](bool pairs) {
+    double a = 0.0, c = 0.0;
+    const double* x = d.x;
+    product([&](unsigned j) { return x[j]; }, [](double v) { return v; },
+            [&](int i, double s) {
+              const double ri = __dsub_rn(d.b[i], __dsub_rn(__dmul_rn(d.diag[i], d.x[i]), s));
+              d.r[i] = ri;
+              a = __dadd_rn(a, __dmul_rn(ri, ri));
+              if (pairs) {
+                const double zi = __ddiv_rn(ri, d.diag[i]);
+                d.inv[i] = reciprocal(d.diag[i]);
+                d.zp[cur][i] = make_double2(zi, 0.0);
+                c = __dadd_rn(c, __dmul_rn(ri, zi));
+              }
+            });
+    put(a, c, pairs ? 2 : 1);
   };
 
-  // r = b - A x, z = r / D, p = z; |r|^2 and <r, z>
-  {
-    double a = 0.0, c = 0.0;
-    for (int i = pb * blockDim.x + threadIdx.x; i < n; i += stride) {
-      const double ri = __dsub_rn(d.b[i], row_product(d, d.x, i));
-      const double zi = __ddiv_rn(ri, d.diag[i]);
-      d.r[i] = ri;
-      d.z[i] = zi;
-      d.p[i] = zi;
-      a = __dadd_rn(a, __dmul_rn(ri, ri));
-      c = __dadd_rn(c, __dmul_rn(ri, zi));
-    }
-    put(PS_A, a);
-    put(PS_B, c);
-  }
+  residual(true);
   if (!sync_fold(2)) return;
-  if (threadIdx.x == 0) {
-    rr = fv[PS_A].d;
-    if (pb == 0) d.out->initial_rr = rr;
-    target = fmax(rr, 2.220446049250313e-16) * kPcgTolerance;
-    rho = fv[PS_B].d;
+  if (tid == 0) {
+    S.rr = S.fv[PS_A].d;
+    if (pb == 0) d.out->initial_rr = S.rr;
+    S.target = fmax(S.rr, 2.220446049250313e-16) * kPcgTolerance;
+    S.rho = S.fv[PS_B].d;
   }
   __syncthreads();
 
   for (int loop = 0; loop < n; ++loop) {
-    if (rr <= target) break;
-    // q = A p and <p, q>
+    if (S.rr <= S.target) break;
+    // p = z + beta p, q = (D - W) p and <p, q>
     {
+      const double2* zp = d.zp[cur];
+      const double bt = S.beta;
       double a = 0.0;
-      for (int i = pb * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const double qi = row_product(d, d.p, i);
+      auto direction = [&](double2 v) { return __fma_rn(bt, v.y, v.x); };
+      product([&](unsigned j) { return zp[j]; }, direction, [&](int i, double s) {
+        const double pi = direction(zp[i]);
+        const double qi = __dsub_rn(__dmul_rn(d.diag[i], pi), s);
+        d.p[i] = pi;
         d.q[i] = qi;
-        a = __dadd_rn(a, __dmul_rn(d.p[i], qi));
-      }
-      put(PS_A, a);
+        a = __dadd_rn(a, __dmul_rn(pi, qi));
+      });
+      put(a, 0.0, 1);
     }
     if (!sync_fold(1)) return;
-    if (threadIdx.x == 0) {
-      const double den = fv[PS_A].d;
-      action = 0;
-      if (!isfinite(den) || den <= 0.0 || !isfinite(rho) || rho <= 0.0) {
-        action = 1;
+    if (tid == 0) {
+      const double den = S.fv[PS_A].d;
+      S.action = 0;
+      if (!isfinite(den) || den <= 0.0 || !isfinite(S.rho) || S.rho <= 0.0) {
+        S.action = 1;
       } else {
-        alpha = __ddiv_rn(rho, den);
-        if (!isfinite(alpha)) action = 1;
+        S.alpha = __ddiv_rn(S.rho, den);
+        if (!isfinite(S.alpha)) S.action = 1;
       }
-      if (action) stop = 1;
+      if (S.action) S.stop = 1;
     }
     __syncthreads();
-    if (action) break;
+    if (S.action) break;
     // x += alpha p, r -= alpha q; |r|^2, z = r / D, <r, z>
+    cur ^= 1;
     {
       double a = 0.0, c = 0.0;
-      for (int i = pb * blockDim.x + threadIdx.x; i < n; i += stride) {
-        d.x[i] = __dadd_rn(d.x[i], __dmul_rn(alpha, d.p[i]));
-        const double ri = __dsub_rn(d.r[i], __dmul_rn(alpha, d.q[i]));
-        const double zi = __ddiv_rn(ri, d.diag[i]);
+      const double al = S.alpha;
+      for (int t = pb; t < d.tiles; t += np) {
+        const PcgTile tile = d.tile[t];
+        if (tid >= (int)tile.rows) continue;
+        const int i = (int)tile.row0 + tid;
+        const double pi = d.p[i];
+        d.x[i] = __dadd_rn(d.x[i], __dmul_rn(al, pi));
+        const double ri = __dsub_rn(d.r[i], __dmul_rn(al, d.q[i]));
+        const double zi = quotient(ri, d.diag[i], d.inv[i]);
         d.r[i] = ri;
-        d.z[i] = zi;
+        d.zp[cur][i] = make_double2(zi, pi);
         a = __dadd_rn(a, __dmul_rn(ri, ri));
         c = __dadd_rn(c, __dmul_rn(ri, zi));
       }
-      put(PS_A, a);
-      put(PS_B, c);
+      put(a, c, 2);
     }
     if (!sync_fold(2)) return;
-    if (threadIdx.x == 0) {
-      iterations++;
-      rr = fv[PS_A].d;
-      action = rr <= target ? 2 : 0;
-      if (!action) {
-        const double next = fv[PS_B].d;
+    if (tid == 0) {
+      S.iterations++;
+      S.rr = S.fv[PS_A].d;
+      S.action = S.rr <= S.target ? 2 : 0;
+      if (!S.action) {
+        const double next = S.fv[PS_B].d;
         if (!isfinite(next) || next <= 0.0) {
-          stop = 1;
-          action = 1;
+          S.stop = 1;
+          S.action = 1;
         } else {
-          beta = __ddiv_rn(next, rho);
-          rho = next;
+          S.beta = __ddiv_rn(next, S.rho);
+          S.rho = next;
         }
       }
     }
     __syncthreads();
-    if (action == 1) break;
-    if (action == 2) {
+    if (S.action == 1) break;
+    if (S.action == 2) {
       // the recursive residual says converged: recompute the true one
       // (lib.rs:4656-4677) and restart from it when it is not small enough
-      {
-        double a = 0.0, c = 0.0;
-        for (int i = pb * blockDim.x + threadIdx.x; i < n; i += stride) {
-          const double ri = __dsub_rn(d.b[i], row_product(d, d.x, i));
-          const double zi = __ddiv_rn(ri, d.diag[i]);
-          d.r[i] = ri;
-          d.z[i] = zi;
-          d.p[i] = zi;   // the restart direction, used only if the check fails
-          a = __dadd_rn(a, __dmul_rn(ri, ri));
-          c = __dadd_rn(c, __dmul_rn(ri, zi));
-        }
-        put(PS_A, a);
-        put(PS_B, c);
-      }
+      // (p = z: the pairs' second parts are zero)
+      residual(true);
       if (!sync_fold(2)) return;
-      if (threadIdx.x == 0) {
-        rr = fv[PS_A].d;
-        action = 0;
-        if (rr > target) {
-          const double next = fv[PS_B].d;
-          restarts++;
+      if (tid == 0) {
+        S.rr = S.fv[PS_A].d;
+        S.action = 0;
+        if (S.rr > S.target) {
+          const double next = S.fv[PS_B].d;
+          S.restarts++;
+          S.beta = 0.0;
           if (!isfinite(next) || next <= 0.0) {
-            stop = 1;
-            action = 1;
+            S.stop = 1;
+            S.action = 1;
           } else {
-            rho = next;
+            S.rho = next;
           }
         }
       }
       __syncthreads();
-      if (action == 1) break;
-      continue;   // p = z is already in place (or the loop test ends the solve)
+      if (S.action == 1) break;
     }
-    // p = z + beta p
-    for (int i = pb * blockDim.x + threadIdx.x; i < n; i += stride)
-      d.p[i] = __dadd_rn(d.z[i], __dmul_rn(beta, d.p[i]));
-    if (!sync_only()) return;
   }
 
   // the true final residual (finish_quadratic_solve, lib.rs:4702-4752)
-  {
-    double a = 0.0;
-    for (int i = pb * blockDim.x + threadIdx.x; i < n; i += stride) {
-      const double ri = __dsub_rn(d.b[i], row_product(d, d.x, i));
-      a = __dadd_rn(a, __dmul_rn(ri, ri));
-    }
-    put(PS_A, a);
-  }
+  residual(false);
   if (!sync_fold(1)) return;
-  if (pb == 0 && threadIdx.x == 0) {
+  if (pb == 0 && tid == 0) {
     PcgResult& o = *d.out;
-    o.final_rr = fv[PS_A].d;
-    o.target = target;
-    o.iterations = iterations;
-    o.restarts = restarts;
-    o.converged = o.final_rr <= target ? 1 : 0;
-    o.stop = o.converged ? 0 : stop;
+    o.final_rr = S.fv[PS_A].d;
+    o.target = S.target;
+    o.iterations = S.iterations;
+    o.restarts = S.restarts;
+    o.converged = o.final_rr <= S.target ? 1 : 0;
+    o.stop = o.converged ? 0 : S.stop;
   }
+}
+
+// Cuts the rows into tiles of about equal work, at most kPcgThreads segments
+// each, and as many on each multiprocessor; a small system into tiles of 64
+// segments or more (fewer blocks meet sooner at the barriers). `padded`: the
+// entries with what fills the warps up, which is less than 32 of a tile's
+// longest segment.
+std::vector<PcgTile> cut_tiles(uint32_t n, const uint32_t* ptr, int sms, int* blocks, uint64_t* padded) {
+  uint64_t segments = 0;
+  for (uint32_t i = 0; i < n; ++i)
+    segments += std::min<uint64_t>(std::max<uint64_t>(1, ((uint64_t)ptr[i + 1] - ptr[i] + kSegment - 1) / kSegment),
+                                   kPcgThreads);
+  const uint64_t fit = kPcgThreads - kPcgThreads / 8;   // boundaries fall up to a row late
+  uint64_t want = std::max<uint64_t>(1, segments / 64);
+  if (want > (uint64_t)sms) want = (segments + fit * sms - 1) / (fit * sms) * sms;
+  constexpr uint64_t kRowCost = 16;   // a row's own operations, in entries
+  const uint64_t cost = ptr[n] + kRowCost * n;
+  std::vector<PcgTile> tiles;
+  uint64_t base = 0, done = 0, in_tile = 0;
+  for (uint32_t i = 0; i < n; ++i) {
+    const uint64_t len = (uint64_t)ptr[i + 1] - ptr[i];
+    uint64_t segs = std::max<uint64_t>(1, (len + kSegment - 1) / kSegment);
+    const bool alone = segs > kPcgThreads;   // a long row is its own tile, of longer segments
+    const bool due = done * want >= (uint64_t)tiles.size() * cost;
+    if (tiles.empty() || due || in_tile + segs > kPcgThreads) {
+      if (!tiles.empty()) base += (uint64_t)ptr[i] - ptr[tiles.back().row0] + 32ull * tiles.back().segment;
+      tiles.push_back({i, 0, alone ? (unsigned)((len + kPcgThreads - 1) / kPcgThreads) : kSegment, base});
+      in_tile = 0;
+    }
+    tiles.back().rows++;
+    in_tile += alone ? (uint64_t)kPcgThreads : segs;
+    done += len + kRowCost;
+  }
+  *padded = base + ((uint64_t)ptr[n] - ptr[tiles.back().row0]) + 32ull * tiles.back().segment;
+  *blocks = (int)std::min<uint64_t>((uint64_t)sms, tiles.size());
+  return tiles;
 }
 
 }  // namespace
@@ -279,21 +497,27 @@ extern "C" int32_t texo_gp_quadratic_solve(int32_t device, uint32_t n, const dou
   if (cudaSetDevice(device) != cudaSuccess) return fail(TEXO_GP_ERR_CUDA, "cudaSetDevice failed");
   static const int per_sm = [] {   // thread-safe one-time initialisation
     int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pcg, kThreads, 0) != cudaSuccess) b = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pcg, kPcgThreads, 0) != cudaSuccess) b = 0;
     return b;
   }();
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   if (per_sm <= 0 || sms <= 0) return fail(TEXO_GP_ERR_CUDA, "k_pcg cannot be resident");
-  const int blocks = (int)std::min<uint64_t>(std::min<uint64_t>((uint64_t)std::min(per_sm, 2) * sms, kMaxPcgBlocks),
-                                             std::max<uint64_t>(1, (n + kThreads - 1) / kThreads));
+  int blocks = 0;
+  uint64_t padded = 0;
+  const std::vector<PcgTile> tiles = cut_tiles(n, adjacency_ptr, std::min(sms, kMaxPcgBlocks), &blocks, &padded);
 
   // one allocation: vectors, matrix, partials, barrier, result
   auto round = [](size_t b) { return (b + 255) & ~(size_t)255; };
   const size_t vec = round((size_t)n * 8), nz8 = round(std::max<uint64_t>(nnz, 1) * 8),
                nz4 = round(std::max<uint64_t>(nnz, 1) * 4), p4 = round(((size_t)n + 1) * 4);
   const size_t part = round((size_t)2 * kPcgSlots * kMaxPcgBlocks * 8);
-  const size_t total = 8 * vec + nz8 + nz4 + p4 + part + round(sizeof(GridBarrier)) + round(sizeof(PcgResult));
+  const size_t pad8 = round(padded * 8), pad4 = round(padded * 4), rows4 = round((size_t)n * 4),
+               tile_bytes = round(tiles.size() * sizeof(PcgTile)),
+               warp_bytes = round(tiles.size() * kPcgWarps * sizeof(uint2)),
+               place_bytes = round(tiles.size() * kPcgThreads * sizeof(unsigned short));
+  const size_t total = 11 * vec + nz8 + nz4 + p4 + part + pad8 + pad4 + rows4 + tile_bytes + warp_bytes + place_bytes +
+                       round(sizeof(GridBarrier)) + round(sizeof(PcgResult));
   cudaStream_t s = nullptr;
   if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return fail(TEXO_GP_ERR_CUDA, "stream");
   char* base = nullptr;
@@ -313,13 +537,22 @@ extern "C" int32_t texo_gp_quadratic_solve(int32_t device, uint32_t n, const dou
   double* b = (double*)take(vec);
   d.x = (double*)take(vec);
   d.r = (double*)take(vec);
-  d.z = (double*)take(vec);
   d.p = (double*)take(vec);
   d.q = (double*)take(vec);
-  take(vec);   // spare (keeps the layout 256-byte aligned for any n)
+  d.inv = (double*)take(vec);
+  d.zp[0] = (double2*)take(2 * vec);
+  d.zp[1] = (double2*)take(2 * vec);
   double* w = (double*)take(nz8);
   unsigned* idx = (unsigned*)take(nz4);
   unsigned* ptr = (unsigned*)take(p4);
+  d.dealt_w = (double*)take(pad8);
+  d.dealt_i = (unsigned*)take(pad4);
+  d.row_segments = (unsigned*)take(rows4);
+  PcgTile* tile = (PcgTile*)take(tile_bytes);
+  d.warp = (uint2*)take(warp_bytes);
+  d.place = (unsigned short*)take(place_bytes);
+  d.tile = tile;
+  d.tiles = (int)tiles.size();
   d.part = (double*)take(part);
   d.bar = (GridBarrier*)take(round(sizeof(GridBarrier)));
   d.out = (PcgResult*)take(round(sizeof(PcgResult)));
@@ -341,11 +574,12 @@ extern "C" int32_t texo_gp_quadratic_solve(int32_t device, uint32_t n, const dou
             cudaMemcpyAsync(ptr, adjacency_ptr, ((size_t)n + 1) * 4, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             (!nnz || (cudaMemcpyAsync(idx, adjacency_index, nnz * 4, cudaMemcpyHostToDevice, s) == cudaSuccess &&
                       cudaMemcpyAsync(w, adjacency_weight, nnz * 8, cudaMemcpyHostToDevice, s) == cudaSuccess)) &&
+            cudaMemcpyAsync(tile, tiles.data(), tiles.size() * sizeof(PcgTile), cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemsetAsync(d.bar, 0, sizeof(GridBarrier), s) == cudaSuccess &&
             cudaMemsetAsync(d.out, 0, sizeof(PcgResult), s) == cudaSuccess;
   if (ok) {
     void* args[] = {&d};
-    ok = cudaLaunchCooperativeKernel((const void*)k_pcg, dim3(blocks), dim3(kThreads), args, 0, s) == cudaSuccess;
+    ok = cudaLaunchCooperativeKernel((const void*)k_pcg, dim3(blocks), dim3(kPcgThreads), args, 0, s) == cudaSuccess;
     if (ok) note_launch();
   }
   GridBarrier hb{};
