@@ -38,6 +38,7 @@
 #include <string>
 #include <vector>
 
+#include "call.h"
 #include "engine.h"
 #include "persistent_body.cuh"
 
@@ -512,14 +513,11 @@ int32_t run_auction(int32_t device, AucHost& h, int32_t* assignment, uint32_t* p
   const size_t sz_occ = round(h.occ ? m : 1), sz_txy = round(2 * std::max<uint64_t>(n, 1) * 4);
   const size_t total = 2 * sz_m4 + sz_bid + 5 * sz_n4 + sz_act + sz_touch + 2 * sz_nnz + sz_ptr + sz_occ + sz_txy +
                        round(32) + round(sizeof(GridBarrier)) + round(sizeof(AucResult));
-  cudaStream_t s = nullptr;
-  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess)
-    return fail_with(st, TEXO_GP_ERR_CUDA, "cudaStreamCreate failed");
-  char* base = nullptr;
-  if (cudaMallocAsync((void**)&base, total, s) != cudaSuccess) {
-    cudaStreamDestroy(s);
-    return fail_with(st, TEXO_GP_ERR_OUT_OF_MEMORY, "cudaMallocAsync failed");
-  }
+  Call call(device);
+  if (!call.ok()) return fail_with(st, TEXO_GP_ERR_CUDA, "cudaStreamCreate failed");
+  const cudaStream_t s = call.stream();
+  char* base = call.memory(total);
+  if (!base) return fail_with(st, TEXO_GP_ERR_OUT_OF_MEMORY, "cudaMallocAsync failed");
   char* at = base;
   auto take = [&](size_t b) {
     char* r = at;
@@ -551,10 +549,7 @@ int32_t run_auction(int32_t device, AucHost& h, int32_t* assignment, uint32_t* p
   d.cnt = (unsigned*)take(round(32));
   d.bar = (GridBarrier*)take(round(sizeof(GridBarrier)));
   d.out = (AucResult*)take(round(sizeof(AucResult)));
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  cudaEventRecord(e0, s);   // timed: the input copies, the launch, the copies back
+  call.start();   // timed: the input copies, the launch, the copies back
   const size_t ptr_bytes = ((h.grid ? slots : n) + 1) * 4;
   bool ok = cudaMemcpyAsync(ptr, h.grid ? h.tptr : h.dptr, ptr_bytes, cudaMemcpyHostToDevice, s) == cudaSuccess;
   if (nnz)
@@ -593,15 +588,8 @@ int32_t run_auction(int32_t device, AucHost& h, int32_t* assignment, uint32_t* p
        cudaMemcpyAsync(&hb, d.bar, sizeof(GridBarrier), cudaMemcpyDeviceToHost, s) == cudaSuccess;
   if (prices_out && m)
     ok = ok && cudaMemcpyAsync(prices_out, d.price, m * 4, cudaMemcpyDeviceToHost, s) == cudaSuccess;
-  cudaEventRecord(e1, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess) ok = false;
   float ms = 0.f;
-  cudaEventElapsedTime(&ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  cudaFreeAsync(base, s);
-  cudaStreamSynchronize(s);
-  cudaStreamDestroy(s);
+  if (!call.finish(&ms)) ok = false;
   int32_t code = TEXO_GP_OK;
   if (!ok) {
     code = TEXO_GP_ERR_CUDA;

@@ -35,9 +35,12 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <limits>
+#include <new>
 #include <string>
 #include <vector>
 
+#include "call.h"
 #include "engine.h"
 #include "persistent_body.cuh"
 
@@ -52,6 +55,7 @@ struct PcgResult {
   unsigned iterations, restarts;
   int stop;             // 0 residual, 1 breakdown, 2 dimension
   int converged;
+  int wrong_entry;      // an entry's index or weight is refused
   double initial_rr, target, final_rr;
 };
 
@@ -173,10 +177,22 @@ __device__ void lay_out(const PcgDev& d, int t, PcgShared& S) {
   d.place[(size_t)t * kPcgThreads + tid] = (unsigned short)seg;
   const unsigned have = some ? S.lay.length[seg] : 0;
   const size_t from = (size_t)e0 + (some ? S.lay.first[seg] : 0), to = tile.base + start + lane;
+  bool wrong = false;
   for (unsigned k = 0; k < width; ++k) {   // a lane with fewer entries adds zeros times a row of its tile
-    d.dealt_w[to + 32 * (size_t)k] = k < have ? d.w[from + k] : 0.0;
-    d.dealt_i[to + 32 * (size_t)k] = k < have ? d.idx[from + k] : tile.row0;
+    double w = 0.0;
+    unsigned idx = tile.row0;
+    if (k < have) {
+      w = d.w[from + k];
+      idx = d.idx[from + k];
+      if (idx >= (unsigned)d.n || (__double2hiint(w) & 0x7ff00000) == 0x7ff00000) {   // infinite or not a number
+        wrong = true;
+        idx = tile.row0;
+      }
+    }
+    d.dealt_w[to + 32 * (size_t)k] = w;
+    d.dealt_i[to + 32 * (size_t)k] = idx;
   }
+  if (wrong) atomicExch(&d.out->wrong_entry, 1);
   __syncthreads();
 }
 
@@ -309,6 +325,7 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg(PcgDev d) {
 
   residual(true);
   if (!sync_fold(2)) return;
+  if (__ldcg(&d.out->wrong_entry)) return;   // set before the barrier: every block leaves
   if (tid == 0) {
     S.rr = S.fv[PS_A].d;
     if (pb == 0) d.out->initial_rr = S.rr;
@@ -483,18 +500,26 @@ extern "C" int32_t texo_gp_quadratic_solve(int32_t device, uint32_t n, const dou
   const uint64_t nnz = adjacency_ptr[n];
   if (adjacency_ptr[0] != 0 || (nnz && (!adjacency_index || !adjacency_weight)))
     return fail(TEXO_GP_ERR_INVALID_ARGUMENT, "adjacency_ptr must start at 0");
-  for (uint32_t i = 0; i < n; ++i) {
-    if (adjacency_ptr[i + 1] < adjacency_ptr[i]) return fail(TEXO_GP_ERR_INVALID_ARGUMENT, "adjacency_ptr decreases");
-    if (!(std::isfinite(diagonal[i]) && diagonal[i] > 0.0))
-      return fail(TEXO_GP_ERR_INVALID_ARGUMENT, "diagonal entries must be finite and positive");
-    if (!std::isfinite(rhs[i]) || !std::isfinite(solution[i]))
-      return fail(TEXO_GP_ERR_INVALID_ARGUMENT, "non-finite right-hand side or initial solution");
-  }
-  for (uint64_t k = 0; k < nnz; ++k)
-    if (adjacency_index[k] >= n || !std::isfinite(adjacency_weight[k]))
-      return fail(TEXO_GP_ERR_INVALID_ARGUMENT, "adjacency index out of range or non-finite weight");
+  // no early way out: these loops are vectorized
+  constexpr double kMax = std::numeric_limits<double>::max();
+  unsigned decreases = 0, diagonals = 0, vectors = 0;
+  for (uint32_t i = 0; i < n; ++i) decreases |= adjacency_ptr[i + 1] < adjacency_ptr[i];
+  for (uint32_t i = 0; i < n; ++i) diagonals |= !(diagonal[i] > 0.0) | !(diagonal[i] <= kMax);
+  for (uint32_t i = 0; i < n; ++i) vectors |= !(std::fabs(rhs[i]) <= kMax) | !(std::fabs(solution[i]) <= kMax);
+  if (decreases) return fail(TEXO_GP_ERR_INVALID_ARGUMENT, "adjacency_ptr decreases");
+  if (diagonals) return fail(TEXO_GP_ERR_INVALID_ARGUMENT, "diagonal entries must be finite and positive");
+  if (vectors) return fail(TEXO_GP_ERR_INVALID_ARGUMENT, "non-finite right-hand side or initial solution");
+  // The entries are checked where the kernel deals them; without a device,
+  // here, so that a wrong system is refused as such.
+  const char* const kWrongEntry = "adjacency index out of range or non-finite weight";
+  auto no_device = [&](int32_t st, const std::string& why) {
+    for (uint64_t k = 0; k < nnz; ++k)
+      if (adjacency_index[k] >= n || !std::isfinite(adjacency_weight[k]))
+        return fail(TEXO_GP_ERR_INVALID_ARGUMENT, kWrongEntry);
+    return fail(st, why);
+  };
 
-  if (cudaSetDevice(device) != cudaSuccess) return fail(TEXO_GP_ERR_CUDA, "cudaSetDevice failed");
+  if (cudaSetDevice(device) != cudaSuccess) return no_device(TEXO_GP_ERR_CUDA, "cudaSetDevice failed");
   static const int per_sm = [] {   // thread-safe one-time initialisation
     int b = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_pcg, kPcgThreads, 0) != cudaSuccess) b = 0;
@@ -502,10 +527,15 @@ extern "C" int32_t texo_gp_quadratic_solve(int32_t device, uint32_t n, const dou
   }();
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  if (per_sm <= 0 || sms <= 0) return fail(TEXO_GP_ERR_CUDA, "k_pcg cannot be resident");
+  if (per_sm <= 0 || sms <= 0) return no_device(TEXO_GP_ERR_CUDA, "k_pcg cannot be resident");
   int blocks = 0;
   uint64_t padded = 0;
-  const std::vector<PcgTile> tiles = cut_tiles(n, adjacency_ptr, std::min(sms, kMaxPcgBlocks), &blocks, &padded);
+  std::vector<PcgTile> tiles;
+  try {
+    tiles = cut_tiles(n, adjacency_ptr, std::min(sms, kMaxPcgBlocks), &blocks, &padded);
+  } catch (const std::bad_alloc&) {
+    return no_device(TEXO_GP_ERR_OUT_OF_MEMORY, "no memory for the tiles");
+  }
 
   // one allocation: vectors, matrix, partials, barrier, result
   auto round = [](size_t b) { return (b + 255) & ~(size_t)255; };
@@ -518,13 +548,11 @@ extern "C" int32_t texo_gp_quadratic_solve(int32_t device, uint32_t n, const dou
                place_bytes = round(tiles.size() * kPcgThreads * sizeof(unsigned short));
   const size_t total = 11 * vec + nz8 + nz4 + p4 + part + pad8 + pad4 + rows4 + tile_bytes + warp_bytes + place_bytes +
                        round(sizeof(GridBarrier)) + round(sizeof(PcgResult));
-  cudaStream_t s = nullptr;
-  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return fail(TEXO_GP_ERR_CUDA, "stream");
-  char* base = nullptr;
-  if (cudaMallocAsync((void**)&base, total, s) != cudaSuccess) {
-    cudaStreamDestroy(s);
-    return fail(TEXO_GP_ERR_OUT_OF_MEMORY, "cudaMallocAsync failed");
-  }
+  Call call(device);
+  if (!call.ok()) return no_device(TEXO_GP_ERR_CUDA, "stream");
+  const cudaStream_t s = call.stream();
+  char* base = call.memory(total);
+  if (!base) return no_device(TEXO_GP_ERR_OUT_OF_MEMORY, "cudaMallocAsync failed");
   char* at = base;
   auto take = [&](size_t b) {
     char* r = at;
@@ -562,12 +590,9 @@ extern "C" int32_t texo_gp_quadratic_solve(int32_t device, uint32_t n, const dou
   d.idx = idx;
   d.ptr = ptr;
 
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
   int32_t st = TEXO_GP_OK;
   PcgResult res{};
-  cudaEventRecord(e0, s);
+  call.start();
   bool ok = cudaMemcpyAsync(diag, diagonal, (size_t)n * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(b, rhs, (size_t)n * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(d.x, solution, (size_t)n * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
@@ -586,21 +611,16 @@ extern "C" int32_t texo_gp_quadratic_solve(int32_t device, uint32_t n, const dou
   ok = ok && cudaMemcpyAsync(solution, d.x, (size_t)n * 8, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
        cudaMemcpyAsync(&res, d.out, sizeof(PcgResult), cudaMemcpyDeviceToHost, s) == cudaSuccess &&
        cudaMemcpyAsync(&hb, d.bar, sizeof(GridBarrier), cudaMemcpyDeviceToHost, s) == cudaSuccess;
-  cudaEventRecord(e1, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess) ok = false;
   float ms = 0.f;
-  cudaEventElapsedTime(&ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  cudaFreeAsync(base, s);
-  cudaStreamSynchronize(s);
-  cudaStreamDestroy(s);
+  if (!call.finish(&ms)) ok = false;
   if (!ok) {
     st = TEXO_GP_ERR_CUDA;
     set_last_error(std::string("quadratic solve: ") + cudaGetErrorString(cudaGetLastError()));
   } else if (hb.error) {
     st = TEXO_GP_ERR_DEVICE_TIMEOUT;
     set_last_error("quadratic solve: a grid barrier wait ran out");
+  } else if (res.wrong_entry) {   // the solution came back as it was
+    return fail(TEXO_GP_ERR_INVALID_ARGUMENT, kWrongEntry);
   } else if (!res.converged) {
     st = TEXO_GP_ERR_PCG_NOT_CONVERGED;
     set_last_error(std::string("analytical PCG ") + (res.stop == 1 ? "breakdown" : "dimension") + " after " +

@@ -15,9 +15,11 @@
 // rectangle and tile) is the difference from the reference's FP64 sums.
 #include <cmath>
 #include <cstring>
+#include <limits>
 #include <string>
 
 #include "common.cuh"
+#include "call.h"
 #include "engine.h"
 #include "kernels.cuh"
 
@@ -164,7 +166,13 @@ extern "C" int32_t texo_gp_routing_demand(int32_t device, uint32_t width, uint32
   if (elapsed_ms) *elapsed_ms = 0.0;
   if (!horizontal || !vertical || (num_boxes && !boxes)) return TEXO_GP_ERR_INVALID_ARGUMENT;
   if (width == 0 || height == 0 || (uint64_t)width * height > (1ull << 26)) return TEXO_GP_ERR_INVALID_NORMALIZATION;
+  unsigned wrong = 0;   // no early way out: this loop is vectorized
+  constexpr double kMax = std::numeric_limits<double>::max();
   for (uint64_t i = 0; i < num_boxes; ++i) {
+    const double* b = boxes + 4 * i;
+    wrong |= !(b[0] <= b[1]) | !(b[2] <= b[3]) | !(b[0] >= -kMax) | !(b[1] <= kMax) | !(b[2] >= -kMax) | !(b[3] <= kMax);
+  }
+  for (uint64_t i = 0; wrong && i < num_boxes; ++i) {
     const double* b = boxes + 4 * i;
     if (!(std::isfinite(b[0]) && std::isfinite(b[1]) && std::isfinite(b[2]) && std::isfinite(b[3])) ||
         b[0] > b[1] || b[2] > b[3]) {
@@ -176,24 +184,19 @@ extern "C" int32_t texo_gp_routing_demand(int32_t device, uint32_t width, uint32
   if (cudaSetDevice(device) != cudaSuccess) return TEXO_GP_ERR_CUDA;
   const int W = (int)width, H = (int)height;
   const size_t tiles = (size_t)W * H, plane = (size_t)(W + 1) * (H + 1);
-  cudaStream_t s = nullptr;
-  if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return TEXO_GP_ERR_CUDA;
-  char* base = nullptr;
+  Call call(device);
+  if (!call.ok()) return TEXO_GP_ERR_CUDA;
+  const cudaStream_t s = call.stream();
   const size_t b_bytes = ((std::max<uint64_t>(num_boxes, 1) * 32) + 255) & ~(size_t)255;
   const size_t d_bytes = ((2 * plane * 8) + 255) & ~(size_t)255;
   const size_t o_bytes = ((tiles * 8) + 255) & ~(size_t)255;
-  if (cudaMallocAsync((void**)&base, b_bytes + d_bytes + 2 * o_bytes, s) != cudaSuccess) {
-    cudaStreamDestroy(s);
-    return TEXO_GP_ERR_OUT_OF_MEMORY;
-  }
+  char* base = call.memory(b_bytes + d_bytes + 2 * o_bytes);
+  if (!base) return TEXO_GP_ERR_OUT_OF_MEMORY;
   double* dbox = (double*)base;
   unsigned long long* diff = (unsigned long long*)(base + b_bytes);
   double* dh = (double*)(base + b_bytes + d_bytes);
   double* dv = (double*)(base + b_bytes + d_bytes + o_bytes);
-  cudaEvent_t e0 = nullptr, e1 = nullptr;
-  cudaEventCreate(&e0);
-  cudaEventCreate(&e1);
-  cudaEventRecord(e0, s);
+  call.start();
   bool ok = (!num_boxes || cudaMemcpyAsync(dbox, boxes, num_boxes * 32, cudaMemcpyHostToDevice, s) == cudaSuccess) &&
             cudaMemsetAsync(diff, 0, 2 * plane * 8, s) == cudaSuccess;
   if (ok && num_boxes) {
@@ -210,15 +213,8 @@ extern "C" int32_t texo_gp_routing_demand(int32_t device, uint32_t width, uint32
          cudaMemcpyAsync(horizontal, dh, tiles * 8, cudaMemcpyDeviceToHost, s) == cudaSuccess &&
          cudaMemcpyAsync(vertical, dv, tiles * 8, cudaMemcpyDeviceToHost, s) == cudaSuccess;
   }
-  cudaEventRecord(e1, s);
-  if (cudaStreamSynchronize(s) != cudaSuccess) ok = false;
   float ms = 0.f;
-  cudaEventElapsedTime(&ms, e0, e1);
-  cudaEventDestroy(e0);
-  cudaEventDestroy(e1);
-  cudaFreeAsync(base, s);
-  cudaStreamSynchronize(s);
-  cudaStreamDestroy(s);
+  if (!call.finish(&ms)) ok = false;
   if (elapsed_ms) *elapsed_ms = ms;
   if (!ok) {
     set_last_error(std::string("routing demand: ") + cudaGetErrorString(cudaGetLastError()));
