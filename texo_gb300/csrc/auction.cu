@@ -30,7 +30,8 @@
 // active bidders alone, not on the order threads reach the atomics: the
 // result is deterministic. The bid slots, touched lists and active lists
 // alternate between two buffers and the list counters rotate over four
-// slots, so no phase clears what another block may still read.
+// slots, so no phase clears what another block may still read. Once few
+// bidders are left one block runs the rounds alone (`tail_rounds`).
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -45,10 +46,10 @@
 namespace tgp {
 namespace {
 
-constexpr int kAucThreads = 256;
+constexpr int kAucThreads = 1024;
 constexpr int kAucWarps = kAucThreads / 32;
-constexpr int kAucBlocksPerSm = 2;   // resident blocks a multiprocessor runs
-constexpr int kTailPerWarp = 2;      // active bidders per warp at which block 0 finishes alone
+constexpr int kAucBlocksPerSm = 1;   // resident blocks a multiprocessor runs
+constexpr int kTailBidders = 64;     // active bidders at which block 0 finishes alone
 constexpr unsigned kNone = 0xFFFFFFFFu;
 constexpr unsigned long long kNoKey = ~0ull;                      // "no candidate"
 constexpr unsigned long long kTimeLimitNs = 20ull * 1000000000ull; // the whole auction
@@ -120,6 +121,23 @@ __device__ __forceinline__ void warp_best2(unsigned long long& a1, unsigned long
   }
 }
 
+// A word of the auction's state. One block alone reads it through its L1, which
+// its own writes reach; among several it comes from the L2.
+template <bool ALONE, class T>
+__device__ __forceinline__ T state(const T* p) {
+  return ALONE ? *p : __ldcg(p);
+}
+
+// What a bidder looks through: an explicit domain's range, or a target tile
+// (x, y) and a kind of the grid.
+struct Bidder {
+  unsigned id, from, to, kind;
+};
+__device__ __forceinline__ Bidder bidder(const AucDev& d, unsigned b) {
+  if (!d.grid) return {b, __ldg(d.dptr + b), __ldg(d.dptr + b + 1), 0};
+  return {b, __ldg(d.txy + 2 * b), __ldg(d.txy + 2 * b + 1), __ldg(d.kind + b)};
+}
+
 // Objects of one tile a lane reads per batch in the ring walk.
 constexpr int kTileBatch = 8;
 
@@ -134,91 +152,113 @@ __device__ __forceinline__ unsigned ring_of(unsigned p) {
   return r;
 }
 
-// The two least (reduced cost, object) keys among bidder b's candidates, the
-// same in every lane of the warp. Returns the candidates this lane visited.
+// Point p >= 1 of the diamond, its ring r and offsets, packed in bytes for the
+// first kPoints (rings to 22), which each block keeps in shared memory.
+constexpr unsigned kPoints = 1024;
+struct Point {
+  int dx, dy;
+  unsigned r;
+};
+__device__ __forceinline__ Point point(unsigned p) {
+  const unsigned r = ring_of(p);
+  if (r == 0) return {0, 0, 0};
+  // ring r as four quarter turns of (r - i, i)
+  const unsigned j = p - (1u + 2u * r * (r - 1u)), q = j / r, i = j - q * r;
+  const int u = (int)(r - i), v = (int)i;
+  return {q == 0 ? u : q == 1 ? -v : q == 2 ? -u : v, q == 0 ? v : q == 1 ? u : q == 2 ? -v : -u, r};
+}
+__device__ __forceinline__ Point point(const char4* table, unsigned p) {
+  if (p >= kPoints) return point(p);
+  const char4 c = table[p];
+  return {c.x, c.y, (unsigned)c.z};
+}
+
+// The two least (reduced cost, object) keys among bidder `who`'s candidates,
+// the same in every lane of the warp. Returns the candidates this lane visited.
 //
 // The ring walk hands the warp 32 consecutive points of the diamond at a
 // time and stops once the second best is below the least cost an unseen
 // object can have, s times the first ring not fully seen. Visiting rings
 // past the reference's stopping ring adds only objects that cannot enter
 // the best two, so the result is the reference's exact best two.
-__device__ __forceinline__ unsigned long long best_two(const AucDev& d, unsigned b, int lane, unsigned long long& k1,
-                                                       unsigned long long& k2) {
+//
+// A walk is one chain of loads (tile, object, price) after another, with the
+// arithmetic of the points between them and the warp's second best behind:
+// the points come from a table, the second least cost from two integer
+// reductions (objects are looked at once, at the end), and one block alone,
+// which has nothing else in flight, reads the next points' prices ahead.
+template <bool ALONE>
+__device__ __forceinline__ unsigned long long best_two(const AucDev& d, const Bidder& who, const char4* table, int lane,
+                                                       unsigned long long& k1, unsigned long long& k2) {
+  const unsigned all = 0xffffffffu;
   unsigned long long a1 = kNoKey, a2 = kNoKey, seen = 0;
   if (!d.grid) {
-    const unsigned e = __ldg(d.dptr + b + 1);
-    for (unsigned k = __ldg(d.dptr + b) + lane; k < e; k += 32) {
+    for (unsigned k = who.from + lane; k < who.to; k += 32) {
       const unsigned o = __ldg(d.dobj + k);
-      insert2(a1, a2, make_key(d.scale * __ldg(d.dcost + k) + __ldcg(d.price + o), o));
+      insert2(a1, a2, make_key(d.scale * __ldg(d.dcost + k) + state<ALONE>(d.price + o), o));
       ++seen;
     }
-    warp_best2(a1, a2);
   } else {
-    const int tx = (int)__ldg(d.txy + 2 * b), ty = (int)__ldg(d.txy + 2 * b + 1);
+    const int tx = (int)who.from, ty = (int)who.to;
     const int W = (int)d.W, H = (int)d.H;
-    const unsigned* tp = d.tptr + (size_t)__ldg(d.kind + b) * d.W * d.H;
+    const unsigned* tp = d.tptr + (size_t)who.kind * d.W * d.H;
     const unsigned R = d.max_radius;
     const unsigned total = 1u + 2u * R * (R + 1u);   // points of the whole diamond
-    unsigned long long m1 = kNoKey, m2 = kNoKey;
+    struct Tile {
+      unsigned ring_cost, kb, e, o, price;   // its objects; the first one and its price (kNone: taken or none)
+    };
+    auto look = [&](unsigned p) {
+      Tile t{0, 0, 0, kNone, 0};
+      if (p >= total) return t;
+      const Point q = point(table, p);
+      const int x = tx + q.dx, y = ty + q.dy;
+      if (x < 0 || y < 0 || x >= W || y >= H) return t;
+      t.ring_cost = d.scale * q.r;
+      t.kb = __ldg(tp + y * W + x);
+      t.e = __ldg(tp + y * W + x + 1);
+      if (t.e == t.kb) return t;
+      t.o = __ldg(d.tobj + t.kb);
+      t.price = state<ALONE>(d.price + t.o);
+      if (d.occ && __ldg(d.occ + t.o)) t.o = kNone;
+      return t;
+    };
+    Tile t = look(lane);
     for (unsigned p0 = 0;; p0 += 32) {
-      const unsigned p = p0 + lane;
-      if (p < total) {
-        const unsigned r = ring_of(p);
-        int dx = 0, dy = 0;
-        if (r) {
-          // ring r as four quarter turns of (r - i, i)
-          const unsigned j = p - (1u + 2u * r * (r - 1u)), q = j / r, i = j - q * r;
-          const int u = (int)(r - i), v = (int)i;
-          dx = q == 0 ? u : q == 1 ? -v : q == 2 ? -u : v;
-          dy = q == 0 ? v : q == 1 ? u : q == 2 ? -v : -u;
+      Tile next;
+      if (ALONE) next = look(p0 + 32 + lane);
+      seen += t.e - t.kb;
+      if (t.o != kNone) insert2(a1, a2, make_key(t.ring_cost + t.price, t.o));
+      // a tile's further objects kTileBatch at a time, their loads issued together
+      // (keys are distinct, so the order of insertion does not matter)
+      for (unsigned k0 = t.kb + 1; k0 < t.e; k0 += kTileBatch) {
+        unsigned o[kTileBatch], pr[kTileBatch];
+        bool use[kTileBatch];
+#pragma unroll
+        for (int i = 0; i < kTileBatch; ++i) o[i] = k0 + i < t.e ? __ldg(d.tobj + k0 + i) : kNone;
+#pragma unroll
+        for (int i = 0; i < kTileBatch; ++i) {
+          use[i] = o[i] != kNone && !(d.occ && __ldg(d.occ + o[i]));
+          pr[i] = o[i] != kNone ? state<ALONE>(d.price + o[i]) : 0u;
         }
-        const int x = tx + dx, y = ty + dy;
-        if (x >= 0 && y >= 0 && x < W && y < H) {
-          const int t = y * W + x;
-          const unsigned ring_cost = d.scale * r, e = __ldg(tp + t + 1);
-          // a tile's objects kTileBatch at a time, their loads issued together
-          // (keys are distinct, so the order of insertion does not matter);
-          // a tile with one object takes the short path
-          const unsigned kb = __ldg(tp + t);
-          if (e == kb + 1) {
-            const unsigned o = __ldg(d.tobj + kb);
-            ++seen;
-            if (!(d.occ && __ldg(d.occ + o))) insert2(a1, a2, make_key(ring_cost + __ldcg(d.price + o), o));
-          } else
-          for (unsigned k0 = kb; k0 < e; k0 += kTileBatch) {
-            unsigned o[kTileBatch], pr[kTileBatch];
-            bool use[kTileBatch];
 #pragma unroll
-            for (int i = 0; i < kTileBatch; ++i) o[i] = k0 + i < e ? __ldg(d.tobj + k0 + i) : kNone;
-#pragma unroll
-            for (int i = 0; i < kTileBatch; ++i) {
-              use[i] = o[i] != kNone && !(d.occ && __ldg(d.occ + o[i]));
-              pr[i] = o[i] != kNone ? __ldcg(d.price + o[i]) : 0u;
-            }
-#pragma unroll
-            for (int i = 0; i < kTileBatch; ++i) {
-              seen += o[i] != kNone;
-              if (use[i]) insert2(a1, a2, make_key(ring_cost + pr[i], o[i]));
-            }
-          }
-        }
+        for (int i = 0; i < kTileBatch; ++i)
+          if (use[i]) insert2(a1, a2, make_key(t.ring_cost + pr[i], o[i]));
       }
-      // the warp's best two so far, merged from copies: each lane keeps the
-      // best two of the points it visited itself, so the merge always joins
-      // disjoint candidate sets
-      m1 = a1;
-      m2 = a2;
-      warp_best2(m1, m2);
       const unsigned last = min(p0 + 32u, total) - 1u;
       if (last == total - 1u) break;   // every ring seen
-      const unsigned rl = ring_of(last);
+      const unsigned rl = point(table, last).r;
       const unsigned unseen = last == 2u * rl * (rl + 1u) ? rl + 1u : rl;   // first ring not fully seen
+      // the warp's second least reduced cost: the least without one lane's
+      const unsigned c1 = (unsigned)(a1 >> 32), least = __reduce_min_sync(all, c1);
+      const int holder = __ffs(__ballot_sync(all, c1 == least)) - 1;
+      const unsigned second = __reduce_min_sync(all, lane == holder ? (unsigned)(a2 >> 32) : c1);
       // strict: an unseen object could tie the second best
-      if (m2 != kNoKey && (unsigned)(m2 >> 32) < d.scale * unseen) break;
+      if (second < d.scale * unseen) break;   // never with fewer than two seen: the largest cost there is
+      if (!ALONE) next = look(p0 + 32 + lane);
+      t = next;
     }
-    a1 = m1;
-    a2 = m2;
   }
+  warp_best2(a1, a2);
   k1 = a1;
   k2 = a2;
   return seen;
@@ -226,7 +266,7 @@ __device__ __forceinline__ unsigned long long best_two(const AucDev& d, unsigned
 
 // Bid phase of round k: warps [w0, w0 + nw) of the launch take the active
 // bidders in turn.
-__device__ __forceinline__ void bid_phase(const AucDev& d, unsigned k, unsigned nA, unsigned w0, unsigned nw, int lane,
+__device__ __forceinline__ void bid_phase(const AucDev& d, const char4* table, unsigned k, unsigned nA, unsigned w0, unsigned nw, int lane,
                                           unsigned long long& bids, unsigned long long& seen) {
   const unsigned cur = k & 1u;
   const unsigned* A = d.act + (size_t)cur * d.n;
@@ -235,7 +275,7 @@ __device__ __forceinline__ void bid_phase(const AucDev& d, unsigned k, unsigned 
   for (unsigned j = w0; j < nA; j += nw) {
     const unsigned b = __ldcg(A + j);
     unsigned long long k1, k2;
-    seen += best_two(d, b, lane, k1, k2);
+    seen += best_two<false>(d, bidder(d, b), table, lane, k1, k2);
     if (lane == 0) {
       const unsigned long long dummy = make_key(d.dummy, kNone);
       if (k1 > dummy) {
@@ -288,7 +328,8 @@ __device__ __forceinline__ void resolve_phase(const AucDev& d, unsigned k, unsig
       ++dmatched;
     }
   }
-  for (unsigned j = t0; j < nA; j += nt) {
+  // (threads from the other end, so that both lists are walked at once)
+  for (unsigned j = nt - 1 - t0; j < nA; j += nt) {
     const unsigned b = __ldcg(A + j);
     const unsigned o = __ldcg(d.want + b);
     if (o == kNone) continue;
@@ -298,28 +339,103 @@ __device__ __forceinline__ void resolve_phase(const AucDev& d, unsigned k, unsig
   const unsigned nP = __ldcg(cntT + ((k + 3) & 3u));
   const unsigned* P = d.touched + (size_t)nxt * d.cap;
   unsigned long long* bidp = d.bid + (size_t)nxt * d.m;
-  for (unsigned t = t0; t < nP; t += nt) bidp[__ldcg(P + t)] = 0;
+  for (unsigned t = (t0 + nt / 2) % nt; t < nP; t += nt) bidp[__ldcg(P + t)] = 0;
 }
 
-// Adds the block's changes of the held totals to the result (one atomic each
-// when nonzero).
-__device__ __forceinline__ void publish_totals(const AucDev& d, long long dbase, long long dmatched, long long* sh) {
-  if (threadIdx.x == 0) sh[0] = sh[1] = 0;
+// The rounds of at most kTailBidders bidders, by one block: the bidders and
+// their bids in shared memory, one warp a bidder and one thread a bid, the
+// auction's state through the L1. The round's outcome is that of the phases
+// above. Returns the number of the round in which no bidder was left (or the
+// time limit had run out).
+// What bounds a round is its chain of dependent loads. With lists, bids and
+// prices in global memory one took about 6 us, this takes 3 (9 us with all
+// blocks, two grid barriers of 1.7 us among them). 42,000 bidders, 174 rounds:
+// kernel and copies 1.83 -> 1.06 ms; 32 or 256 bidders in place of 64 take 0.06
+// or 0.15 ms longer.
+struct TailRound {
+  Bidder who[2][kTailBidders];
+  unsigned object[kTailBidders], offer[kTailBidders], base[kTailBidders];
+  int owner[kTailBidders];   // of the object bid on
+  unsigned count[2];
+  int stop;
+};
+__device__ __forceinline__ unsigned tail_rounds(const AucDev& d, const char4* table, unsigned k, unsigned nA, unsigned long long t_start,
+                                                TailRound& S, unsigned long long& bids, unsigned long long& seen,
+                                                long long& dbase, long long& dmatched) {
+  const unsigned tid = threadIdx.x, lane = tid & 31;
+  int cur = 0;
+  if (tid < nA) S.who[0][tid] = bidder(d, __ldcg(d.act + (size_t)(k & 1u) * d.n + tid));
+  if (tid == 0) {
+    S.count[0] = nA;
+    S.stop = 0;
+  }
   __syncthreads();
-  if (dbase) atomicAdd((unsigned long long*)&sh[0], (unsigned long long)dbase);
-  if (dmatched) atomicAdd((unsigned long long*)&sh[1], (unsigned long long)dmatched);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    if (sh[0]) atomicAdd(&d.out->total_base, (unsigned long long)sh[0]);
-    if (sh[1]) atomicAdd(&d.out->matched, (unsigned long long)sh[1]);
+  for (;; ++k, cur ^= 1) {
+    nA = S.count[cur];
+    if (nA == 0 || S.stop) return k;
+    for (unsigned j = tid >> 5; j < nA; j += kAucWarps) {
+      const Bidder who = S.who[cur][j];
+      unsigned long long k1, k2;
+      seen += best_two<true>(d, who, table, (int)lane, k1, k2);
+      if (lane == 0) {
+        const unsigned long long dummy = make_key(d.dummy, kNone);
+        unsigned o = kNone;   // the private dummy is strictly better: unmatched for good
+        if (k1 <= dummy) {
+          o = (unsigned)k1;
+          const unsigned price = state<true>(d.price + o);
+          const unsigned second = (unsigned)(min(k2, dummy) >> 32), best = (unsigned)(k1 >> 32);
+          S.owner[j] = state<true>(d.owner + o);
+          S.offer[j] = price + (second - best) + 1u;
+          S.base[j] = (best - price) / d.scale;
+          ++bids;
+        }
+        S.object[j] = o;
+      }
+    }
+    if (tid == 0) S.count[cur ^ 1] = 0;
+    __syncthreads();
+    if (tid < nA && S.object[tid] != kNone) {
+      const Bidder me = S.who[cur][tid];
+      const unsigned o = S.object[tid];
+      const unsigned long long mine = make_key(S.offer[tid], kNone - me.id);
+      bool won = true;
+      for (unsigned j = 0; j < nA; ++j)
+        if (S.object[j] == o && make_key(S.offer[j], kNone - S.who[cur][j].id) > mine) won = false;
+      Bidder out = me;
+      bool back = true;
+      if (won) {
+        const int prev = S.owner[tid];
+        d.owner[o] = (int)me.id;
+        d.price[o] = S.offer[tid];
+        d.assign[me.id] = (int)o;
+        d.held_base[me.id] = S.base[tid];
+        dbase += S.base[tid];
+        back = prev >= 0;
+        if (back) {
+          d.assign[prev] = -1;
+          dbase -= state<true>(d.held_base + prev);
+          out = bidder(d, (unsigned)prev);
+        } else {
+          ++dmatched;
+        }
+      }
+      if (back) S.who[cur ^ 1][atomicAdd(&S.count[cur ^ 1], 1u)] = out;
+    }
+    if (tid == 0 && now_ns() - t_start > kTimeLimitNs) {
+      S.stop = 1;
+      d.out->stop_round = k + 1;
+    }
+    __syncthreads();
   }
 }
 
 __global__ void __launch_bounds__(kAucThreads, kAucBlocksPerSm) k_auction(AucDev d) {
   __shared__ unsigned gen;
-  __shared__ int failed, s_stop;
+  __shared__ int failed;
   __shared__ unsigned long long s_bids, s_seen;
-  __shared__ long long s_tot[2];
+  __shared__ long long s_base, s_matched;
+  __shared__ TailRound s_tail;
+  __shared__ char4 s_table[kPoints];
   const int pb = blockIdx.x, np = gridDim.x;
   const int lane = threadIdx.x & 31;
   const unsigned gtid = pb * blockDim.x + threadIdx.x, gstride = np * blockDim.x;
@@ -331,6 +447,11 @@ __global__ void __launch_bounds__(kAucThreads, kAucBlocksPerSm) k_auction(AucDev
   if (threadIdx.x == 0) {
     gen = 0;
     s_bids = s_seen = 0;
+    s_base = s_matched = 0;
+  }
+  for (unsigned p = threadIdx.x; p < kPoints; p += kAucThreads) {
+    const Point q = point(p);
+    s_table[p] = make_char4((signed char)q.dx, (signed char)q.dy, (signed char)q.r, 0);
   }
   // initial state: every bidder active in index order, prices zero
   for (unsigned o = gtid; o < d.m; o += gstride) {
@@ -349,6 +470,7 @@ __global__ void __launch_bounds__(kAucThreads, kAucBlocksPerSm) k_auction(AucDev
 
   unsigned k = 0;
   bool tail = false;
+  long long dbase = 0, dmatched = 0;
   for (;; ++k) {
     const unsigned nA = __ldcg(cntA + (k & 3u));
     // block 0 may set the stop round during this round's bid phase; it names
@@ -358,7 +480,7 @@ __global__ void __launch_bounds__(kAucThreads, kAucBlocksPerSm) k_auction(AucDev
     // The active set never grows (a bidder wins, displacing at most one
     // holder, loses or leaves), so once it fits one block that block
     // finishes the auction alone, without grid barriers.
-    if (nA <= (unsigned)kAucWarps * kTailPerWarp) {
+    if (nA <= (unsigned)kTailBidders) {
       tail = true;
       break;
     }
@@ -367,38 +489,23 @@ __global__ void __launch_bounds__(kAucThreads, kAucBlocksPerSm) k_auction(AucDev
       cntT[(k + 1) & 3u] = 0;
       if (now_ns() - t_start > kTimeLimitNs) d.out->stop_round = k + 1;
     }
-    bid_phase(d, k, nA, gwarp, nwarps, lane, my_bids, my_seen);
+    bid_phase(d, s_table, k, nA, gwarp, nwarps, lane, my_bids, my_seen);
     if (!grid_sync(d.bar, (unsigned)np, &gen, &nbar, nullptr, &failed)) return;
-    long long dbase = 0, dmatched = 0;
     resolve_phase(d, k, nA, gtid, gstride, dbase, dmatched);
-    publish_totals(d, dbase, dmatched, s_tot);
     if (!grid_sync(d.bar, (unsigned)np, &gen, &nbar, nullptr, &failed)) return;
   }
   const unsigned grid_rounds = k;
-  if (tail && pb == 0) {
-    for (;; ++k) {
-      const unsigned nA = __ldcg(cntA + (k & 3u));
-      if (threadIdx.x == 0) {
-        s_stop = now_ns() - t_start > kTimeLimitNs;
-        if (s_stop) d.out->stop_round = k + 1;
-        cntA[(k + 2) & 3u] = 0;
-        cntT[(k + 1) & 3u] = 0;
-      }
-      __syncthreads();
-      if (nA == 0 || s_stop) break;
-      bid_phase(d, k, nA, threadIdx.x >> 5, kAucWarps, lane, my_bids, my_seen);
-      __syncthreads();
-      long long dbase = 0, dmatched = 0;
-      resolve_phase(d, k, nA, threadIdx.x, blockDim.x, dbase, dmatched);
-      publish_totals(d, dbase, dmatched, s_tot);   // ends with the block barrier the next round needs
-    }
-  }
+  if (tail && pb == 0) k = tail_rounds(d, s_table, k, __ldcg(cntA + (k & 3u)), t_start, s_tail, my_bids, my_seen, dbase, dmatched);
+  if (dbase) atomicAdd((unsigned long long*)&s_base, (unsigned long long)dbase);
+  if (dmatched) atomicAdd((unsigned long long*)&s_matched, (unsigned long long)dmatched);
   atomicAdd(&s_bids, my_bids);
   atomicAdd(&s_seen, my_seen);
   __syncthreads();
   if (threadIdx.x == 0) {
     atomicAdd(&d.out->bids, s_bids);
     atomicAdd(&d.out->examined, s_seen);
+    if (s_base) atomicAdd(&d.out->total_base, (unsigned long long)s_base);
+    if (s_matched) atomicAdd(&d.out->matched, (unsigned long long)s_matched);
     if (pb == 0) {
       d.out->rounds = k;
       d.out->tail_rounds = k - grid_rounds;
