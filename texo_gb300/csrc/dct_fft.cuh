@@ -42,6 +42,8 @@ namespace fft {
 // the tables of one axis up to 256 points. Lengths up to 512 take 512 points
 // a group, 1024 takes 1024 (two butterflies a thread).
 constexpr int kBuf = 2048;
+constexpr int kLogPoints = 9;                    // log2 of the points of a group
+static_assert(1 << kLogPoints == 2 * kThreads, "one butterfly a thread");
 constexpr int kStage = 640;                      // float2 slots of one staged copy, padding included (512 points)
 constexpr int kTables = 512 + kStage;            // the tables' first slot
 
@@ -143,9 +145,24 @@ __device__ __forceinline__ bool tables_stay(const Dev& d) {
 }
 
 // Vectors transformed together: one butterfly per thread per stage (n/2
-// butterflies per vector), at least one vector; many small groups keep every
-// SM busy on small grids.
-__device__ __forceinline__ int group_size(int logn) { return max(1, (2 * kThreads) >> logn); }
+// butterflies per vector), at least one vector, and no more than spreads the
+// groups over `blocks` blocks (the warps of the absent vectors then leave the
+// multiprocessor to the others: 64 x 64 bins on 21 blocks took 8 vectors on 8
+// of them, 4 on 16 save 0.8 us of an evaluation's 20). 0 blocks: as many as
+// fit. Lengths and groups are powers of two, so a group's field and first
+// vector are found by shifts.
+struct Groups {
+  int log_vectors, log_per_field;   // vectors a group, groups a field
+  __device__ __forceinline__ Groups(int logn, int log_count, int fields, int blocks) {
+    log_vectors = min(max(kLogPoints - logn, 0), log_count);
+    while (log_vectors > 0 && fields << (log_count - log_vectors + 1) <= blocks) --log_vectors;
+    log_per_field = log_count - log_vectors;
+  }
+  __device__ __forceinline__ int vectors() const { return 1 << log_vectors; }
+  __device__ __forceinline__ int count(int fields) const { return fields << log_per_field; }
+  __device__ __forceinline__ int field(int t) const { return t >> log_per_field; }
+  __device__ __forceinline__ int first(int t) const { return (t & ((1 << log_per_field) - 1)) << log_vectors; }
+};
 
 __device__ __forceinline__ int brev(int m, int logn) {
   return logn ? (int)(__brev((unsigned)m) >> (32 - logn)) : 0;
@@ -266,14 +283,13 @@ __device__ __forceinline__ int out_index(const Place<NB>& at, int r) {
   return (at.p >> 1) | r;
 }
 
-// Forward: the vectors' real samples staged in Makhoul's order (st[vec * n +
-// m], conflict-free) -> V. The inputs are real and stage 0's twiddle is one,
+// Stages 0 and 1 of a forward transform: the vectors' real samples staged in Makhoul's order (st[vec * n +
+// m], conflict-free). The inputs are real and stage 0's twiddle is one,
 // so stage 0 is two real sums, formed from four staged samples by each of the
 // two threads that would trade them (no exchange before stage 1); the
 // products by one and the sums with zero that are left out change no value.
-template <int NB, class G>
-__device__ __forceinline__ void forward(const G& g, const Place<NB>& at, const float2* st, const Axis& a,
-                                        float4* exch, Pair (&x)[NB]) {
+template <int NB>
+__device__ __forceinline__ void forward_start(const Place<NB>& at, const float2* st, const Axis& a, Pair (&x)[NB]) {
   const DF zero{0.f, 0.f};
   auto sample = [&](int m) {
     const float2 v = st[(at.vec << at.L) + m];
@@ -296,7 +312,6 @@ __device__ __forceinline__ void forward(const G& g, const Place<NB>& at, const f
     x[r].a = CDF{df_add(u, t.re), t.im};
     x[r].b = CDF{df_sub(u, t.re), df_neg(t.im)};
   }
-  stages(g, at, 2, x, a, exch);
 }
 // X_k = Re(post_k V_k)
 __device__ __forceinline__ DF coef(const Axis& a, const CDF& v, int k) {
@@ -304,11 +319,11 @@ __device__ __forceinline__ DF coef(const Axis& a, const CDF& v, int k) {
   return df_sub(df_mul(p.re, v.re), df_mul(p.im, v.im));
 }
 
-// Inverse: the coefficients X_k / s_k staged (st[vec * stride + pad_k(k)]) ->
-// F; sample unmak(m) of the vector is Re F_m / n.
-template <int NB, class G>
-__device__ __forceinline__ void inverse(const G& g, const Place<NB>& at, const float2* st, int stride, const Axis& a,
-                                        float4* exch, Pair (&x)[NB]) {
+// Stage 0 of an inverse transform: the coefficients X_k / s_k staged (st[vec *
+// stride + pad_k(k)]); at the end sample unmak(m) of the vector is Re F_m / n.
+template <int NB>
+__device__ __forceinline__ void inverse_start(const Place<NB>& at, const float2* st, int stride, const Axis& a,
+                                              Pair (&x)[NB]) {
   const float2* v = st + at.vec * stride;
   auto w = [&](int k) {
     const float2 c = v[pad_k(k)];
@@ -327,7 +342,6 @@ __device__ __forceinline__ void inverse(const G& g, const Place<NB>& at, const f
     x[r].a = CDF{df_add(u.re, t.re), df_add(u.im, t.im)};   // stage 0: twiddle one
     x[r].b = CDF{df_sub(u.re, t.re), df_sub(u.im, t.im)};
   }
-  stages(g, at, 1, x, a, exch);
 }
 // an inverse output times 1/n (a power of two)
 __device__ __forceinline__ DF out_sample(const CDF& v, float inv_n) { return df_scale(v.re, inv_n); }
@@ -341,34 +355,100 @@ __device__ __forceinline__ DF df_at(const float* g, size_t i) {
 // read by a vector of one or two warps, whose transforms cross no block
 // barrier), NB = 2 one (its exchanges' barriers lie between)
 template <int NB>
-__device__ __forceinline__ float2* stage_in(float4* buf) {
-  return reinterpret_cast<float2*>(buf + (NB == 1 ? 512 : 1024));
-}
+constexpr int kStageIn = 2 * (NB == 1 ? 512 : 1024);         // first float2 slot
 template <int NB>
-__device__ __forceinline__ float2* stage_out(float4* buf) {
-  return stage_in<NB>(buf) + (NB == 1 ? kStage : 0);
+constexpr int kStageOut = kStageIn<NB> + (NB == 1 ? kStage : 0);
+__device__ __forceinline__ float2* staged(float4* buf, int slot) { return reinterpret_cast<float2*>(buf) + slot; }
+
+// The transform of a group's `vectors` staged vectors, from slot `src` to slot
+// `dst` of the buffer:
+//   FORWARD  samples (Makhoul's order) -> coefficients (four apart)
+//   SCALED   the same, the coefficients times `ie` (1 / eigenvalue) and 1 / s_k
+//   INVERSE  coefficients over s_k -> samples (eight apart), times 1/n
+enum Direction { FORWARD, SCALED, INVERSE };
+template <int NB, class G>
+__device__ __forceinline__ void transform(const G& g, const Axis& a, int direction, int vectors, float4* buf, int src,
+                                          int dst, const float (&ie)[2 * NB]) {
+  const Place<NB> at(g.tid, a.logn);
+  const bool mine = at.vec < vectors;   // fewer vectors than a group holds
+  const int across = at.L - NB - at.lanes;   // index bits that warps trade: a barrier each
+  if (!__any_sync(0xffffffffu, mine)) {
+#pragma unroll 1
+    for (int w = 0; w < across; ++w) g.sync();
+    return;
+  }
+  Place<NB> pl = at;
+  if (!mine) pl.vec = 0;                // idle threads of a warp that works trade what is not kept
+  const int stride = pad_k(a.n), h = a.n >> 1;
+  const float2* in = staged(buf, src);
+  float2* out = staged(buf, dst);
+  Pair x[NB];
+  int from;
+  if (direction == INVERSE) {
+    inverse_start(pl, in, stride, a, x);
+    from = 1;
+  } else {
+    forward_start(pl, in, a, x);
+    from = 2;
+  }
+  stages(g, pl, from, x, a, buf);
+  if (!mine) return;
+  if (direction == INVERSE) {
+    const int ostride = pad_i(a.n);
+    const float inv_n = __int_as_float((127 - a.logn) << 23);   // 2^-logn
+#pragma unroll
+    for (int r = 0; r < NB; ++r) {
+      const int m = out_index(at, r);
+      const DF v0 = out_sample(x[r].a, inv_n), v1 = out_sample(x[r].b, inv_n);
+      out[at.vec * ostride + pad_i(unmak(m, a.n))] = make_float2(v0.hi, v0.lo);
+      out[at.vec * ostride + pad_i(unmak(m + h, a.n))] = make_float2(v1.hi, v1.lo);
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < NB; ++r) {
+      const int k = out_index(at, r);
+      DF c0 = coef(a, x[r].a, k), c1 = coef(a, x[r].b, k + h);
+      if (direction == SCALED) {
+        const float2 s0 = a.inv_s[k], s1 = a.inv_s[k + h];
+        c0 = df_mul(df_mul(c0, DF{ie[2 * r], 0.f}), DF{s0.x, s0.y});
+        c1 = df_mul(df_mul(c1, DF{ie[2 * r + 1], 0.f}), DF{s1.x, s1.y});
+      }
+      out[at.vec * stride + pad_k(k)] = make_float2(c0.hi, c0.lo);
+      out[at.vec * stride + pad_k(k + h)] = make_float2(c1.hi, c1.lo);
+    }
+  }
 }
+// The passes take the transform as a callable, `run(g, axis, direction,
+// vectors, buf, src, dst, ie)`: the standalone kernels have it inlined, with
+// its direction known; the persistent loop shares one copy among its passes.
+struct Inlined {
+  template <int NB, class G>
+  __device__ __forceinline__ void run(const G& g, const Axis& a, Direction direction, int vectors, float4* buf, int src,
+                                      int dst, const float (&ie)[2 * NB]) const {
+    transform<NB>(g, a, direction, vectors, buf, src, dst, ie);
+  }
+};
 
 // Pass 1: t1 = rows-DCT(rho). With `mean` (fixed-point mean per field) the
 // density preparation is folded in: rho = (phys + fill - mean) 2^-32 enters
 // the transform exactly (EXACT, as a double-float) or as the FP32 value that
 // is stored, and the physical overflow is counted into the IS_OVERFLOW /
 // IS_OVER_BINS partials.
-template <int NB, bool EXACT, class G>
+template <int NB, bool EXACT, class G, class T>
 static __device__ __forceinline__ void rows_fwd(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
-                                                Shared& sh, const long long* mean, bool tables) {
-  const int W = d.g.Wb, H = d.g.Hb, L = d.logW, GV = min(group_size(L), H), per = GV << L;
-  const int gpf = (H + GV - 1) / GV, groups = gpf * d.K;
+                                                Shared& sh, const long long* mean, bool tables, int spread, const T& dct) {
+  const int W = d.g.Wb, L = d.logW;
+  const Groups grp(L, d.logH, d.K, spread);
+  const int GV = grp.vectors(), per = GV << L, groups = grp.count(d.K);
   const Axis a = vb < groups ? stage_tables(g, axis_x(d), buf, tables) : axis_x(d);
-  const Place<NB> at(g.tid, L);
   const int stride = pad_k(W);
-  float2 *in = stage_in<NB>(buf), *out = stage_out<NB>(buf);
+  float2 *in = staged(buf, kStageIn<NB>), *out = staged(buf, kStageOut<NB>);
   long long ov[kMaxFields], cnt[kMaxFields];
 #pragma unroll
   for (int f = 0; f < kMaxFields; ++f) ov[f] = cnt[f] = 0;
 #pragma unroll 1
   for (int t = vb; t < groups; t += nvb) {
-    const int f = t / gpf, y0 = (t % gpf) * GV;
+    const int f = grp.field(t), y0 = grp.first(t);
     const size_t base = (size_t)f * d.B + (size_t)y0 * W;
     g.sync();   // earlier readers of the buffer are done
     long long o = 0, c = 0;
@@ -400,19 +480,8 @@ static __device__ __forceinline__ void rows_fwd(const G& g, const Dev& d, Partia
         cnt[ff] += c;
       }
     g.sync();
-    Pair x[NB];
-    const bool mine = at.vec < GV;   // fewer vectors than a group holds: idle threads trade zeros
-    Place<NB> pl = at;
-    if (!mine) pl.vec = 0;
-    forward(g, pl, in, a, buf, x);
-    if (mine)
-#pragma unroll
-      for (int r = 0; r < NB; ++r) {
-        const int k = out_index(at, r);
-        const DF c0 = coef(a, x[r].a, k), c1 = coef(a, x[r].b, k + (W >> 1));
-        out[at.vec * stride + pad_k(k)] = make_float2(c0.hi, c0.lo);
-        out[at.vec * stride + pad_k(k + (W >> 1))] = make_float2(c1.hi, c1.lo);
-      }
+    const float none[2 * NB] = {};
+    dct.template run<NB>(g, a, FORWARD, GV, buf, kStageIn<NB>, kStageOut<NB>, none);
     g.sync();
 #pragma unroll
     for (int q = 0; q < 2 * NB; ++q) {
@@ -431,18 +500,19 @@ static __device__ __forceinline__ void rows_fwd(const G& g, const Dev& d, Partia
 
 // Pass 2: t2 = cols-IDCT(cols-DCT(t1) * inv_eig), whole columns per group;
 // the scaled coefficients stay double-floats between the two transforms.
-template <int NB, class G>
-static __device__ __forceinline__ void cols(const G& g, const Dev& d, int vb, int nvb, float4* buf, bool tables) {
-  const int W = d.g.Wb, H = d.g.Hb, L = d.logH, GV = min(group_size(L), W), per = GV << L;
-  const int gpf = (W + GV - 1) / GV, groups = gpf * d.K;
+template <int NB, class G, class T>
+static __device__ __forceinline__ void cols(const G& g, const Dev& d, int vb, int nvb, float4* buf, bool tables, int spread,
+                                            const T& dct) {
+  const int W = d.g.Wb, H = d.g.Hb, L = d.logH;
+  const Groups grp(L, d.logW, d.K, spread);
+  const int GV = grp.vectors(), per = GV << L, groups = grp.count(d.K);
   const Axis a = vb < groups ? stage_tables(g, axis_y(d), buf, tables) : axis_y(d);
   const Place<NB> at(g.tid, L);
-  const int stride = pad_k(H), logG = 31 - __clz(GV);
-  float2 *in = stage_in<NB>(buf), *mid = stage_out<NB>(buf);
-  const float inv_n = 1.0f / (float)H;
+  const int logG = grp.log_vectors;
+  float2* in = staged(buf, kStageIn<NB>);
 #pragma unroll 1
   for (int t = vb; t < groups; t += nvb) {
-    const int f = t / gpf, x0 = (t % gpf) * GV;
+    const int f = grp.field(t), x0 = grp.first(t);
     const size_t base = (size_t)f * d.B + x0;
     g.sync();   // earlier readers of the buffer are done
 #pragma unroll
@@ -450,40 +520,19 @@ static __device__ __forceinline__ void cols(const G& g, const Dev& d, int vb, in
       const int e = g.tid + q * kThreads, v = e & (GV - 1), y = e >> logG;
       if (e < per) in[(v << L) + mak(y, H)] = df_grid(d.t1)[base + (size_t)y * W + v];
     }
-    const bool mine = at.vec < GV;
-    Place<NB> pl = at;
-    if (!mine) pl.vec = 0;
+    const int column = x0 + (at.vec < GV ? at.vec : 0);
     float ie[2 * NB];   // in flight while the samples are staged
 #pragma unroll
     for (int r = 0; r < NB; ++r) {
       const int k = out_index(at, r);
-      ie[2 * r] = d.inv_eig[(size_t)k * W + x0 + pl.vec];
-      ie[2 * r + 1] = d.inv_eig[(size_t)(k + (H >> 1)) * W + x0 + pl.vec];
+      ie[2 * r] = d.inv_eig[(size_t)k * W + column];
+      ie[2 * r + 1] = d.inv_eig[(size_t)(k + (H >> 1)) * W + column];
     }
     g.sync();
-    Pair x[NB];
-    forward(g, pl, in, a, buf, x);
-    if (mine)
-#pragma unroll
-      for (int r = 0; r < NB; ++r) {
-        const int k = out_index(at, r);
-        const float2 s0 = a.inv_s[k], s1 = a.inv_s[k + (H >> 1)];
-        const DF c0 = df_mul(df_mul(coef(a, x[r].a, k), DF{ie[2 * r], 0.f}), DF{s0.x, s0.y});
-        const DF c1 = df_mul(df_mul(coef(a, x[r].b, k + (H >> 1)), DF{ie[2 * r + 1], 0.f}), DF{s1.x, s1.y});
-        mid[at.vec * stride + pad_k(k)] = make_float2(c0.hi, c0.lo);
-        mid[at.vec * stride + pad_k(k + (H >> 1))] = make_float2(c1.hi, c1.lo);
-      }
+    dct.template run<NB>(g, a, SCALED, GV, buf, kStageIn<NB>, kStageOut<NB>, ie);
     g.sync();
-    inverse(g, pl, mid, stride, a, buf, x);
+    dct.template run<NB>(g, a, INVERSE, GV, buf, kStageOut<NB>, kStageIn<NB>, ie);
     const int ostride = pad_i(H);
-    if (mine)
-#pragma unroll
-      for (int r = 0; r < NB; ++r) {
-        const int m = out_index(at, r);
-        const DF v0 = out_sample(x[r].a, inv_n), v1 = out_sample(x[r].b, inv_n);
-        in[at.vec * ostride + pad_i(unmak(m, H))] = make_float2(v0.hi, v0.lo);
-        in[at.vec * ostride + pad_i(unmak(m + (H >> 1), H))] = make_float2(v1.hi, v1.lo);
-      }
     g.sync();
 #pragma unroll
     for (int q = 0; q < 2 * NB; ++q) {
@@ -494,21 +543,19 @@ static __device__ __forceinline__ void cols(const G& g, const Dev& d, int vb, in
 }
 
 // Pass 3: phi = rows-IDCT(t2) and the energy partials <rho, phi>.
-template <int NB, class G>
+template <int NB, class G, class T>
 static __device__ __forceinline__ void rows_inv(const G& g, const Dev& d, Partials p, int vb, int nvb, float4* buf,
-                                                Shared& sh, bool tables) {
-  const int W = d.g.Wb, H = d.g.Hb, L = d.logW, GV = min(group_size(L), H), per = GV << L;
-  const int gpf = (H + GV - 1) / GV, groups = gpf * d.K;
+                                                Shared& sh, bool tables, const T& dct) {
+  const int W = d.g.Wb, L = d.logW;
+  const Groups grp(L, d.logH, d.K, 0);   // fixed: the energy's partials are a group's sums
+  const int GV = grp.vectors(), per = GV << L, groups = grp.count(d.K);
   const Axis a = vb < groups ? stage_tables(g, axis_x(d), buf, tables) : axis_x(d);
-  const Place<NB> at(g.tid, L);
   const int stride = pad_k(W), ostride = pad_i(W);
-  float2* mid = stage_in<NB>(buf);
-  float* out = reinterpret_cast<float*>(stage_out<NB>(buf));
-  const float inv_n = 1.0f / (float)W;
+  float2 *mid = staged(buf, kStageIn<NB>), *out = staged(buf, kStageOut<NB>);
   double eacc[kMaxFields] = {0.0, 0.0, 0.0, 0.0};
 #pragma unroll 1
   for (int t = vb; t < groups; t += nvb) {
-    const int f = t / gpf, y0 = (t % gpf) * GV;
+    const int f = grp.field(t), y0 = grp.first(t);
     const size_t base = (size_t)f * d.B + (size_t)y0 * W;
     float rho[2 * NB];
     g.sync();   // earlier readers of the buffer are done
@@ -524,24 +571,15 @@ static __device__ __forceinline__ void rows_inv(const G& g, const Dev& d, Partia
       }
     }
     g.sync();
-    Pair x[NB];
-    const bool mine = at.vec < GV;
-    Place<NB> pl = at;
-    if (!mine) pl.vec = 0;
-    inverse(g, pl, mid, stride, a, buf, x);
-    if (mine)
-#pragma unroll
-      for (int r = 0; r < NB; ++r) {
-        const int m = out_index(at, r);
-        out[at.vec * ostride + pad_i(unmak(m, W))] = df_float(out_sample(x[r].a, inv_n));
-        out[at.vec * ostride + pad_i(unmak(m + (W >> 1), W))] = df_float(out_sample(x[r].b, inv_n));
-      }
+    const float none[2 * NB] = {};
+    dct.template run<NB>(g, a, INVERSE, GV, buf, kStageIn<NB>, kStageOut<NB>, none);
     g.sync();
 #pragma unroll
     for (int q = 0; q < 2 * NB; ++q) {
       const int e = g.tid + q * kThreads;
       if (e < per) {
-        const float v = out[(e >> L) * ostride + pad_i(e & (W - 1))];
+        const float2 c = out[(e >> L) * ostride + pad_i(e & (W - 1))];
+        const float v = df_float(DF{c.x, c.y});
         d.phi[base + e] = v;
 #pragma unroll
         for (int ff = 0; ff < kMaxFields; ++ff)

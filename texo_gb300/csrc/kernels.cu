@@ -24,18 +24,19 @@ __global__ void __launch_bounds__(kThreads, 4) k_fft_rows_fwd(Dev d, Partials p)
     }
     __syncthreads();
   }
-  fft::rows_fwd<NB, false>(whole_block(), d, p, blockIdx.x, gridDim.x, sm.buf, sh, PREP ? mean : nullptr, false);
+  fft::rows_fwd<NB, false>(whole_block(), d, p, blockIdx.x, gridDim.x, sm.buf, sh, PREP ? mean : nullptr, false, 0,
+                           fft::Inlined());
 }
 template <int NB>
 __global__ void __launch_bounds__(kThreads, NB == 2 ? 4 : 1) k_fft_cols(Dev d) {
   __shared__ fft::Smem sm;
-  fft::cols<NB>(whole_block(), d, blockIdx.x, gridDim.x, sm.buf, false);
+  fft::cols<NB>(whole_block(), d, blockIdx.x, gridDim.x, sm.buf, false, 0, fft::Inlined());
 }
 template <int NB>
 __global__ void __launch_bounds__(kThreads, 4) k_fft_rows_inv(Dev d, Partials p) {
   __shared__ fft::Smem sm;
   __shared__ Shared sh;
-  fft::rows_inv<NB>(whole_block(), d, p, blockIdx.x, gridDim.x, sm.buf, sh, false);
+  fft::rows_inv<NB>(whole_block(), d, p, blockIdx.x, gridDim.x, sm.buf, sh, false, fft::Inlined());
 }
 
 // The slice phase before tensor-core pass `step` (memory-bound, every block).
