@@ -200,7 +200,7 @@ struct LoopShared {
   Shared a;                                   // half A's (the block's) folds
   double pair[2 * (kThreads + 4)];            // two FP64 sums at once (half A)
   double wa[SETS == 2 ? kThreads + 4 : 1];    // half B's WA value
-  long long tot[kMaxFields][kThreads / 32];
+  long long tot[kMaxFields][SETS * kThreads / 32];
   unsigned u[3][SETS * kThreads / 32];
   unsigned x[2][kThreads / 32];               // half B's combination
 };
@@ -468,21 +468,23 @@ struct Ctx {
       f = __float_as_int(m.w);
     }
   }
-  // half A: its warps' totals, then (after the group's barrier) partial v
-  __device__ __forceinline__ void stage_totals(const GA& g, const long long (&tot)[kMaxFields]) {
+  // the warps' totals, then (after a barrier, half A) partial v of half A's or
+  // all warps' totals
+  __device__ __forceinline__ void stage_totals(const long long (&tot)[kMaxFields]) {
 #pragma unroll
     for (int f = 0; f < kMaxFields; ++f)
       if (f < d.K) {
         const long long t = warp_sum(tot[f]);
-        if ((g.tid & 31) == 0) sh.tot[f][g.tid >> 5] = t;
+        if ((threadIdx.x & 31) == 0) sh.tot[f][threadIdx.x >> 5] = t;
       }
   }
+  template <int WARPS = kThreads / 32>
   __device__ __forceinline__ void write_totals(const GA& g, int v) {
     const int f = g.tid - 128;
     if (f >= 0 && f < d.K) {
       long long t = 0;
 #pragma unroll
-      for (int w = 0; w < kThreads / 32; ++w) t += sh.tot[f][w];
+      for (int w = 0; w < WARPS; ++w) t += sh.tot[f][w];
       islot(r.p, IS_GRID_SUM + f)[v] = t;
     }
   }
@@ -496,7 +498,7 @@ struct Ctx {
       deposit(member(j, o), o, p, tot);
     }
     g.sync();   // earlier readers of the scratch are done
-    stage_totals(g, tot);
+    stage_totals(tot);
     g.sync();
     write_totals(g, v);
   }
@@ -969,7 +971,7 @@ struct Ctx {
     const unsigned hi = __reduce_max_sync(0xffffffffu, __float_as_uint(pmax));
     const unsigned c = __reduce_add_sync(0xffffffffu, diff) | (__any_sync(0xffffffffu, badp) ? 0x80000000u : 0u);
     g.sync();   // earlier readers of the scratch are done
-    stage_totals(g, tot);
+    stage_totals(tot);
     if ((g.tid & 31) == 0) {
       sh.u[0][g.tid >> 5] = lo;
       sh.u[1][g.tid >> 5] = hi;
@@ -994,12 +996,16 @@ struct Ctx {
     if (deposits) write_totals(g, v);
   }
 
-  // Half A: c = clamp(y - g / (L P)), scattered as it is formed; changed
-  // count, <g, c - y>, sum P (c - y)^2. Each thread's objects and the order of
-  // its sums are those of the 256-thread stage (the sums are FP32), the next
-  // object's loads in flight.
+  // The block: c = clamp(y - g / (L P)) and its scatter; changed count,
+  // <g, c - y>, sum P (c - y)^2. Half A forms the points (each thread's objects
+  // and the order of its sums are those of the 256-thread stage, the sums are
+  // FP32), the next object's loads in flight. Then both halves scatter them,
+  // which is most of the phase and integer arithmetic, so of any order: by half
+  // A alone, each object as it was formed, the phase and its barrier took 13.9
+  // us at 42,000 cells, this takes 12.9 (2,000 cells: 9.3, 8.9).
   __device__ void candidate(const float2* y, const float2* gy, float invL, float2* c, int v) {
     const GA g = half_a();
+    const bool a_half = in_a();
     unsigned diff = 0;
     float dot = 0.f, msn = 0.f;
     long long tot[kMaxFields] = {0, 0, 0, 0};
@@ -1022,7 +1028,7 @@ struct Ctx {
       if (resident(j)) res->pos[j] = t;
       return t;
     };
-    int j = g.tid, o = object(v, j);
+    int j = g.tid, o = a_half ? object(v, j) : d.nobj;
     In cur, next;
     if (o < d.nobj) cur = load(j, o);
 #pragma unroll 1
@@ -1030,26 +1036,34 @@ struct Ctx {
       const int o2 = object(v, j + kThreads);
       if (o2 < d.nobj) next = load(j + kThreads, o2);
       const float2 t = step(cur, j, o);
-      deposit(cur.mem, o, t, tot);
+      if constexpr (SETS == 1) deposit(cur.mem, o, t, tot);
       cur = next;
       j += kThreads;
       o = o2;
     }
-    // both FP64 sums at once, each in block_fold_fp64's order
+    __syncthreads();   // the points are there, and earlier readers of the scratch are done
     double *b0 = sh.pair, *b1 = sh.pair + kThreads + 4;
-    const unsigned n = __reduce_add_sync(0xffffffffu, diff);
-    g.sync();   // earlier readers of the scratch are done
-    stage_totals(g, tot);
-    b0[g.tid] = (double)dot;
-    b1[g.tid] = (double)msn;
-    if ((g.tid & 31) == 0) sh.u[0][g.tid >> 5] = n;
-    g.sync();
+    if (a_half) {
+      b0[g.tid] = (double)dot;
+      b1[g.tid] = (double)msn;
+      const unsigned n = __reduce_add_sync(0xffffffffu, diff);
+      if ((g.tid & 31) == 0) sh.u[0][g.tid >> 5] = n;
+    }
+    if constexpr (SETS == 2) {
+#pragma unroll 1
+      for (j = threadIdx.x; (o = object(v, j)) < d.nobj; j += kBlock)
+        deposit(member(j, o), o, resident(j) ? res->pos[j] : c[o], tot);
+    }
+    stage_totals(tot);
+    __syncthreads();
+    if (!a_half) return;
+    // both FP64 sums at once, each in block_fold_fp64's order
     if (g.tid == 64) {
       long long t = 0;
       for (int w = 0; w < kThreads / 32; ++w) t += sh.u[0][w];
       islot(set(), IS_DIFF)[v] = t;
     }
-    write_totals(g, v);
+    write_totals<kWarps>(g, v);
     {
       const int w = g.tid >> 5, at = (w & 3) * 32 + (g.tid & 31);
       double* b = w < 4 ? b0 : b1;
@@ -1668,7 +1682,7 @@ static __device__ void run_body(int pb, int np, Resident* resident) {
             VLOOP c.reset_grids(v);
             SYNC_OR_EXIT(PC_EXTRAP)
           }
-          if (c.in_a()) run_candidate<LARGE, SETS>(ybuf, gy, c.C());
+          run_candidate<LARGE, SETS>(ybuf, gy, c.C());
           SYNC_OR_EXIT(PC_CANDIDATE)
           {
             const Partials q = c.set();
