@@ -1,8 +1,8 @@
 """The kernels at the sizes where their tiles, groups and shared-memory copies
 end.
 
-- transforms of every length from 2 to 1024, square and not, alone and several
-  vectors to a group: potential against the FP64 oracle, 1e-6 normwise as for
+- transforms of every length from 2 to 1024, square and not, alone, several
+  vectors to a group and fewer than a group holds: potential against the FP64 oracle, 1e-6 normwise as for
   the other grids of this form (double-float butterflies, the FP32 storage
   between the passes decides).
 - the placement loop with objects beyond the ones a block keeps in shared
@@ -27,7 +27,8 @@ from texo_gb300.placer import Batch, Placer, default_params
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("W,H", [(2, 2), (4, 2), (2, 64), (8, 16), (16, 1024), (32, 4), (128, 512), (512, 8), (1024, 2)])
+@pytest.mark.parametrize("W,H", [(2, 2), (4, 2), (2, 64), (8, 16), (16, 1024), (32, 4), (128, 512), (512, 8), (1024, 2),
+                                 (128, 2), (2, 128), (256, 2), (2, 256)])
 def test_transform_lengths(W, H):
     i = np.arange(W * H)
     d = ((i * 31 + 7) % 101) - 50.0 + ((i * 13 + 5) % 17) / 17.0
@@ -40,7 +41,8 @@ def test_transform_lengths(W, H):
 
 @pytest.mark.parametrize("side,cells,bins_x,bins_y,iterations,stacked", [
     (520, 3000, 512, 512, 2, False), (48, 2000, 64, 32, 4, False), (48, 2000, 16, 8, 4, False),
-    (24, 400, 4, 2, 4, False), (48, 2000, 64, 64, 3, True), (48, 2000, 104, 40, 3, True)])
+    (24, 400, 4, 2, 4, False), (96, 9000, 128, 128, 3, False), (140, 18000, 128, 128, 3, False),
+    (140, 18000, 128, 64, 3, False), (48, 2000, 64, 64, 3, True), (48, 2000, 104, 40, 3, True)])
 def test_the_loop_alone_equals_the_loop_in_a_batch(side, cells, bins_x, bins_y, iterations, stacked):
     prob = P.synthetic(side, cells, 60, cells + cells // 5, 6.0, 1)
     if stacked:

@@ -19,7 +19,7 @@ struct PerDevice {
   int count;
   cudaMemPool_t pool;
 };
-// plain data, so nothing runs at exit, when the driver may be gone
+// plain data, so nothing runs at exit, when CUDA may be gone
 PerDevice g_devices[kDevices];
 std::mutex g_mu;
 PerDevice* of(int device) { return device >= 0 && device < kDevices ? g_devices + device : nullptr; }

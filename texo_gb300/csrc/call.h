@@ -1,8 +1,8 @@
 // call.h — the stream, events and device memory of one self-contained call
 // (an auction, a quadratic solve, a demand map, the register clustering).
 //
-// Creating and destroying a stream and two events, and device memory that the
-// driver maps and unmaps, took 100 to 300 us of each call. Streams and events
+// Creating and destroying a stream and two events, and device memory that
+// CUDA maps and unmaps, took 100 to 300 us of each call. Streams and events
 // are kept for the next call, at most kKept of each device; memory comes from a
 // pool of the device that keeps at most kKeptBytes between calls and gives
 // back the rest. Any number of threads may call: each has its own stream.

@@ -191,7 +191,7 @@ __device__ __forceinline__ int pad_i(int i) { return i + (i >> 3); }   // sample
 // values are the same, operation for operation. Measured: the three passes
 // of a 256 x 256 solve in the persistent loop, its three grid barriers
 // included, 28.8 -> 25.3 us; a 1024 x 1024 solve in the host engine (rows
-// forward / columns / rows inverse) 37 / 80 / 55 -> 25 / 68 / 33 us.
+// forward / columns / rows inverse) 37 / 80 / 55 -> 24 / 60 / 30 us.
 // NB = 2 (1024 points): a thread runs two butterflies, whose points differ in
 // position bit 1 at stage 0.
 template <int NB>
@@ -220,6 +220,11 @@ __device__ __forceinline__ void butterfly(Pair& x, const CDF& w) {
   x.a = CDF{df_add(x.a.re, t.re), df_add(x.a.im, t.im)};
 }
 
+// Whether the exchange before stage s is between warps (a barrier of the group).
+template <int NB>
+__device__ __forceinline__ bool crosses_warps(const Place<NB>& at, int s) {
+  return s >= NB && s - NB < at.L - NB - at.lanes;
+}
 // Brings position bit s into the pairs (s >= 1).
 template <int NB, class G>
 __device__ __forceinline__ void exchange(const G& g, const Place<NB>& at, int s, Pair (&x)[NB], float4* exch) {
@@ -230,8 +235,8 @@ __device__ __forceinline__ void exchange(const G& g, const Place<NB>& at, int s,
     return;
   }
   const bool up = (at.p >> s) & 1;
-  const int w = s - NB;                          // warp bit
-  if (w < at.L - NB - at.lanes) {                // through shared memory, the two buffers in turn
+  if (crosses_warps<NB>(at, s)) {                // through shared memory, the two buffers in turn
+    const int w = s - NB;                        // warp bit
     float4* e = exch + (w & 1) * NB * kThreads;
 #pragma unroll
     for (int r = 0; r < NB; ++r) e[r * kThreads + g.tid] = cdf_store(up ? x[r].a : x[r].b);
@@ -371,10 +376,11 @@ __device__ __forceinline__ void transform(const G& g, const Axis& a, int directi
                                           int dst, const float (&ie)[2 * NB]) {
   const Place<NB> at(g.tid, a.logn);
   const bool mine = at.vec < vectors;   // fewer vectors than a group holds
-  const int across = at.L - NB - at.lanes;   // index bits that warps trade: a barrier each
-  if (!__any_sync(0xffffffffu, mine)) {
+  const int from = direction == INVERSE ? 1 : 2;   // the first stage after an exchange
+  if (!__any_sync(0xffffffffu, mine)) {   // only the barriers of the exchanges between warps
 #pragma unroll 1
-    for (int w = 0; w < across; ++w) g.sync();
+    for (int s = from; s < at.L; ++s)
+      if (crosses_warps<NB>(at, s)) g.sync();
     return;
   }
   Place<NB> pl = at;
@@ -383,14 +389,10 @@ __device__ __forceinline__ void transform(const G& g, const Axis& a, int directi
   const float2* in = staged(buf, src);
   float2* out = staged(buf, dst);
   Pair x[NB];
-  int from;
-  if (direction == INVERSE) {
+  if (direction == INVERSE)
     inverse_start(pl, in, stride, a, x);
-    from = 1;
-  } else {
+  else
     forward_start(pl, in, a, x);
-    from = 2;
-  }
   stages(g, pl, from, x, a, buf);
   if (!mine) return;
   if (direction == INVERSE) {

@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kThreads) k_hpwl(Dev d, Partials p, const floa
 // warps, one per SM sub-partition) in block_reduce_array's order, eight slots
 // side by side: a slot is a round trip to memory and a chain of FP64 adds of
 // 64 cycles each; the nine slots of an evaluation took 14.6 us one after
-// another at 1M cells and take 9.3 this way (two rounds of eight).
+// another at 1M cells and take 7.5 this way (two rounds of eight).
 constexpr int kFinThreads = 1024;
 constexpr int kMaxFinJobs = 6 * kMaxFields + 16;
 struct FinJob {
