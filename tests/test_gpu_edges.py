@@ -42,7 +42,8 @@ def test_transform_lengths(W, H):
 @pytest.mark.parametrize("side,cells,bins_x,bins_y,iterations,stacked", [
     (520, 3000, 512, 512, 2, False), (48, 2000, 64, 32, 4, False), (48, 2000, 16, 8, 4, False),
     (24, 400, 4, 2, 4, False), (96, 9000, 128, 128, 3, False), (140, 18000, 128, 128, 3, False),
-    (140, 18000, 128, 64, 3, False), (48, 2000, 64, 64, 3, True), (48, 2000, 104, 40, 3, True)])
+    (140, 18000, 128, 64, 3, False), (140, 18000, 256, 64, 3, False), (140, 18000, 64, 256, 3, False),
+    (48, 2000, 64, 64, 3, True), (48, 2000, 104, 40, 3, True)])
 def test_the_loop_alone_equals_the_loop_in_a_batch(side, cells, bins_x, bins_y, iterations, stacked):
     prob = P.synthetic(side, cells, 60, cells + cells // 5, 6.0, 1)
     if stacked:
