@@ -840,11 +840,12 @@ struct Controller {
       for (int st = 0; st < 4; ++st) launch_dct(D, I.r, st, nvb, s, &I.tmaps, true);
       launch_gather(D, I.r, pos, nvb, s);
       CU(cudaStreamWaitEvent(s, side_ev[1], 0));
+      launch_finalize_joined(D, I.r, nvb, FIN_ENERGY | fin, s);
       density_evaluations++;
     } else {
       launch_wa(D, I.r, pos, gam, nvb, s);
+      launch_finalize(D, I.r, nvb, FIN_WA | fin, s);
     }
-    launch_finalize(D, I.r, nvb, (density ? FIN_ENERGY : FIN_WA) | fin, s);
     launch_combine(D, I.r, g, nvb, s, kkt ? pos : nullptr);
     launch_finalize(D, I.r, nvb, FIN_COMBINE | (kkt ? FIN_KKT : 0), s);
     device_evaluations++;

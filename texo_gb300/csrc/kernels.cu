@@ -6,15 +6,15 @@
 
 namespace tgp {
 
-// The kernels of an evaluation follow one another within microseconds, and the
-// gap between two of them (the last blocks' ends, the launch, the first blocks'
-// starts) is about one. Launched with `follow` a kernel is set up while its
-// predecessor in the stream still runs, and its blocks wait here until that has
-// completed and its writes can be seen (so no kernel that is launched so reads
-// its predecessors' results through the read-only cache, and none follows an
-// event of another stream). Two microseconds a kernel: an evaluation at 250,000
-// cells with the tensor-core transforms, 19 launches, 245 -> 215 us; a whole
-// evaluate call at 2,000 cells 166 -> 148.
+// The kernels of an evaluation follow one another within microseconds. Launched
+// with `follow` a kernel is set up while its predecessor in the stream still
+// runs, and its blocks wait here until that kernel has completed and its writes
+// can be seen (so no kernel that is launched so reads its predecessors' results
+// through the read-only cache). The wait covers the kernel before it in its
+// own stream and nothing else: the kernel after a cudaStreamWaitEvent is launched
+// plainly (`launch_finalize_joined`), as is k_wa, whose predecessor is in
+// another stream. An evaluation at 250,000 cells with the tensor-core transforms,
+// 19 launches, 245 -> 215 us; a whole evaluate call at 2,000 cells 166 -> 148.
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -470,7 +470,7 @@ void launch_gather(const Dev& d, const Reduce& r, const float2* pos, int nvb, cu
 }
 void launch_combine(const Dev& d, const Reduce& r, float2* gout, int nvb, cudaStream_t s, const float2* kkt_pos) {
   COUNT;
-  k_combine<<<nvb, kThreads, 0, s>>>(d, r.p, r.scal + SC_COEF, gout, kkt_pos);
+  follow(k_combine, nvb, kThreads, 0, s, d, r.p, r.scal + SC_COEF, gout, kkt_pos);
 }
 void launch_extrapolate(const Dev& d, const Reduce& r, const float2* x, const float2* xp, float e, float2* y,
                         int nvb, cudaStream_t s, bool reset) {
@@ -498,6 +498,10 @@ void launch_hpwl(const Dev& d, const Reduce& r, const float2* pos, int nvb, cuda
 void launch_finalize(const Dev& d, const Reduce& r, int nvb, int mask, cudaStream_t s) {
   COUNT;
   follow(k_finalize, 1, kFinThreads, 0, s, d, r, nvb, mask);
+}
+void launch_finalize_joined(const Dev& d, const Reduce& r, int nvb, int mask, cudaStream_t s) {
+  COUNT;
+  k_finalize<<<1, kFinThreads, 0, s>>>(d, r, nvb, mask);
 }
 static inline int wide_blocks(size_t n) { return (int)std::min<size_t>((n + kThreads - 1) / kThreads, 2048); }
 void launch_narrow(const double* src, float* dst, size_t n, long long* nonfinite, long long mark, cudaStream_t s) {

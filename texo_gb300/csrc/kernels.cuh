@@ -82,6 +82,8 @@ void launch_kkt(const Dev& d, const Reduce& r, const float2* x, const float2* g,
 void launch_precond(const Dev& d, const Reduce& r, int nvb, cudaStream_t s);
 void launch_hpwl(const Dev& d, const Reduce& r, const float2* pos, int nvb, cudaStream_t s);
 void launch_finalize(const Dev& d, const Reduce& r, int nvb, int mask, cudaStream_t s);
+// The same where the stream has just waited for another stream's event.
+void launch_finalize_joined(const Dev& d, const Reduce& r, int nvb, int mask, cudaStream_t s);
 // FP64 host arrays staged on the device -> FP32 (raising *nonfinite to mark
 // when a value is not finite), and the results' FP64 and integer arrays from device state.
 void launch_narrow(const double* src, float* dst, size_t n, long long* nonfinite, long long mark, cudaStream_t s);
