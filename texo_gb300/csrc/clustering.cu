@@ -34,8 +34,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
-#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -61,13 +59,10 @@ struct Window {
 
 // The table, formed once in extended precision (erf' = 2 / sqrt(pi)
 // exp(-x^2), and its n-th derivative times (-1)^n H_n(x), the Hermite
-// polynomials' three-term recurrence) and kept on each device.
-cudaError_t window_table(int device, const Window** out) {
-  static std::mutex mu;
-  static std::map<int, Window*> cache;
-  std::lock_guard<std::mutex> lk(mu);
-  auto it = cache.find(device);
-  if (it == cache.end()) {
+// polynomials' three-term recurrence). Each call sends it (20 KB) with its own
+// inputs, on its own stream: nothing is kept on a device between calls.
+const std::vector<Window>& window_table() {
+  static const std::vector<Window> table = [] {   // thread-safe one-time initialisation
     std::vector<Window> t(kIntervals);
     const long double h = 2.5L / sqrtl(2.0L), two_over_sqrt_pi = 2.0L / sqrtl(3.14159265358979323846264338327950288L);
     for (int k = 0; k < kIntervals; ++k) {
@@ -88,14 +83,9 @@ cudaError_t window_table(int device, const Window** out) {
       }
       for (int n = 0; n < kTerms; ++n) t[k].c[n] = (double)c[n];
     }
-    Window* d = nullptr;
-    cudaError_t e = cudaMalloc(&d, t.size() * sizeof(Window));
-    if (e == cudaSuccess) e = cudaMemcpy(d, t.data(), t.size() * sizeof(Window), cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return e;
-    it = cache.emplace(device, d).first;
-  }
-  *out = it->second;
-  return cudaSuccess;
+    return t;
+  }();
+  return table;
 }
 
 // soft_division_ceiling (register_clustering.rs:89-97); the divisors are
@@ -374,8 +364,9 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
   if (!call.ok()) return TEXO_GP_ERR_CUDA;
   const cudaStream_t s = call.stream();
   auto round = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const size_t s8 = round(n * 8), s4 = round(n * 4);
-  char* base = call.memory(5 * s8 + 4 * s4 + 256);
+  const std::vector<Window>& table = window_table();
+  const size_t s8 = round(n * 8), s4 = round(n * 4), st = round(table.size() * sizeof(Window));
+  char* base = call.memory(5 * s8 + 4 * s4 + st + 256);
   if (!base) return TEXO_GP_ERR_OUT_OF_MEMORY;
   ClusterDev d{};
   d.n = (unsigned)n;
@@ -390,6 +381,8 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
   float2* d32 = (float2*)(base + 4 * s8 + 3 * s4);
   unsigned* dfoc = (unsigned*)(base + 5 * s8 + 3 * s4);
   d.bad = (int*)(base + 5 * s8 + 4 * s4);
+  Window* dtable = (Window*)(base + 5 * s8 + 4 * s4 + 256);
+  d.table = dtable;
   d.xy32 = d32;
   d.focal = dfoc;
   d.cutoff32 = cutoff32;
@@ -399,7 +392,7 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
   d.group_end = dge;
   d.order = dord;
   call.start();
-  bool ok = window_table(device, &d.table) == cudaSuccess &&
+  bool ok = cudaMemcpyAsync(dtable, table.data(), table.size() * sizeof(Window), cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(dxy, sxy.data(), n * 16, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(dce, sce.data(), n * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(dgb, gb.data(), n * 4, cudaMemcpyHostToDevice, s) == cudaSuccess &&
