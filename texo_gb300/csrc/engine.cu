@@ -96,14 +96,18 @@ struct Staged {
 };
 // Host FP64 coordinates -> device FP32 optimizer buffer, on the instance's
 // stream; `src` is read until the caller synchronizes.
-// With a `mark` (growing from call to call) SI_NONFINITE becomes it when a
-// coordinate is not finite.
-int32_t upload_coords(Instance& I, float2* dst, const double* src, size_t nobj, long long mark = 0) {
+int32_t upload_coords(Instance& I, float2* dst, const double* src, size_t nobj) {
   Staged buf(I.stream);
   CU(buf.get(2 * nobj * sizeof(double)));
   CU(cudaMemcpyAsync(buf.p, src, 2 * nobj * sizeof(double), cudaMemcpyHostToDevice, I.stream));
-  launch_narrow((const double*)buf.p, (float*)dst, 2 * nobj, mark ? I.r.iscal + SI_NONFINITE : nullptr, mark, I.stream);
+  launch_narrow((const double*)buf.p, (float*)dst, 2 * nobj, I.stream);
   return TEXO_GP_OK;
+}
+bool all_finite(const double* v, size_t n) {   // no early way out: this loop is vectorized
+  constexpr double kMax = std::numeric_limits<double>::max();
+  unsigned wrong = 0;
+  for (size_t i = 0; i < n; ++i) wrong |= !(std::fabs(v[i]) <= kMax);
+  return !wrong;
 }
 std::vector<double> dct_basis(uint32_t n) {
   const double nf = (double)n;
@@ -755,11 +759,7 @@ struct Controller {
   std::vector<double> fixed_scales;
   uint64_t iter_offset = 0;
 
-  explicit Controller(Instance& i) : I(i), coordinate_calls(i.coordinate_calls), hr(i.h_run->run) { std::memset(&hr, 0, sizeof(hr)); }
-  // texo_gp_evaluate's coordinate check: the event behind its flag, and the
-  // calls made (a flag equal to the call's number is this call's)
-  cudaEvent_t check_ev = nullptr;
-  long long& coordinate_calls;
+  explicit Controller(Instance& i) : I(i), hr(i.h_run->run) { std::memset(&hr, 0, sizeof(hr)); }
 
   // WA's stream and the events around it (the host engine's evaluations)
   cudaStream_t side = nullptr;
@@ -772,7 +772,6 @@ struct Controller {
     }
     for (cudaEvent_t e : side_ev)
       if (e) cudaEventDestroy(e);
-    if (check_ev) cudaEventDestroy(check_ev);
     if (step_exec) cudaGraphExecDestroy(step_exec);
     for (cudaEvent_t e : step_ev)
       if (e) cudaEventDestroy(e);
@@ -1936,16 +1935,19 @@ int32_t texo_gp_evaluate(texo_gp_handle h, const double* coordinates, double gam
   Instance& I = *h->inst;
   Controller& C = *h->ctl;
   const size_t nobj = (size_t)I.d.nobj, B = I.m.bins(), K = I.m.K;
-  // The coordinates' finiteness is checked while they are narrowed; the
-  // evaluation is queued behind (a non-finite coordinate lands on the grid's
-  // edge there), and while it runs the host reads the check: nothing is given
-  // out unless it has passed.
-  const long long mark = ++C.coordinate_calls;
-  if (!C.check_ev) CU(cudaEventCreateWithFlags(&C.check_ev, cudaEventDisableTiming));
-  TRY(upload_coords(I, I.bufY, coordinates, nobj, mark));
-  CU(cudaMemcpyAsync(I.h_iscal + SI_NONFINITE, I.r.iscal + SI_NONFINITE, sizeof(long long), cudaMemcpyDeviceToHost,
-                     I.stream));
-  CU(cudaEventRecord(C.check_ev, I.stream));
+  // A refused call leaves the handle as it was. Between two calls Y holds
+  // nothing, and without a density at X neither does what an evaluation writes:
+  // then the coordinates are checked while the evaluation runs (12 us at 42k
+  // cells; one that is not finite lands on the grid's edge), and its
+  // counts are taken back; else before it is queued.
+  auto refuse = [&]() -> int32_t {
+    CU(cudaStreamSynchronize(I.stream));
+    return TEXO_GP_ERR_NONFINITE_UNIT_COORDINATE;
+  };
+  TRY(upload_coords(I, I.bufY, coordinates, nobj));
+  const bool check_first = C.density_at_x;
+  if (check_first && !all_finite(coordinates, 2 * nobj)) return refuse();
+  const uint64_t counts_before[2] = {C.density_evaluations, C.device_evaluations};
   C.density_at_x = false;
   TRY(C.enqueue_eval(I.bufY, I.gY, gamma, false));
   Staged buf(I.stream);
@@ -1965,10 +1967,10 @@ int32_t texo_gp_evaluate(texo_gp_handle h, const double* coordinates, double gam
       }
     launch_widen_eval(I.d, dev[0], dev[1], dev[2], dev[3], I.stream);
   }
-  CU(cudaEventSynchronize(C.check_ev));
-  if (I.h_iscal[SI_NONFINITE] == mark) {
-    CU(cudaStreamSynchronize(I.stream));
-    return TEXO_GP_ERR_NONFINITE_UNIT_COORDINATE;
+  if (!check_first && !all_finite(coordinates, 2 * nobj)) {
+    C.density_evaluations = counts_before[0];
+    C.device_evaluations = counts_before[1];
+    return refuse();
   }
   CU(cudaMemcpyAsync(I.h_iscal, I.r.iscal, kIScalars * sizeof(long long), cudaMemcpyDeviceToHost, I.stream));
   CU(cudaMemcpyAsync(I.h_scal, I.r.scal, kScalars * sizeof(double), cudaMemcpyDeviceToHost, I.stream));

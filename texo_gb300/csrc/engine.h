@@ -86,7 +86,6 @@ struct Instance {
   double* h_scal = nullptr;                      // pinned host mirror
   long long* h_iscal = nullptr;
   uint64_t bytes = 0;
-  long long coordinate_calls = 0;                // texo_gp_evaluate calls (the mark of SI_NONFINITE)
   tc::TcMaps tmaps{};                            // tensor maps of the tensor-core DCT operands
 
   ~Instance();
