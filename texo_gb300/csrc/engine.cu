@@ -82,8 +82,8 @@ cudaError_t keep_pool(int device) {
   return e;
 }
 // Device memory for one call's FP64 arrays, from the stream-ordered pool and
-// back to it when the call's work on the stream is done: nothing is added to
-// an instance's footprint.
+// back to it when the call's work on the stream is done. No footprint counts
+// it, so no call relies on it: where there is none, the host converts.
 struct Staged {
   cudaStream_t s;
   char* p = nullptr;
@@ -92,15 +92,35 @@ struct Staged {
   ~Staged() {
     if (p) cudaFreeAsync(p, s);
   }
-  cudaError_t get(size_t n) { return cudaMallocAsync((void**)&p, std::max<size_t>(n, 16), s); }
+  bool get(size_t n) {
+    if (cudaMallocAsync((void**)&p, n, s) == cudaSuccess) return true;
+    cudaGetLastError();
+    p = nullptr;
+    return false;
+  }
 };
 // Host FP64 coordinates -> device FP32 optimizer buffer, on the instance's
 // stream; `src` is read until the caller synchronizes.
 int32_t upload_coords(Instance& I, float2* dst, const double* src, size_t nobj) {
+  if (!nobj) return TEXO_GP_OK;
   Staged buf(I.stream);
-  CU(buf.get(2 * nobj * sizeof(double)));
-  CU(cudaMemcpyAsync(buf.p, src, 2 * nobj * sizeof(double), cudaMemcpyHostToDevice, I.stream));
-  launch_narrow((const double*)buf.p, (float*)dst, 2 * nobj, I.stream);
+  if (buf.get(2 * nobj * sizeof(double))) {
+    CU(cudaMemcpyAsync(buf.p, src, 2 * nobj * sizeof(double), cudaMemcpyHostToDevice, I.stream));
+    launch_narrow((const double*)buf.p, (float*)dst, 2 * nobj, I.stream);
+  } else {
+    const std::vector<float> narrow(src, src + 2 * nobj);
+    CU(cudaMemcpyAsync(dst, narrow.data(), nobj * sizeof(float2), cudaMemcpyHostToDevice, I.stream));
+    CU(cudaStreamSynchronize(I.stream));
+  }
+  return TEXO_GP_OK;
+}
+// An array of the device -> the host's, each value through `convert`.
+template <class T, class Convert>
+int32_t read_converted(Instance& I, const T* src, size_t n, Convert convert) {
+  std::vector<T> v(n);
+  CU(cudaMemcpyAsync(v.data(), src, n * sizeof(T), cudaMemcpyDeviceToHost, I.stream));
+  CU(cudaStreamSynchronize(I.stream));
+  for (size_t i = 0; i < n; ++i) convert(i, v[i]);
   return TEXO_GP_OK;
 }
 bool all_finite(const double* v, size_t n) {   // no early way out: this loop is vectorized
@@ -1747,13 +1767,17 @@ int32_t handle_targets(texo_gp_handle h, uint32_t* out, double* coords, texo_gp_
     Staged buf(I.stream);
     const bool rounded = out && I.m.has_density && U;   // without a density field the checkpoint is the initial point
     const size_t cb = coords ? 2 * nobj * sizeof(double) : 0, tb = rounded ? 2 * U * sizeof(uint32_t) : 0;
-    if (cb + tb) {
-      CU(buf.get(cb + tb));
+    if (cb + tb && buf.get(cb + tb)) {
       double* c = cb ? (double*)buf.p : nullptr;
       uint32_t* t = tb ? (uint32_t*)(buf.p + cb) : nullptr;
       launch_widen_point(I.d, I.best, I.bufX, t, c, I.stream);
       if (cb) CU(cudaMemcpyAsync(coords, c, cb, cudaMemcpyDeviceToHost, I.stream));
       if (tb) CU(cudaMemcpyAsync(out, t, tb, cudaMemcpyDeviceToHost, I.stream));
+    } else {
+      if (cb) TRY(read_converted(I, (const float*)I.bufX, 2 * nobj, [&](size_t i, float v) { coords[i] = v; }));
+      if (tb)
+        TRY(read_converted(I, (const float*)I.best, 2 * U,
+                           [&](size_t i, float v) { out[i] = round_coord(v, i & 1 ? I.m.H : I.m.W); }));
     }
     CU(cudaStreamSynchronize(I.stream));
     CU(cudaGetLastError());
@@ -1957,8 +1981,8 @@ int32_t texo_gp_evaluate(texo_gp_handle h, const double* coordinates, double gam
   double* dev[4] = {nullptr, nullptr, nullptr, nullptr};
   size_t total = 0;
   for (size_t c : counts) total += (c + 1) & ~(size_t)1;   // each array starts on 16 bytes
-  if (total) {
-    CU(buf.get(total * sizeof(double)));
+  const bool widened = total && buf.get(total * sizeof(double));
+  if (widened) {
     double* at = (double*)buf.p;
     for (int i = 0; i < 4; ++i)
       if (counts[i]) {
@@ -1975,8 +1999,27 @@ int32_t texo_gp_evaluate(texo_gp_handle h, const double* coordinates, double gam
   CU(cudaMemcpyAsync(I.h_iscal, I.r.iscal, kIScalars * sizeof(long long), cudaMemcpyDeviceToHost, I.stream));
   CU(cudaMemcpyAsync(I.h_scal, I.r.scal, kScalars * sizeof(double), cudaMemcpyDeviceToHost, I.stream));
   for (int i = 0; i < 4; ++i)
-    if (counts[i])
-      CU(cudaMemcpyAsync(host[i], dev[i], counts[i] * sizeof(double), cudaMemcpyDeviceToHost, I.stream));
+    if (dev[i]) CU(cudaMemcpyAsync(host[i], dev[i], counts[i] * sizeof(double), cudaMemcpyDeviceToHost, I.stream));
+  if (total && !widened) {
+    if (counts[0])
+      TRY(read_converted(I, I.d.wa_fix, counts[0], [&](size_t i, unsigned long long v) {
+        wa_gradient[i] = (double)(long long)v * kInvFix;
+      }));
+    if (counts[1])
+      TRY(read_converted(I, (const float*)I.d.graw, counts[1], [&](size_t i, float v) {
+        const size_t f = i / (2 * nobj), o = i / 2 % nobj;
+        field_gradient[i] = o < I.m.U || (size_t)I.m.fil_field[o - I.m.U] == f ? v : 0.f;
+      }));
+    if (counts[2]) {
+      TRY(read_converted(I, I.d.phys, counts[2], [&](size_t i, long long v) { std::memcpy(density + i, &v, 8); }));
+      TRY(read_converted(I, I.d.fill, counts[2], [&](size_t i, long long v) {
+        long long a;
+        std::memcpy(&a, density + i, 8);
+        density[i] = (double)(a + v) * kInvFix;
+      }));
+    }
+    if (counts[3]) TRY(read_converted(I, I.d.phi, counts[3], [&](size_t i, float v) { potential[i] = v; }));
+  }
   CU(cudaStreamSynchronize(I.stream));
   CU(cudaGetLastError());
   if (I.h_iscal[SI_TC_FAIL]) {
