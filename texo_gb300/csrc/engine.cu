@@ -44,8 +44,53 @@ void set_last_error(const std::string& s) { g_last_error = s; }
 
 void release_mirror(RunBlock* run);
 
+namespace {
+// Second streams with their events, kept for the next instance of the device
+// (made and destroyed with each restart they took 27 us of its 198 with one
+// evaluation at 2,000 cells).
+constexpr size_t kKeptSides = 8;   // in all
+std::mutex g_side_mu;
+std::vector<std::pair<int, Side>> g_side_free;
+
+void destroy_side(Side& d) {
+  if (d.s) cudaStreamDestroy(d.s);
+  if (d.ready) cudaEventDestroy(d.ready);
+  if (d.done) cudaEventDestroy(d.done);
+  d = Side{};
+}
+cudaError_t acquire_side(int device, Side& out) {
+  {
+    std::lock_guard<std::mutex> lk(g_side_mu);
+    for (auto it = g_side_free.begin(); it != g_side_free.end(); ++it)
+      if (it->first == device) {
+        out = it->second;
+        g_side_free.erase(it);
+        return cudaSuccess;
+      }
+  }
+  cudaError_t e = cudaStreamCreateWithFlags(&out.s, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&out.ready, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&out.done, cudaEventDisableTiming);
+  if (e != cudaSuccess) destroy_side(out);
+  return e;
+}
+void release_side(int device, Side& d) {
+  if (!d.s) return;
+  if (cudaStreamSynchronize(d.s) == cudaSuccess) {
+    std::lock_guard<std::mutex> lk(g_side_mu);
+    if (g_side_free.size() < kKeptSides) {
+      g_side_free.emplace_back(device, d);
+      d = Side{};
+      return;
+    }
+  }
+  destroy_side(d);
+}
+}  // namespace
+
 Instance::~Instance() {
   if (stream) cudaStreamSynchronize(stream);
+  release_side(device, side);
   for (void* p : allocations) cudaFreeAsync(p, stream);
   if (stream) {
     cudaStreamSynchronize(stream);
@@ -781,17 +826,7 @@ struct Controller {
 
   explicit Controller(Instance& i) : I(i), hr(i.h_run->run) { std::memset(&hr, 0, sizeof(hr)); }
 
-  // WA's stream and the events around it (the host engine's evaluations)
-  cudaStream_t side = nullptr;
-  cudaEvent_t side_ev[2] = {nullptr, nullptr};
-
   ~Controller() {
-    if (side) {
-      cudaStreamSynchronize(side);
-      cudaStreamDestroy(side);
-    }
-    for (cudaEvent_t e : side_ev)
-      if (e) cudaEventDestroy(e);
     if (step_exec) cudaGraphExecDestroy(step_exec);
     for (cudaEvent_t e : step_ev)
       if (e) cudaEventDestroy(e);
@@ -846,19 +881,16 @@ struct Controller {
     const bool density = !reuse && I.m.has_density;
     if (!cleared) launch_init(D, density, true, nvb, s);
     if (density) {
-      if (!side) {
-        CU(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-        for (cudaEvent_t& e : side_ev) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-      }
-      CU(cudaEventRecord(side_ev[0], s));
-      CU(cudaStreamWaitEvent(side, side_ev[0], 0));
-      launch_wa(D, I.r, pos, gam, nvb, side);
-      CU(cudaEventRecord(side_ev[1], side));
+      if (!I.side.s) CU(acquire_side(I.device, I.side));
+      CU(cudaEventRecord(I.side.ready, s));
+      CU(cudaStreamWaitEvent(I.side.s, I.side.ready, 0));
+      launch_wa(D, I.r, pos, gam, nvb, I.side.s);
+      CU(cudaEventRecord(I.side.done, I.side.s));
       launch_scatter(D, I.r, pos, nvb, s);
       if (!D.fft) launch_prep(D, I.r, nvb, s);
       for (int st = 0; st < 4; ++st) launch_dct(D, I.r, st, nvb, s, &I.tmaps, true);
       launch_gather(D, I.r, pos, nvb, s);
-      CU(cudaStreamWaitEvent(s, side_ev[1], 0));
+      CU(cudaStreamWaitEvent(s, I.side.done, 0));
       launch_finalize_joined(D, I.r, nvb, FIN_ENERGY | fin, s);
       density_evaluations++;
     } else {

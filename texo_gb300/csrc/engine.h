@@ -62,6 +62,13 @@ struct HostModel {
 
 int32_t build_model(const texo_gp_problem* p, const texo_gp_params* prm, HostModel& m, uint64_t* err_index);
 
+// A second stream beside an instance's own, and the events that lead to it and
+// back: the wirelength of the host engine's evaluations.
+struct Side {
+  cudaStream_t s = nullptr;
+  cudaEvent_t ready = nullptr, done = nullptr;
+};
+
 // Device-resident instance: every buffer one placement needs.
 struct Instance {
   HostModel m;
@@ -69,6 +76,7 @@ struct Instance {
   int sms = 152;
   int nvb = 1;
   cudaStream_t stream = nullptr;
+  Side side;   // from its first evaluation on
   std::vector<void*> allocations;
   Dev d{};
   Reduce r{};
