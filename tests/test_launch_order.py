@@ -95,3 +95,13 @@ def test_handles_of_many_threads_restarted_give_what_each_gives_alone():
         assert all(np.array_equal(a, b) for a, b in zip(alone[k], alone[k][6:]))   # a restart changes nothing
         for r in got[k]:
             assert all(np.array_equal(a, b) for a, b in zip(alone[k], r))
+
+
+def test_tables_sent_from_pageable_memory_have_arrived_before_another_stream_reads_them():
+    """Each function of the engine that fills a table with cudaMemcpy waits for the legacy stream before it publishes it."""
+    s = text("engine.cu")
+    for m in re.finditer(r"cudaError_t shared_\w+\([^)]*\) \{", s):
+        body = s[m.end():block_end(s, m.end() - 1)]
+        if "cudaMemcpy(" in body:
+            assert "sent(" in body and body.index("sent(") < body.index("cache.emplace"), m.group()
+    assert re.search(r"cudaError_t sent\(.*cudaStreamSynchronize\(cudaStreamLegacy\)", s)

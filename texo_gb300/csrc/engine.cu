@@ -187,6 +187,10 @@ std::vector<double> dct_basis(uint32_t n) {
 // Spectral tables of a bin grid (DCT basis and its transpose per axis, the
 // inverse Laplacian eigenvalues), read-only and identical for every
 // instance with the same grid: built once per device and size and shared.
+// The instances read them on non-blocking streams, which do not wait for the
+// legacy stream, and cudaMemcpy from pageable memory may return with the
+// transfer still under way there: `sent` is past it.
+cudaError_t sent(cudaError_t e) { return e == cudaSuccess ? cudaStreamSynchronize(cudaStreamLegacy) : e; }
 struct SpectralTables {
   float *Cx = nullptr, *CxT = nullptr, *Cy = nullptr, *CyT = nullptr, *inv_eig = nullptr;
 };
@@ -252,7 +256,7 @@ cudaError_t shared_basis(int device, uint32_t n, BasisTables* out) {
     up(&t.cA, cA);
     up(&t.ctA, ctA);
     up(&t.e, e);
-    if (err != cudaSuccess) return err;
+    if ((err = sent(err)) != cudaSuccess) return err;
     it = cache.emplace(std::make_pair(device, n), t).first;
   }
   *out = it->second;
@@ -304,7 +308,7 @@ cudaError_t shared_fft(int device, uint32_t n, FftTables* out) {
     up(&t.post, post);
     up(&t.pre, pre);
     up(&t.inv_s, inv_s);
-    if (e != cudaSuccess) return e;
+    if ((e = sent(e)) != cudaSuccess) return e;
     it = cache.emplace(std::make_pair(device, n), t).first;
   }
   *out = it->second;
@@ -342,7 +346,7 @@ cudaError_t shared_inv_eig(int device, uint32_t Wb, uint32_t Hb, float** out) {
     float* d = nullptr;
     cudaError_t e = cudaMalloc(&d, ie.size() * 4);
     if (e == cudaSuccess) e = cudaMemcpy(d, ie.data(), ie.size() * 4, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) return e;
+    if ((e = sent(e)) != cudaSuccess) return e;
     it = cache.emplace(std::make_tuple(device, Wb, Hb), d).first;
   }
   *out = it->second;
