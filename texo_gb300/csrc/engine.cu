@@ -1073,9 +1073,11 @@ struct Controller {
     const double next = midpoint1(std::sqrt(1.0 + 4.0 * a * a));
     const double e = std::isfinite(next) ? (a - 1.0) / next : 0.0;
     const bool ahead = std::isfinite(next) && (float)e != 0.f;
+    const bool known = density_at_x;
     launch_precond(D, I.r, nvb, s);
-    TRY(enqueue_eval(I.bufX, I.gX, gam, density_at_x, false, FIN_PRECOND));
+    TRY(enqueue_eval(I.bufX, I.gX, gam, known, false, FIN_PRECOND));
     if (ahead) {
+      density_at_x = false;   // Y's from here on, also for a call that goes on after a failure below
       CU(cudaMemcpyAsync(I.h_scal + kScalars, I.r.scal, kScalars * sizeof(double), cudaMemcpyDeviceToHost, s));
       CU(cudaMemcpyAsync(I.h_iscal + kIScalars, I.r.iscal, kIScalars * sizeof(long long), cudaMemcpyDeviceToHost, s));
       launch_extrapolate(D, I.r, I.bufX, I.bufXp, e, I.bufY, nvb, s, true);
@@ -1093,11 +1095,9 @@ struct Controller {
     TRY(checked(eo));
     bool origin = !ahead || I.h_iscal[SI_DIFF] == 0;   // the extrapolated point is the origin
     double origin_kkt = I.h_scal[SC_KKT];
-    if (ahead) {
-      if (origin)
-        density_evaluations--;   // the device still describes the origin's coordinates
-      else
-        density_at_x = false;
+    if (ahead && origin) {   // the device still describes the origin's coordinates
+      density_at_x = known;
+      density_evaluations--;
     }
     bool restart = false;
     bool has_wL = has_L;
