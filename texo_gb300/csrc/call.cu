@@ -50,7 +50,14 @@ Call::Call(int device) : device_(device) {
 
 Call::~Call() {
   if (!stream_) return;
-  if (base_) cudaFreeAsync(base_, stream_);
+  if (base_) {
+    cudaFreeAsync(base_, stream_);
+    // a pool gives memory back when a stream is waited for, not when it is freed
+    unsigned long long held = 0;
+    if (!pool_ || cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        held > kKeptBytes)
+      cudaStreamSynchronize(stream_);
+  }
   if (PerDevice* d = sound_ ? of(device_) : nullptr) {
     std::lock_guard<std::mutex> lk(g_mu);
     if (d->count < kKept) {
@@ -65,7 +72,6 @@ Call::~Call() {
 }
 
 char* Call::memory(size_t bytes) {
-  cudaMemPool_t pool = nullptr;
   if (PerDevice* d = of(device_)) {
     std::lock_guard<std::mutex> lk(g_mu);
     if (!d->pool) {
@@ -82,12 +88,13 @@ char* Call::memory(size_t bytes) {
           cudaMemPoolDestroy(made);
       }
     }
-    pool = d->pool;
+    pool_ = d->pool;
   }
   void* p = nullptr;
-  if (!pool || cudaMallocFromPoolAsync(&p, bytes, pool, stream_) != cudaSuccess) {
+  if (!pool_ || cudaMallocFromPoolAsync(&p, bytes, pool_, stream_) != cudaSuccess) {
     // the device's default pool may hold what this one cannot get
     cudaGetLastError();
+    pool_ = nullptr;
     if (cudaMallocAsync(&p, bytes, stream_) != cudaSuccess) {
       sound_ = false;
       return nullptr;

@@ -32,6 +32,7 @@ class Call {
   cudaStream_t stream_ = nullptr;
   cudaEvent_t e0_ = nullptr, e1_ = nullptr;
   char* base_ = nullptr;
+  cudaMemPool_t pool_ = nullptr;   // the device's pool, where the memory is its
   bool sound_ = true;   // no error seen: the stream may serve another call
 };
 
