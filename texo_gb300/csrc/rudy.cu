@@ -57,6 +57,11 @@ __device__ __forceinline__ Pieces axis_pieces(double lo, double hi, int extent) 
   p.v[2] = overlap(ib + 1.0);
   return p;
 }
+// Pieces without overlap given no tile.
+__device__ __forceinline__ void drop_empty(Pieces& p) {
+  if (p.v[0] == 0.0) p.c[0] = p.c[1];
+  if (p.v[2] == 0.0) p.c[3] = p.c[2];
+}
 
 // diff: [2][(H + 1) x (W + 1)] int64, zeroed. The nine rectangles of a box share
 // their corners: their rounded values are differenced in registers along both
@@ -70,7 +75,12 @@ __global__ void k_rudy_boxes(const double* boxes, long long nbox, int W, int H, 
   const double dx = x1 - x0, dy = y1 - y0;
   const double area = (dx + 1.0) * (dy + 1.0);
   const double hd = dx / area, vd = dy / area;
-  const Pieces px = axis_pieces(x0, x1, W), py = axis_pieces(y0, y1, H);
+  Pieces px = axis_pieces(x0, x1, W), py = axis_pieces(y0, y1, H);
+  if (__double2hiint(dx) == 0x7ff00000 || __double2hiint(dy) == 0x7ff00000) {
+    // wider than FP64: its density is no number, nor is zero times that
+    drop_empty(px);
+    drop_empty(py);
+  }
   const size_t plane = (size_t)(W + 1) * (H + 1);
   long long above_h[3] = {0, 0, 0}, above_v[3] = {0, 0, 0};   // the row of rectangles before
 #pragma unroll
