@@ -118,7 +118,7 @@ struct ClusterDev {
   const unsigned *group_begin, *group_end;   // per sorted register: its control set's range
   const unsigned* order;               // sorted position -> input index
   const Window* table;
-  double inv_scale, cutoff;
+  double half_window, inv_scale, cutoff;
   float cutoff32;                      // cutoff plus a margin that covers the FP32 rounding
   double* areas;                       // by input index
   int* bad;
@@ -194,7 +194,9 @@ __global__ void __launch_bounds__(kClusterThreads) k_clustering(ClusterDev d) {
   total = __dadd_rn(total, soft_ceiling(sum, 2.0, 0.5));
   if (cur == focal_ce) focal = sum;
   const unsigned out = __ldg(d.order + p);
-  if (!(isfinite(focal) && focal > 0.0)) {
+  // so far out that the window's edges round to the register's own place
+  auto no_window = [&](double v) { return __dadd_rn(v, d.half_window) == __dsub_rn(v, d.half_window); };
+  if (!(isfinite(focal) && focal > 0.0) || no_window(at.x) || no_window(at.y)) {
     atomicExch(d.bad, 1);
     d.areas[out] = 0.0;
     return;
@@ -370,6 +372,7 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
   if (!base) return TEXO_GP_ERR_OUT_OF_MEMORY;
   ClusterDev d{};
   d.n = (unsigned)n;
+  d.half_window = half_window;
   d.inv_scale = 1.0 / scale;
   d.cutoff = cutoff;
   double2* dxy = (double2*)base;
