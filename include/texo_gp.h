@@ -872,6 +872,9 @@ int32_t texo_gp_repair(uint32_t width, uint32_t height, uint32_t num_bels, const
  * (flags set to 1) and return without faulting; the device stays usable. No
  * counterpart in the reference. */
 int32_t texo_gp_selftest_waits(int32_t device, int32_t* barrier_timed_out, int32_t* mbarrier_timed_out);
+/* Self test of the quadratic solve's division by the diagonal: out[i] = a[i] /
+ * b[i] as the solve forms it, for n <= 2^26 pairs. */
+int32_t texo_gp_selftest_quotient(int32_t device, uint32_t n, const double* a, const double* b, double* out);
 
 #ifdef __cplusplus
 }

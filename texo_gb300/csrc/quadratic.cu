@@ -110,9 +110,13 @@ struct PcgShared {
 };
 
 // a / b from b's rounded reciprocal and one correction by the remainder
-// (Markstein 1990): three operations for the divide's nine, the result the
-// same but for the rarest ties. A diagonal near the ends of the range of
-// exponents has no such reciprocal (zero) and is divided by.
+// (Markstein 1990). The corrected value is within 1.5 * 2^-53 units in the last
+// place of a / b before it is rounded, so the result is the rounded quotient but
+// where a / b lies that close to the middle of two numbers, and then the other
+// of the two (0.04 ms of a 42,000-cell solve's 0.43 against the divide). A
+// diagonal near the ends of the range of exponents has no such reciprocal
+// (zero) and is divided by; a quotient beyond FP64 may be no number instead of
+// infinite, and either is a breakdown.
 __device__ __forceinline__ double reciprocal(double b) { return b > 1e-200 && b < 1e200 ? __drcp_rn(b) : 0.0; }
 __device__ __forceinline__ double quotient(double a, double b, double inverse) {
   if (__double2hiint(inverse) == 0) return __ddiv_rn(a, b);
@@ -443,6 +447,11 @@ __global__ void __launch_bounds__(kPcgThreads, 1) k_pcg(PcgDev d) {
   }
 }
 
+__global__ void k_quotient_selftest(unsigned n, const double* a, const double* b, double* out) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = quotient(a[i], b[i], reciprocal(b[i]));
+}
+
 // Cuts the rows into tiles of about equal work, at most kPcgThreads segments
 // each, and as many on each multiprocessor; a small system into tiles of 64
 // segments or more (fewer blocks meet sooner at the barriers). `padded`: the
@@ -638,4 +647,25 @@ extern "C" int32_t texo_gp_quadratic_solve(int32_t device, uint32_t n, const dou
     stats->kernel_launches = 1;
   }
   return st;
+}
+
+extern "C" int32_t texo_gp_selftest_quotient(int32_t device, uint32_t n, const double* a, const double* b, double* out) {
+  if (n == 0 || n > (1u << 26) || !a || !b || !out) return TEXO_GP_ERR_INVALID_ARGUMENT;
+  Call call(device);
+  if (!call.ok()) return TEXO_GP_ERR_CUDA;
+  const size_t bytes = (size_t)n * 8;
+  double* d = (double*)call.memory(3 * bytes);
+  if (!d) return TEXO_GP_ERR_OUT_OF_MEMORY;
+  const cudaStream_t s = call.stream();
+  call.start();
+  bool ok = cudaMemcpyAsync(d, a, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+            cudaMemcpyAsync(d + n, b, bytes, cudaMemcpyHostToDevice, s) == cudaSuccess;
+  if (ok) {
+    k_quotient_selftest<<<(n + kPcgThreads - 1) / kPcgThreads, kPcgThreads, 0, s>>>(n, d, d + n, d + 2 * (size_t)n);
+    ok = cudaGetLastError() == cudaSuccess &&
+         cudaMemcpyAsync(out, d + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost, s) == cudaSuccess;
+  }
+  float ms = 0.f;
+  if (!call.finish(&ms)) ok = false;
+  return ok ? TEXO_GP_OK : TEXO_GP_ERR_CUDA;
 }
