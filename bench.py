@@ -118,6 +118,12 @@ def stage_bytes(stage, n):
     }.get(stage, 0)
 
 
+def timed_stage_bytes(stage, n):
+    """The bytes of a stage as texo_gp_stage_times launches it: the combination
+    forms the KKT residual too (it reads positions, bounds and P)."""
+    return stage_bytes(stage, n) + ((n["U"] + n["F"]) * 28 if stage == "combine" else 0)
+
+
 def aggregate_ranks(total_ms, steps, dist=None, device="cuda"):
     """Replicas: every rank places its own instance (seeded by its rank); the
     whole-job value is all ranks' steps over the slowest rank's time."""
@@ -530,7 +536,7 @@ def stage_report(workload, dct_name, reps):
         torch.cuda.nvtx.range_pop()
     out = {}
     for k, ms in st.items():
-        b = stage_bytes(k, n)
+        b = timed_stage_bytes(k, n)
         out[k] = {"us": round(ms * 1000, 2), "algorithmic_bytes": b,
                   "gbs": round(b / (ms * 1e-3) / 1e9, 1) if ms > 0 and b else None,
                   "frac": round(b / (ms * 1e-3) / 1e9 / peak, 4) if ms > 0 and b else None}
@@ -1233,8 +1239,8 @@ def main():
     # per-stage device times (standalone stage kernels) and the roofline
     stages = named_stages(g.stage_times(reps=20), n)
     peak, peak_kind = peaks()
-    stage_roofline = {k: {"ms": v, "algorithmic_bytes": stage_bytes(k, n),
-                          "gbs": stage_bytes(k, n) / (v * 1e-3) / 1e9 if v > 0 else None}
+    stage_roofline = {k: {"ms": v, "algorithmic_bytes": timed_stage_bytes(k, n),
+                          "gbs": timed_stage_bytes(k, n) / (v * 1e-3) / 1e9 if v > 0 else None}
                       for k, v in stages.items()}
     if engine == abi.ENGINE_DEVICE:
         # one persistent launch per step runs the whole iteration: its

@@ -1083,7 +1083,7 @@ struct Controller {
       launch_extrapolate(D, I.r, I.bufX, I.bufXp, e, I.bufY, nvb, s, true);
       TRY(enqueue_eval(I.bufY, I.gY, gam, false, true, FIN_DIFF, true));
     } else {
-      launch_kkt(D, I.r, I.bufX, I.gX, nullptr, nvb, s);
+      launch_kkt(D, I.r, I.bufX, I.gX, nvb, s);
       launch_finalize(D, I.r, nvb, FIN_KKT, s);
     }
     TRY(sync_read());
@@ -1118,7 +1118,7 @@ struct Controller {
         TRY(checked(ey));
         f_y = ey.value;
       } else if (restart && !origin) {   // the origin's own residual was not needed so far
-        launch_kkt(D, I.r, I.bufX, I.gX, nullptr, nvb, s);
+        launch_kkt(D, I.r, I.bufX, I.gX, nvb, s);
         launch_finalize(D, I.r, nvb, FIN_KKT, s);
         TRY(sync_read());
         y_stat = origin_kkt = I.h_scal[SC_KKT];
@@ -2315,11 +2315,11 @@ int32_t texo_gp_stage_times(texo_gp_handle h, uint32_t reps, double* ms, uint32_
         case 3: launch_prep(D, I.r, nvb, s); break;
         case 4: case 5: case 6: case 7: launch_dct(D, I.r, (int)st - 4, nvb, s, &I.tmaps); break;
         case 8: launch_gather(D, I.r, I.bufX, nvb, s); break;
-        case 9: launch_combine(D, I.r, I.gX, nvb, s); break;
+        case 9: launch_combine(D, I.r, I.gX, nvb, s, I.bufX); break;
         case 10: launch_finalize(D, I.r, nvb, FIN_ENERGY | FIN_COMBINE, s); break;
         case 11: launch_extrapolate(D, I.r, I.bufX, I.bufXp, 0.5, I.bufY, nvb, s); break;
         case 12: launch_candidate(D, I.r, I.bufX, I.gX, 1.0, I.bufC, nvb, s); break;
-        case 13: launch_kkt(D, I.r, I.bufX, I.gX, I.bufXp, nvb, s); break;
+        case 13: launch_kkt(D, I.r, I.bufX, I.gX, nvb, s); break;
         default: launch_precond(D, I.r, nvb, s); break;
       }
     }

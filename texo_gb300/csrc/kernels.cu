@@ -184,11 +184,10 @@ __global__ void __launch_bounds__(kThreads) k_candidate(Dev d, Partials p, const
   if (reset) stage_init(whole_block(), d, blockIdx.x, gridDim.x, true, true);
   stage_candidate(whole_block(), d, y, gy, invL, c, p, blockIdx.x, gridDim.x, sh, buf);
 }
-__global__ void __launch_bounds__(kThreads) k_kkt(Dev d, Partials p, const float2* x, const float2* g,
-                                                 const float2* ref) {
+__global__ void __launch_bounds__(kThreads) k_kkt(Dev d, Partials p, const float2* x, const float2* g) {
   after_previous();
   __shared__ Shared sh;
-  stage_kkt(whole_block(), d, x, g, ref, p, blockIdx.x, gridDim.x, sh);
+  stage_kkt(whole_block(), d, x, g, p, blockIdx.x, gridDim.x, sh);
 }
 __global__ void __launch_bounds__(kThreads) k_precond(Dev d, Partials p, const double* lambda) {
   after_previous();
@@ -275,10 +274,7 @@ __global__ void __launch_bounds__(kFinThreads) k_finalize(Dev d, Reduce r, int n
       add(pslot(p, SLOT_DOT), 0, SC_DOT);
       add(pslot(p, SLOT_MSN), 0, SC_MSN);
     }
-    if (mask & FIN_KKT) {
-      add(mslot(p, MS_KKT), 3, SC_KKT);
-      add(mslot(p, MS_CHANGE), 3, SC_CHANGE);
-    }
+    if (mask & FIN_KKT) add(mslot(p, MS_KKT), 3, SC_KKT);
     if (mask & FIN_PRECOND) {
       add(mslot(p, MS_PMIN), 4, SC_PMIN);
       add(mslot(p, MS_PMAX), 3, SC_PMAX);
@@ -476,10 +472,9 @@ void launch_candidate(const Dev& d, const Reduce& r, const float2* y, const floa
   COUNT;
   follow(k_candidate, nvb, kThreads, 0, s, d, r.p, y, gy, invL, c, reset);
 }
-void launch_kkt(const Dev& d, const Reduce& r, const float2* x, const float2* g, const float2* ref, int nvb,
-                cudaStream_t s) {
+void launch_kkt(const Dev& d, const Reduce& r, const float2* x, const float2* g, int nvb, cudaStream_t s) {
   COUNT;
-  follow(k_kkt, nvb, kThreads, 0, s, d, r.p, x, g, ref);
+  follow(k_kkt, nvb, kThreads, 0, s, d, r.p, x, g);
 }
 void launch_precond(const Dev& d, const Reduce& r, int nvb, cudaStream_t s) {
   COUNT;

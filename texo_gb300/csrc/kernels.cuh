@@ -18,7 +18,6 @@ enum Scalar {
   SC_DOT = 23,
   SC_MSN = 24,
   SC_KKT = 25,
-  SC_CHANGE = 26,
   SC_PMIN = 27,
   SC_PMAX = 28,
   SC_HPWL = 29,
@@ -76,8 +75,7 @@ void launch_extrapolate(const Dev& d, const Reduce& r, const float2* x, const fl
                         int nvb, cudaStream_t s, bool reset = false);
 void launch_candidate(const Dev& d, const Reduce& r, const float2* y, const float2* gy, float invL, float2* c,
                       int nvb, cudaStream_t s, bool reset = false);
-void launch_kkt(const Dev& d, const Reduce& r, const float2* x, const float2* g, const float2* ref, int nvb,
-                cudaStream_t s);
+void launch_kkt(const Dev& d, const Reduce& r, const float2* x, const float2* g, int nvb, cudaStream_t s);
 void launch_precond(const Dev& d, const Reduce& r, int nvb, cudaStream_t s);
 void launch_hpwl(const Dev& d, const Reduce& r, const float2* pos, int nvb, cudaStream_t s);
 void launch_finalize(const Dev& d, const Reduce& r, int nvb, int mask, cudaStream_t s);

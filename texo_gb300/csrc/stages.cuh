@@ -22,7 +22,7 @@ enum ISlot {
   kISlots
 };
 // Max/min partial slots (doubles).
-enum MSlot { MS_KKT = 0, MS_CHANGE, MS_PMIN, MS_PMAX, kMSlots };
+enum MSlot { MS_KKT = 0, MS_PMIN, MS_PMAX, kMSlots };
 
 struct Partials {
   double* sum;        // [kSlots][kMaxPartials]
@@ -969,26 +969,19 @@ static __device__ void stage_candidate(const G& g, const Dev& d, const float2* y
   write_partials(g, sums, 2, [&](int i) { return pslot(p, i == 0 ? SLOT_DOT : SLOT_MSN); }, vb, buf, 2);
 }
 
-// box_metric_kkt_residual (global_placement.rs:648-663) and, optionally, the
-// max coordinate change against `ref`.
+// box_metric_kkt_residual (global_placement.rs:648-663).
 template <class G>
-static __device__ void stage_kkt(const G& g, const Dev& d, const float2* x, const float2* grad,
-                                 const float2* ref, Partials p, int vb, int nvb, Shared& sh) {
-  float r = 0.f, ch = 0.f;
+static __device__ void stage_kkt(const G& g, const Dev& d, const float2* x, const float2* grad, Partials p, int vb,
+                                 int nvb, Shared& sh) {
+  float r = 0.f;
   const int stride = nvb * kThreads;
   for (int o = vb * kThreads + g.tid; o < d.nobj; o += stride) {
     const float2 a = x[o], gg = grad[o], lo = d.lo[o], hi = d.hi[o];
     const float s = rsqrtf(d.P[o]);
     r = fmaxf(r, kkt_comp(gg.x, a.x, lo.x, hi.x) * s);
     r = fmaxf(r, kkt_comp(gg.y, a.y, lo.y, hi.y) * s);
-    if (ref) {
-      const float2 b = ref[o];
-      ch = fmaxf(ch, fabsf(a.x - b.x));
-      ch = fmaxf(ch, fabsf(a.y - b.y));
-    }
   }
   write_partial_max(g, r, mslot(p, MS_KKT), vb, sh.f, false);
-  if (ref) write_partial_max(g, ch, mslot(p, MS_CHANGE), vb, sh.f, false);
 }
 
 // diagonal_preconditioner (eplace.rs:1046-1100).
