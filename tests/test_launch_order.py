@@ -60,6 +60,18 @@ def test_a_kernel_behind_another_streams_event_is_launched_plainly():
         assert "<<<" in body and "follow(" not in body, (name, launcher)
 
 
+def test_a_kernel_behind_a_stream_ordered_allocation_is_launched_plainly():
+    """The memory may have been freed by another stream, which the allocation then makes this one wait for."""
+    kernels, engine = text("kernels.cu"), text("engine.cu")
+    uses = [m.end() for m in re.finditer(r"buf\.get\(", engine)]
+    assert len(uses) == 3   # coordinates in, a point out, an evaluation out
+    for i in uses:
+        launcher = next_launch(engine, i)
+        body = re.search(r"void %s\([^)]*\) \{" % launcher, kernels)
+        body = kernels[body.end():block_end(kernels, body.end() - 1)]
+        assert "<<<" in body and "follow(" not in body, launcher
+
+
 FORMS = [dict(bins_x=128, bins_y=128), dict(bins_x=96, bins_y=80), dict(bins_x=128, bins_y=128, dct_mode=abi.DCT_TENSOR)]
 
 

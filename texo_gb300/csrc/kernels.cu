@@ -13,7 +13,8 @@ namespace tgp {
 // through the read-only cache). The wait covers the kernel before it in its
 // own stream and nothing else: the kernel after a cudaStreamWaitEvent is launched
 // plainly (`launch_finalize_joined`), as is k_wa, whose predecessor is in
-// another stream. An evaluation at 250,000 cells with the tensor-core transforms,
+// another stream, and as are the kernels after a stream-ordered allocation, which
+// may make the stream wait for the one that freed the memory. An evaluation at 250,000 cells with the tensor-core transforms,
 // 19 launches, 245 -> 215 us; a whole evaluate call at 2,000 cells 166 -> 148.
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -352,7 +353,6 @@ __global__ void __launch_bounds__(kThreads) k_widen_point(Dev d, const float2* b
 // texo_gp_evaluate's arrays; each may be null.
 __global__ void __launch_bounds__(kThreads) k_widen_eval(Dev d, double* wa, double2* field, double* density,
                                                          double* potential) {
-  after_previous();
   const int first = blockIdx.x * kThreads + threadIdx.x, stride = gridDim.x * kThreads;
   if (wa)
     for (int i = first; i < 2 * d.U; i += stride) wa[i] = (double)(long long)d.wa_fix[i] * kInvFix;
@@ -506,8 +506,8 @@ void launch_widen_point(const Dev& d, const float2* best, const float2* x, uint3
 }
 void launch_widen_eval(const Dev& d, double* wa, double* field, double* density, double* potential, cudaStream_t s) {
   COUNT;
-  follow(k_widen_eval, wide_blocks(std::max<size_t>((size_t)d.nobj, (size_t)d.B)), kThreads, 0, s, d, wa,
-         (double2*)field, density, potential);
+  k_widen_eval<<<wide_blocks(std::max<size_t>((size_t)d.nobj, (size_t)d.B)), kThreads, 0, s>>>(
+      d, wa, (double2*)field, density, potential);
 }
 void launch_round_compare(const Dev& d, const float2* x, uint32_t* prev, int W, int H, unsigned long long* mismatch,
                           int nvb, cudaStream_t s) {
