@@ -34,6 +34,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <numeric>
 #include <string>
 #include <vector>
@@ -59,33 +61,48 @@ struct Window {
 
 // The table, formed once in extended precision (erf' = 2 / sqrt(pi)
 // exp(-x^2), and its n-th derivative times (-1)^n H_n(x), the Hermite
-// polynomials' three-term recurrence). Each call sends it (20 KB) with its own
-// inputs, on its own stream: nothing is kept on a device between calls.
-const std::vector<Window>& window_table() {
-  static const std::vector<Window> table = [] {   // thread-safe one-time initialisation
-    std::vector<Window> t(kIntervals);
-    const long double h = 2.5L / sqrtl(2.0L), two_over_sqrt_pi = 2.0L / sqrtl(3.14159265358979323846264338327950288L);
-    for (int k = 0; k < kIntervals; ++k) {
-      const long double m = (k + 0.5L) / kPerUnit;
-      t[k].middle = (double)m;
-      long double c[kTerms] = {0.5L * (erfcl(m - h) - erfcl(m + h))};
-      for (int side = 0; side < 2; ++side) {
-        const long double x = side ? m - h : m + h, e = (side ? -0.5L : 0.5L) * two_over_sqrt_pi * expl(-x * x);
-        long double h0 = 1.0L, h1 = 2.0L * x, sign = 1.0L, factorial = 1.0L;
-        for (int n = 0; n + 1 < kTerms; ++n) {   // c[n + 1]: the n-th derivative of erf' over (n + 1)!
-          factorial *= n + 1;
-          c[n + 1] += sign * h0 * e / factorial;
-          const long double h2 = 2.0L * x * h1 - 2.0L * (n + 1) * h0;
-          h0 = h1;
-          h1 = h2;
-          sign = -sign;
-        }
+// polynomials' three-term recurrence).
+std::vector<Window> form_table() {
+  std::vector<Window> t(kIntervals);
+  const long double h = 2.5L / sqrtl(2.0L), two_over_sqrt_pi = 2.0L / sqrtl(3.14159265358979323846264338327950288L);
+  for (int k = 0; k < kIntervals; ++k) {
+    const long double m = (k + 0.5L) / kPerUnit;
+    t[k].middle = (double)m;
+    long double c[kTerms] = {0.5L * (erfcl(m - h) - erfcl(m + h))};
+    for (int side = 0; side < 2; ++side) {
+      const long double x = side ? m - h : m + h, e = (side ? -0.5L : 0.5L) * two_over_sqrt_pi * expl(-x * x);
+      long double h0 = 1.0L, h1 = 2.0L * x, sign = 1.0L, factorial = 1.0L;
+      for (int n = 0; n + 1 < kTerms; ++n) {   // c[n + 1]: the n-th derivative of erf' over (n + 1)!
+        factorial *= n + 1;
+        c[n + 1] += sign * h0 * e / factorial;
+        const long double h2 = 2.0L * x * h1 - 2.0L * (n + 1) * h0;
+        h0 = h1;
+        h1 = h2;
+        sign = -sign;
       }
-      for (int n = 0; n < kTerms; ++n) t[k].c[n] = (double)c[n];
     }
-    return t;
-  }();
-  return table;
+    for (int n = 0; n < kTerms; ++n) t[k].c[n] = (double)c[n];
+  }
+  return t;
+}
+// The table on a device: sent by its first call, on that call's stream, and
+// published once it has arrived (sent with each call's inputs it cost 2 to 9 us
+// of a call). nullptr where it could not be.
+const Window* window_table(int device, cudaStream_t s) {
+  static std::mutex mu;
+  static std::map<int, const Window*> on_device;
+  std::lock_guard<std::mutex> lk(mu);
+  const auto it = on_device.find(device);
+  if (it != on_device.end()) return it->second;
+  const std::vector<Window> t = form_table();
+  Window* d = nullptr;
+  if (cudaMallocAsync((void**)&d, t.size() * sizeof(Window), s) != cudaSuccess) return nullptr;
+  if (cudaMemcpyAsync(d, t.data(), t.size() * sizeof(Window), cudaMemcpyHostToDevice, s) != cudaSuccess ||
+      cudaStreamSynchronize(s) != cudaSuccess) {
+    cudaFreeAsync(d, s);
+    return nullptr;
+  }
+  return on_device[device] = d;
 }
 
 // soft_division_ceiling (register_clustering.rs:89-97); the divisors are
@@ -366,11 +383,10 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
   if (!call.ok()) return TEXO_GP_ERR_CUDA;
   const cudaStream_t s = call.stream();
   auto round = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  const std::vector<Window>& table = window_table();
-  const size_t s8 = round(n * 8), s4 = round(n * 4), st = round(table.size() * sizeof(Window));
-  char* base = call.memory(5 * s8 + 4 * s4 + st + 256);
-  if (!base) return TEXO_GP_ERR_OUT_OF_MEMORY;
+  const size_t s8 = round(n * 8), s4 = round(n * 4);
+  char* base = call.memory(5 * s8 + 4 * s4 + 256);
   ClusterDev d{};
+  if (!base || !(d.table = window_table(device, s))) return TEXO_GP_ERR_OUT_OF_MEMORY;
   d.n = (unsigned)n;
   d.half_window = half_window;
   d.inv_scale = 1.0 / scale;
@@ -384,8 +400,6 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
   float2* d32 = (float2*)(base + 4 * s8 + 3 * s4);
   unsigned* dfoc = (unsigned*)(base + 5 * s8 + 3 * s4);
   d.bad = (int*)(base + 5 * s8 + 4 * s4);
-  Window* dtable = (Window*)(base + 5 * s8 + 4 * s4 + 256);
-  d.table = dtable;
   d.xy32 = d32;
   d.focal = dfoc;
   d.cutoff32 = cutoff32;
@@ -395,8 +409,7 @@ extern "C" int32_t texo_gp_register_clustering_areas(int32_t device, uint64_t nu
   d.group_end = dge;
   d.order = dord;
   call.start();
-  bool ok = cudaMemcpyAsync(dtable, table.data(), table.size() * sizeof(Window), cudaMemcpyHostToDevice, s) == cudaSuccess &&
-            cudaMemcpyAsync(dxy, sxy.data(), n * 16, cudaMemcpyHostToDevice, s) == cudaSuccess &&
+  bool ok = cudaMemcpyAsync(dxy, sxy.data(), n * 16, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(dce, sce.data(), n * 8, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(dgb, gb.data(), n * 4, cudaMemcpyHostToDevice, s) == cudaSuccess &&
             cudaMemcpyAsync(dge, ge.data(), n * 4, cudaMemcpyHostToDevice, s) == cudaSuccess &&
