@@ -810,7 +810,7 @@ struct Controller {
   double a = 1.0;
   bool has_L = false;
   double L = 0.0;
-  bool density_at_x = false;  // graw/phi/energies describe bufX
+  bool density_at_x = false;  // graw/phi/energies describe bufX (host engine; the device engine's own: hr.density_at_x)
   // statistics
   uint64_t evaluations = 0, device_evaluations = 0, trials = 0;
   uint64_t density_evaluations = 0;   // evaluations that rebuilt the density side
@@ -1996,7 +1996,8 @@ int32_t texo_gp_evaluate(texo_gp_handle h, const double* coordinates, double gam
   Controller& C = *h->ctl;
   const size_t nobj = (size_t)I.d.nobj, B = I.m.bins(), K = I.m.K;
   // A refused call leaves the handle as it was. Between two calls Y holds
-  // nothing, and without a density at X neither does what an evaluation writes:
+  // nothing, and without a density at X (either engine's) neither does what an
+  // evaluation writes:
   // then the coordinates are checked while the evaluation runs (12 us at 42k
   // cells; one that is not finite lands on the grid's edge), and its
   // counts are taken back; else before it is queued.
@@ -2005,10 +2006,11 @@ int32_t texo_gp_evaluate(texo_gp_handle h, const double* coordinates, double gam
     return TEXO_GP_ERR_NONFINITE_UNIT_COORDINATE;
   };
   TRY(upload_coords(I, I.bufY, coordinates, nobj));
-  const bool check_first = C.density_at_x;
+  const bool check_first = C.density_at_x || C.hr.density_at_x;
   if (check_first && !all_finite(coordinates, 2 * nobj)) return refuse();
   const uint64_t counts_before[2] = {C.density_evaluations, C.device_evaluations};
   C.density_at_x = false;
+  C.hr.density_at_x = 0;
   TRY(C.enqueue_eval(I.bufY, I.gY, gamma, false));
   Staged buf(I.stream);
   const size_t counts[4] = {wa_gradient ? 2 * (size_t)I.m.U : 0, field_gradient ? K * 2 * nobj : 0,
