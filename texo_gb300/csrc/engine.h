@@ -63,10 +63,11 @@ struct HostModel {
 int32_t build_model(const texo_gp_problem* p, const texo_gp_params* prm, HostModel& m, uint64_t* err_index);
 
 // A second stream beside an instance's own, and the events that lead to it and
-// back: the wirelength of the host engine's evaluations.
+// back: the wirelength of the host engine's evaluations. `checked` is behind the
+// flag of texo_gp_evaluate's coordinates.
 struct Side {
   cudaStream_t s = nullptr;
-  cudaEvent_t ready = nullptr, done = nullptr;
+  cudaEvent_t ready = nullptr, done = nullptr, checked = nullptr;
 };
 
 // Device-resident instance: every buffer one placement needs.
@@ -94,6 +95,7 @@ struct Instance {
   double* h_scal = nullptr;                      // pinned host mirror
   long long* h_iscal = nullptr;
   uint64_t bytes = 0;
+  long long coordinate_calls = 0;                // texo_gp_evaluate calls that flag (the mark of SI_NONFINITE)
   tc::TcMaps tmaps{};                            // tensor maps of the tensor-core DCT operands
 
   ~Instance();

@@ -329,9 +329,15 @@ __global__ void __launch_bounds__(kFinThreads) k_finalize(Dev d, Reduce r, int n
 // (on this machine a copy from or to pageable memory runs at the pinned rate)
 // and narrowed or widened here. On one host core the conversions of a
 // million-cell call took 6.5 ms of its 15.
-__global__ void __launch_bounds__(kThreads) k_narrow(const double* __restrict__ src, float* __restrict__ dst, size_t n) {
-  for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += (size_t)gridDim.x * kThreads)
-    dst[i] = __double2float_rn(src[i]);
+__global__ void __launch_bounds__(kThreads) k_narrow(const double* __restrict__ src, float* __restrict__ dst, size_t n,
+                                                     long long* nonfinite, long long mark) {
+  bool bad = false;
+  for (size_t i = (size_t)blockIdx.x * kThreads + threadIdx.x; i < n; i += (size_t)gridDim.x * kThreads) {
+    const double v = src[i];
+    dst[i] = __double2float_rn(v);
+    bad = bad || !isfinite(v);
+  }
+  if (nonfinite && bad) atomicMax(nonfinite, mark);
 }
 // rounded_targets_from_coordinates (eplace.rs:954-971) of the checkpoint, and
 // the current coordinates; either output may be null.
@@ -493,10 +499,10 @@ void launch_finalize_joined(const Dev& d, const Reduce& r, int nvb, int mask, cu
   k_finalize<<<1, kFinThreads, 0, s>>>(d, r, nvb, mask);
 }
 static inline int wide_blocks(size_t n) { return (int)std::min<size_t>((n + kThreads - 1) / kThreads, 2048); }
-void launch_narrow(const double* src, float* dst, size_t n, cudaStream_t s) {
+void launch_narrow(const double* src, float* dst, size_t n, long long* nonfinite, long long mark, cudaStream_t s) {
   if (!n) return;
   COUNT;
-  k_narrow<<<wide_blocks(n), kThreads, 0, s>>>(src, dst, n);
+  k_narrow<<<wide_blocks(n), kThreads, 0, s>>>(src, dst, n, nonfinite, mark);
 }
 void launch_widen_point(const Dev& d, const float2* best, const float2* x, uint32_t* targets, double* coords,
                         cudaStream_t s) {

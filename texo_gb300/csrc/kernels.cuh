@@ -37,7 +37,8 @@ enum IScalar {
   SI_PBAD = 10,
   SI_GRID_SUM = 11,              // + field
   SI_TC_FAIL = 15,               // set when a tensor-core DCT wait ran out
-  kIScalars = 16
+  SI_NONFINITE = 16,             // the mark of the last call that gave a coordinate that is not finite
+  kIScalars = 32
 };
 
 enum FinalizeMask {
@@ -81,9 +82,9 @@ void launch_hpwl(const Dev& d, const Reduce& r, const float2* pos, int nvb, cuda
 void launch_finalize(const Dev& d, const Reduce& r, int nvb, int mask, cudaStream_t s);
 // The same where the stream has just waited for another stream's event.
 void launch_finalize_joined(const Dev& d, const Reduce& r, int nvb, int mask, cudaStream_t s);
-// FP64 host arrays staged on the device -> FP32, and the results' FP64 and
-// integer arrays from device state.
-void launch_narrow(const double* src, float* dst, size_t n, cudaStream_t s);
+// FP64 host arrays staged on the device -> FP32 (raising *nonfinite to mark
+// when a value is not finite), and the results' FP64 and integer arrays from device state.
+void launch_narrow(const double* src, float* dst, size_t n, long long* nonfinite, long long mark, cudaStream_t s);
 void launch_widen_point(const Dev& d, const float2* best, const float2* x, uint32_t* targets, double* coords,
                         cudaStream_t s);
 void launch_widen_eval(const Dev& d, double* wa, double* field, double* density, double* potential, cudaStream_t s);
