@@ -18,6 +18,7 @@ struct PerDevice {
   Idle idle[kKept];
   int count;
   cudaMemPool_t pool;
+  unsigned long long live, held;   // bytes of the pool in use, and the most since it last gave back
 };
 // plain data, so nothing runs at exit, when CUDA may be gone
 PerDevice g_devices[kDevices];
@@ -53,10 +54,14 @@ Call::~Call() {
   if (base_) {
     cudaFreeAsync(base_, stream_);
     // a pool gives memory back when a stream is waited for, not when it is freed
-    unsigned long long held = 0;
-    if (!pool_ || cudaMemPoolGetAttribute(pool_, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
-        held > kKeptBytes)
-      cudaStreamSynchronize(stream_);
+    bool wait = true;
+    if (PerDevice* d = bytes_ ? of(device_) : nullptr) {
+      std::lock_guard<std::mutex> lk(g_mu);
+      d->live -= bytes_;
+      wait = d->held > kKeptBytes;
+      if (wait) d->held = d->live;
+    }
+    if (wait) cudaStreamSynchronize(stream_);
   }
   if (PerDevice* d = sound_ ? of(device_) : nullptr) {
     std::lock_guard<std::mutex> lk(g_mu);
@@ -72,7 +77,9 @@ Call::~Call() {
 }
 
 char* Call::memory(size_t bytes) {
-  if (PerDevice* d = of(device_)) {
+  PerDevice* const d = of(device_);
+  cudaMemPool_t pool = nullptr;
+  if (d) {
     std::lock_guard<std::mutex> lk(g_mu);
     if (!d->pool) {
       cudaMemPoolProps props{};
@@ -88,13 +95,17 @@ char* Call::memory(size_t bytes) {
           cudaMemPoolDestroy(made);
       }
     }
-    pool_ = d->pool;
+    pool = d->pool;
   }
   void* p = nullptr;
-  if (!pool_ || cudaMallocFromPoolAsync(&p, bytes, pool_, stream_) != cudaSuccess) {
+  if (pool && cudaMallocFromPoolAsync(&p, bytes, pool, stream_) == cudaSuccess) {
+    bytes_ = bytes;
+    std::lock_guard<std::mutex> lk(g_mu);
+    d->live += bytes;
+    if (d->held < d->live) d->held = d->live;
+  } else {
     // the device's default pool may hold what this one cannot get
     cudaGetLastError();
-    pool_ = nullptr;
     if (cudaMallocAsync(&p, bytes, stream_) != cudaSuccess) {
       sound_ = false;
       return nullptr;

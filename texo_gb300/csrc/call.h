@@ -32,7 +32,7 @@ class Call {
   cudaStream_t stream_ = nullptr;
   cudaEvent_t e0_ = nullptr, e1_ = nullptr;
   char* base_ = nullptr;
-  cudaMemPool_t pool_ = nullptr;   // the device's pool, where the memory is its
+  size_t bytes_ = 0;    // of the device's kept pool
   bool sound_ = true;   // no error seen: the stream may serve another call
 };
 
